@@ -820,6 +820,7 @@ static int32_t bind_blocks(lc_model* m) {
             tq->view = buf; tk->view = buf + tq->nbytes; tv->view = buf + tq->nbytes + tk->nbytes;
             w.fused_buf = buf;
             w.fused_qkv = true;
+            w.q = w.k = w.v = QWeight();  // their own copies are gone
             LC_TRY(qweight_init(&w.qkv, tq->typ, buf, m->nqkv, H));
         }
         LC_TRY(weight_of(m, p + "attn_output.weight", H, nq, &w.o, nullptr));
@@ -850,6 +851,29 @@ static int32_t bind_blocks(lc_model* m) {
         LC_CHECK((int)e.rows == m->cfg.vocab_size, LC_ERR_INVALID, "token_embd.weight has %zu rows, vocabulary is %d", e.rows, m->cfg.vocab_size);
         const size_t row_bytes = e.nbytes / e.rows;
         LC_TRY(qweight_init(&m->head, e.typ, (const uint8_t*)e.view + (size_t)m->v0 * row_bytes, V, H));
+    }
+    return LC_OK;
+}
+
+// The rows' powers of two of every matrix that the many-token product reads, in one buffer.
+static int32_t bind_row_scales(lc_model* m) {
+    std::vector<QWeight*> all = {&m->head};
+    for (LayerW& w : m->layers) {
+        for (QWeight* q : {&w.qkv, &w.q, &w.k, &w.v, &w.o, &w.gate, &w.up, &w.down}) all.push_back(q);
+        for (auto* set : {&w.egate, &w.eup, &w.edown})
+            for (QWeight& q : *set) all.push_back(&q);
+    }
+    all.erase(std::remove_if(all.begin(), all.end(), [](QWeight* q) { return !q->data || !qgemm_split_weight_ok(*q); }), all.end());
+    size_t rows = 0;
+    for (QWeight* q : all) rows += q->n;
+    if (rows == 0) return LC_OK;
+    float* down = nullptr;
+    LC_TRY(dalloc(&down, rows));
+    m->owned.push_back(down);
+    for (QWeight* q : all) {
+        LC_TRY(launch_row_scales(*q, down, m->stream));
+        q->row_down = down;
+        down += q->n;
     }
     return LC_OK;
 }
@@ -920,6 +944,7 @@ int32_t lc_model_finalize(lc_model* m) {
     LC_CHECK(!m->finalized, LC_ERR_STATE, "model already finalized");
     DeviceGuard dg(m->device);
     if (!m->stack) LC_TRY(bind_blocks(m));
+    if (!m->stack) LC_TRY(bind_row_scales(m));
     const int H = m->H, V = m->V;
 
     // weight sanity scan (loader.rs:241-249) and resident byte count

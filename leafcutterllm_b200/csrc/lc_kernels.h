@@ -54,8 +54,9 @@ struct QWeight {
     int n = 0, k = 0;
     size_t row_bytes = 0;
     alignas(64) unsigned char tmap[128];      // CUtensorMap for the TMA-staged kernels: box = one 256-element unit x 32 rows
-    alignas(64) unsigned char tmap_wide[128]; // the same tensor with a box of 128 rows (tcgen05 kernel)
+    alignas(64) unsigned char tmap_wide[128]; // the same tensor with a box of 128 rows (tcgen05 kernel of up to 64 tokens)
     bool has_tmap = false;
+    const float* row_down = nullptr;  // device: the rows' powers of two for the many-token product (launch_row_scales), or null
 };
 int32_t qweight_init(QWeight* w, uint32_t typ, const void* data_dev, int n, int k);
 
@@ -123,24 +124,32 @@ struct GemmWorkspace {
     float* tok_scale = nullptr;  // [t_cap]
     float* partial = nullptr;    // sums of the shares of k when a product is split over several CTAs per tile
     size_t partial_bytes = 0;
+    float* row_tmp = nullptr;    // row scales of matrices that come without (QWeight::row_down)
+    size_t row_cap = 0;
     int t_cap = 0, k_max = 0;
     // what xh / sx / tok_scale hold when the summing kernel of the previous product prepared them (see GemvArgs::prep_next);
     // valid for the very next product only
-    mutable const float* prep_x = nullptr;
-    mutable const float* prep_norm = nullptr;
-    mutable int prep_k = 0, prep_t = 0;
+    const float* prep_x = nullptr;
+    const float* prep_norm = nullptr;
+    int prep_k = 0, prep_t = 0;
 };
 int32_t run_tcgen05_probe(double* out16_host, cudaStream_t s);
 int32_t qgemm_workspace_alloc(GemmWorkspace* ws, int t_cap, int k_max);
 void qgemm_workspace_free(GemmWorkspace* ws);
-// true when launch_qgemm implements these arguments for T tokens (Q4_K weights, T at least LC_GEMM_MIN_TOKENS, default 5: up to four tokens the
+// true when the many-token product can read this matrix (Q4_K, Q5_K, Q6_K, Q4_0, Q8_0, rows of whole 256-element units)
+bool qgemm_split_weight_ok(const QWeight& w);
+// the rows' powers of two (QWeight::row_down) of such a matrix: down[n]
+int32_t launch_row_scales(const QWeight& w, float* down, cudaStream_t s);
+// true when launch_qgemm implements these arguments for T tokens (T at least LC_GEMM_MIN_TOKENS, default 5: up to four tokens the
 // matrix-vector kernels are faster, from five on they would run their 8-token form, which this product beats)
 bool qgemm_applies(const GemvArgs& a, int T, const GemmWorkspace& ws);
 // a.m = number of tokens; queues two kernels (activation preparation, product), three when k is split (reduction)
-int32_t launch_qgemm(const GemvArgs& a, const GemmWorkspace& ws, cudaStream_t s, int* launches = nullptr);
-// Tensor map over f16 activations [2 halves][rows][k] with a box of 64 elements x box_rows rows x both halves, 128-byte swizzle.
+int32_t launch_qgemm(const GemvArgs& a, GemmWorkspace& ws, cudaStream_t s, int* launches = nullptr);// Tensor map over f16 activations [2 halves][rows][k] with a box of 64 elements x box_rows rows x both halves, 128-byte swizzle.
 bool make_act_tmap(void* out128, const void* base, uint64_t k, uint64_t rows, uint32_t box_rows);
 bool make_act_tmap_chunks(void* out128, const void* base, uint64_t k, uint64_t rows, uint32_t box_rows, uint32_t box_chunks);
+// ---- qgemm_split.cu ----
+// the product alone, for launch_qgemm: *slices > 0 says that shares of k are left in ws.partial; *launches counts on
+int32_t launch_qgemm_split(const GemvArgs& a, GemmWorkspace& ws, int* slices, int* launches, cudaStream_t s);
 
 // ---- attention.cu ----
 struct KvLayout {

@@ -1,0 +1,840 @@
+// Quantised weights (Q4_K, Q5_K, Q6_K, Q4_0, Q8_0) times MANY tokens (prompts, batched decode steps) on the 5th-generation tensor
+// cores: the dense contraction of the path (Tensor::matmul with m > 1, rust/src/tensor.rs:107-135,
+// over weights that the reference dequantises per call, rust/src/model/loader.rs:213-224).
+//
+//   y[t, r] = sum_k x[t, k] * w[r, k]
+//
+// Weights stay as raw GGUF blocks in HBM; nothing dequantised is ever written back.  Both factors enter the tensor cores as sums
+// of two f16: a weight, times a power of two of its row, is hi + lo with 22 bits (every type but Q6_K has at most 21, so it is
+// exact), an activation, times a power of two of its token, is hi + lo with 22 bits.  Three of the four products count
+// (lo * lo is 2^-22 of the result): per 16 elements of k
+//
+//   main  += W_hi * X_hi                       one tcgen05.mma with N = 2 * tokens over [X_hi | X_lo] forms the first two,
+//   small += W_hi * X_lo,  small += W_lo * X_hi    a second with N = tokens the third.
+//
+// The tensor cores truncate when they add to an f32 accumulator: the error grows with the number of additions (measured on
+// N(0,1) products: 3.5e-7 of the result after 256 elements of k, 1.2e-6 after 1024, 9.6e-6 after 8192; 3 terms into one accumulator
+// 1.0e-6 after 256).  So `main`, 2^11 times larger than `small`, is emptied into registers every 256 elements and those sums are
+// rounded to nearest; `small` runs to the end.
+//
+// Q4_K / Q5_K weights are d * sc * q - dmin * m: the first part is the weight above, the second joins as more k: -dmin * m (17
+// bits, two f16) of a sub-block against the sum of the activations over it, 16 values per 256-element unit, behind the last unit.
+//
+// One CTA owns 128 weight rows (the M of tcgen05.mma; for gate/up 64 rows of each, so that SiLU(gate) * up happens here) and up to 128
+// tokens, and walks k in chunks of 32 elements:
+//
+//   producers  one thread requests the activation tiles (64 elements x N tokens, hi and lo, 128-byte swizzle), one the raw blocks of a
+//              256-element unit (TMA boxes of 32 rows; Q6_K's 210-byte blocks have no 16-byte alignment: two warps copy them by words);
+//   unpack     sixteen warps in four groups that take the chunks in turn (two at a time up to 64 tokens): thread r owns row r, turns the chunk's 32
+//              elements into f16 integers by byte permutes, hi = d' q and lo = d' q - hi by two f16x2 instructions (exact), and stores both with
+//              tcgen05.st as the A operand in TENSOR MEMORY (lane = row, column = two consecutive k).  A group has a tensor-memory
+//              stage of its own, so every barrier has one waiter that sees all of its phases;
+//   multiply   one warp, whose elected lane issues;
+//   drain      the unpack warps again: when a unit is through, group g adds tokens 32 g ... 32 g + 31 of `main` to its registers, one
+//              unit behind its unpacking, so it never waits for the products it feeds.  `main` has two places that units take in turn.
+//
+// What bounds it: the tensor pipe.  192 cycles per 128 rows x 128 tokens x 16 elements (128 + 64 for the two instructions; measured
+// 128 / 64 / 45 / 45 cycles at N = 256 / 128 / 64 / 32 and below), i.e. a third of the f16 rate; few tokens are bound by the 45
+// cycles that any instruction takes.  Unpacking takes 2.4 instructions per weight (Q6_K five), a quarter of the issue slots at 128 tokens.
+#include <algorithm>
+#include <cstdlib>
+#include <cuda_fp16.h>
+#include "lc_kernels.h"
+#include "lc_quant.cuh"
+#include "lc_tma.cuh"
+#include "lc_umma.cuh"
+
+namespace lc {
+
+namespace {
+
+constexpr int kRows = 128;       // weight rows per CTA = MMA M
+constexpr int kMaxTok = 128;     // most tokens per CTA
+constexpr int kMaxRaw = 8;       // raw units in flight
+constexpr int kMaxB = 8;         // activation chunks (64 elements) in flight
+constexpr int kGroups = 4;       // unpack groups of four warps
+constexpr int kControl = 4;      // warps ahead of them: activation producer, issuer, raw producer (Q6_K: two)
+constexpr int kThreads = 32 * (kControl + 4 * kGroups);
+// Tensor-memory columns: main of even units [128 - N, 128), small [128, 128 + N), main of odd units [128 + N, 128 + 2 N): small borders on
+// both, so that one instruction covers main and small of either (odd units have their activations as [lo | hi]).  Behind them
+// the A stages, 32 columns each: 16 of W_hi, 16 of W_lo for 32 elements of k; four, or eight where 64 tokens and fewer leave the room.
+constexpr uint32_t kColSmall = 128;
+__host__ __device__ constexpr uint32_t col_a(int N) { return N <= 64 ? 256u : 384u; }
+
+template <uint32_t TYPE> struct RawUnit;  // bytes of a row's unit in shared memory
+template <> struct RawUnit<LC_TYPE_Q4_K> { static constexpr int pitch = 144; };
+template <> struct RawUnit<LC_TYPE_Q5_K> { static constexpr int pitch = 176; };
+template <> struct RawUnit<LC_TYPE_Q4_0> { static constexpr int pitch = 144; };
+template <> struct RawUnit<LC_TYPE_Q8_0> { static constexpr int pitch = 272; };
+template <> struct RawUnit<LC_TYPE_Q6_K> { static constexpr int pitch = 212; };  // 210 from a word boundary on; an odd number of words: no bank conflicts
+template <uint32_t TYPE> constexpr bool kHasMin = TYPE == LC_TYPE_Q4_K || TYPE == LC_TYPE_Q5_K;
+
+struct GemmParams {
+    float* out;             // [T, n]
+    const float* residual;  // or null
+    const float* tok_scale; // [T] power of two that the preparation divided token t by
+    const float* row_down0; // [n] power of two that brings row r's weights back (and of the second matrix)
+    const float* row_down1;
+    const unsigned char *w0, *w1;  // raw blocks
+    size_t row_bytes;
+    int n, k, T;
+    int N;                  // tokens per CTA, a multiple of 16: the box height of the activation tensor maps
+    int epi;                // GemvEpilogue; EPI_SILU_MUL: 64 rows of each matrix per CTA
+    int raw_stages, b_stages;
+    int ksplit;             // CTAs along k per tile (gridDim.z)
+    int row_dynamic;        // row_down comes from a kernel ahead of this one in the stream
+    float* partial;         // [ksplit][matrices][T][n] f32 for the summing kernel, or null: the CTA holds the whole sum and writes `out`
+    int* error_flag;
+};
+
+// ---- tcgen05 wrappers -------------------------------------------------------------------------------------------------
+// f32 accumulate, f16 x f16, both K-major, M = 128
+__host__ __device__ constexpr uint32_t idesc_f16(int n_tok) {
+    return (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(n_tok >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
+}
+// D[tmem] (+)= A[tmem] * B[smem]^T
+__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(db), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+        "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
+}
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(r));
+    return r != 0;
+}
+// ---- unpacking ---------------------------------------------------------------------------------------------------------
+// bytes b0, b1 (or b2, b3) of v as the f16 pair (1024 + b0, 1024 + b1): 0x64 is the high byte of 1024.0
+__device__ __forceinline__ uint32_t bias_pair(uint32_t v, int upper) { return __byte_perm(v, 0x64646464u, upper ? 0x5342u : 0x5140u); }
+__device__ __forceinline__ uint32_t h2_fma(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+__device__ __forceinline__ uint32_t h2_mul(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t h2_add(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t h2_neg(uint32_t a) { return a ^ 0x80008000u; }
+__device__ __forceinline__ uint32_t h2_pair(float v) {  // (v, v) as f16x2
+    const __half2 h = __float2half2_rn(v);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+__device__ __forceinline__ uint32_t f16_at(const unsigned char* p) { return *reinterpret_cast<const uint16_t*>(p); }
+// words [0, OUT) of the bytes that begin `shift` (even, below 16) bytes into w; `shift` is the same for the whole warp
+template <int IN, int OUT>
+__device__ __forceinline__ void shift_words(uint32_t (&w)[IN], int shift, uint32_t (&o)[OUT]) {
+    if (shift & 8) {
+#pragma unroll
+        for (int i = 0; i + 2 < IN; i++) w[i] = w[i + 2];
+    }
+    if (shift & 4) {
+#pragma unroll
+        for (int i = 0; i + 1 < IN; i++) w[i] = w[i + 1];
+    }
+    const uint32_t bits = (uint32_t)(shift & 2) * 8u;
+#pragma unroll
+    for (int i = 0; i < OUT; i++) o[i] = __funnelshift_r(w[i], w[i + 1 < IN ? i + 1 : i], bits);
+}
+// hi = s q rounded to f16, lo = what that lost: exact where s q has 22 bits and less
+__device__ __forceinline__ void split_product(uint32_t s, uint32_t q, uint32_t& hi, uint32_t& lo) {
+    hi = h2_mul(s, q);
+    lo = h2_fma(s, q, h2_neg(hi));
+}
+// Elements 32 j ... 32 j + 31 of a row's unit times `up`, as f16 pairs: column c holds elements 2 c and 2 c + 1.
+// Q4_K (mod.rs:66-98): sub-block j has the low (even j) or high nibbles of bytes 32 (j / 2) ... under scale sc[j];
+// (1024 + q) sc - 1024 sc is one fused multiply-add with the exact result sc q <= 945.  Q5_K (mod.rs:101-142): a fifth bit, <= 1953.
+struct UnitHead { float d; uint32_t sc_lo, sc_hi; };  // d times `up`, the eight scales (of the types that have them)
+template <uint32_t TYPE>
+__device__ __forceinline__ UnitHead load_head(const unsigned char* rp, float up) {
+    UnitHead h{0.f, 0u, 0u};
+    if constexpr (kHasMin<TYPE>) {
+        const uint4 w = *reinterpret_cast<const uint4*>(rp);  // d, dmin, 12 scale bytes
+        uint32_t mn_lo, mn_hi;
+        unpack_scales_k4(w.y, w.z, w.w, &h.sc_lo, &h.sc_hi, &mn_lo, &mn_hi);
+        h.d = h2f((uint16_t)(w.x & 0xFFFFu)) * up;
+    } else if constexpr (TYPE == LC_TYPE_Q6_K) {
+        h.d = h2f((uint16_t)f16_at(rp + 208)) * up;
+    }
+    return h;
+}
+template <uint32_t TYPE>
+__device__ __forceinline__ void unpack_chunk(const unsigned char* rp, const UnitHead& head, int j, float up, uint32_t (&hi)[16], uint32_t (&lo)[16]) {
+    if constexpr (kHasMin<TYPE>) {
+        // high nibbles stay where they are: (1024 + 16 q) (sc / 16) - 1024 (sc / 16)
+        const float sub = (float)(((j < 4 ? head.sc_lo : head.sc_hi) >> (8 * (j & 3))) & 0xFFu);
+        constexpr bool fifth = TYPE == LC_TYPE_Q5_K;
+        const float fs = (j & 1) && !fifth ? sub * 0.0625f : sub;
+        const uint32_t mask = (j & 1) && !fifth ? 0xF0F0F0F0u : 0x0F0F0F0Fu;
+        const uint32_t d = h2_pair(head.d), sc = h2_pair(fs), bias = h2_pair(-1024.0f * fs);
+        const uint4* q = reinterpret_cast<const uint4*>(rp + (TYPE == LC_TYPE_Q5_K ? 48 : 16) + 32 * (j >> 1));
+        const int sh = (j & 1) * 4;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const uint4 v = q[h];
+            const uint32_t vv[4] = {v.x, v.y, v.z, v.w};
+            uint32_t hb[4] = {0u, 0u, 0u, 0u};
+            if constexpr (TYPE == LC_TYPE_Q5_K) {
+                const uint4 hq = *reinterpret_cast<const uint4*>(rp + 16 + 16 * h);
+                hb[0] = hq.x; hb[1] = hq.y; hb[2] = hq.z; hb[3] = hq.w;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                uint32_t b = (fifth ? vv[i] >> sh : vv[i]) & mask;
+                if constexpr (TYPE == LC_TYPE_Q5_K) b |= ((hb[i] >> j) & 0x01010101u) << 4;
+                const int c = h * 8 + i * 2;
+                split_product(d, h2_fma(bias_pair(b, 0), sc, bias), hi[c], lo[c]);
+                split_product(d, h2_fma(bias_pair(b, 1), sc, bias), hi[c + 1], lo[c + 1]);
+            }
+        }
+    } else if constexpr (TYPE == LC_TYPE_Q4_0) {  // mod.rs:16-34: 18 bytes: scale, low nibbles = elements 0..15, high = 16..31
+        const int at = 18 * j;
+        const uint4* p = reinterpret_cast<const uint4*>(rp + (at & ~15));
+        const uint4 a = p[0], b = p[1];  // j <= 7: the block ends within two pieces (at most byte 14 + 18 of them)
+        uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}, o[5];
+        shift_words(w, at & 15, o);
+        const uint32_t d = h2_pair(h2f((uint16_t)(o[0] & 0xFFFFu)) * up), m8 = 0xE408E408u;  // -1032
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const uint32_t v = __funnelshift_r(o[i], o[i + 1], 16);
+            const uint32_t bl = v & 0x0F0F0F0Fu, bh = (v >> 4) & 0x0F0F0F0Fu;
+            split_product(d, h2_add(bias_pair(bl, 0), m8), hi[2 * i], lo[2 * i]);
+            split_product(d, h2_add(bias_pair(bl, 1), m8), hi[2 * i + 1], lo[2 * i + 1]);
+            split_product(d, h2_add(bias_pair(bh, 0), m8), hi[8 + 2 * i], lo[8 + 2 * i]);
+            split_product(d, h2_add(bias_pair(bh, 1), m8), hi[9 + 2 * i], lo[9 + 2 * i]);
+        }
+    } else if constexpr (TYPE == LC_TYPE_Q8_0) {  // mod.rs:37-51: 34 bytes: scale, 32 signed bytes
+        const int at = 34 * j;
+        const uint4* p = reinterpret_cast<const uint4*>(rp + (at & ~15));
+        const uint4 a = p[0], b = p[1], e = p[2];  // ends at most at byte 14 + 34 of the three pieces
+        uint32_t w[12] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, e.x, e.y, e.z, e.w}, o[9];
+        shift_words(w, at & 15, o);
+        const uint32_t d = h2_pair(h2f((uint16_t)(o[0] & 0xFFFFu)) * up), m = 0xE480E480u;  // -1152 = -(1024 + 128)
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const uint32_t v = __funnelshift_r(o[i], o[i + 1], 16) ^ 0x80808080u;  // byte + 128
+            split_product(d, h2_add(bias_pair(v, 0), m), hi[2 * i], lo[2 * i]);
+            split_product(d, h2_add(bias_pair(v, 1), m), hi[2 * i + 1], lo[2 * i + 1]);
+        }
+    } else {  // Q6_K, mod.rs:145-180; rp: the block's first byte, on an even address
+        const int n = j >> 2, quad = j & 3;
+        const uint32_t off = (uint32_t)(uintptr_t)rp & 2u, bits = off * 8u;
+        const uint32_t* wl = reinterpret_cast<const uint32_t*>(rp - off) + 16 * n + 8 * (quad & 1);
+        const uint32_t* wh = reinterpret_cast<const uint32_t*>(rp - off) + 32 + 8 * n;
+        uint32_t l[9], h[9];
+#pragma unroll
+        for (int i = 0; i < 9; i++) { l[i] = wl[i]; h[i] = wh[i]; }
+        uint32_t sh[2], sl[2];
+#pragma unroll
+        for (int i = 0; i < 2; i++) {  // d sc has 18 bits: two f16
+            const float s = head.d * (float)*reinterpret_cast<const int8_t*>(rp + 192 + 8 * n + 2 * quad + i);
+            const float top = __half2float(__float2half_rn(s));
+            sh[i] = h2_pair(s);
+            sl[i] = h2_pair(s - top);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const uint32_t vl = __funnelshift_r(l[i], l[i + 1], bits), vh = __funnelshift_r(h[i], h[i + 1], bits);
+            const uint32_t b = ((vl >> (4 * (quad >> 1))) & 0x0F0F0F0Fu) | (((vh >> (2 * quad)) & 0x03030303u) << 4);
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const uint32_t q = h2_add(bias_pair(b, k), 0xE420E420u);  // -1056 = -(1024 + 32)
+                const int c = 2 * i + k;
+                split_product(sh[i >> 2], q, hi[c], lo[c]);
+                lo[c] = h2_fma(sl[i >> 2], q, lo[c]);
+            }
+        }
+    }
+}
+// The offset operand of a unit: p[i] = -dmin * m[i] has at most 17 significant bits, so hi = f16(p) and lo = f16(p - hi)
+// carry it exactly.  Columns 0-3: the eight hi as pairs (k' = 0..7), columns 4-7: the eight lo (k' = 8..15); the sums tile holds
+// each sub-block sum at k' and k' + 8.
+__device__ __forceinline__ void unpack_mins(uint4 w, float up, uint32_t* col) {
+    uint32_t sc_lo, sc_hi, mn_lo, mn_hi;
+    unpack_scales_k4(w.y, w.z, w.w, &sc_lo, &sc_hi, &mn_lo, &mn_hi);
+    const float dmin = h2f((uint16_t)(w.x >> 16)) * up;
+#pragma unroll
+    for (int j2 = 0; j2 < 4; j2++) {
+        __half hi[2], lo[2];
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int i = 2 * j2 + e;
+            const float pr = -dmin * (float)(((i < 4 ? mn_lo : mn_hi) >> (8 * (i & 3))) & 0xFFu);
+            hi[e] = __float2half_rn(pr);
+            lo[e] = __float2half_rn(pr - __half2float(hi[e]));
+        }
+        const __half2 a = __halves2half2(hi[0], hi[1]), b = __halves2half2(lo[0], lo[1]);
+        col[j2] = *reinterpret_cast<const uint32_t*>(&a);
+        col[4 + j2] = *reinterpret_cast<const uint32_t*>(&b);
+    }
+}
+
+// ---- row scales ----------------------------------------------------------------------------------------------------------
+// A power of two per row that brings its weights up to 2^13 ... 2^14: the low half of a weight then keeps its bits above
+// 2^-24, f16's smallest step, unless it is 2^-17 of the row's largest.  One warp per row; down[r] = 2^-s.
+__global__ void __launch_bounds__(256) row_scale_kernel(uint32_t typ, const unsigned char* __restrict__ w, size_t row_bytes, int n, int k, float* __restrict__ down) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (row >= n) return;
+    const unsigned char* rp = w + (size_t)row * row_bytes;
+    float bound = 0.f;
+    const int blocks = typ == LC_TYPE_Q4_0 || typ == LC_TYPE_Q8_0 ? k / 32 : k / 256;
+    for (int b = lane; b < blocks; b += 32) {
+        float v = 0.f;
+        if (typ == LC_TYPE_Q4_K || typ == LC_TYPE_Q5_K) {
+            const unsigned char* p = rp + (size_t)b * (typ == LC_TYPE_Q4_K ? 144 : 176);
+            const uint4 h = *reinterpret_cast<const uint4*>(p);
+            uint32_t sl, sh, ml, mh;
+            unpack_scales_k4(h.y, h.z, h.w, &sl, &sh, &ml, &mh);
+            const uint32_t s = __vmaxu4(sl, sh), m = __vmaxu4(ml, mh);
+            const float sm = (float)max(max(s & 0xFFu, (s >> 8) & 0xFFu), max((s >> 16) & 0xFFu, s >> 24));
+            const float mm = (float)max(max(m & 0xFFu, (m >> 8) & 0xFFu), max((m >> 16) & 0xFFu, m >> 24));
+            const float d = fabsf(h2f((uint16_t)(h.x & 0xFFFFu))), dm = fabsf(h2f((uint16_t)(h.x >> 16)));
+            v = fmaxf(d * fmaxf(sm, 1.f) * (typ == LC_TYPE_Q4_K ? 15.f : 31.f), dm * fmaxf(mm, 1.f));
+        } else if (typ == LC_TYPE_Q4_0) {
+            v = 8.f * fabsf(h2f((uint16_t)f16_at(rp + (size_t)b * 18)));
+        } else if (typ == LC_TYPE_Q8_0) {
+            v = 128.f * fabsf(h2f((uint16_t)f16_at(rp + (size_t)b * 34)));
+        } else {
+            const unsigned char* p = rp + (size_t)b * 210;
+            int s = 1;
+            for (int i = 0; i < 16; i++) s = max(s, abs((int)*reinterpret_cast<const int8_t*>(p + 192 + i)));
+            v = 32.f * (float)s * fabsf(h2f((uint16_t)f16_at(p + 208)));
+        }
+        if (v < INFINITY) bound = fmaxf(bound, v);  // a broken block gives NaN in its row whatever the scale
+    }
+    bound = warp_max(bound);
+    if (lane == 0) {
+        int e = 0;
+        if (bound > 0.f) (void)frexpf(bound, &e);  // bound = f 2^e, f in [0.5, 1)
+        down[row] = ldexpf(1.0f, e - 14);          // e within f16's range times 63 * 31 or 127 * 32
+    }
+}
+
+// grid = (row tiles, token tiles, shares of k).  tm0 / tm1: raw blocks of the
+// matrix (and of `up` for EPI_SILU_MUL), box = one unit x 32 rows.  tmx: the prepared activations [2 halves][t_cap rows][k] f16, box = 64
+// elements x N rows of one half; tms: the sub-block sums [2][t_cap rows][k / 16], the same box.
+// WIDE: more than 64 tokens.  Sub-chunk j (32 elements) of a unit then belongs to group j & 3, stage by stage; else group g has the 64 elements
+// from 64 g on as one stage, so that the issuer waits half as often for products that are soon over.
+template <uint32_t TYPE, bool WIDE>
+__global__ void __launch_bounds__(kThreads, 1)
+qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1, const __grid_constant__ CUtensorMap tmx,
+                  const __grid_constant__ CUtensorMap tms, GemmParams p) {
+    constexpr int kPitch = RawUnit<TYPE>::pitch;
+    constexpr bool kWords = TYPE == LC_TYPE_Q6_K;  // raw units copied by words
+    constexpr uint32_t raw_bytes = kPitch * kRows;
+    constexpr int kOwn = WIDE ? 32 : 16;           // tokens whose sums a thread keeps
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const bool pair = p.epi == EPI_SILU_MUL;
+    const int N = p.N;
+    const int RS = p.raw_stages, BS = p.b_stages;
+    const uint32_t b_half = (uint32_t)N * 128u;
+
+    unsigned char* bt = smem;                          // [BS][two tiles of N x 128 B]
+    unsigned char* raw = bt + (size_t)BS * 2 * b_half;  // [RS][raw_bytes]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(raw + (size_t)RS * raw_bytes);
+    uint64_t* raw_full = bars;                 // [kMaxRaw] producer -> unpack
+    uint64_t* raw_empty = raw_full + kMaxRaw;  // [kMaxRaw] unpack (a warp each) -> producer
+    uint64_t* b_full = raw_empty + kMaxRaw;    // [kMaxB]   producer -> issuer
+    uint64_t* b_empty = b_full + kMaxB;        // [kMaxB]   commit -> producer
+    uint64_t* a_full = b_empty + kMaxB;        // [4]       a group's four warps -> issuer
+    uint64_t* a_empty = a_full + 4;            // [4]       commit -> that group
+    uint64_t* d_full = a_empty + 4;            // [2]       commit -> drain
+    uint64_t* d_empty = d_full + 2;            // [2]       drain (a warp each) -> issuer
+    uint64_t* wound = d_empty + 2;             // [1]       products in flight when a wait of the issuer ran out
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(wound + 1);
+
+    const int drains = WIDE ? 4 * ((N + 31) / 32) : 4 * kGroups;  // warps that keep sums
+    if (warp == 0 && lane == 0) {
+        for (int i = 0; i < kMaxRaw; i++) { mbar_init(&raw_full[i], kWords ? 64 : 1); mbar_init(&raw_empty[i], 4 * kGroups); }
+        for (int i = 0; i < kMaxB; i++) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
+        for (int i = 0; i < kGroups; i++) { mbar_init(&a_full[i], 4); mbar_init(&a_empty[i], 1); }
+        for (int i = 0; i < 2; i++) { mbar_init(&d_full[i], 1); mbar_init(&d_empty[i], drains); }
+        mbar_init(wound, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 1) tmem_alloc(tmem_slot, 512);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    bool ok = true;
+
+    // this CTA's share of k: whole groups of four units (one chunk of sub-block sums); unit v below is u_begin + v
+    const int row0 = blockIdx.x * (pair ? kRows / 2 : kRows), tok0 = blockIdx.y * N, nquads = (p.k / kUnitElems + 3) / 4;
+    const int u_begin = (int)((long long)blockIdx.z * nquads / p.ksplit) * 4;
+    const int nu = min((int)((long long)(blockIdx.z + 1) * nquads / p.ksplit) * 4, p.k / kUnitElems) - u_begin;
+    const int sum_chunks = kHasMin<TYPE> ? (nu + 3) / 4 : 0;  // chunks of sub-block sums behind the units, four units each,
+    const int nv = nu + (sum_chunks + 3) / 4;                 // as further units of up to four chunks
+    auto chunks_of = [&](int v) { return v < nu ? 4 : min(4, sum_chunks - 4 * (v - nu)); };
+
+    // Stages are counted along, never by division: one takes a single thread 100 cycles.
+    if (warp == 0) {
+        // ---------------------------------------------------------------- producer of the activations
+        if (lane == 0) {
+            pdl_wait();
+            int sb = 0, in_flight = 0;
+            uint32_t phase = 1;
+            {
+                for (int v = 0; v < nv && ok; v++) {
+                    unsigned char* const hi_first = bt + (v & 1) * b_half;  // odd units: [lo | hi]
+                    unsigned char* const lo_first = bt + (1 - (v & 1)) * b_half;
+                    const int nc = chunks_of(v);
+                    for (int c = 0; c < nc; c++) {
+                        if (!mbar_wait(&b_empty[sb], phase)) { ok = false; break; }
+                        const CUtensorMap* m = v < nu ? &tmx : &tms;
+                        const int x = v < nu ? (u_begin + v) * kUnitElems + c * 64 : (u_begin / 4 + (v - nu) * 4 + c) * 64;
+                        mbar_expect_tx(&b_full[sb], 2 * b_half);
+                        tma_load_3d(hi_first + (size_t)sb * 2 * b_half, m, x, tok0, 0, &b_full[sb]);
+                        tma_load_3d(lo_first + (size_t)sb * 2 * b_half, m, x, tok0, 1, &b_full[sb]);
+                        in_flight = min(in_flight + 1, BS);
+                        if (++sb == BS) { sb = 0; phase ^= 1; }
+                    }
+                }
+            }
+            if (!ok)  // copies in flight land first: the newest of each stage (phase: that of `empty` for stage sb)
+                for (int i = 0; i < in_flight; i++) {
+                    if (sb == 0) { sb = BS; phase ^= 1; }
+                    mbar_wait(&b_full[--sb], phase ^ 1);
+                }
+        }
+    } else if (!kWords && warp == 2) {
+        // ---------------------------------------------------------------- producer of the raw units
+        // the weights do not depend on the kernel ahead of this one, so this stream starts before the wait for it
+        if (lane == 0) {
+            int sr = 0, in_flight = 0;
+            uint32_t phase = 1;
+            {
+                for (int v = 0; v < nu; v++) {
+                    if (!mbar_wait(&raw_empty[sr], phase)) { ok = false; break; }
+                    mbar_expect_tx(&raw_full[sr], raw_bytes);
+#pragma unroll
+                    for (int b = 0; b < 4; b++)
+                        tma_load_2d(raw + (size_t)sr * raw_bytes + b * 32 * kPitch, pair && b >= 2 ? &tm1 : &tm0, (u_begin + v) * (kPitch / 4),
+                                    row0 + (pair ? b & 1 : b) * 32, &raw_full[sr]);
+                    in_flight = min(in_flight + 1, RS);
+                    if (++sr == RS) { sr = 0; phase ^= 1; }
+                }
+            }
+            if (!ok)
+                for (int i = 0; i < in_flight; i++) {
+                    if (sr == 0) { sr = RS; phase ^= 1; }
+                    mbar_wait(&raw_full[--sr], phase ^ 1);
+                }
+        }
+    } else if (kWords && (warp == 2 || warp == 3)) {
+        // ---------------------------------------------------------------- the same by words: a warp per row, every other row
+        int sr = 0;
+        uint32_t phase = 1;
+        {
+            for (int v = 0; v < nu; v++) {
+                ok = __all_sync(0xffffffffu, mbar_wait(&raw_empty[sr], phase));
+                if (!ok) break;
+                uint32_t dst = smem_u32(raw + (size_t)sr * raw_bytes + (warp - 2) * kPitch) + lane * 4;
+#pragma unroll 1
+                for (int half = 0; half < 2; half++) {  // rows 0 .. 63, 64 .. 127 (pair: of the second matrix)
+                    const int first = row0 + (pair ? 0 : half * 64) + warp - 2;
+                    const unsigned char* src = (pair && half ? p.w1 : p.w0) + (size_t)(u_begin + v) * 210;
+                    const size_t step = 2 * p.row_bytes;
+                    const int live = min(32, (p.n - first + 1) / 2);  // rows past the end: any data, dropped at the end
+                    const unsigned char* row = src + (size_t)first * p.row_bytes;
+#pragma unroll 4
+                    for (int r = 0; r < live; r++, row += step, dst += 2 * kPitch) {
+                        const unsigned char* base = reinterpret_cast<const unsigned char*>((uintptr_t)row & ~(uintptr_t)2) + lane * 4;
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(base) : "memory");
+                        // words 32 ... 52; of the last one only two bytes where the block began on a word
+                        const uint32_t take = lane < 20 ? 4u : 2u + ((uint32_t)(uintptr_t)row & 2u);
+                        if (lane < 21) asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + 128), "l"(base + 128), "r"(take) : "memory");
+                    }
+                    dst += (32 - max(live, 0)) * 2 * kPitch;
+                }
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&raw_full[sr])) : "memory");
+                if (++sr == RS) { sr = 0; phase ^= 1; }
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else if (warp == 1) {
+        // ---------------------------------------------------------------- multiply
+        // the whole warp walks the loop and waits (uniform control flow, so that operands live in uniform registers: one lane walking it alone
+        // issues a product every 57 cycles at best, and every 200 here), one lane issues
+        const bool one = elect_one();
+        const uint32_t id1 = idesc_f16(N), id2 = idesc_f16(2 * N), d_small = tmem + kColSmall, a0 = tmem + col_a(N);
+        int sb = 0;
+        uint32_t b_phase = 0;
+        const uint64_t b_first = umma_desc_sw128(smem_u32(bt)), b_step = (2 * b_half) >> 4, b_tile = b_half >> 4;
+        uint64_t b_both = b_first;
+        for (int v = 0; v < nu && ok; v++) {
+            const uint32_t odd = v & 1;
+            const uint32_t d_both = odd ? d_small : d_small - (uint32_t)N, d_main = odd ? d_small + (uint32_t)N : d_both;
+            const uint64_t to_hi = odd ? b_tile : 0, to_lo = odd ? 0 : b_tile;
+            if (v >= 2) ok = mbar_wait(&d_empty[odd], ((v >> 1) - 1) & 1);
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                ok = ok && mbar_wait(&b_full[sb], b_phase);
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const uint32_t st = WIDE ? (2 * c + h) & 3 : c, a = a0 + (WIDE ? st * 32 : st * 64 + h * 32);
+                    if (WIDE || h == 0) ok = ok && mbar_wait(&a_full[st], WIDE ? (uint32_t)(c >> 1) : odd);  // the stage's uses: WIDE 2 v and 2 v + 1, else v
+                    tc_fence_after();
+                    if (one && ok) {
+                        const uint64_t bb = b_both + 4 * h;
+                        if (c == 0 && h == 0) {  // the unit's first: main starts anew
+                            umma_f16_ts(d_main, a, bb + to_hi, id1, 0u);
+                            umma_f16_ts(d_small, a, bb + to_lo, id1, (uint32_t)(v > 0));
+                        } else {
+                            umma_f16_ts(d_both, a, bb, id2, 1u);
+                        }
+                        umma_f16_ts(d_small, a + 16, bb + to_hi, id1, 1u);
+                        umma_f16_ts(d_both, a + 8, bb + 2, id2, 1u);
+                        umma_f16_ts(d_small, a + 24, bb + 2 + to_hi, id1, 1u);
+                        if (WIDE || h == 1) umma_commit(&a_empty[st]);
+                        if (h == 1) umma_commit(&b_empty[sb]);
+                        if (h == 1 && c == 3) umma_commit(&d_full[odd]);
+                    }
+                    __syncwarp();
+                }
+                b_both += b_step;
+                if (++sb == BS) { sb = 0; b_phase ^= 1; b_both = b_first; }
+            }
+        }
+        for (int v = nu; kHasMin<TYPE> && v < nv && ok; v++) {  // the offsets: no low halves beside the high ones
+            const uint32_t odd = v & 1;
+            const uint32_t d_both = odd ? d_small : d_small - (uint32_t)N, d_main = odd ? d_small + (uint32_t)N : d_both;
+            const int nc = chunks_of(v);
+            if (v >= 2) ok = mbar_wait(&d_empty[odd], ((v >> 1) - 1) & 1);
+            for (int c = 0; c < nc && ok; c++) {
+                ok = mbar_wait(&b_full[sb], b_phase);
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const uint32_t st = WIDE ? (2 * c + h) & 3 : c, a = a0 + (WIDE ? st * 32 : st * 64 + h * 32);
+                    if (WIDE || h == 0) ok = ok && mbar_wait(&a_full[st], WIDE ? (uint32_t)(c >> 1) : odd);
+                    tc_fence_after();
+                    if (one && ok) {
+                        const uint64_t bb = b_both + 4 * h;
+                        if (c == 0 && h == 0) {
+                            umma_f16_ts(d_main, a, bb + (odd ? b_tile : 0), id1, 0u);
+                            umma_f16_ts(d_small, a, bb + (odd ? 0 : b_tile), id1, 1u);
+                        } else {
+                            umma_f16_ts(d_both, a, bb, id2, 1u);
+                        }
+                        umma_f16_ts(d_both, a + 8, bb + 2, id2, 1u);
+                        if (WIDE || h == 1) umma_commit(&a_empty[st]);
+                        if (h == 1) umma_commit(&b_empty[sb]);
+                        if (h == 1 && c == nc - 1) umma_commit(&d_full[odd]);
+                    }
+                    __syncwarp();
+                }
+                b_both += b_step;
+                if (++sb == BS) { sb = 0; b_phase ^= 1; b_both = b_first; }
+            }
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) {
+            if (one) umma_commit(wound);
+            mbar_wait(wound, 0);
+        }
+    } else if (warp >= kControl) {
+        // ---------------------------------------------------------------- unpack and drain, then the epilogue
+        const int g = (warp - kControl) >> 2, quarter = warp & 3;
+        const int row = quarter * 32 + lane;  // of the tile; also the tensor-memory lane
+        const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16), a_stage = lane_base + col_a(N) + (uint32_t)g * (WIDE ? 32 : 64);
+        const int mat = pair ? quarter >> 1 : 0;
+        const unsigned char* const weights = mat ? p.w1 : p.w0;
+        const int own = WIDE ? max(0, min(32, N - 32 * g)) : N / 4, tbase = g * (WIDE ? 32 : N / 4);  // this thread's tokens of the tile
+        auto wait_all = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); };
+        float y[kOwn];
+        auto add_columns = [&](uint32_t col) {
+            col += lane_base + tbase;
+            if constexpr (WIDE) {
+#pragma unroll
+                for (int t0 = 0; t0 < 32; t0 += 16)
+                    if (t0 < own) {
+                        uint32_t a[16];
+                        tmem_ld16(col + t0, a);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                        for (int t = 0; t < 16; t++) y[t0 + t] += __uint_as_float(a[t]);
+                    }
+            } else {
+                uint32_t a[16];
+#pragma unroll
+                for (int t0 = 0; t0 < 16; t0 += 4)
+                    if (t0 < own) tmem_ld4(col + t0, a + t0);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int t0 = 0; t0 < 16; t0 += 4)
+                    if (t0 < own) {
+#pragma unroll
+                        for (int t = t0; t < t0 + 4; t++) y[t] += __uint_as_float(a[t]);
+                    }
+            }
+        };
+        auto drain = [&](uint32_t w) {  // unit w
+            if (own <= 0) return;
+            ok = wait_all(&d_full[w & 1], (w >> 1) & 1);
+            if (!ok) return;
+            tc_fence_after();
+            add_columns(w & 1 ? kColSmall + (uint32_t)N : kColSmall - (uint32_t)N);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&d_empty[w & 1]);
+        };
+        int sr = 0;
+        uint32_t raw_phase = 0, a_phase = 1;
+        if (p.row_dynamic) pdl_wait();
+        {
+            const int grow = row0 + (pair ? row & 63 : row);
+            const bool live = grow < p.n;
+            const unsigned char* const wrow = weights + (size_t)min(grow, p.n - 1) * p.row_bytes;
+            const float down = live ? (mat ? p.row_down1 : p.row_down0)[grow] : 1.0f, up = live ? 1.0f / down : 0.0f;
+#pragma unroll
+            for (int t = 0; t < kOwn; t++) y[t] = 0.f;
+            for (int v = 0; v < nu && ok; v++) {
+                ok = wait_all(&raw_full[sr], raw_phase);
+                if (!ok) break;
+                const unsigned char* rp = raw + (size_t)sr * raw_bytes + (size_t)row * kPitch;
+                if constexpr (kWords) rp += (uint32_t)(uintptr_t)(wrow + (size_t)(u_begin + v) * 210) & 2u;
+                const UnitHead head = load_head<TYPE>(rp, up);
+#pragma unroll 1
+                for (int jj = 0; jj < 2; jj++) {
+                    if (!WIDE && jj == 0) {  // the products of the stage's use before are complete
+                        ok = wait_all(&a_empty[g], a_phase);
+                        if (!ok) break;
+                        a_phase ^= 1;
+                        tc_fence_after();
+                    }
+                    uint32_t hi[16], lo[16];
+                    unpack_chunk<TYPE>(rp, head, WIDE ? g + 4 * jj : 2 * g + jj, up, hi, lo);
+                    if (jj == 1) {
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&raw_empty[sr]);
+                    }
+                    if (WIDE) {
+                        ok = wait_all(&a_empty[g], a_phase);
+                        if (!ok) break;
+                        a_phase ^= 1;
+                        tc_fence_after();
+                    }
+                    tmem_st16(a_stage + (WIDE ? 0 : jj * 32), hi);
+                    tmem_st16(a_stage + (WIDE ? 0 : jj * 32) + 16, lo);
+                    if (WIDE || jj == 1) {
+                        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&a_full[g]);
+                    }
+                }
+                if (ok && v > 0) drain(v - 1);
+                if (++sr == RS) { sr = 0; raw_phase ^= 1; }
+            }
+            for (int v = nu; kHasMin<TYPE> && v < nv && ok; v++) {
+                // the offset operand: two units' sixteen values per sub-chunk, from their headers in global memory (L2: the units passed through it)
+                const int last_j = 2 * chunks_of(v);
+#pragma unroll 1
+                for (int jj = 0; jj < 2; jj++) {
+                    const int j = WIDE ? g + 4 * jj : 2 * g + jj;
+                    if (j >= last_j) break;
+                    if (WIDE || jj == 0) {
+                        ok = wait_all(&a_empty[g], a_phase);
+                        if (!ok) break;
+                        a_phase ^= 1;
+                        tc_fence_after();
+                    }
+                    const int u = u_begin + ((v - nu) * 4 + (j >> 1)) * 4 + (j & 1) * 2;
+                    uint32_t col[16];
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        uint4 hd = make_uint4(0u, 0u, 0u, 0u);
+                        if (live && u + e < u_begin + nu) hd = *reinterpret_cast<const uint4*>(wrow + (size_t)(u + e) * kPitch);
+                        unpack_mins(hd, up, col + 8 * e);
+                    }
+                    tmem_st16(a_stage + (WIDE ? 0 : jj * 32), col);
+                    if (WIDE || jj == 1) {
+                        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&a_full[g]);
+                    }
+                }
+                if (ok) drain(v - 1);
+            }
+            if (ok) drain(nv - 1);
+            if (ok && own > 0) add_columns(kColSmall);  // complete: the last unit's d_full followed every product
+            pdl_wait();
+            const int t_first = tok0 + tbase, mine = ok ? min(own, p.T - t_first) : 0;
+            // a lane has one token's scale: a load beside each result's store would wait for it
+            const float scale = lane < mine ? __ldg(p.tok_scale + t_first + lane) : 0.f;
+#pragma unroll
+            for (int t = 0; t < kOwn; t++) y[t] *= down * __shfl_sync(0xffffffffu, scale, t);
+            if (p.partial) {
+                float* dst = p.partial + ((size_t)(blockIdx.z * (pair ? 2 : 1) + mat) * p.T + t_first) * p.n + grow;
+#pragma unroll
+                for (int t = 0; t < kOwn; t++)
+                    if (live && t < mine) dst[(size_t)t * p.n] = y[t];
+            } else if (pair) {
+                // rows 0 .. 63 of the tile are gate, 64 .. 127 up: the halves meet in the activation stages, which nothing uses any more
+                float* const ex = reinterpret_cast<float*>(bt) + (size_t)tbase * 64 + (row & 63);
+                float* const dst = p.out + (size_t)t_first * p.n + grow;
+                if (mat == 0) {
+#pragma unroll
+                    for (int t = 0; t < kOwn; t++)
+                        if (t < mine) ex[t * 64] = silu_f(y[t]);
+                }
+                asm volatile("bar.sync %0, 128;" ::"r"(1 + g) : "memory");  // all of the group's warps come here, whatever their waits gave
+                if (mat == 1) {
+#pragma unroll
+                    for (int t = 0; t < kOwn; t++)
+                        if (live && t < mine) dst[(size_t)t * p.n] = __fmul_rn(ex[t * 64], y[t]);
+                }
+            } else {
+                const size_t o = (size_t)t_first * p.n + grow;
+#pragma unroll
+                for (int t = 0; t < kOwn; t++)
+                    if (live && t < mine) {
+                        float r = y[t];
+                        if (p.epi == EPI_ADD_RESIDUAL) r = __fadd_rn(p.residual[o + (size_t)t * p.n], r);
+                        p.out[o + (size_t)t * p.n] = r;
+                    }
+            }
+        }
+    }
+    if (!ok && p.error_flag) atomicCAS(p.error_flag, 0, 3);
+    tc_fence_before();
+    __syncthreads();
+    pdl_launch_dependents();  // at the very end: CTAs of the next kernel that move in earlier take SMs from this one's
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_free(tmem, 512);
+    }
+}
+
+}  // namespace
+
+// ---- host side --------------------------------------------------------------------------------------------------------
+bool qgemm_split_weight_ok(const QWeight& w) {
+    switch (w.typ) {
+        case LC_TYPE_Q4_K: case LC_TYPE_Q5_K: case LC_TYPE_Q4_0: case LC_TYPE_Q8_0: return w.has_tmap && w.k % kUnitElems == 0;
+        case LC_TYPE_Q6_K: return w.k % kUnitElems == 0 && (uintptr_t)w.data % 4 == 0;
+        default: return false;
+    }
+}
+int32_t launch_row_scales(const QWeight& w, float* down, cudaStream_t s) {
+    LC_CUDA(launch_pdl(row_scale_kernel, dim3((unsigned)((w.n + 7) / 8)), dim3(256), 0, s, w.typ, (const unsigned char*)w.data, w.row_bytes, w.n, w.k, down));
+    return LC_OK;
+}
+
+namespace {
+struct GemmShape { int N, raw_stages, b_stages; size_t smem; };
+// Tokens per CTA: the fewest tiles, filled evenly.  Stages: five activation chunks (with few tokens eight) and the raw units that fit.
+template <uint32_t TYPE>
+GemmShape shape_for(int T) {
+    GemmShape g;
+    const int tt = (T + kMaxTok - 1) / kMaxTok;
+    g.N = (((T + tt - 1) / tt) + 15) & ~15;
+    const size_t raw = (size_t)RawUnit<TYPE>::pitch * kRows, fixed = 1024 + 512, b = (size_t)2 * g.N * 128;
+    g.b_stages = g.N <= 64 ? kMaxB : 5;
+    while (g.b_stages > 3 && fixed + g.b_stages * b + 3 * raw > kMaxSmem) g.b_stages--;
+    g.raw_stages = std::min<int>(kMaxRaw, (int)((kMaxSmem - fixed - g.b_stages * b) / raw));
+    g.smem = fixed + g.b_stages * b + g.raw_stages * raw;
+    return g;
+}
+// cycles of the tensor pipe per 256-element unit
+long unit_cycles(int N) {
+    const long one = std::max(45, N / 2), two = std::max(45, N);
+    return 16 * (one + two);
+}
+
+template <uint32_t TYPE>
+int32_t launch_type(const GemvArgs& a, const GemmWorkspace& ws, GemmParams& p, int* summed_slices, cudaStream_t s) {
+    const GemmShape g = shape_for<TYPE>(p.T);
+    p.N = g.N; p.raw_stages = g.raw_stages; p.b_stages = g.b_stages;
+    auto kern = g.N <= 64 ? qgemm_split_kernel<TYPE, false> : qgemm_split_kernel<TYPE, true>;
+    LC_CUDA(ensure_smem_limit((const void*)kern, g.smem));
+    alignas(64) CUtensorMap tmx, tms;
+    const size_t rows = (size_t)ws.t_cap;
+    LC_CHECK(make_bf16_tmap_3d(&tmx, ws.xh, (uint64_t)p.k, rows, 2, (uint64_t)p.k, rows * p.k, 64, (uint32_t)g.N, 1) &&
+                 make_bf16_tmap_3d(&tms, ws.sx, (uint64_t)p.k / 16, rows, 2, (uint64_t)p.k / 16, rows * (p.k / 16), 64, (uint32_t)g.N, 1),
+             LC_ERR_CUDA, "qgemm: activation tensor maps");
+    const int nmat = a.epi == EPI_SILU_MUL ? 2 : 1;
+    const int tiles = (p.n * nmat + kRows - 1) / kRows, ttiles = (p.T + g.N - 1) / g.N, nquads = (p.k / kUnitElems + 3) / 4;
+    // Few tiles (a batched decode step, a short prompt): k is cut over several CTAs so that all SMs work, and a second kernel adds
+    // the shares in a fixed order.  Cost in cycles: waves of units plus a fixed part (launch, first unit, drain) per wave, and the
+    // shares' trip through L2 at 3000 bytes per cycle.
+    int ks = 1;
+    double best = 0;
+    for (int c = 1; c <= std::min(8, nquads); c++) {
+        const size_t bytes = (size_t)c * nmat * p.T * p.n * sizeof(float);
+        if (c > 1 && (bytes > ws.partial_bytes || p.n % 4 != 0)) break;
+        const long waves = ((long)tiles * ttiles * c + sm_count() - 1) / sm_count();
+        const double cost = (double)waves * (std::min((nquads + c - 1) / c * 4, p.k / kUnitElems) * unit_cycles(g.N) + 6000) + (c > 1 ? 4000 + 2.0 * bytes / 3000 : 0);
+        if (c == 1 || cost < best) { best = cost; ks = c; }
+    }
+    p.ksplit = ks;
+    p.partial = ks > 1 ? ws.partial : nullptr;
+    *summed_slices = ks > 1 ? ks * nmat : 0;
+    const CUtensorMap* t0 = (const CUtensorMap*)a.w->tmap;
+    const CUtensorMap* t1 = a.w2 ? (const CUtensorMap*)a.w2->tmap : t0;
+    LC_CUDA(launch_pdl(kern, dim3((unsigned)tiles, (unsigned)ttiles, (unsigned)ks), dim3(kThreads), g.smem, s, *t0, *t1, tmx, tms, p));
+    return LC_OK;
+}
+}  // namespace
+
+// The product of prepared activations (ws.xh, ws.sx, ws.tok_scale).  *slices > 0: the shares are in ws.partial, still to be summed.
+int32_t launch_qgemm_split(const GemvArgs& a, GemmWorkspace& ws, int* slices, int* launches, cudaStream_t s) {
+    const int n = a.w->n;
+    const bool pair = a.epi == EPI_SILU_MUL;
+    GemmParams p{};
+    p.row_down0 = a.w->row_down;
+    p.row_down1 = pair ? a.w2->row_down : p.row_down0;
+    if (!p.row_down0 || !p.row_down1) {  // a matrix that was not laid out for this product when it was bound
+        const size_t need = (size_t)n * 2;
+        if (ws.row_cap < need) {
+            if (ws.row_tmp) cudaFree(ws.row_tmp);
+            ws.row_tmp = nullptr; ws.row_cap = 0;
+            LC_CUDA(cudaMalloc((void**)&ws.row_tmp, need * sizeof(float)));
+            ws.row_cap = need;
+        }
+        LC_TRY(launch_row_scales(*a.w, ws.row_tmp, s));
+        if (pair) LC_TRY(launch_row_scales(*a.w2, ws.row_tmp + n, s));
+        p.row_down0 = ws.row_tmp; p.row_down1 = ws.row_tmp + n;
+        p.row_dynamic = 1;
+        *launches += pair ? 2 : 1;
+    }
+    p.out = a.out; p.residual = a.residual; p.tok_scale = ws.tok_scale;
+    p.w0 = (const unsigned char*)a.w->data; p.w1 = pair ? (const unsigned char*)a.w2->data : p.w0;
+    p.row_bytes = a.w->row_bytes;
+    p.n = n; p.k = a.w->k; p.T = a.m; p.epi = (int)a.epi;
+    p.error_flag = gemv_error_flag_dev();
+    *launches += 1;
+    switch (a.w->typ) {
+        case LC_TYPE_Q4_K: return launch_type<LC_TYPE_Q4_K>(a, ws, p, slices, s);
+        case LC_TYPE_Q5_K: return launch_type<LC_TYPE_Q5_K>(a, ws, p, slices, s);
+        case LC_TYPE_Q4_0: return launch_type<LC_TYPE_Q4_0>(a, ws, p, slices, s);
+        case LC_TYPE_Q8_0: return launch_type<LC_TYPE_Q8_0>(a, ws, p, slices, s);
+        default: return launch_type<LC_TYPE_Q6_K>(a, ws, p, slices, s);
+    }
+}
+
+}  // namespace lc

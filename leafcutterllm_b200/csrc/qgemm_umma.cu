@@ -37,6 +37,7 @@
 //
 // Every wait is bounded; a wait that runs out sets the library's device error flag and the CTA winds down (tensor
 // memory freed, no copy left in flight).
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cuda_fp16.h>
@@ -870,6 +871,9 @@ void qgemm_workspace_free(GemmWorkspace* ws) {
     if (ws->tok_scale) cudaFree(ws->tok_scale);
     if (ws->partial) cudaFree(ws->partial);
     ws->partial = nullptr;
+    if (ws->row_tmp) cudaFree(ws->row_tmp);
+    ws->row_tmp = nullptr;
+    ws->row_cap = 0;
     ws->xh = nullptr;
     ws->sx = nullptr;
     ws->tok_scale = nullptr;
@@ -880,32 +884,17 @@ static int gemm_min_tokens() {
     return v;
 }
 bool qgemm_applies(const GemvArgs& a, int T, const GemmWorkspace& ws) {
-    if (!a.w || !ws.xh) return false;
-    if ((a.w->typ != LC_TYPE_Q4_K && a.w->typ != LC_TYPE_Q5_K) || !a.w->has_tmap || a.w->k % kUnitElems != 0) return false;
-    if (a.epi == EPI_SILU_MUL && (!a.w2 || a.w2->typ != a.w->typ || !a.w2->has_tmap)) return false;
+    if (!a.w || !ws.xh || a.group || !qgemm_split_weight_ok(*a.w)) return false;
+    if (a.epi == EPI_SILU_MUL && (!a.w2 || a.w2->typ != a.w->typ || !qgemm_split_weight_ok(*a.w2))) return false;
     if (T < gemm_min_tokens() || T > ws.t_cap || a.w->k > ws.k_max) return false;
     if (((uintptr_t)a.x % 16) != 0 || (a.norm_w && ((uintptr_t)a.norm_w % 16) != 0)) return false;
     return true;
 }
 
-int32_t launch_qgemm(const GemvArgs& a, const GemmWorkspace& ws, cudaStream_t s, int* launches) {
+// The product of prepared activations through the kernel above.  *slices > 0: the shares (or gate's and up's sums) are in ws.partial.
+static int32_t launch_qgemm_tile(const GemvArgs& a, GemmWorkspace& ws, int* slices, cudaStream_t s) {
     const int T = a.m, K = a.w->k, n = a.w->n;
-    LC_CHECK(qgemm_applies(a, T, ws), LC_ERR_INVALID, "qgemm: arguments outside what the kernel implements");
-    if (a.epi == EPI_ADD_RESIDUAL) LC_CHECK(a.residual != nullptr, LC_ERR_INVALID, "qgemm: residual missing");
     const int terms = (getenv("LC_GEMM_TERMS") && atoi(getenv("LC_GEMM_TERMS")) == 1) ? 1 : 3;  // read per call so that a test can switch it
-    // activations: [t_cap rows of high halves | t_cap rows of low halves], each row k elements of this matrix
-    const size_t lo_offset = (size_t)ws.t_cap * K, sx_lo_offset = (size_t)ws.t_cap * (K / 16);
-    // the summing kernel of the product before this one may have prepared exactly this input (GemvArgs::prep_next)
-    const bool prepared = ws.prep_x == a.x && ws.prep_norm == a.norm_w && ws.prep_k == K && ws.prep_t == T && a.x != nullptr;
-    ws.prep_x = nullptr;
-    if (!prepared) {
-        const size_t smem = (size_t)K * sizeof(float);
-        if (smem > 48 * 1024) LC_CUDA(ensure_smem_limit((const void*)xprep_kernel, smem));
-        // a token's row is short (16 - 44 KB) and its three passes are latency: many threads, one or a few float4 each
-        // (64 sequences, 4 layers: 2.43 / 2.40 / 2.40 ms per step with 256 / 512 / 1024 threads)
-        LC_CUDA(launch_pdl(xprep_kernel, dim3(T), dim3(K >= 4096 ? 1024 : 256), smem, s, a.x, a.norm_w, a.eps, K, (__half*)ws.xh, lo_offset, (__half*)ws.sx,
-                           sx_lo_offset, ws.tok_scale));
-    }
     const int N = std::min(kMaxTok, (T + 15) & ~15);
     alignas(64) CUtensorMap tmx, tms;
     LC_CHECK(make_act_tmap_chunks(&tmx, ws.xh, (uint64_t)K, (uint64_t)ws.t_cap, (uint32_t)N, 2), LC_ERR_CUDA, "qgemm: activation tensor map");
@@ -969,22 +958,7 @@ int32_t launch_qgemm(const GemvArgs& a, const GemmWorkspace& ws, cudaStream_t s,
     p.partial = summed ? ws.partial : nullptr;
     dim3 grid((unsigned)(tiles * nmat), (unsigned)ttiles, (unsigned)ks);
     LC_CUDA(launch_pdl(kern, grid, dim3(kThreads), smem, s, *t0, *t1, tmx, tms, p));
-    if (summed) {
-        const size_t plane = (size_t)T * n;
-        if (a.prep_next && n % kUnitElems == 0 && n <= ws.k_max) {
-            // one CTA per token sums the shares and prepares the row for the next product, whose k is this n
-            const size_t rsmem = (size_t)n * sizeof(float);
-            if (rsmem > 48 * 1024) LC_CUDA(ensure_smem_limit((const void*)qgemm_reduce_prep_kernel, rsmem));
-            LC_CUDA(launch_pdl(qgemm_reduce_prep_kernel, dim3(T), dim3(n >= 4096 ? 1024 : 256), rsmem, s, (const float*)ws.partial, nmat * ks, T, n,
-                               (int)a.epi, a.residual, a.out, a.next_norm_w, a.next_eps, (__half*)ws.xh, (size_t)ws.t_cap * n, (__half*)ws.sx,
-                               (size_t)ws.t_cap * (n / 16), ws.tok_scale));
-            ws.prep_x = a.out; ws.prep_norm = a.next_norm_w; ws.prep_k = n; ws.prep_t = T;
-        } else {
-            LC_CUDA(launch_pdl(qgemm_reduce_kernel, dim3((unsigned)((plane / 4 + 255) / 256)), dim3(256), 0, s, (const float*)ws.partial, nmat * ks,
-                               plane, (int)a.epi, a.residual, a.out));
-        }
-    }
-    if (launches) *launches = (prepared ? 1 : 2) + (summed ? 1 : 0);
+    *slices = summed ? nmat * ks : 0;
     if (want_trace) {
         unsigned h[56];
         LC_CUDA(cudaStreamSynchronize(s));
@@ -998,6 +972,56 @@ int32_t launch_qgemm(const GemvArgs& a, const GemmWorkspace& ws, cudaStream_t s,
             fprintf(stderr, " | %8u\n", h[r * 8 + 7]);
         }
     }
+    return LC_OK;
+}
+
+// One token tile of Q4_K / Q5_K stays with the kernel above: it multiplies twice per weight where qgemm_split.cu does three times, and up to
+// 64 tokens its instructions are too short for that to be free.  Measured with the activation preparation, 64 tokens, us here / there:
+// [4096 -> 12288] 40 / 44, [11008 -> 4096] 35 / 38, gate and up 71 / 90; 128 tokens 75 / 48, 68 / 41, 130 / 95; 512 tokens 207 / 136,
+// 190 / 118, 350 / 240.
+static bool use_split(uint32_t typ, int T) { return T > kMaxTok || (typ != LC_TYPE_Q4_K && typ != LC_TYPE_Q5_K); }
+
+int32_t launch_qgemm(const GemvArgs& a, GemmWorkspace& ws, cudaStream_t s, int* launches) {
+    const int T = a.m, K = a.w->k, n = a.w->n;
+    LC_CHECK(qgemm_applies(a, T, ws), LC_ERR_INVALID, "qgemm: arguments outside what the kernel implements");
+    if (a.epi == EPI_ADD_RESIDUAL) LC_CHECK(a.residual != nullptr, LC_ERR_INVALID, "qgemm: residual missing");
+    // activations: [t_cap rows of high halves | t_cap rows of low halves], each row k elements of this matrix
+    const size_t lo_offset = (size_t)ws.t_cap * K, sx_lo_offset = (size_t)ws.t_cap * (K / 16);
+    // the summing kernel of the product before this one may have prepared exactly this input (GemvArgs::prep_next)
+    const bool prepared = ws.prep_x == a.x && ws.prep_norm == a.norm_w && ws.prep_k == K && ws.prep_t == T && a.x != nullptr;
+    ws.prep_x = nullptr;
+    if (!prepared) {
+        const size_t smem = (size_t)K * sizeof(float);
+        if (smem > 48 * 1024) LC_CUDA(ensure_smem_limit((const void*)xprep_kernel, smem));
+        // a token's row is short (16 - 44 KB) and its three passes are latency: many threads, one or a few float4 each
+        // (64 sequences, 4 layers: 2.43 / 2.40 / 2.40 ms per step with 256 / 512 / 1024 threads)
+        LC_CUDA(launch_pdl(xprep_kernel, dim3(T), dim3(K >= 4096 ? 1024 : 256), smem, s, a.x, a.norm_w, a.eps, K, (__half*)ws.xh, lo_offset, (__half*)ws.sx,
+                           sx_lo_offset, ws.tok_scale));
+    }
+    int slices = 0, count = prepared ? 0 : 1;
+    if (use_split(a.w->typ, T)) {
+        LC_TRY(launch_qgemm_split(a, ws, &slices, &count, s));
+    } else {
+        LC_TRY(launch_qgemm_tile(a, ws, &slices, s));
+        count += 1;
+    }
+    if (slices) {
+        count += 1;
+        const size_t plane = (size_t)T * n;
+        if (a.prep_next && n % kUnitElems == 0 && n <= ws.k_max) {
+            // one CTA per token sums the shares and prepares the row for the next product, whose k is this n
+            const size_t rsmem = (size_t)n * sizeof(float);
+            if (rsmem > 48 * 1024) LC_CUDA(ensure_smem_limit((const void*)qgemm_reduce_prep_kernel, rsmem));
+            LC_CUDA(launch_pdl(qgemm_reduce_prep_kernel, dim3(T), dim3(n >= 4096 ? 1024 : 256), rsmem, s, (const float*)ws.partial, slices, T, n,
+                               (int)a.epi, a.residual, a.out, a.next_norm_w, a.next_eps, (__half*)ws.xh, (size_t)ws.t_cap * n, (__half*)ws.sx,
+                               (size_t)ws.t_cap * (n / 16), ws.tok_scale));
+            ws.prep_x = a.out; ws.prep_norm = a.next_norm_w; ws.prep_k = n; ws.prep_t = T;
+        } else {
+            LC_CUDA(launch_pdl(qgemm_reduce_kernel, dim3((unsigned)((plane / 4 + 255) / 256)), dim3(256), 0, s, (const float*)ws.partial, slices,
+                               plane, (int)a.epi, a.residual, a.out));
+        }
+    }
+    if (launches) *launches = count;
     return LC_OK;
 }
 

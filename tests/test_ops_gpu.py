@@ -149,6 +149,36 @@ def test_qmatmul_q4k_many_tokens_tensor_core_gemm(gpu, oracle, monkeypatch, typ,
         assert_close(fast[t], want[t], 4e-3 * np.abs(want[t]).max(), 0, f"one-term gemm token {t}")
 
 
+# one unit, odd numbers of units (rows of Q6_K blocks then start two bytes off a word), token counts on both sides of the 16-token steps
+# and of the tiles of 64 and 128, row counts off the 128-row tile, k cut over several CTAs (few tiles) and not
+@pytest.mark.parametrize("m,k,n", [(5, 256, 1), (17, 768, 130), (64, 4096, 256), (65, 2816, 100), (128, 1024, 384), (129, 11008, 129), (300, 1280, 4100)])
+@pytest.mark.parametrize("typ", [2, 8, 12, 13, 14])
+def test_many_token_product_vs_oracle(gpu, oracle, typ, m, k, n):
+    """Weights of both signs whose block scales differ by 2^12 inside a row and by 2^24 between rows, tokens that differ by e^12.
+    A weight keeps 22 bits beside its row's largest (2^-23), an activation 22 beside its token's, and 256 products are added with
+    truncation before each rounded sum (measured 3.5e-7 of the sum of squares' root): 2e-5 of the largest result leaves ten times that."""
+    r = rng(typ * 1000 + k + n + m)
+    be, bb = gpu.QUANT_GEOMETRY[typ]
+    w = r.integers(0, 256, n * k // be * bb, dtype=np.uint8).reshape(n, -1, bb)
+    size = np.exp2(r.uniform(-18, 6, (n, 1))) * np.exp2(r.uniform(-12, 0, w.shape[:2])) / {2: 8, 8: 128, 12: 945, 13: 1953, 14: 4064}[typ]
+    sc = (np.maximum(size, 2.0 ** -24) * r.choice([-1, 1], w.shape[:2])).astype(np.float16).view(np.uint16)
+    at = 208 if typ == 14 else 0
+    w[..., at], w[..., at + 1] = sc & 0xFF, sc >> 8
+    if typ in (12, 13):
+        w[..., 2], w[..., 3] = sc & 0xFF, sc >> 8
+    w = w.ravel()
+    a = (r.standard_normal((m, k)) * np.exp(r.uniform(-6, 6, (m, 1)))).astype(np.float32)
+    got = gpu.qmatmul(typ, a.ravel(), w, m, k, n).reshape(m, n)
+    dense = gpu.dequantize(typ, w, n * k).reshape(n, k).astype(np.float64)  # bit-exact with the oracle's (tested above)
+    want = a.astype(np.float64) @ dense.T
+    bound = 2e-5 * np.sqrt((a.astype(np.float64) ** 2) @ (dense.T ** 2))  # per result: the root of the products' sum of squares
+    assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / bound).max()
+    rows = r.choice(n, min(n, 8), replace=False)
+    rb = w.size // n
+    sub = np.concatenate([w[i * rb:(i + 1) * rb] for i in rows])
+    assert_close(want[:5, rows], oracle.qmatmul(typ, a[:5].ravel(), sub, 5, k, len(rows)).reshape(5, len(rows)), 2e-5 * np.abs(want[:5, rows]).max(), 1e-4, "oracle sample")
+
+
 def test_qmatmul_linearity_full_size(gpu, oracle):
     """7B-shape matrices: A(x+y) = Ax + Ay and a sample of rows against the oracle."""
     from leafcutterllm_b200 import synth
