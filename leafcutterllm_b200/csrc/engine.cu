@@ -248,8 +248,12 @@ int32_t attention_block(lc_model* m, int l, const float* x, const float* norm_w,
         if (T >= 16 && m->n_tiles > 0 && !no_tc && attention_prefill_applies(kv, m->nh))  // a prefill chunk: tiles of 64 queries on the tensor cores
             LC_TRY(launch_attention_prefill(q, m->nqkv, m->d_attn, m->nh, kv, m->d_tiles, m->n_tiles, m->d_page_table, m->pages_per_seq, m->stream));
         else
-            LC_TRY(launch_attention(q, m->nqkv, m->d_attn, T, m->nh, kv, m->d_tok_seq, m->d_tok_pos, m->d_page_table, m->pages_per_seq,
-                                    m->cfg.max_seq_len, m->d_attn_scratch, m->d_attn_counters, nullptr, m->stream));
+            for (int t0 = 0; t0 < T; t0 += kAttnSlice) {
+                LC_TRY(launch_attention(q + (size_t)t0 * m->nqkv, m->nqkv, m->d_attn + (size_t)t0 * m->nh * m->hd, std::min(kAttnSlice, T - t0), m->nh, kv,
+                                        m->d_tok_seq + t0, m->d_tok_pos + t0, m->d_page_table, m->pages_per_seq, m->cfg.max_seq_len, m->d_attn_scratch,
+                                        m->d_attn_counters, nullptr, m->stream));
+                if (t0 > 0) m->launches_in_call += 1;
+            }
         m->launches_in_call += 2;
     }
     GemvArgs o;
@@ -265,13 +269,13 @@ int32_t attention_block(lc_model* m, int l, const float* x, const float* norm_w,
     return gemv_tiled(m, o, T, m->H, m->nh * m->hd);
 }
 
-// Mixture-of-experts FFN in place of ffn_forward (moe.cu has the definition): router, then either ONE grouped launch per
-// projection over the experts that received tokens (Q4_K experts, calls of up to 64 tokens), or every expert on every
-// token through the ordinary products (prefill chunks, other quant types), then the weighted sum of the chosen experts.
+// Mixture-of-experts FFN in place of ffn_forward (moe.cu has the definition): router, then ONE grouped launch per projection over
+// the experts that received tokens (Q4_K experts: matrix-vector kernels for few rows per expert, else the many-token product), or every
+// expert on every token through the ordinary products (other quant types), then the weighted sum of the chosen experts.
 int32_t moe_block(lc_model* m, int l, const float* x, const float* norm_w, int T, const float* residual, float* out) {
     LayerW& w = m->layers[l];
     const int E = m->cfg.n_experts, K = m->cfg.top_k, El = m->El, e0 = m->e0;  // this rank's experts: e0 .. e0 + El - 1
-    const bool grouped = w.grouped_ok && T <= kMoeGroupedTokens;
+    const bool product = w.grouped_ok && (T > kMoeGroupedTokens || T * K > kMoeProductRows * E), grouped = w.grouped_ok && !product;
     if (m->tp > 1 && m->rank != 0) residual = nullptr;  // the residual enters the sum over the ranks once
     out = partial_dst(m, out);
     MoeRouteArgs r;
@@ -306,7 +310,27 @@ int32_t moe_block(lc_model* m, int l, const float* x, const float* norm_w, int T
         m->launches_in_call += 5;
         return LC_OK;
     }
-    (void)E;
+    if (product) {  // the experts' rows in expert order, one many-token product per projection
+        int launches = 2;
+        LC_TRY(launch_moe_order(m->d_moe_sel, T * K, e0, El, m->d_moe_off, m->d_moe_rows, T <= kMoeGroupedTokens ? m->d_moe_touched : nullptr, m->stream));
+        const int mean = (T * K + E - 1) / E;
+        GemmGroup gg;
+        gg.maps0 = w.tm_gate; gg.maps1 = w.tm_up; gg.refs0 = w.ref_gate; gg.refs1 = w.ref_up;
+        gg.offsets = m->d_moe_off; gg.n_experts = El;
+        gg.typical = std::min(T, mean + (int)sqrtf((float)mean));  // most experts fit the tiles that this many rows take
+        GemvArgs a;
+        a.w = &w.egate[0]; a.w2 = &w.eup[0]; a.x = x; a.norm_w = norm_w; a.eps = m->cfg.rms_eps; a.out = m->d_moe_h; a.epi = EPI_SILU_MUL; a.m = T * K;
+        LC_TRY(launch_qgemm_group(a, m->gemm_ws, gg, m->d_moe_rows, K, m->stream, &launches));
+        GemmGroup gd = gg;
+        gd.maps0 = w.tm_down; gd.maps1 = nullptr; gd.refs0 = w.ref_down; gd.refs1 = nullptr;
+        gd.row_map = m->d_moe_rows;
+        GemvArgs d;
+        d.w = &w.edown[0]; d.x = m->d_moe_h; d.out = m->d_moe_y; d.m = T * K;
+        LC_TRY(launch_qgemm_group(d, m->gemm_ws, gd, nullptr, 1, m->stream, &launches));
+        LC_TRY(launch_moe_combine(m->d_moe_y, m->d_moe_sel, m->d_moe_w, K, m->H, T, 0, 0, e0, El, residual, out, m->stream));
+        m->launches_in_call += launches;
+        return LC_OK;
+    }
     for (int e = 0; e < El; e++) {
         GemvArgs g;
         g.w = &w.egate[e]; g.w2 = &w.eup[e]; g.x = x; g.norm_w = norm_w; g.eps = m->cfg.rms_eps; g.out = m->d_ffn; g.epi = EPI_SILU_MUL;
@@ -573,7 +597,9 @@ static int32_t create_handle(const lc_model_config* cfg, std::unique_ptr<LayerSt
     int64_t pool = m->cfg.kv_pool_tokens > 0 ? m->cfg.kv_pool_tokens : (int64_t)m->max_seqs * m->pages_per_seq * m->page_tokens;
     m->pages_total = (int)((pool + m->page_tokens - 1) / m->page_tokens);
     m->kv_elt = m->cfg.kv_dtype ? 4 : 2;
-    m->t_cap = std::max(m->stack ? kStackChunk : kPrefillChunk, m->max_seqs);
+    // a pass holds no more tokens than the handle's sequences can have: the step buffers, and the time to allocate them, follow
+    const long most = std::min<long>(kPrefillChunk, (long)m->max_seqs * m->cfg.max_seq_len);
+    m->t_cap = std::max({m->stack ? kStackChunk : (int)most, m->max_seqs, 16});
     m->head_rows = std::max(16, m->max_seqs);
     m->seq_open.assign(m->max_seqs, 0);
     m->stream = lc::stream();
@@ -855,7 +881,7 @@ static int32_t bind_blocks(lc_model* m) {
     return LC_OK;
 }
 
-// The rows' powers of two of every matrix that the many-token product reads, in one buffer.
+// The rows' powers of two of every matrix that the many-token product reads, in one buffer; and where it finds a mixture's experts.
 static int32_t bind_row_scales(lc_model* m) {
     std::vector<QWeight*> all = {&m->head};
     for (LayerW& w : m->layers) {
@@ -874,6 +900,21 @@ static int32_t bind_row_scales(lc_model* m) {
         LC_TRY(launch_row_scales(*q, down, m->stream));
         q->row_down = down;
         down += q->n;
+    }
+    for (LayerW& w : m->layers) {
+        if (!w.grouped_ok) continue;
+        const std::vector<QWeight>* sets[3] = {&w.egate, &w.eup, &w.edown};
+        const ExpertRef** dst[3] = {&w.ref_gate, &w.ref_up, &w.ref_down};
+        for (int i = 0; i < 3; i++) {
+            std::vector<ExpertRef> host;
+            for (const QWeight& q : *sets[i]) host.push_back(ExpertRef{(const unsigned char*)q.data, q.row_down});
+            ExpertRef* dev = nullptr;
+            LC_TRY(dalloc(&dev, host.size()));
+            m->owned.push_back(dev);
+            LC_CUDA(cudaMemcpyAsync(dev, host.data(), host.size() * sizeof(ExpertRef), cudaMemcpyHostToDevice, m->stream));
+            LC_CUDA(cudaStreamSynchronize(m->stream));
+            *dst[i] = dev;
+        }
     }
     return LC_OK;
 }
@@ -909,16 +950,22 @@ static int32_t alloc_block_buffers(lc_model* m) {
     const int T = m->t_cap, H = m->H, F = m->F, nq = m->nh * m->hd;
     LC_TRY(dalloc(&m->d_hidden2, (size_t)T * H));
     LC_TRY(dalloc(&m->d_qkv, (size_t)T * m->nqkv)); LC_TRY(dalloc(&m->d_attn, (size_t)T * nq));
-    LC_TRY(dalloc(&m->d_ffn, (size_t)T * F));
-    LC_TRY(qgemm_workspace_alloc(&m->gemm_ws, T, std::max(std::max(H, F), nq)));
+    bool dense = m->cfg.n_experts == 0;  // some layer runs a feed-forward or every expert on every token
+    for (const LayerW& w : m->layers) dense = dense || !w.grouped_ok;
+    if (dense) LC_TRY(dalloc(&m->d_ffn, (size_t)T * F));
+    LC_TRY(qgemm_workspace_alloc(&m->gemm_ws, m->cfg.n_experts > 0 ? T * m->cfg.top_k : T, std::max(std::max(H, F), nq)));  // rows: a token's, once per expert it goes to
     if (m->any_unfused_qkv) LC_TRY(dalloc(&m->d_qkv_parts, (size_t)T * m->nqkv));
     if (m->cfg.n_experts > 0) {
         const int E = m->cfg.n_experts, K = m->cfg.top_k;
         LC_TRY(dalloc(&m->d_moe_sel, (size_t)T * K)); LC_TRY(dalloc(&m->d_moe_w, (size_t)T * K));
         LC_TRY(dalloc(&m->d_moe_cnt, (size_t)E + 1)); LC_TRY(dalloc(&m->d_moe_lists, (size_t)E * kMoeGroupedTokens));
         LC_CUDA(cudaMemsetAsync(m->d_moe_cnt, 0, ((size_t)E + 1) * sizeof(int32_t), m->stream));  // the word behind the counts is the router's ticket
-        LC_TRY(dalloc(&m->d_moe_h, (size_t)kMoeGroupedTokens * K * F)); LC_TRY(dalloc(&m->d_moe_y, (size_t)kMoeGroupedTokens * K * H));
-        LC_TRY(dalloc(&m->d_moe_yall, (size_t)E * T * H));
+        bool any = false, all = true;  // layers whose experts have the grouped forms
+        for (const LayerW& w : m->layers) { any = any || w.grouped_ok; all = all && w.grouped_ok; }
+        const size_t slots = (size_t)(any ? std::max(T, kMoeGroupedTokens) : kMoeGroupedTokens) * K;
+        LC_TRY(dalloc(&m->d_moe_h, slots * F)); LC_TRY(dalloc(&m->d_moe_y, slots * H));
+        LC_TRY(dalloc(&m->d_moe_off, (size_t)m->El + 1)); LC_TRY(dalloc(&m->d_moe_rows, slots));
+        if (!all) LC_TRY(dalloc(&m->d_moe_yall, (size_t)E * T * H));
         auto planes_alloc = [&](GemvPlanes* pl, size_t rows, int k) -> int32_t {
             const size_t units = rows * (size_t)(k / 256);
             if (units == 0) return LC_OK;
@@ -931,7 +978,7 @@ static int32_t alloc_block_buffers(lc_model* m) {
         LC_CUDA(cudaMemsetAsync(m->d_moe_touched, 0, 8, m->stream));
     }
     size_t sc = 16;
-    for (int t = 1; t <= T; t++) sc = std::max(sc, attention_scratch_bytes(t, m->nh, m->hd, m->cfg.max_seq_len));
+    for (int t = 1; t <= std::max(kAttnSlice, m->max_seqs); t++) sc = std::max(sc, attention_scratch_bytes(t, m->nh, m->hd, m->cfg.max_seq_len));
     m->attn_scratch_bytes = sc;
     LC_TRY(dalloc((uint8_t**)&m->d_attn_scratch, sc));
     LC_TRY(dalloc(&m->d_attn_counters, (size_t)T * m->nh));
@@ -1020,7 +1067,7 @@ int32_t lc_model_destroy(lc_model* m) {
         mem.clear();
     }
     for (lc_model* x : m->members) if (x != m) x->leader = nullptr;
-    void* bufs[] = {m->d_tiles, m->d_part, m->d_key, m->d_key_max, m->d_logits_all, m->d_moe_sel, m->d_moe_w, m->d_moe_cnt, m->d_moe_lists, m->d_moe_h, m->d_moe_y, m->d_moe_yall, m->d_moe_touched,
+    void* bufs[] = {m->d_tiles, m->d_part, m->d_key, m->d_key_max, m->d_logits_all, m->d_moe_sel, m->d_moe_off, m->d_moe_rows, m->d_moe_w, m->d_moe_cnt, m->d_moe_lists, m->d_moe_h, m->d_moe_y, m->d_moe_yall, m->d_moe_touched,
                     m->moe_planes_x.planes, m->moe_planes_x.sxf, m->moe_planes_x.inv2s, m->moe_planes_h.planes, m->moe_planes_h.sxf, m->moe_planes_h.inv2s,
                     m->d_stream_slots, m->d_page_table, m->d_tokens, m->d_tok_seq, m->d_tok_pos, m->d_tok_rope, m->d_last_idx, m->d_hidden, m->d_hidden2,
                     m->d_qkv, m->d_attn, m->d_ffn, m->d_last, m->d_logits, m->d_next, m->d_out_tokens, m->d_step_ctr,

@@ -148,8 +148,20 @@ int32_t launch_qgemm(const GemvArgs& a, GemmWorkspace& ws, cudaStream_t s, int* 
 bool make_act_tmap(void* out128, const void* base, uint64_t k, uint64_t rows, uint32_t box_rows);
 bool make_act_tmap_chunks(void* out128, const void* base, uint64_t k, uint64_t rows, uint32_t box_rows, uint32_t box_chunks);
 // ---- qgemm_split.cu ----
+// The experts of one mixture layer as one many-token product: GemvArgs.w / w2 give the experts' common shape and type, GemvArgs.m the
+// number of activation rows, which lie in expert order.  All pointers are device memory.
+struct ExpertRef { const unsigned char* w; const float* down; };  // an expert's raw blocks and its rows' powers of two
+struct GemmGroup {
+    const void *maps0 = nullptr, *maps1 = nullptr;     // [n_experts] tensor maps of the first matrix, of `up`
+    const ExpertRef *refs0 = nullptr, *refs1 = nullptr;  // [n_experts]
+    const int32_t* offsets = nullptr;  // [n_experts + 1] expert e has activation rows offsets[e] .. offsets[e + 1] - 1
+    const int32_t* row_map = nullptr;  // row of `out` for each activation row (null: the same)
+    int n_experts = 0, typical = 0;    // typical: rows that an expert receives on average, rounded up
+};
 // the product alone, for launch_qgemm: *slices > 0 says that shares of k are left in ws.partial; *launches counts on
-int32_t launch_qgemm_split(const GemvArgs& a, GemmWorkspace& ws, int* slices, int* launches, cudaStream_t s);
+int32_t launch_qgemm_split(const GemvArgs& a, GemmWorkspace& ws, const GemmGroup* group, int* slices, int* launches, cudaStream_t s);
+// Preparation and product of the experts (a.m activation rows).  rows: activation row r is row rows[r] / div of a.x (null: r).
+int32_t launch_qgemm_group(const GemvArgs& a, GemmWorkspace& ws, const GemmGroup& group, const int32_t* rows, int div, cudaStream_t s, int* launches);
 
 // ---- attention.cu ----
 struct KvLayout {
@@ -222,6 +234,9 @@ struct MoeRouteArgs {
     unsigned* ticket = nullptr;            // with `lists`: a device word, zero between launches (the CTA that finishes last builds the lists)
 };
 int32_t launch_moe_route(const MoeRouteArgs& a, cudaStream_t s);
+// The slots (token * top_k + choice) of experts first .. first + count - 1 in expert order, and where each expert's begin: offsets[count + 1],
+// rows[offsets[count]].  touched (optional) is increased by the number of those experts that have a slot.
+int32_t launch_moe_order(const int32_t* sel, int slots, int first, int count, int32_t* offsets, int32_t* rows, unsigned long long* touched, cudaStream_t s);
 // out[t] = residual[t] + sum_j wsel[t][j] * y[row(t, j)] in ascending expert order; mode 0: row = t * top_k + j,
 // mode 1: row = (sel[t][j] - local_first) * t_stride + t (every local expert's outputs for every token, a plane of t_stride
 // rows per expert); only the experts local_first .. local_first + local_count - 1 are added

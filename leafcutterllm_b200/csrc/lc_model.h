@@ -34,14 +34,21 @@ struct LayerW {
     std::vector<QWeight> egate, eup, edown;
     void *tm_gate = nullptr, *tm_up = nullptr, *tm_down = nullptr;
     bool grouped_ok = false;
+    const ExpertRef *ref_gate = nullptr, *ref_up = nullptr, *ref_down = nullptr;  // with grouped_ok: the same experts for the many-token product
 };
 
-constexpr int kPrefillChunk = 512;
+// Tokens per pass.  The experts of a mixture receive a share of them each, and the fuller their tiles the better (Mixtral shape, 4 layers,
+// 1,600 tokens: 36.9 ms in passes of 1,024, 33.1 in one); the step buffers grow with it.
+constexpr int kPrefillChunk = 2048;
+constexpr int kAttnSlice = 512;          // tokens per launch of the attention kernels that split a context (their scratch grows with both)
 constexpr int kTileRun = 16;             // runs of fewer tokens attend token by token
 constexpr int kChunkRun = 32;            // runs of fewer tokens walk the gated delta rule token by token
 constexpr int kStackChunk = 2048;      // tokens per pass of a checkpoint-directory design
 constexpr int kTokTile = 8;
-constexpr int kMoeGroupedTokens = 64;  // calls of at most this many tokens run the experts as one grouped launch
+constexpr int kMoeGroupedTokens = 64;  // most tokens of a call whose experts run as one grouped matrix-vector launch
+// Rows per expert from which the experts run as a grouped many-token product instead: the matrix-vector kernel reads the experts again for
+// every four rows.  Mixtral shape, gate/up + down of a layer: 4 rows 420 us (matrix-vector), a hundred rows 2.4 ms (product).
+constexpr int kMoeProductRows = 5;
 
 }  // namespace lc
 
@@ -106,8 +113,9 @@ struct lc_model {
     int32_t* d_step_ctr = nullptr;
     unsigned long long* d_stream_slots = nullptr;  // cross-CTA merge slots of the single-token attention kernel (zero between launches)
     // mixture-of-experts scratch: the router's picks and weights per token, per-expert slot counts and lists, the slots'
-    // FFN hidden rows and outputs (calls of up to kMoeGroupedTokens tokens), every expert's output plane (larger calls)
+    // FFN hidden rows and outputs, every expert's output plane (experts that have no grouped form)
     int32_t *d_moe_sel = nullptr, *d_moe_cnt = nullptr, *d_moe_lists = nullptr;
+    int32_t *d_moe_off = nullptr, *d_moe_rows = nullptr;  // of the grouped product: where each expert's slots begin; the slots in expert order
     float *d_moe_w = nullptr, *d_moe_h = nullptr, *d_moe_y = nullptr, *d_moe_yall = nullptr;
     GemvPlanes moe_planes_x, moe_planes_h;  // fixed-point activations of the grouped launches: the layer's input per token, the experts' hidden rows per slot
     unsigned long long* d_moe_touched = nullptr;  // experts that received a token, summed over layers and steps since the last read

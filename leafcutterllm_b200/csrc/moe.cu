@@ -11,6 +11,7 @@
 //                    -- for calls of up to 64 tokens -- the CTA that finishes last lists, per expert and in token order, the
 //                    (token, choice) slots it received, for the grouped expert product.
 // moe_combine_kernel out[t] = residual[t] + sum_j w[t][j] * y[row(t, j)], j in ascending expert order.
+#include <algorithm>
 #include "lc_kernels.h"
 
 namespace lc {
@@ -120,6 +121,41 @@ moe_route_kernel(const float* __restrict__ x, const float* __restrict__ norm_w, 
     if (threadIdx.x == 0) *ticket = 0;  // every CTA has taken its ticket: ready for the next launch
 }
 
+// The slots of this rank's experts in expert order, each expert's ascending: one CTA, a warp per expert (in turn) counts its slots, then
+// writes them behind those of the experts before.  `sel` has 4,096 words for a prompt chunk of 2,048 tokens and two experts each: 128 steps of a warp.
+__global__ void __launch_bounds__(1024)
+moe_order_kernel(const int32_t* __restrict__ sel, int slots, int first, int count, int32_t* __restrict__ offsets, int32_t* __restrict__ rows,
+                 unsigned long long* __restrict__ touched) {
+    __shared__ int n_s[kMaxExperts];
+    pdl_wait();
+    pdl_launch_dependents();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    for (int e = warp; e < count; e += warps) {
+        int n = 0;
+#pragma unroll 4
+        for (int i = lane; i < slots; i += 32) n += sel[i] == first + e;
+        for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+        if (lane == 0) n_s[e] = n;
+    }
+    __syncthreads();
+    for (int e = warp; e < count; e += warps) {
+        int at = 0;
+        for (int i = 0; i < e; i++) at += n_s[i];
+        if (lane == 0) {
+            offsets[e] = at;
+            if (e == count - 1) offsets[count] = at + n_s[e];
+            if (touched && n_s[e] > 0) atomicAdd(touched, 1ull);
+        }
+#pragma unroll 4
+        for (int i0 = 0; i0 < slots; i0 += 32) {
+            const bool hit = i0 + lane < slots && sel[i0 + lane] == first + e;
+            const unsigned m = __ballot_sync(0xffffffffu, hit);
+            if (hit) rows[at + __popc(m & ((1u << lane) - 1u))] = i0 + lane;
+            at += __popc(m);
+        }
+    }
+}
+
 // mode 0: row(t, j) = t * K + j (one row per slot); mode 1: row(t, j) = (sel[t][j] - local_first) * T_stride + t (a plane per
 // local expert).  Only experts local_first .. local_first + local_count - 1 are added (a rank of a cut model adds its own).
 __global__ void moe_combine_kernel(const float* __restrict__ y, const int32_t* __restrict__ sel, const float* __restrict__ wsel, int K, int H, int T,
@@ -192,6 +228,12 @@ int32_t launch_moe_route(const MoeRouteArgs& a, cudaStream_t s) {
              LC_ERR_INVALID, "moe route: rows must be 16-byte aligned multiples of four elements");
     LC_CUDA(launch_dep_smem(moe_route_kernel, dim3((unsigned)a.T), dim3(kRouteThreads), (size_t)a.H * sizeof(float), s, a.x, a.norm_w, a.eps, a.H, a.T, a.w_router, a.n_experts, a.top_k, a.sel,
                        a.wsel, a.counts, a.lists, a.list_stride, a.touched, a.local_first, a.local_count > 0 ? a.local_count : a.n_experts, a.ticket));
+    return LC_OK;
+}
+
+int32_t launch_moe_order(const int32_t* sel, int slots, int first, int count, int32_t* offsets, int32_t* rows, unsigned long long* touched, cudaStream_t s) {
+    LC_CHECK(sel && offsets && rows && slots >= 1 && count >= 1 && count <= kMaxExperts, LC_ERR_INVALID, "moe order: bad argument");
+    LC_CUDA(launch_dep(moe_order_kernel, dim3(1), dim3(std::min(1024, 32 * count)), s, sel, slots, first, count, offsets, rows, touched));
     return LC_OK;
 }
 

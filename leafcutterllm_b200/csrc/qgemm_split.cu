@@ -84,6 +84,12 @@ struct GemmParams {
     int ksplit;             // CTAs along k per tile (gridDim.z)
     int row_dynamic;        // row_down comes from a kernel ahead of this one in the stream
     float* partial;         // [ksplit][matrices][T][n] f32 for the summing kernel, or null: the CTA holds the whole sum and writes `out`
+    // the experts of a mixture layer (see GemmGroup): activation rows in expert order, expert e's from offsets[e] on; null for a plain product
+    const CUtensorMap *maps0, *maps1;
+    const ExpertRef *refs0, *refs1;
+    const int32_t* offsets;
+    const int32_t* row_map; // row of `out` that activation row r's result goes to (null: r)
+    int n_experts;
     int* error_flag;
 };
 
@@ -350,6 +356,23 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
     const int N = p.N;
     const int RS = p.raw_stages, BS = p.b_stages;
     const uint32_t b_half = (uint32_t)N * 128u;
+    const int row0 = blockIdx.x * (pair ? kRows / 2 : kRows), nquads = (p.k / kUnitElems + 3) / 4;
+    int tok0 = blockIdx.y * N, tok_end = p.T;
+    const CUtensorMap *map0 = &tm0, *map1 = &tm1;
+    ExpertRef ref0{p.w0, p.row_down0}, ref1{p.w1, p.row_down1};
+    if (p.offsets) {  // this CTA's expert and its tile of that expert's rows; the grid has room for the last, short tile of each
+        pdl_wait();
+        int left = blockIdx.y, e = 0, first = __ldg(p.offsets);
+        for (; e < p.n_experts; e++) {
+            const int end = __ldg(p.offsets + e + 1), tiles = (end - first + N - 1) / N;
+            if (left < tiles) { tok0 = first + left * N; tok_end = end; break; }
+            left -= tiles;
+            first = end;
+        }
+        if (e == p.n_experts) return;
+        map0 = p.maps0 + e; ref0 = p.refs0[e];
+        if (pair) { map1 = p.maps1 + e; ref1 = p.refs1[e]; }
+    }
 
     unsigned char* bt = smem;                          // [BS][two tiles of N x 128 B]
     unsigned char* raw = bt + (size_t)BS * 2 * b_half;  // [RS][raw_bytes]
@@ -383,7 +406,6 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
     bool ok = true;
 
     // this CTA's share of k: whole groups of four units (one chunk of sub-block sums); unit v below is u_begin + v
-    const int row0 = blockIdx.x * (pair ? kRows / 2 : kRows), tok0 = blockIdx.y * N, nquads = (p.k / kUnitElems + 3) / 4;
     const int u_begin = (int)((long long)blockIdx.z * nquads / p.ksplit) * 4;
     const int nu = min((int)((long long)(blockIdx.z + 1) * nquads / p.ksplit) * 4, p.k / kUnitElems) - u_begin;
     const int sum_chunks = kHasMin<TYPE> ? (nu + 3) / 4 : 0;  // chunks of sub-block sums behind the units, four units each,
@@ -432,7 +454,7 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
                     mbar_expect_tx(&raw_full[sr], raw_bytes);
 #pragma unroll
                     for (int b = 0; b < 4; b++)
-                        tma_load_2d(raw + (size_t)sr * raw_bytes + b * 32 * kPitch, pair && b >= 2 ? &tm1 : &tm0, (u_begin + v) * (kPitch / 4),
+                        tma_load_2d(raw + (size_t)sr * raw_bytes + b * 32 * kPitch, pair && b >= 2 ? map1 : map0, (u_begin + v) * (kPitch / 4),
                                     row0 + (pair ? b & 1 : b) * 32, &raw_full[sr]);
                     in_flight = min(in_flight + 1, RS);
                     if (++sr == RS) { sr = 0; phase ^= 1; }
@@ -456,7 +478,7 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
 #pragma unroll 1
                 for (int half = 0; half < 2; half++) {  // rows 0 .. 63, 64 .. 127 (pair: of the second matrix)
                     const int first = row0 + (pair ? 0 : half * 64) + warp - 2;
-                    const unsigned char* src = (pair && half ? p.w1 : p.w0) + (size_t)(u_begin + v) * 210;
+                    const unsigned char* src = (pair && half ? ref1.w : ref0.w) + (size_t)(u_begin + v) * 210;
                     const size_t step = 2 * p.row_bytes;
                     const int live = min(32, (p.n - first + 1) / 2);  // rows past the end: any data, dropped at the end
                     const unsigned char* row = src + (size_t)first * p.row_bytes;
@@ -561,7 +583,7 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
         const int row = quarter * 32 + lane;  // of the tile; also the tensor-memory lane
         const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16), a_stage = lane_base + col_a(N) + (uint32_t)g * (WIDE ? 32 : 64);
         const int mat = pair ? quarter >> 1 : 0;
-        const unsigned char* const weights = mat ? p.w1 : p.w0;
+        const unsigned char* const weights = mat ? ref1.w : ref0.w;
         const int own = WIDE ? max(0, min(32, N - 32 * g)) : N / 4, tbase = g * (WIDE ? 32 : N / 4);  // this thread's tokens of the tile
         auto wait_all = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); };
         float y[kOwn];
@@ -608,7 +630,7 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
             const int grow = row0 + (pair ? row & 63 : row);
             const bool live = grow < p.n;
             const unsigned char* const wrow = weights + (size_t)min(grow, p.n - 1) * p.row_bytes;
-            const float down = live ? (mat ? p.row_down1 : p.row_down0)[grow] : 1.0f, up = live ? 1.0f / down : 0.0f;
+            const float down = live ? (mat ? ref1.down : ref0.down)[grow] : 1.0f, up = live ? 1.0f / down : 0.0f;
 #pragma unroll
             for (int t = 0; t < kOwn; t++) y[t] = 0.f;
             for (int v = 0; v < nu && ok; v++) {
@@ -683,7 +705,7 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
             if (ok) drain(nv - 1);
             if (ok && own > 0) add_columns(kColSmall);  // complete: the last unit's d_full followed every product
             pdl_wait();
-            const int t_first = tok0 + tbase, mine = ok ? min(own, p.T - t_first) : 0;
+            const int t_first = tok0 + tbase, mine = ok ? min(own, tok_end - t_first) : 0;
             // a lane has one token's scale: a load beside each result's store would wait for it
             const float scale = lane < mine ? __ldg(p.tok_scale + t_first + lane) : 0.f;
 #pragma unroll
@@ -707,6 +729,13 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
 #pragma unroll
                     for (int t = 0; t < kOwn; t++)
                         if (live && t < mine) dst[(size_t)t * p.n] = __fmul_rn(ex[t * 64], y[t]);
+                }
+            } else if (p.row_map) {
+                const int to = lane < mine ? __ldg(p.row_map + t_first + lane) : 0;
+#pragma unroll
+                for (int t = 0; t < kOwn; t++) {
+                    const int r = __shfl_sync(0xffffffffu, to, t);
+                    if (live && t < mine) p.out[(size_t)r * p.n + grow] = y[t];
                 }
             } else {
                 const size_t o = (size_t)t_first * p.n + grow;
@@ -767,8 +796,8 @@ long unit_cycles(int N) {
 }
 
 template <uint32_t TYPE>
-int32_t launch_type(const GemvArgs& a, const GemmWorkspace& ws, GemmParams& p, int* summed_slices, cudaStream_t s) {
-    const GemmShape g = shape_for<TYPE>(p.T);
+int32_t launch_type(const GemvArgs& a, const GemmWorkspace& ws, GemmParams& p, const GemmGroup* group, int* summed_slices, cudaStream_t s) {
+    const GemmShape g = shape_for<TYPE>(group ? group->typical : p.T);
     p.N = g.N; p.raw_stages = g.raw_stages; p.b_stages = g.b_stages;
     auto kern = g.N <= 64 ? qgemm_split_kernel<TYPE, false> : qgemm_split_kernel<TYPE, true>;
     LC_CUDA(ensure_smem_limit((const void*)kern, g.smem));
@@ -778,13 +807,13 @@ int32_t launch_type(const GemvArgs& a, const GemmWorkspace& ws, GemmParams& p, i
                  make_bf16_tmap_3d(&tms, ws.sx, (uint64_t)p.k / 16, rows, 2, (uint64_t)p.k / 16, rows * (p.k / 16), 64, (uint32_t)g.N, 1),
              LC_ERR_CUDA, "qgemm: activation tensor maps");
     const int nmat = a.epi == EPI_SILU_MUL ? 2 : 1;
-    const int tiles = (p.n * nmat + kRows - 1) / kRows, ttiles = (p.T + g.N - 1) / g.N, nquads = (p.k / kUnitElems + 3) / 4;
+    const int tiles = (p.n * nmat + kRows - 1) / kRows, ttiles = group ? p.T / g.N + group->n_experts : (p.T + g.N - 1) / g.N, nquads = (p.k / kUnitElems + 3) / 4;
     // Few tiles (a batched decode step, a short prompt): k is cut over several CTAs so that all SMs work, and a second kernel adds
     // the shares in a fixed order.  Cost in cycles: waves of units plus a fixed part (launch, first unit, drain) per wave, and the
     // shares' trip through L2 at 3000 bytes per cycle.
     int ks = 1;
     double best = 0;
-    for (int c = 1; c <= std::min(8, nquads); c++) {
+    for (int c = 1; c <= (group ? 1 : std::min(8, nquads)); c++) {
         const size_t bytes = (size_t)c * nmat * p.T * p.n * sizeof(float);
         if (c > 1 && (bytes > ws.partial_bytes || p.n % 4 != 0)) break;
         const long waves = ((long)tiles * ttiles * c + sm_count() - 1) / sm_count();
@@ -802,13 +831,17 @@ int32_t launch_type(const GemvArgs& a, const GemmWorkspace& ws, GemmParams& p, i
 }  // namespace
 
 // The product of prepared activations (ws.xh, ws.sx, ws.tok_scale).  *slices > 0: the shares are in ws.partial, still to be summed.
-int32_t launch_qgemm_split(const GemvArgs& a, GemmWorkspace& ws, int* slices, int* launches, cudaStream_t s) {
+int32_t launch_qgemm_split(const GemvArgs& a, GemmWorkspace& ws, const GemmGroup* group, int* slices, int* launches, cudaStream_t s) {
     const int n = a.w->n;
     const bool pair = a.epi == EPI_SILU_MUL;
     GemmParams p{};
     p.row_down0 = a.w->row_down;
     p.row_down1 = pair ? a.w2->row_down : p.row_down0;
-    if (!p.row_down0 || !p.row_down1) {  // a matrix that was not laid out for this product when it was bound
+    if (group) {
+        p.maps0 = (const CUtensorMap*)group->maps0; p.maps1 = (const CUtensorMap*)group->maps1;
+        p.refs0 = group->refs0; p.refs1 = group->refs1;
+        p.offsets = group->offsets; p.row_map = group->row_map; p.n_experts = group->n_experts;
+    } else if (!p.row_down0 || !p.row_down1) {  // a matrix that was not laid out for this product when it was bound
         const size_t need = (size_t)n * 2;
         if (ws.row_cap < need) {
             if (ws.row_tmp) cudaFree(ws.row_tmp);
@@ -829,11 +862,11 @@ int32_t launch_qgemm_split(const GemvArgs& a, GemmWorkspace& ws, int* slices, in
     p.error_flag = gemv_error_flag_dev();
     *launches += 1;
     switch (a.w->typ) {
-        case LC_TYPE_Q4_K: return launch_type<LC_TYPE_Q4_K>(a, ws, p, slices, s);
-        case LC_TYPE_Q5_K: return launch_type<LC_TYPE_Q5_K>(a, ws, p, slices, s);
-        case LC_TYPE_Q4_0: return launch_type<LC_TYPE_Q4_0>(a, ws, p, slices, s);
-        case LC_TYPE_Q8_0: return launch_type<LC_TYPE_Q8_0>(a, ws, p, slices, s);
-        default: return launch_type<LC_TYPE_Q6_K>(a, ws, p, slices, s);
+        case LC_TYPE_Q4_K: return launch_type<LC_TYPE_Q4_K>(a, ws, p, group, slices, s);
+        case LC_TYPE_Q5_K: return launch_type<LC_TYPE_Q5_K>(a, ws, p, group, slices, s);
+        case LC_TYPE_Q4_0: return launch_type<LC_TYPE_Q4_0>(a, ws, p, group, slices, s);
+        case LC_TYPE_Q8_0: return launch_type<LC_TYPE_Q8_0>(a, ws, p, group, slices, s);
+        default: return launch_type<LC_TYPE_Q6_K>(a, ws, p, group, slices, s);
     }
 }
 

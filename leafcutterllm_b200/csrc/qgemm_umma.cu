@@ -257,14 +257,15 @@ __device__ __forceinline__ void xprep_row(float* row, float acc, float amax, con
 }
 
 __global__ void __launch_bounds__(1024)
-xprep_kernel(const float* __restrict__ x, const float* __restrict__ norm_w, float eps, int K, __half* __restrict__ xh,
-             size_t lo_offset, __half* __restrict__ sx, size_t sx_lo_offset, float* __restrict__ tok_scale) {
+xprep_kernel(const float* __restrict__ x, const int32_t* __restrict__ rows, int div, const int32_t* __restrict__ live, const float* __restrict__ norm_w, float eps, int K,
+             __half* __restrict__ xh, size_t lo_offset, __half* __restrict__ sx, size_t sx_lo_offset, float* __restrict__ tok_scale) {
     extern __shared__ float row[];
     __shared__ float sh[64];
     pdl_wait();
     pdl_launch_dependents();
     const int t = blockIdx.x;
-    const float* xr = x + (size_t)t * K;
+    if (live && t >= __ldg(live)) return;  // slots of experts that other ranks hold
+    const float* xr = x + (size_t)(rows ? __ldg(rows + t) / div : t) * K;  // rows: those of a mixture's experts, in expert order
     float acc = 0.f, amax = 0.f;
     for (int i = threadIdx.x * 4; i < K; i += blockDim.x * 4) {
         const float4 v = *reinterpret_cast<const float4*>(xr + i);
@@ -859,8 +860,8 @@ int32_t qgemm_workspace_alloc(GemmWorkspace* ws, int t_cap, int k_max) {
     LC_CUDA(cudaMalloc(&ws->sx, bytes / 16));
     LC_CUDA(cudaMemset(ws->sx, 0, bytes / 16));
     LC_CUDA(cudaMalloc((void**)&ws->tok_scale, (size_t)ws->t_cap * sizeof(float)));
-    // shares of k of the batched decode step, and the two matrices of gate/up at any number of tokens
-    ws->partial_bytes = std::max((size_t)64 << 20, (size_t)2 * ws->t_cap * k_max * sizeof(float));
+    // shares of k of the batched decode step, and the two matrices of gate/up of one token tile
+    ws->partial_bytes = std::max((size_t)64 << 20, (size_t)2 * kMaxTok * k_max * sizeof(float));
     LC_CUDA(cudaMalloc((void**)&ws->partial, ws->partial_bytes));
     return LC_OK;
 }
@@ -995,12 +996,12 @@ int32_t launch_qgemm(const GemvArgs& a, GemmWorkspace& ws, cudaStream_t s, int* 
         if (smem > 48 * 1024) LC_CUDA(ensure_smem_limit((const void*)xprep_kernel, smem));
         // a token's row is short (16 - 44 KB) and its three passes are latency: many threads, one or a few float4 each
         // (64 sequences, 4 layers: 2.43 / 2.40 / 2.40 ms per step with 256 / 512 / 1024 threads)
-        LC_CUDA(launch_pdl(xprep_kernel, dim3(T), dim3(K >= 4096 ? 1024 : 256), smem, s, a.x, a.norm_w, a.eps, K, (__half*)ws.xh, lo_offset, (__half*)ws.sx,
+        LC_CUDA(launch_pdl(xprep_kernel, dim3(T), dim3(K >= 4096 ? 1024 : 256), smem, s, a.x, (const int32_t*)nullptr, 1, (const int32_t*)nullptr, a.norm_w, a.eps, K, (__half*)ws.xh, lo_offset, (__half*)ws.sx,
                            sx_lo_offset, ws.tok_scale));
     }
     int slices = 0, count = prepared ? 0 : 1;
     if (use_split(a.w->typ, T)) {
-        LC_TRY(launch_qgemm_split(a, ws, &slices, &count, s));
+        LC_TRY(launch_qgemm_split(a, ws, nullptr, &slices, &count, s));
     } else {
         LC_TRY(launch_qgemm_tile(a, ws, &slices, s));
         count += 1;
@@ -1023,6 +1024,20 @@ int32_t launch_qgemm(const GemvArgs& a, GemmWorkspace& ws, cudaStream_t s, int* 
     }
     if (launches) *launches = count;
     return LC_OK;
+}
+
+int32_t launch_qgemm_group(const GemvArgs& a, GemmWorkspace& ws, const GemmGroup& group, const int32_t* rows, int div, cudaStream_t s, int* launches) {
+    const int K = a.w->k;
+    LC_CHECK(a.m >= 1 && a.m <= ws.t_cap && K <= ws.k_max && qgemm_split_weight_ok(*a.w) && group.offsets && group.n_experts >= 1 && group.typical >= 1,
+             LC_ERR_INVALID, "grouped qgemm: %d rows of %d elements do not fit", a.m, K);
+    ws.prep_x = nullptr;
+    const size_t smem = (size_t)K * sizeof(float);
+    if (smem > 48 * 1024) LC_CUDA(ensure_smem_limit((const void*)xprep_kernel, smem));
+    LC_CUDA(launch_pdl(xprep_kernel, dim3(a.m), dim3(K >= 4096 ? 1024 : 256), smem, s, a.x, rows, div, group.offsets + group.n_experts, a.norm_w, a.eps, K, (__half*)ws.xh, (size_t)ws.t_cap * K,
+                       (__half*)ws.sx, (size_t)ws.t_cap * (K / 16), ws.tok_scale));
+    int slices = 0;
+    *launches += 1;
+    return launch_qgemm_split(a, ws, &group, &slices, launches, s);
 }
 
 }  // namespace lc

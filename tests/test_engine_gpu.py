@@ -90,6 +90,17 @@ def test_chunked_prefill_matches(gpu, oracle):
     eng.close()
 
 
+@pytest.mark.parametrize("types,heads", [((12, 12, 12), 2), ((2, 8, 8), 8)])
+def test_prompt_longer_than_a_pass(gpu, oracle, types, heads):
+    """2,100 tokens: a full pass of 2,048 and a short one behind it; heads of 128 (tiled prefill attention) and of 32 (in slices of 512 tokens)."""
+    from leafcutterllm_b200 import synth
+    spec = small_spec(*types, layers=1, hidden=256, heads=heads, kv=heads, ffn=256, vocab=300)
+    eng, om = make_pair(gpu, oracle, spec, max_seq_len=2112)
+    prompt = synth.prompt_tokens(2100, spec.vocab_size, 1)
+    assert_close(eng.forward(prompt), om.forward(prompt), LOGIT_ABS, LOGIT_REL, "2100-token prefill")
+    eng.close()
+
+
 def test_batched_sequences_match_single(gpu, oracle):
     from leafcutterllm_b200 import synth
     spec = small_spec(12, 12, 12)
