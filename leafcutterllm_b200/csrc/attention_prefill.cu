@@ -210,7 +210,151 @@ attention_prefill_kernel(const float* __restrict__ q, int q_stride, float* __res
     }
 }
 
+// The same for every other head size, cache type and page size, in f32: the tile's queries lie in shared memory, each of eight warps takes
+// eight of them; keys and values come 32 at a time.  Scores with a lane per key (four dims a step: one 16-byte read of the
+// key, one broadcast read per query), values with HD / 32 dims a lane.  Scores, softmax and sums are f32 FMAs in a fixed order.
+// Why: the kernel it takes prompts from has one CTA per (token, head) and reads the whole context for each.  Bound by the issue of shared-memory
+// reads (12 wavefronts beside 32 FMAs of a warp).
+constexpr int kRowsQ = 64, kRowsK = 32, kRowsWarps = 8, kRowsPer = kRowsQ / kRowsWarps;
+template <int HD> constexpr size_t rows_smem() { return sizeof(float) * ((size_t)kRowsQ * HD + kRowsK * (HD + 4) + kRowsK * HD + kRowsQ * kRowsK); }
+template <int HD, bool F32>
+__global__ void __launch_bounds__(32 * kRowsWarps)
+attention_rows_kernel(const float* __restrict__ q, int q_stride, float* __restrict__ out, int out_stride, KvLayout kv,
+                      const PrefillTile* __restrict__ tiles, const int32_t* __restrict__ page_table, int pages_per_seq, int n_heads) {
+    extern __shared__ __align__(16) float rows_sm[];
+    float* const sq = rows_sm;                     // [kRowsQ][HD]
+    float* const sk = sq + kRowsQ * HD;            // [kRowsK][HD + 4]: 16-byte reads a row apart meet every bank once
+    float* const sv = sk + kRowsK * (HD + 4);      // [kRowsK][HD]
+    constexpr int DPL = HD / 32;
+    pdl_launch_dependents();
+    pdl_wait();
+    const PrefillTile tl = tiles[blockIdx.x];
+    const int head = blockIdx.y, kvh = head / (n_heads / kv.n_kv);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r0 = warp * kRowsPer;
+    float* const sp = sv + kRowsK * HD + r0 * kRowsK;  // this warp's weights [kRowsPer][kRowsK]
+    const int32_t* pt = page_table + (size_t)tl.seq * pages_per_seq;
+    const int ctx_end = tl.pos0 + tl.n, mine = min(kRowsPer, tl.n - r0);  // rows of this warp (may be none)
+    const int last = tl.pos0 + r0 + mine - 1;                            // the newest position that they see
+    for (int i = tid; i < kRowsQ * (HD / 4); i += blockDim.x) {
+        const int r = i / (HD / 4), c = i % (HD / 4) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < tl.n) v = *reinterpret_cast<const float4*>(q + (size_t)(tl.tok0 + r) * q_stride + (size_t)head * HD + c);
+        *reinterpret_cast<float4*>(sq + r * HD + c) = v;
+    }
+    float m[kRowsPer], l[kRowsPer], acc[kRowsPer][DPL];  // l: this lane's keys only, until the end
+#pragma unroll
+    for (int r = 0; r < kRowsPer; r++) {
+        m[r] = -INFINITY; l[r] = 0.f;
+#pragma unroll
+        for (int d = 0; d < DPL; d++) acc[r][d] = 0.f;
+    }
+    const float root = sqrtf((float)HD);  // attention.rs:93: dot / sqrt(head_dim)
+    for (int t0 = 0; t0 < ctx_end; t0 += kRowsK) {
+        __syncthreads();  // the tile before has been read
+        for (int i = tid; i < kRowsK * (HD / 4); i += blockDim.x) {
+            const int t = i / (HD / 4), c = i % (HD / 4) * 4, pos = t0 + t;
+            float4 k4 = make_float4(0.f, 0.f, 0.f, 0.f), v4 = k4;  // past the end: weight zero, and zero times what lies there would not be
+            if (pos < ctx_end) {
+                const size_t at = (((size_t)pt[pos / kv.page_tokens] * kv.n_kv + kvh) * kv.page_tokens + pos % kv.page_tokens) * HD + c;
+                if constexpr (F32) {
+                    k4 = *reinterpret_cast<const float4*>((const float*)kv.k_pool + at);
+                    v4 = *reinterpret_cast<const float4*>((const float*)kv.v_pool + at);
+                } else {
+                    const uint2 kh = *reinterpret_cast<const uint2*>((const __half*)kv.k_pool + at), vh = *reinterpret_cast<const uint2*>((const __half*)kv.v_pool + at);
+                    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&kh.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&kh.y));
+                    const float2 e = __half22float2(*reinterpret_cast<const __half2*>(&vh.x)), f = __half22float2(*reinterpret_cast<const __half2*>(&vh.y));
+                    k4 = make_float4(a.x, a.y, b.x, b.y);
+                    v4 = make_float4(e.x, e.y, f.x, f.y);
+                }
+            }
+            *reinterpret_cast<float4*>(sk + t * (HD + 4) + c) = k4;
+            *reinterpret_cast<float4*>(sv + t * HD + c) = v4;
+        }
+        __syncthreads();
+        if (mine <= 0 || t0 > last) continue;
+        float s[kRowsPer];
+#pragma unroll
+        for (int r = 0; r < kRowsPer; r++) s[r] = 0.f;
+#pragma unroll 4
+        for (int c = 0; c < HD; c += 4) {
+            const float4 k4 = *reinterpret_cast<const float4*>(sk + lane * (HD + 4) + c);
+#pragma unroll
+            for (int r = 0; r < kRowsPer; r++) {
+                const float4 q4 = *reinterpret_cast<const float4*>(sq + (r0 + r) * HD + c);
+                s[r] = fmaf(q4.x, k4.x, s[r]); s[r] = fmaf(q4.y, k4.y, s[r]); s[r] = fmaf(q4.z, k4.z, s[r]); s[r] = fmaf(q4.w, k4.w, s[r]);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < kRowsPer; r++) {
+            const float z = t0 + lane <= tl.pos0 + r0 + r ? s[r] / root : -INFINITY;
+            const float mn = fmaxf(m[r], warp_max(z));  // finite from the first tile on: every row sees position 0
+            const float alpha = expf(m[r] - mn), w = expf(z - mn);
+            m[r] = mn;
+            l[r] = fmaf(l[r], alpha, w);
+#pragma unroll
+            for (int d = 0; d < DPL; d++) acc[r][d] *= alpha;
+            sp[r * kRowsK + lane] = w;
+        }
+        __syncwarp();
+#pragma unroll 2
+        for (int t = 0; t < kRowsK; t += 4) {
+            float v[4][DPL];
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+#pragma unroll
+                for (int d = 0; d < DPL; d++) v[k][d] = sv[(t + k) * HD + d * 32 + lane];
+#pragma unroll
+            for (int r = 0; r < kRowsPer; r++) {
+                const float4 w4 = *reinterpret_cast<const float4*>(sp + r * kRowsK + t);
+#pragma unroll
+                for (int d = 0; d < DPL; d++) {
+                    acc[r][d] = fmaf(w4.x, v[0][d], acc[r][d]); acc[r][d] = fmaf(w4.y, v[1][d], acc[r][d]);
+                    acc[r][d] = fmaf(w4.z, v[2][d], acc[r][d]); acc[r][d] = fmaf(w4.w, v[3][d], acc[r][d]);
+                }
+            }
+        }
+        __syncwarp();  // the weights have been read
+    }
+#pragma unroll
+    for (int r = 0; r < kRowsPer; r++) {
+        const float sum = warp_sum(l[r]);
+        if (r < mine) {
+            float* dst = out + (size_t)(tl.tok0 + r0 + r) * out_stride + (size_t)head * HD + lane;
+#pragma unroll
+            for (int d = 0; d < DPL; d++) dst[d * 32] = acc[r][d] / sum;
+        }
+    }
+}
+
+template <int HD, bool F32>
+int32_t launch_rows(const float* q, int q_stride, float* out, int n_heads, const KvLayout& kv, const PrefillTile* tiles_dev, int n_tiles, const int32_t* page_table,
+                    int pages_per_seq, cudaStream_t s) {
+    LC_CUDA(ensure_smem_limit((const void*)attention_rows_kernel<HD, F32>, rows_smem<HD>()));
+    LC_CUDA(launch_pdl(attention_rows_kernel<HD, F32>, dim3((unsigned)n_tiles, (unsigned)n_heads), dim3(32 * kRowsWarps), rows_smem<HD>(), s, q, q_stride, out, n_heads * HD,
+                       kv, tiles_dev, page_table, pages_per_seq, n_heads));
+    return LC_OK;
+}
+
 }  // namespace
+
+bool attention_rows_applies(const KvLayout& kv, int n_heads, const float* q, int q_stride) {
+    return (kv.hd == 32 || kv.hd == 64 || kv.hd == 128 || kv.hd == 256) && kv.n_kv > 0 && n_heads % kv.n_kv == 0 && (uintptr_t)q % 16 == 0 && q_stride % 4 == 0;
+}
+int32_t launch_attention_rows(const float* q, int q_stride, float* out, int n_heads, const KvLayout& kv, const PrefillTile* tiles_dev, int n_tiles,
+                              const int32_t* page_table, int pages_per_seq, cudaStream_t s) {
+    if (n_tiles <= 0) return LC_OK;
+    LC_CHECK(attention_rows_applies(kv, n_heads, q, q_stride), LC_ERR_INVALID, "attention rows: head_dim %d or unaligned queries", kv.hd);
+    switch (kv.hd * 2 + (kv.kv_f32 ? 1 : 0)) {
+        case 64: return launch_rows<32, false>(q, q_stride, out, n_heads, kv, tiles_dev, n_tiles, page_table, pages_per_seq, s);
+        case 65: return launch_rows<32, true>(q, q_stride, out, n_heads, kv, tiles_dev, n_tiles, page_table, pages_per_seq, s);
+        case 128: return launch_rows<64, false>(q, q_stride, out, n_heads, kv, tiles_dev, n_tiles, page_table, pages_per_seq, s);
+        case 129: return launch_rows<64, true>(q, q_stride, out, n_heads, kv, tiles_dev, n_tiles, page_table, pages_per_seq, s);
+        case 256: return launch_rows<128, false>(q, q_stride, out, n_heads, kv, tiles_dev, n_tiles, page_table, pages_per_seq, s);
+        case 257: return launch_rows<128, true>(q, q_stride, out, n_heads, kv, tiles_dev, n_tiles, page_table, pages_per_seq, s);
+        case 512: return launch_rows<256, false>(q, q_stride, out, n_heads, kv, tiles_dev, n_tiles, page_table, pages_per_seq, s);
+        default: return launch_rows<256, true>(q, q_stride, out, n_heads, kv, tiles_dev, n_tiles, page_table, pages_per_seq, s);
+    }
+}
 
 bool attention_prefill_applies(const KvLayout& kv, int n_heads) {
     return kv.hd == kHD && !kv.kv_f32 && kv.page_tokens == kPage && kv.n_kv > 0 && n_heads % kv.n_kv == 0;

@@ -247,6 +247,8 @@ int32_t attention_block(lc_model* m, int l, const float* x, const float* norm_w,
         static const bool no_tc = getenv("LC_PREFILL_FMA") != nullptr;  // diagnostics: the one-CTA-per-(token, head) kernel for every call
         if (T >= 16 && m->n_tiles > 0 && !no_tc && attention_prefill_applies(kv, m->nh))  // a prefill chunk: tiles of 64 queries on the tensor cores
             LC_TRY(launch_attention_prefill(q, m->nqkv, m->d_attn, m->nh, kv, m->d_tiles, m->n_tiles, m->d_page_table, m->pages_per_seq, m->stream));
+        else if (T >= 16 && m->n_tiles > 0 && T >= kRowsRun * m->n_tiles && !no_tc && attention_rows_applies(kv, m->nh, q, m->nqkv))
+            LC_TRY(launch_attention_rows(q, m->nqkv, m->d_attn, m->nh, kv, m->d_tiles, m->n_tiles, m->d_page_table, m->pages_per_seq, m->stream));
         else
             for (int t0 = 0; t0 < T; t0 += kAttnSlice) {
                 LC_TRY(launch_attention(q + (size_t)t0 * m->nqkv, m->nqkv, m->d_attn + (size_t)t0 * m->nh * m->hd, std::min(kAttnSlice, T - t0), m->nh, kv,

@@ -209,6 +209,10 @@ bool attention_prefill_applies(const KvLayout& kv, int n_heads);
 // q is already rotated and the new keys / values are already in the cache (launch_rope_kv_append); out is [tokens, n_heads * 128]
 int32_t launch_attention_prefill(const float* q, int q_stride, float* out, int n_heads, const KvLayout& kv, const PrefillTile* tiles_dev, int n_tiles,
                                  const int32_t* page_table, int pages_per_seq, cudaStream_t s);
+// the same in f32 for the other head sizes (32, 64, 128, 256), cache types and page sizes
+bool attention_rows_applies(const KvLayout& kv, int n_heads, const float* q, int q_stride);
+int32_t launch_attention_rows(const float* q, int q_stride, float* out, int n_heads, const KvLayout& kv, const PrefillTile* tiles_dev, int n_tiles,
+                              const int32_t* page_table, int pages_per_seq, cudaStream_t s);
 // Bytes of merge slots the single-token streaming kernel needs for this head geometry (0: the kernel does not apply).
 size_t attention_stream_slot_bytes(int n_heads, int n_kv);
 

@@ -40,6 +40,9 @@ struct LayerW {
 // Tokens per pass.  The experts of a mixture receive a share of them each, and the fuller their tiles the better (Mixtral shape, 4 layers,
 // 1,600 tokens: 36.9 ms in passes of 1,024, 33.1 in one); the step buffers grow with it.
 constexpr int kPrefillChunk = 2048;
+// Tokens per tile from which prompts attend tile by tile where the tensor-core kernel does not apply; shorter runs would leave most warps of a
+// tile idle while one of them walks the whole context, which the split-context kernel shares out.
+constexpr int kRowsRun = 8;
 constexpr int kAttnSlice = 512;          // tokens per launch of the attention kernels that split a context (their scratch grows with both)
 constexpr int kTileRun = 16;             // runs of fewer tokens attend token by token
 constexpr int kChunkRun = 32;            // runs of fewer tokens walk the gated delta rule token by token
