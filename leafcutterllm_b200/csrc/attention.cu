@@ -14,47 +14,48 @@
 
 namespace lc {
 
+// One thread has a pair (d, d + hd / 2) of one token and takes it through several heads: the angle's power, sine and cosine are the same for all of
+// them and cost more than the rotation (a thread per pair and head: 27 us for 512 tokens of 32 + 32 heads, against 8 us of memory traffic).
 __global__ void rope_kv_append_kernel(float* __restrict__ q, float* __restrict__ k, const float* __restrict__ v, int row_stride,
-                                      int n_tok, int n_heads, KvLayout kv, const int32_t* __restrict__ tok_seq,
+                                      int n_heads, KvLayout kv, const int32_t* __restrict__ tok_seq,
                                       const int32_t* __restrict__ tok_pos, const int32_t* __restrict__ tok_rope,
                                       const int32_t* __restrict__ page_table, int pages_per_seq, float theta) {
     pdl_launch_dependents();
     pdl_wait();
-    const int hd = kv.hd, half = hd / 2;
-    const int per_tok = (n_heads + kv.n_kv) * half;
-    long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (long long)n_tok * per_tok) return;
-    int tok = (int)(idx / per_tok), r = (int)(idx % per_tok);
-    int h = r / half, d = r % half;
+    const int hd = kv.hd, half = hd / 2, tok = blockIdx.x, d = threadIdx.x % half;
+    const int lanes = blockDim.x / half, step = lanes * gridDim.y;
     // attention.rs:16-20
-    float freq = __fdiv_rn(1.0f, powf(theta, __fdiv_rn(__fmul_rn(2.0f, (float)d), (float)hd)));
-    float angle = __fmul_rn((float)tok_rope[tok], freq);
-    float ca = cosf(angle), sa = sinf(angle);
-    if (h < n_heads) {
-        float* p = q + (size_t)tok * row_stride + h * hd;
-        float x1 = p[d], x2 = p[d + half];
-        p[d] = __fsub_rn(__fmul_rn(x1, ca), __fmul_rn(x2, sa));
-        p[d + half] = __fadd_rn(__fmul_rn(x1, sa), __fmul_rn(x2, ca));
-    } else {
-        int kh = h - n_heads;
-        float* p = k + (size_t)tok * row_stride + kh * hd;
-        const float* pv = v + (size_t)tok * row_stride + kh * hd;
-        float x1 = p[d], x2 = p[d + half];
-        float r1 = __fsub_rn(__fmul_rn(x1, ca), __fmul_rn(x2, sa));
-        float r2 = __fadd_rn(__fmul_rn(x1, sa), __fmul_rn(x2, ca));
-        p[d] = r1;
-        p[d + half] = r2;
-        int pos = tok_pos[tok];
-        int page = page_table[(size_t)tok_seq[tok] * pages_per_seq + pos / kv.page_tokens];
-        size_t base = (((size_t)page * kv.n_kv + kh) * kv.page_tokens + pos % kv.page_tokens) * hd;
-        if (kv.kv_f32) {
-            float* K = (float*)kv.k_pool; float* V = (float*)kv.v_pool;
-            K[base + d] = r1; K[base + d + half] = r2;
-            V[base + d] = pv[d]; V[base + d + half] = pv[d + half];
+    const float freq = __fdiv_rn(1.0f, powf(theta, __fdiv_rn(__fmul_rn(2.0f, (float)d), (float)hd)));
+    const float angle = __fmul_rn((float)tok_rope[tok], freq);
+    const float ca = cosf(angle), sa = sinf(angle);
+    const int pos = tok_pos[tok];
+    const int page = page_table[(size_t)tok_seq[tok] * pages_per_seq + pos / kv.page_tokens];
+#pragma unroll 4
+    for (int h = blockIdx.y * lanes + threadIdx.x / half; h < n_heads + kv.n_kv; h += step) {
+        if (h < n_heads) {
+            float* p = q + (size_t)tok * row_stride + h * hd;
+            const float x1 = p[d], x2 = p[d + half];
+            p[d] = __fsub_rn(__fmul_rn(x1, ca), __fmul_rn(x2, sa));
+            p[d + half] = __fadd_rn(__fmul_rn(x1, sa), __fmul_rn(x2, ca));
         } else {
-            __half* K = (__half*)kv.k_pool; __half* V = (__half*)kv.v_pool;
-            K[base + d] = __float2half_rn(r1); K[base + d + half] = __float2half_rn(r2);
-            V[base + d] = __float2half_rn(pv[d]); V[base + d + half] = __float2half_rn(pv[d + half]);
+            const int kh = h - n_heads;
+            float* p = k + (size_t)tok * row_stride + kh * hd;
+            const float* pv = v + (size_t)tok * row_stride + kh * hd;
+            const float x1 = p[d], x2 = p[d + half];
+            const float r1 = __fsub_rn(__fmul_rn(x1, ca), __fmul_rn(x2, sa));
+            const float r2 = __fadd_rn(__fmul_rn(x1, sa), __fmul_rn(x2, ca));
+            p[d] = r1;
+            p[d + half] = r2;
+            const size_t base = (((size_t)page * kv.n_kv + kh) * kv.page_tokens + pos % kv.page_tokens) * hd;
+            if (kv.kv_f32) {
+                float* K = (float*)kv.k_pool; float* V = (float*)kv.v_pool;
+                K[base + d] = r1; K[base + d + half] = r2;
+                V[base + d] = pv[d]; V[base + d + half] = pv[d + half];
+            } else {
+                __half* K = (__half*)kv.k_pool; __half* V = (__half*)kv.v_pool;
+                K[base + d] = __float2half_rn(r1); K[base + d + half] = __float2half_rn(r2);
+                V[base + d] = __float2half_rn(pv[d]); V[base + d + half] = __float2half_rn(pv[d + half]);
+            }
         }
     }
 }
@@ -268,10 +269,12 @@ int32_t launch_rope_kv_append(float* q, float* k, const float* v, int row_stride
                               const int32_t* tok_seq, const int32_t* tok_pos, const int32_t* tok_rope,
                               const int32_t* page_table, int pages_per_seq, float theta, cudaStream_t s) {
     if (n_tok <= 0) return LC_OK;
-    long long total = (long long)n_tok * (n_heads + kv.n_kv) * (kv.hd / 2);
-    unsigned grid = (unsigned)((total + 255) / 256);
-    LC_CUDA(launch_k(rope_kv_append_kernel, dim3(grid), dim3(256), s, q, k, v, row_stride, n_tok, n_heads, kv, tok_seq, tok_pos,
-                     tok_rope, page_table, pages_per_seq, theta));
+    const int half = kv.hd / 2, lanes = std::max(1, 256 / half), heads = n_heads + kv.n_kv;
+    LC_CHECK(half >= 1 && half * lanes <= 1024, LC_ERR_UNSUPPORTED, "rope: head_dim %d", kv.hd);
+    // few tokens: the heads over several CTAs, down to one head per thread
+    const int parts = std::min((heads + lanes - 1) / lanes, std::max(1, 8 * sm_count() / n_tok));
+    LC_CUDA(launch_k(rope_kv_append_kernel, dim3((unsigned)n_tok, (unsigned)parts), dim3((unsigned)(half * lanes)), s, q, k, v, row_stride, n_heads, kv, tok_seq,
+                     tok_pos, tok_rope, page_table, pages_per_seq, theta));
     return LC_OK;
 }
 
