@@ -131,7 +131,8 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_staged_kernel(AttnP
         stage(pos);
     }
     const int t_begin = split * p.chunk, t_end = min(pos + 1, t_begin + p.chunk);
-    const int n = t_end - t_begin;
+    const int n = t_end - t_begin, live = (pos + p.chunk) / p.chunk;  // pieces that hold a key of this token; the grid has room for the longest context
+    if (n <= 0) return;
     __syncthreads();  // barrier initialised
     bool ok = true;
     if (n > 0) ok = mbar_wait(&bar, 0);
@@ -216,7 +217,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_staged_kernel(AttnP
             __syncthreads();
             a_out = ((acc_s[tid] + acc_s[HD + tid]) + acc_s[2 * HD + tid]) + acc_s[3 * HD + tid];
         }
-        if (p.n_splits == 1) {
+        if (live == 1) {
             p.out[(size_t)item * HD + tid] = a_out / l;
             continue;
         }
@@ -225,19 +226,19 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_staged_kernel(AttnP
         // the last split of this (token, head) to finish merges all of them, in split order
         __threadfence();
         __syncthreads();
-        if (tid == 0) last_s = (atomicAdd(&p.counters[item], 1) == p.n_splits - 1);
+        if (tid == 0) last_s = (atomicAdd(&p.counters[item], 1) == live - 1);
         __syncthreads();
         if (last_s) {
             __threadfence();
             const float* pp = p.partial + (size_t)item * p.n_splits * (HD + 2);
             float mm = -INFINITY;
-            for (int s2 = 0; s2 < p.n_splits; s2++) mm = fmaxf(mm, __ldcg(pp + (size_t)s2 * (HD + 2)));
+#pragma unroll 4
+            for (int s2 = 0; s2 < live; s2++) mm = fmaxf(mm, __ldcg(pp + (size_t)s2 * (HD + 2)));
             float ll = 0.f, a = 0.f;
-            for (int s2 = 0; s2 < p.n_splits; s2++) {
+#pragma unroll 4
+            for (int s2 = 0; s2 < live; s2++) {  // no branch: the pieces' loads are in flight together
                 const float* ps = pp + (size_t)s2 * (HD + 2);
-                const float ms = __ldcg(ps);
-                if (ms == -INFINITY) continue;  // empty split
-                const float scl = expf(ms - mm);
+                const float scl = expf(__ldcg(ps) - mm);
                 ll += __ldcg(ps + 1) * scl;
                 a += __ldcg(ps + 2 + tid) * scl;
             }

@@ -282,14 +282,14 @@ __device__ __forceinline__ void attention_item(const AttnParams& p, int item, in
             ll += sm_l[w] * sc;
             a += sm_acc[w][d] * sc;
         }
-        if (p.n_splits == 1) {
+        if (live == 1) {  // nothing to merge with, whatever the launch left room for
             p.out[(size_t)tok * n_heads * HD + h * HD + d] = a / ll;
         } else {
             if (d == 0) { pout[0] = mm; pout[1] = ll; }
             pout[2 + d] = a;
         }
     }
-    if (p.n_splits == 1) return;
+    if (live == 1) return;
     // ---- the last split of this (token, head) to finish merges all of them, in split order ----
     __threadfence();
     group_sync<BAR>(bar_id);
@@ -302,14 +302,14 @@ __device__ __forceinline__ void attention_item(const AttnParams& p, int item, in
     __threadfence();
     const float* pp = p.partial + (size_t)item * p.n_splits * (HD + 2);
     float mm = -INFINITY;
+#pragma unroll 4
     for (int s = 0; s < live; s++) mm = fmaxf(mm, __ldcg(pp + (size_t)s * (HD + 2)));
     for (int d = tid; d < HD; d += kAttnWarps * 32) {
         float ll = 0.f, a = 0.f;
-        for (int s = 0; s < live; s++) {
+#pragma unroll 4
+        for (int s = 0; s < live; s++) {  // every one of them has a key; no branch: the pieces' loads are in flight together
             const float* ps = pp + (size_t)s * (HD + 2);
-            const float ms = __ldcg(ps);
-            if (ms == -INFINITY) continue;  // empty split
-            const float sc = expf(ms - mm);
+            const float sc = expf(__ldcg(ps) - mm);
             ll += __ldcg(ps + 1) * sc;
             a += __ldcg(ps + 2 + d) * sc;
         }
