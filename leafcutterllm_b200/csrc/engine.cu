@@ -599,9 +599,10 @@ static int32_t create_handle(const lc_model_config* cfg, std::unique_ptr<LayerSt
     int64_t pool = m->cfg.kv_pool_tokens > 0 ? m->cfg.kv_pool_tokens : (int64_t)m->max_seqs * m->pages_per_seq * m->page_tokens;
     m->pages_total = (int)((pool + m->page_tokens - 1) / m->page_tokens);
     m->kv_elt = m->cfg.kv_dtype ? 4 : 2;
-    // a pass holds no more tokens than the handle's sequences can have: the step buffers, and the time to allocate them, follow
-    const long most = std::min<long>(kPrefillChunk, (long)m->max_seqs * m->cfg.max_seq_len);
-    m->t_cap = std::max({m->stack ? kStackChunk : (int)most, m->max_seqs, 16});
+    // a pass holds no more tokens than the handle's sequences can have, but 512 (the layer probes take as many): the step buffers, and the time to
+    // allocate them, follow
+    const long most = std::max<long>(512, std::min<long>(kPrefillChunk, (long)m->max_seqs * m->cfg.max_seq_len));
+    m->t_cap = std::max(m->stack ? kStackChunk : (int)most, m->max_seqs);
     m->head_rows = std::max(16, m->max_seqs);
     m->seq_open.assign(m->max_seqs, 0);
     m->stream = lc::stream();

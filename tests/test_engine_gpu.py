@@ -90,6 +90,21 @@ def test_chunked_prefill_matches(gpu, oracle):
     eng.close()
 
 
+@pytest.mark.parametrize("rows", [16, 63, 65, 130])  # one tile with idle warps, a row short of a tile, one more, two full ones and a short one
+@pytest.mark.parametrize("hd,kv_dtype,page", [(32, "f16", 16), (32, "f32", 5), (64, "f32", 16), (64, "f16", 32), (128, "f32", 16), (128, "f16", 8), (256, "f16", 16), (256, "f32", 16)])
+def test_prompt_attention_in_tiles(gpu, oracle, hd, kv_dtype, page, rows):
+    """Head sizes, cache types and page sizes that the tensor-core prompt attention does not take; a second run of rows behind the first,
+    so that tiles begin past position 0.  The host's and the device's powf differ by an ulp or two, which is 260 * 2^-22 = 6e-5 of an angle at the
+    last position and of the scores' order: 2e-4 of the largest output; an f16 cache may round a key or value the other way (2^-11 of it): 1e-3."""
+    spec = small_spec(12, 12, 12, layers=1, hidden=512, heads=512 // hd, kv=max(1, 256 // hd), ffn=256, vocab=64)
+    eng, om = make_pair(gpu, oracle, spec, max_seq_len=2 * rows, kv_dtype=kv_dtype, kv_page_tokens=page, rope_mode="absolute")
+    x = np.random.default_rng(hd + rows).standard_normal((2 * rows, 512)).astype(np.float32)
+    for part in (x[:rows], x[rows:]):
+        got, want = eng.probe_attention(0, part), om.attention(0, part)
+        assert_close(got, want, (2e-4 if kv_dtype == "f32" else 1e-3) * np.abs(want).max(), 0, f"{rows} rows of {hd}")
+    eng.close()
+
+
 @pytest.mark.parametrize("types,heads", [((12, 12, 12), 2), ((2, 8, 8), 8)])
 def test_prompt_longer_than_a_pass(gpu, oracle, types, heads):
     """2,100 tokens: a full pass of 2,048 and a short one behind it; heads of 128 (tiled prefill attention) and of 32 (in slices of 512 tokens)."""
