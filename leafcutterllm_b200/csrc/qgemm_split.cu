@@ -34,8 +34,9 @@
 //              unit behind its unpacking, so it never waits for the products it feeds.  `main` has two places that units take in turn.
 //
 // What bounds it: the tensor pipe.  192 cycles per 128 rows x 128 tokens x 16 elements (128 + 64 for the two instructions; measured
-// 128 / 64 / 45 / 45 cycles at N = 256 / 128 / 64 / 32 and below), i.e. a third of the f16 rate; few tokens are bound by the 45
-// cycles that any instruction takes.  Unpacking takes 2.4 instructions per weight (Q6_K five), a quarter of the issue slots at 128 tokens.
+// 128 / 64 / 32 / 13 cycles at N = 256 / 128 / 64 / 16), i.e. a third of the f16 rate.  ncu, 2,048 tokens, Q4_K: tensor pipe active 71 % of the
+// cycles for [4096 -> 12288] (505 us), 68 % for gate and up of 11008 (911 us); issue slots 65 %, two thirds of them unpacking (2.4 instructions per
+// weight, Q6_K five).  512 tokens x [4096 -> 12288]: 138 us, where two products per weight and 64 tokens per CTA (qgemm_umma.cu) took 203.
 #include <algorithm>
 #include <cstdlib>
 #include <cuda_fp16.h>
@@ -412,7 +413,7 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
     const int nv = nu + (sum_chunks + 3) / 4;                 // as further units of up to four chunks
     auto chunks_of = [&](int v) { return v < nu ? 4 : min(4, sum_chunks - 4 * (v - nu)); };
 
-    // Stages are counted along, never by division: one takes a single thread 100 cycles.
+    // Stages are counted along, never by division: one takes a single thread 100 cycles (a tile of 17 units took 163k with them, 112k without).
     if (warp == 0) {
         // ---------------------------------------------------------------- producer of the activations
         if (lane == 0) {
@@ -500,7 +501,7 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
     } else if (warp == 1) {
         // ---------------------------------------------------------------- multiply
         // the whole warp walks the loop and waits (uniform control flow, so that operands live in uniform registers: one lane walking it alone
-        // issues a product every 57 cycles at best, and every 200 here), one lane issues
+        // issues a product every 57 cycles at best, and every 200 here: a tile of 17 units took 112k cycles, now 68k), one lane issues
         const bool one = elect_one();
         const uint32_t id1 = idesc_f16(N), id2 = idesc_f16(2 * N), d_small = tmem + kColSmall, a0 = tmem + col_a(N);
         int sb = 0;
@@ -739,13 +740,21 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
                 }
             } else {
                 const size_t o = (size_t)t_first * p.n + grow;
+                if (p.epi == EPI_ADD_RESIDUAL) {
+                    // the loads of sixteen tokens together (`residual` may be `out`): one beside each store takes a trip to L2 for each,
+                    // 244 us against 197 without a residual for 2,048 tokens x [4096 -> 4096]
+#pragma unroll
+                    for (int t0 = 0; t0 < kOwn; t0 += 16) {
+                        float r[16];
+#pragma unroll
+                        for (int t = 0; t < 16; t++) r[t] = live && t0 + t < mine ? p.residual[o + (size_t)(t0 + t) * p.n] : 0.f;
+#pragma unroll
+                        for (int t = 0; t < 16; t++) y[t0 + t] = __fadd_rn(r[t], y[t0 + t]);
+                    }
+                }
 #pragma unroll
                 for (int t = 0; t < kOwn; t++)
-                    if (live && t < mine) {
-                        float r = y[t];
-                        if (p.epi == EPI_ADD_RESIDUAL) r = __fadd_rn(p.residual[o + (size_t)t * p.n], r);
-                        p.out[o + (size_t)t * p.n] = r;
-                    }
+                    if (live && t < mine) p.out[o + (size_t)t * p.n] = y[t];
             }
         }
     }
