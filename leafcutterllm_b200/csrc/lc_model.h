@@ -49,9 +49,10 @@ constexpr int kChunkRun = 32;            // runs of fewer tokens walk the gated 
 constexpr int kStackChunk = 2048;      // tokens per pass of a checkpoint-directory design
 constexpr int kTokTile = 8;
 constexpr int kMoeGroupedTokens = 64;  // most tokens of a call whose experts run as one grouped matrix-vector launch
-// Rows per expert from which the experts run as a grouped many-token product instead: the matrix-vector kernel reads the experts again for
-// every four rows.  Mixtral shape, gate/up + down of a layer: 4 rows 420 us (matrix-vector), a hundred rows 2.4 ms (product).
-constexpr int kMoeProductRows = 5;
+// Rows per expert beyond which the experts run as a grouped many-token product instead: the matrix-vector kernel reads the experts again for
+// every four rows.  Mixtral shape, us per step of two layers, matrix-vector / product: 24 sequences (6 rows per expert) 1761 / 2169, 32 (8)
+// 2143 / 2263, 48 (12) 2899 / 2563, 64 (16) 3656 / 3028.
+constexpr int kMoeProductRows = 9;
 
 }  // namespace lc
 

@@ -49,9 +49,9 @@ def test_moe_long_call_runs_every_expert(gpu, oracle):
     eng.close()
 
 
-@pytest.mark.parametrize("n_experts,top_k,tokens", [(4, 2, 11), (8, 1, 41), (5, 3, 64), (8, 2, 65), (3, 1, 300), (16, 4, 130)])
+@pytest.mark.parametrize("n_experts,top_k,tokens", [(4, 2, 19), (2, 1, 41), (5, 3, 64), (8, 2, 65), (3, 1, 300), (16, 4, 130)])
 def test_moe_product_of_experts(gpu, oracle, n_experts, top_k, tokens):
-    """Calls in which experts receive more than five rows each: rows in expert order through one many-token product per projection.
+    """Calls in which experts receive more than nine rows each on average: rows in expert order through one many-token product per projection.
     Experts with few rows and with more than a tile, rows that end inside a tile of 16, the next call's decode step on the same cache."""
     from leafcutterllm_b200 import synth
     spec = moe_spec(layers=1, n_experts=n_experts, top_k=top_k)
