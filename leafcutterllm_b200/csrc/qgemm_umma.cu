@@ -977,9 +977,9 @@ static int32_t launch_qgemm_tile(const GemvArgs& a, GemmWorkspace& ws, int* slic
 }
 
 // One token tile of Q4_K / Q5_K stays with the kernel above: it multiplies twice per weight where qgemm_split.cu does three times, and up to
-// 64 tokens its instructions are too short for that to be free.  Measured with the activation preparation, 64 tokens, us here / there:
-// [4096 -> 12288] 40 / 44, [11008 -> 4096] 35 / 38, gate and up 71 / 90; 128 tokens 75 / 48, 68 / 41, 130 / 95; 512 tokens 207 / 136,
-// 190 / 118, 350 / 240.
+// 64 tokens its instructions are too short for that to be free.  Measured with the activation preparation, us here / there:
+// 16 tokens [4096 -> 12288] 30.6 / 38.5, [4096 -> 4096] 14.5 / 16.8, [11008 -> 4096] 26.6 / 32.2, gate and up 53 / 78;
+// 64 tokens [4096 -> 12288] 41 / 44; 512 tokens 212 / 138, gate and up 327 / 237.
 static bool use_split(uint32_t typ, int T) { return T > kMaxTok || (typ != LC_TYPE_Q4_K && typ != LC_TYPE_Q5_K); }
 
 int32_t launch_qgemm(const GemvArgs& a, GemmWorkspace& ws, cudaStream_t s, int* launches) {

@@ -371,3 +371,14 @@ def test_decode_ignores_unwritten_cache_rows(gpu, oracle):
     toks = eng.generate(prompt, 40, stop_on_eos=False)
     assert toks == ref, margins
     eng.close()
+
+
+def test_ffn_probe_of_more_rows_than_the_cache_holds(gpu, oracle):
+    """A pass is 512 rows at least, whatever the sequences' capacity."""
+    spec = small_spec(12, 12, 12, layers=1, hidden=256, heads=2, kv=2, ffn=512, vocab=64)
+    eng, om = make_pair(gpu, oracle, spec, max_seq_len=32)
+    x = np.random.default_rng(3).standard_normal((512, 256)).astype(np.float32)
+    want = om.ffn(0, x)
+    # SiLU(gate) * up of two many-token products (2e-5 of the largest each, tested with the product), then a third
+    assert_close(eng.probe_ffn(0, x), want, 1e-4 * np.abs(want).max(), 1e-4, "512 rows")
+    eng.close()
