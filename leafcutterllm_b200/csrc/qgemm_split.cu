@@ -588,7 +588,7 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
         const int own = WIDE ? max(0, min(32, N - 32 * g)) : N / 4, tbase = g * (WIDE ? 32 : N / 4);  // this thread's tokens of the tile
         auto wait_all = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); };
         float y[kOwn];
-        auto add_columns = [&](uint32_t col) {
+        auto add_columns = [&](uint32_t col, uint32_t skip) {  // skip: a bit for each token that keeps what it has
             col += lane_base + tbase;
             if constexpr (WIDE) {
 #pragma unroll
@@ -598,7 +598,7 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
                         tmem_ld16(col + t0, a);
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                        for (int t = 0; t < 16; t++) y[t0 + t] += __uint_as_float(a[t]);
+                        for (int t = 0; t < 16; t++) y[t0 + t] += (skip >> (t0 + t)) & 1u ? 0.f : __uint_as_float(a[t]);
                     }
             } else {
                 uint32_t a[16];
@@ -610,7 +610,7 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
                 for (int t0 = 0; t0 < 16; t0 += 4)
                     if (t0 < own) {
 #pragma unroll
-                        for (int t = t0; t < t0 + 4; t++) y[t] += __uint_as_float(a[t]);
+                        for (int t = t0; t < t0 + 4; t++) y[t] += (skip >> t) & 1u ? 0.f : __uint_as_float(a[t]);
                     }
             }
         };
@@ -619,7 +619,7 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
             ok = wait_all(&d_full[w & 1], (w >> 1) & 1);
             if (!ok) return;
             tc_fence_after();
-            add_columns(w & 1 ? kColSmall + (uint32_t)N : kColSmall - (uint32_t)N);
+            add_columns(w & 1 ? kColSmall + (uint32_t)N : kColSmall - (uint32_t)N, 0u);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&d_empty[w & 1]);
@@ -704,13 +704,17 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
                 if (ok) drain(v - 1);
             }
             if (ok) drain(nv - 1);
-            if (ok && own > 0) add_columns(kColSmall);  // complete: the last unit's d_full followed every product
             pdl_wait();
             const int t_first = tok0 + tbase, mine = ok ? min(own, tok_end - t_first) : 0;
             // a lane has one token's scale: a load beside each result's store would wait for it
             const float scale = lane < mine ? __ldg(p.tok_scale + t_first + lane) : 0.f;
+            // A negative scale: the token holds an infinity or a NaN (xprep_row).  `main` has its results' signs, W_lo * inf in `small` would be NaN
+            // wherever W_lo is zero.
+            const uint32_t wild = __ballot_sync(0xffffffffu, scale < 0.f);
+            if (ok && own > 0) add_columns(kColSmall, wild);  // complete: the last unit's d_full followed every product
+            // two multiplications: the product of the powers may leave f32's range where the result does not
 #pragma unroll
-            for (int t = 0; t < kOwn; t++) y[t] *= down * __shfl_sync(0xffffffffu, scale, t);
+            for (int t = 0; t < kOwn; t++) y[t] = (y[t] * down) * fabsf(__shfl_sync(0xffffffffu, scale, t));
             if (p.partial) {
                 float* dst = p.partial + ((size_t)(blockIdx.z * (pair ? 2 : 1) + mat) * p.T + t_first) * p.n + grow;
 #pragma unroll

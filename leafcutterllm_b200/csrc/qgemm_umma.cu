@@ -209,10 +209,14 @@ __device__ __forceinline__ void xprep_row(float* row, float acc, float amax, con
         if (norm_w) scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sh[0], (float)K), eps)));  // cpu.rs:52-55
         mx = sh[32] * scale;
     }
-    int e = 0;
-    if (mx > 0.f && mx < INFINITY) (void)frexpf(mx, &e);  // mx = f * 2^e, f in [0.5, 1)
+    // A row that holds an infinity or a NaN has no finite result, only signs: its low halves are zero (inf - inf would make NaN of a result that
+    // is an infinity), its finite elements come below f16's largest, and the scale's sign tells the product (qgemm_split.cu) of it.
+    const bool wild = !(mx < INFINITY);
+    int e = wild ? 126 : 0;
+    if (mx > 0.f && !wild) (void)frexpf(mx, &e);  // mx = f * 2^e, f in [0.5, 1)
+    e = max(-126, min(126, e));  // the power and its inverse are finite: rows at 2^127 come below 4, rows of denormals stay below 1
     const float down = ldexpf(1.0f, -e);
-    if (threadIdx.x == 0) tok_scale[t] = ldexpf(1.0f, e);
+    if (threadIdx.x == 0) tok_scale[t] = ldexpf(wild ? -1.0f : 1.0f, e);
     __half* hi = xh + (size_t)t * K;
     __half* lo = hi + lo_offset;
     __half* sxh = sx + (size_t)t * (K / 16);
@@ -232,7 +236,8 @@ __device__ __forceinline__ void xprep_row(float* row, float acc, float amax, con
             const float a = v.x * down, b = v.y * down, c = v.z * down, d = v.w * down;
             const __half2 h0 = __floats2half2_rn(a, b), h1 = __floats2half2_rn(c, d);
             const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
-            const __half2 l0 = __floats2half2_rn(a - f0.x, b - f0.y), l1 = __floats2half2_rn(c - f1.x, d - f1.y);
+            __half2 l0 = __floats2half2_rn(a - f0.x, b - f0.y), l1 = __floats2half2_rn(c - f1.x, d - f1.y);
+            if (wild) l0 = l1 = __floats2half2_rn(0.f, 0.f);
             uint2 ph, pl;
             ph.x = *reinterpret_cast<const uint32_t*>(&h0); ph.y = *reinterpret_cast<const uint32_t*>(&h1);
             pl.x = *reinterpret_cast<const uint32_t*>(&l0); pl.y = *reinterpret_cast<const uint32_t*>(&l1);
@@ -247,7 +252,7 @@ __device__ __forceinline__ void xprep_row(float* row, float acc, float amax, con
         part += __shfl_xor_sync(0xffffffffu, part, 4);
         if (i < K && (threadIdx.x & 7) == 0) {
             const int sub = i >> 5, unit = sub >> 3, idx = unit * 16 + (sub & 7);
-            const __half sh_ = __float2half_rn(part), sl_ = __float2half_rn(part - __half2float(sh_));
+            const __half sh_ = __float2half_rn(part), sl_ = __float2half_rn(wild ? 0.f : part - __half2float(sh_));
             sxh[idx] = sh_;
             sxl[idx] = sl_;
             sxh[idx + 8] = sh_;  // a second time: the offset operand pairs each sum with the high and with the low part of -dmin * m
@@ -596,7 +601,7 @@ qgemm_umma_q4k_kernel(const __grid_constant__ CUtensorMap tmw0, const __grid_con
 #pragma unroll
                 for (int t = 0; t < kTokD; t++) {
                     const int tok = tok0 + tbase + t;
-                    if (tbase + t < N && tok < p.T) dst[(size_t)tok * p.n + grow] = y[t] * __ldg(p.tok_scale + tok);
+                    if (tbase + t < N && tok < p.T) dst[(size_t)tok * p.n + grow] = y[t] * fabsf(__ldg(p.tok_scale + tok));
                 }
             } else {
 #pragma unroll
@@ -604,7 +609,7 @@ qgemm_umma_q4k_kernel(const __grid_constant__ CUtensorMap tmw0, const __grid_con
                     const int tok = tok0 + tbase + t;
                     if (tbase + t < N && tok < p.T) {
                         const size_t o = (size_t)tok * p.n + grow;
-                        float v = y[t] * __ldg(p.tok_scale + tok);
+                        float v = y[t] * fabsf(__ldg(p.tok_scale + tok));
                         if (p.epi == EPI_ADD_RESIDUAL) v = __fadd_rn(p.residual[o], v);
                         p.out[o] = v;
                     }

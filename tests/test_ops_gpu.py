@@ -179,6 +179,58 @@ def test_many_token_product_vs_oracle(gpu, oracle, typ, m, k, n):
     assert_close(want[:5, rows], oracle.qmatmul(typ, a[:5].ravel(), sub, 5, k, len(rows)).reshape(5, len(rows)), 2e-5 * np.abs(want[:5, rows]).max(), 1e-4, "oracle sample")
 
 
+def scaled_blocks(gpu, typ, n, k, size, r):
+    """Random blocks whose largest weight is about `size` [n, blocks of a row] (offsets as large), and the weights in 64 bits."""
+    be, bb = gpu.QUANT_GEOMETRY[typ]
+    w = r.integers(0, 256, n * k // be * bb, dtype=np.uint8).reshape(n, -1, bb)
+    sc = np.broadcast_to(size / {2: 8, 8: 128, 12: 945, 13: 1953, 14: 4064}[typ], w.shape[:2]).astype(np.float16).view(np.uint16)
+    at = 208 if typ == 14 else 0
+    w[..., at], w[..., at + 1] = sc & 0xFF, sc >> 8
+    if typ in (12, 13):
+        w[..., 2], w[..., 3] = sc & 0xFF, sc >> 8
+    w = w.ravel()
+    return w, gpu.dequantize(typ, w, n * k).reshape(n, k).astype(np.float64)
+
+
+@pytest.mark.parametrize("m", [5, 70])  # the tiles of up to 64 tokens and of more
+@pytest.mark.parametrize("typ", [2, 8, 12, 13, 14])
+def test_many_token_product_at_the_ends_of_f32(gpu, typ, m):
+    """Tokens whose largest element is a denormal, just above 2^-126, or just below f32's end: the power of two that brings them to f16's range has
+    an inverse in f32, and results are as exact as any (the bound of the test above, and half a denormal's step for each of the few roundings)."""
+    k, n = 512, 70
+    r = rng(typ + m)
+    w, dense = scaled_blocks(gpu, typ, n, k, np.exp2(r.uniform(-12, -8, (n, 1))), r)
+    a = r.uniform(-1, 1, (m, k))
+    power = np.resize([-140, -130, -127, -126, -116, 0, 110, 126, 127], m)
+    a = (a * np.exp2(power.astype(np.float64))[:, None]).astype(np.float32)
+    got = gpu.qmatmul(typ, a.ravel(), w, m, k, n).reshape(m, n)
+    want = a.astype(np.float64) @ dense.T
+    bound = 2e-5 * np.sqrt((a.astype(np.float64) ** 2) @ (dense.T ** 2)) + 2.0 ** -147
+    assert np.isfinite(got).all()
+    assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / bound).max(1)
+
+
+@pytest.mark.parametrize("m", [5, 70])
+@pytest.mark.parametrize("typ", [2, 8, 14])
+def test_many_token_product_of_infinities(gpu, typ, m):
+    """A token with one infinity gives infinities of the weights' signs (NaN where the weight is zero), one with a NaN gives NaN, the others what they always give."""
+    k, n = 512, 70
+    r = rng(typ + m + 1)
+    w, dense = scaled_blocks(gpu, typ, n, k, np.ones((n, 1)), r)
+    a = r.standard_normal((m, k)).astype(np.float32)
+    a[0, 300], a[2, 7], a[m - 1, 511] = np.inf, -np.inf, np.nan
+    a[0, 301] = 1e30  # finite, and past f16's largest
+    got = gpu.qmatmul(typ, a.ravel(), w, m, k, n).reshape(m, n)
+    with np.errstate(invalid="ignore"):
+        for t, c in ((0, 300), (2, 7)):
+            want = a[t, c] * dense[:, c]
+            assert np.array_equal(got[t], want.astype(np.float32), equal_nan=True), t
+    assert np.isnan(got[m - 1]).all()
+    rest = [t for t in range(m) if t not in (0, 2, m - 1)]
+    want = a[rest].astype(np.float64) @ dense.T
+    assert (np.abs(got[rest] - want) <= 2e-5 * np.sqrt((a[rest].astype(np.float64) ** 2) @ (dense.T ** 2))).all()
+
+
 def test_qmatmul_linearity_full_size(gpu, oracle):
     """7B-shape matrices: A(x+y) = Ax + Ay and a sample of rows against the oracle."""
     from leafcutterllm_b200 import synth
