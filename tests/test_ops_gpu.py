@@ -231,6 +231,22 @@ def test_many_token_product_of_infinities(gpu, typ, m):
     assert (np.abs(got[rest] - want) <= 2e-5 * np.sqrt((a[rest].astype(np.float64) ** 2) @ (dense.T ** 2))).all()
 
 
+@pytest.mark.parametrize("m", [5, 70])
+@pytest.mark.parametrize("typ", [2, 8, 12, 13, 14])
+def test_many_token_product_beside_a_large_activation(gpu, typ, m):
+    """One element 2^12 times the size of the others, over blocks of zeros: the others keep their 22 bits, and results the bound that they have without it."""
+    k, n = 1024, 70
+    r = rng(typ + m + 2)
+    blocks = k // gpu.QUANT_GEOMETRY[typ][0]
+    w, dense = scaled_blocks(gpu, typ, n, k, np.where(np.arange(blocks) == 0, 0.0, 1.0)[None], r)
+    a = r.standard_normal((m, k)).astype(np.float32)
+    a[:, 3] = 4096 * r.choice([-1, 1], m)
+    got = gpu.qmatmul(typ, a.ravel(), w, m, k, n).reshape(m, n)
+    want = a.astype(np.float64) @ dense.T
+    bound = 2e-5 * np.sqrt((a.astype(np.float64) ** 2) @ (dense.T ** 2))
+    assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / bound).max()
+
+
 def test_qmatmul_linearity_full_size(gpu, oracle):
     """7B-shape matrices: A(x+y) = Ax + Ay and a sample of rows against the oracle."""
     from leafcutterllm_b200 import synth
