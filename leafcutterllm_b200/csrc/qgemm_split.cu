@@ -14,8 +14,13 @@
 //
 // The tensor cores truncate when they add to an f32 accumulator: the error grows with the number of additions (measured on
 // N(0,1) products: 3.5e-7 of the result after 256 elements of k, 1.2e-6 after 1024, 9.6e-6 after 8192; 3 terms into one accumulator
-// 1.0e-6 after 256).  So `main`, 2^11 times larger than `small`, is emptied into registers every 256 elements and those sums are
-// rounded to nearest; `small` runs to the end.
+// 1.0e-6 after 256).  So `main`, 2^11 times larger than `small`, is emptied into registers every 128 or 256 elements and those sums are
+// rounded to nearest; `small` runs to the end.  What is cut off points toward zero, 2.8e-7 of a sum after 256 elements on average and 1.6e-7 after
+// 128, much the same for normal, one-signed and very unequal data, so results are scaled up by about as much: the error's range, one-sided before,
+// then lies around zero.  (Sums that need no cutting, of weights with very few bits, are moved by that much instead.)  Error for normal activations, k = 2048: 3.5e-7
+// uncorrected, 2.0e-7 over 256, 1.4e-7 over 128 elements (additions in f32 in the matrix-vector kernels: 1.0e-7; their fixed-point form 3.0e-7).
+// Emptying every 128 costs 8 % of a 7B prompt, where the tensor pipe is the bound, and 0.7 % of the short prompts of a small Q4_0 / Q8_0 model,
+// whose matrix-vector kernels add in f32: those have it.  Up to 32 tokens tensor memory has room for two sums of 128 elements each, at no cost.
 //
 // Q4_K / Q5_K weights are d * sc * q - dmin * m: the first part is the weight above, the second joins as more k: -dmin * m (17
 // bits, two f16) of a sub-block against the sum of the activations over it, 16 values per 256-element unit, behind the last unit.
@@ -30,8 +35,8 @@
 //              tcgen05.st as the A operand in TENSOR MEMORY (lane = row, column = two consecutive k).  A group has a tensor-memory
 //              stage of its own, so every barrier has one waiter that sees all of its phases;
 //   multiply   one warp, whose elected lane issues;
-//   drain      the unpack warps again: when a unit is through, group g adds tokens 32 g ... 32 g + 31 of `main` to its registers, one
-//              unit behind its unpacking, so it never waits for the products it feeds.  `main` has two places that units take in turn.
+//   drain      the unpack warps again: when a run is through, group g adds tokens 32 g ... 32 g + 31 of `main` to its registers, one
+//              run behind its unpacking, so it never waits for the products it feeds.  `main` has two places that runs take in turn.
 //
 // What bounds it: the tensor pipe.  192 cycles per 128 rows x 128 tokens x 16 elements (128 + 64 for the two instructions; measured
 // 128 / 64 / 32 / 13 cycles at N = 256 / 128 / 64 / 16), i.e. a third of the f16 rate.  ncu, 2,048 tokens, Q4_K: tensor pipe active 71 % of the
@@ -56,8 +61,8 @@ constexpr int kMaxB = 8;         // activation chunks (64 elements) in flight
 constexpr int kGroups = 4;       // unpack groups of four warps
 constexpr int kControl = 4;      // warps ahead of them: activation producer, issuer, raw producer (Q6_K: two)
 constexpr int kThreads = 32 * (kControl + 4 * kGroups);
-// Tensor-memory columns: main of even units [128 - N, 128), small [128, 128 + N), main of odd units [128 + N, 128 + 2 N): small borders on
-// both, so that one instruction covers main and small of either (odd units have their activations as [lo | hi]).  Behind them
+// Tensor-memory columns: main of even runs [128 - N, 128), small [128, 128 + N), main of odd runs [128 + N, 128 + 2 N): small borders on
+// both, so that one instruction covers main and small of either (odd runs have their activations as [lo | hi]).  Behind them
 // the A stages, 32 columns each: 16 of W_hi, 16 of W_lo for 32 elements of k; four, or eight where 64 tokens and fewer leave the room.
 constexpr uint32_t kColSmall = 128;
 __host__ __device__ constexpr uint32_t col_a(int N) { return N <= 64 ? 256u : 384u; }
@@ -68,6 +73,11 @@ template <> struct RawUnit<LC_TYPE_Q5_K> { static constexpr int pitch = 176; };
 template <> struct RawUnit<LC_TYPE_Q4_0> { static constexpr int pitch = 144; };
 template <> struct RawUnit<LC_TYPE_Q8_0> { static constexpr int pitch = 272; };
 template <> struct RawUnit<LC_TYPE_Q6_K> { static constexpr int pitch = 212; };  // 210 from a word boundary on; an odd number of words: no bank conflicts
+// `main` over half a unit at a time (see the header): as runs of their own ...
+template <uint32_t TYPE, bool WIDE> constexpr bool kHalves = WIDE && (TYPE == LC_TYPE_Q4_0 || TYPE == LC_TYPE_Q8_0);
+// ... or, where tensor memory has room, as two sums of one run: then sets of [main of the first half | small | main of the second], for even units
+// from column 0 on and for odd units behind it
+constexpr int kTwoSums = 32;  // most tokens
 template <uint32_t TYPE> constexpr bool kHasMin = TYPE == LC_TYPE_Q4_K || TYPE == LC_TYPE_Q5_K;
 
 struct GemmParams {
@@ -412,6 +422,10 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
     const int sum_chunks = kHasMin<TYPE> ? (nu + 3) / 4 : 0;  // chunks of sub-block sums behind the units, four units each,
     const int nv = nu + (sum_chunks + 3) / 4;                 // as further units of up to four chunks
     auto chunks_of = [&](int v) { return v < nu ? 4 : min(4, sum_chunks - 4 * (v - nu)); };
+    constexpr bool halves = kHalves<TYPE, WIDE>;
+    const bool two = !WIDE && N <= kTwoSums;
+    auto run_of = [&](int v, int c) { return halves ? 2 * v + (c >> 1) : v; };  // of `main`, which has two places that the runs take in turn
+    auto swapped = [&](int v, int c) { return (halves || two) ? c >> 1 : v & 1; };  // activations lie as [lo | hi]: small lies ahead of main
 
     // Stages are counted along, never by division: one takes a single thread 100 cycles (a tile of 17 units took 163k with them, 112k without).
     if (warp == 0) {
@@ -422,16 +436,16 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
             uint32_t phase = 1;
             {
                 for (int v = 0; v < nv && ok; v++) {
-                    unsigned char* const hi_first = bt + (v & 1) * b_half;  // odd units: [lo | hi]
-                    unsigned char* const lo_first = bt + (1 - (v & 1)) * b_half;
                     const int nc = chunks_of(v);
                     for (int c = 0; c < nc; c++) {
                         if (!mbar_wait(&b_empty[sb], phase)) { ok = false; break; }
                         const CUtensorMap* m = v < nu ? &tmx : &tms;
                         const int x = v < nu ? (u_begin + v) * kUnitElems + c * 64 : (u_begin / 4 + (v - nu) * 4 + c) * 64;
+                        unsigned char* const tile = bt + (size_t)sb * 2 * b_half;
+                        const int odd = swapped(v, c);
                         mbar_expect_tx(&b_full[sb], 2 * b_half);
-                        tma_load_3d(hi_first + (size_t)sb * 2 * b_half, m, x, tok0, 0, &b_full[sb]);
-                        tma_load_3d(lo_first + (size_t)sb * 2 * b_half, m, x, tok0, 1, &b_full[sb]);
+                        tma_load_3d(tile + odd * b_half, m, x, tok0, 0, &b_full[sb]);
+                        tma_load_3d(tile + (1 - odd) * b_half, m, x, tok0, 1, &b_full[sb]);
                         in_flight = min(in_flight + 1, BS);
                         if (++sb == BS) { sb = 0; phase ^= 1; }
                     }
@@ -503,29 +517,33 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
         // the whole warp walks the loop and waits (uniform control flow, so that operands live in uniform registers: one lane walking it alone
         // issues a product every 57 cycles at best, and every 200 here: a tile of 17 units took 112k cycles, now 68k), one lane issues
         const bool one = elect_one();
-        const uint32_t id1 = idesc_f16(N), id2 = idesc_f16(2 * N), d_small = tmem + kColSmall, a0 = tmem + col_a(N);
+        const uint32_t id1 = idesc_f16(N), id2 = idesc_f16(2 * N), a0 = tmem + col_a(N);
+        auto small_of = [&](int v) { return tmem + (two ? (uint32_t)((v & 1) * 3 + 1) * (uint32_t)N : kColSmall); };
         int sb = 0;
         uint32_t b_phase = 0;
         const uint64_t b_first = umma_desc_sw128(smem_u32(bt)), b_step = (2 * b_half) >> 4, b_tile = b_half >> 4;
         uint64_t b_both = b_first;
         for (int v = 0; v < nu && ok; v++) {
-            const uint32_t odd = v & 1;
-            const uint32_t d_both = odd ? d_small : d_small - (uint32_t)N, d_main = odd ? d_small + (uint32_t)N : d_both;
-            const uint64_t to_hi = odd ? b_tile : 0, to_lo = odd ? 0 : b_tile;
-            if (v >= 2) ok = mbar_wait(&d_empty[odd], ((v >> 1) - 1) & 1);
 #pragma unroll
             for (int c = 0; c < 4; c++) {
+                const int run = run_of(v, c);
+                const bool begin = halves ? !(c & 1) : c == 0, end = halves ? (c & 1) : c == 3;  // of the run
+                const bool anew = begin || (two && c == 2);
+                const uint32_t d_small = small_of(v), odd = (uint32_t)swapped(v, c);
+                const uint32_t d_both = odd ? d_small : d_small - (uint32_t)N, d_main = odd ? d_small + (uint32_t)N : d_both;
+                const uint64_t to_hi = odd ? b_tile : 0, to_lo = odd ? 0 : b_tile;
+                if (begin && run >= 2) ok = ok && mbar_wait(&d_empty[run & 1], (run / 2 - 1) & 1);
                 ok = ok && mbar_wait(&b_full[sb], b_phase);
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     const uint32_t st = WIDE ? (2 * c + h) & 3 : c, a = a0 + (WIDE ? st * 32 : st * 64 + h * 32);
-                    if (WIDE || h == 0) ok = ok && mbar_wait(&a_full[st], WIDE ? (uint32_t)(c >> 1) : odd);  // the stage's uses: WIDE 2 v and 2 v + 1, else v
+                    if (WIDE || h == 0) ok = ok && mbar_wait(&a_full[st], (uint32_t)(WIDE ? c >> 1 : v & 1));  // the stage's uses: WIDE 2 v and 2 v + 1, else v
                     tc_fence_after();
                     if (one && ok) {
                         const uint64_t bb = b_both + 4 * h;
-                        if (c == 0 && h == 0) {  // the unit's first: main starts anew
+                        if (anew && h == 0) {  // main
                             umma_f16_ts(d_main, a, bb + to_hi, id1, 0u);
-                            umma_f16_ts(d_small, a, bb + to_lo, id1, (uint32_t)(v > 0));
+                            umma_f16_ts(d_small, a, bb + to_lo, id1, (uint32_t)(v > (two ? 1 : 0) || c > 0));
                         } else {
                             umma_f16_ts(d_both, a, bb, id2, 1u);
                         }
@@ -534,7 +552,7 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
                         umma_f16_ts(d_small, a + 24, bb + 2 + to_hi, id1, 1u);
                         if (WIDE || h == 1) umma_commit(&a_empty[st]);
                         if (h == 1) umma_commit(&b_empty[sb]);
-                        if (h == 1 && c == 3) umma_commit(&d_full[odd]);
+                        if (h == 1 && end) umma_commit(&d_full[run & 1]);
                     }
                     __syncwarp();
                 }
@@ -543,29 +561,29 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
             }
         }
         for (int v = nu; kHasMin<TYPE> && v < nv && ok; v++) {  // the offsets: no low halves beside the high ones
-            const uint32_t odd = v & 1;
-            const uint32_t d_both = odd ? d_small : d_small - (uint32_t)N, d_main = odd ? d_small + (uint32_t)N : d_both;
             const int nc = chunks_of(v);
-            if (v >= 2) ok = mbar_wait(&d_empty[odd], ((v >> 1) - 1) & 1);
             for (int c = 0; c < nc && ok; c++) {
-                ok = mbar_wait(&b_full[sb], b_phase);
+                const uint32_t d_small = small_of(v), odd = (uint32_t)swapped(v, c);
+                const uint32_t d_both = odd ? d_small : d_small - (uint32_t)N, d_main = odd ? d_small + (uint32_t)N : d_both;
+                if (c == 0 && v >= 2) ok = mbar_wait(&d_empty[v & 1], (v / 2 - 1) & 1);  // these types' runs are units
+                ok = ok && mbar_wait(&b_full[sb], b_phase);
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     const uint32_t st = WIDE ? (2 * c + h) & 3 : c, a = a0 + (WIDE ? st * 32 : st * 64 + h * 32);
-                    if (WIDE || h == 0) ok = ok && mbar_wait(&a_full[st], WIDE ? (uint32_t)(c >> 1) : odd);
+                    if (WIDE || h == 0) ok = ok && mbar_wait(&a_full[st], (uint32_t)(WIDE ? c >> 1 : v & 1));
                     tc_fence_after();
                     if (one && ok) {
                         const uint64_t bb = b_both + 4 * h;
-                        if (c == 0 && h == 0) {
+                        if ((c == 0 || (two && c == 2)) && h == 0) {
                             umma_f16_ts(d_main, a, bb + (odd ? b_tile : 0), id1, 0u);
-                            umma_f16_ts(d_small, a, bb + (odd ? 0 : b_tile), id1, 1u);
+                            umma_f16_ts(d_small, a, bb + (odd ? 0 : b_tile), id1, (uint32_t)(v > (two ? 1 : 0) || c > 0));
                         } else {
                             umma_f16_ts(d_both, a, bb, id2, 1u);
                         }
                         umma_f16_ts(d_both, a + 8, bb + 2, id2, 1u);
                         if (WIDE || h == 1) umma_commit(&a_empty[st]);
                         if (h == 1) umma_commit(&b_empty[sb]);
-                        if (h == 1 && c == nc - 1) umma_commit(&d_full[odd]);
+                        if (h == 1 && c == nc - 1) umma_commit(&d_full[v & 1]);
                     }
                     __syncwarp();
                 }
@@ -588,14 +606,16 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
         const int own = WIDE ? max(0, min(32, N - 32 * g)) : N / 4, tbase = g * (WIDE ? 32 : N / 4);  // this thread's tokens of the tile
         auto wait_all = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); };
         float y[kOwn];
-        auto add_columns = [&](uint32_t col, uint32_t skip) {  // skip: a bit for each token that keeps what it has
-            col += lane_base + tbase;
+        constexpr uint32_t kNone = ~0u;
+        // skip: a bit for each token that keeps what it has; also: a second column, whose sums are added to the first's (up to 32 tokens, eight a thread)
+        auto add_columns = [&](uint32_t col, uint32_t also, uint32_t skip) {
+            const uint32_t base = lane_base + tbase;
             if constexpr (WIDE) {
 #pragma unroll
                 for (int t0 = 0; t0 < 32; t0 += 16)
                     if (t0 < own) {
                         uint32_t a[16];
-                        tmem_ld16(col + t0, a);
+                        tmem_ld16(base + col + t0, a);
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                         for (int t = 0; t < 16; t++) y[t0 + t] += (skip >> (t0 + t)) & 1u ? 0.f : __uint_as_float(a[t]);
@@ -604,8 +624,17 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
                 uint32_t a[16];
 #pragma unroll
                 for (int t0 = 0; t0 < 16; t0 += 4)
-                    if (t0 < own) tmem_ld4(col + t0, a + t0);
+                    if (t0 < own) tmem_ld4(base + col + t0, a + t0);
+                if (also != kNone) {
+#pragma unroll
+                    for (int t0 = 0; t0 < 8; t0 += 4)
+                        if (t0 < own) tmem_ld4(base + also + t0, a + 8 + t0);
+                }
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (also != kNone) {
+#pragma unroll
+                    for (int t = 0; t < 8; t++) a[t] = __float_as_uint(__uint_as_float(a[t]) + __uint_as_float(a[8 + t]));
+                }
 #pragma unroll
                 for (int t0 = 0; t0 < 16; t0 += 4)
                     if (t0 < own) {
@@ -614,15 +643,17 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
                     }
             }
         };
-        auto drain = [&](uint32_t w) {  // unit w
+        auto drain = [&](int q) {  // run q
             if (own <= 0) return;
-            ok = wait_all(&d_full[w & 1], (w >> 1) & 1);
+            const int place = q & 1;
+            ok = wait_all(&d_full[place], (q >> 1) & 1);
             if (!ok) return;
             tc_fence_after();
-            add_columns(w & 1 ? kColSmall + (uint32_t)N : kColSmall - (uint32_t)N, 0u);
+            if (two) add_columns((uint32_t)(3 * place * N), chunks_of(q) > 2 ? (uint32_t)((3 * place + 2) * N) : kNone, 0u);
+            else add_columns(place ? kColSmall + (uint32_t)N : kColSmall - (uint32_t)N, kNone, 0u);
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&d_empty[w & 1]);
+            if (lane == 0) mbar_arrive(&d_empty[place]);
         };
         int sr = 0;
         uint32_t raw_phase = 0, a_phase = 1;
@@ -668,8 +699,12 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&a_full[g]);
                     }
+                    if (halves && (jj || v > 0)) {  // the run before
+                        drain(2 * v + jj - 1);
+                        if (!ok) break;
+                    }
                 }
-                if (ok && v > 0) drain(v - 1);
+                if (!halves && ok && v > 0) drain(v - 1);
                 if (++sr == RS) { sr = 0; raw_phase ^= 1; }
             }
             for (int v = nu; kHasMin<TYPE> && v < nv && ok; v++) {
@@ -703,7 +738,7 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
                 }
                 if (ok) drain(v - 1);
             }
-            if (ok) drain(nv - 1);
+            if (ok) drain(run_of(nv - 1, 3));
             pdl_wait();
             const int t_first = tok0 + tbase, mine = ok ? min(own, tok_end - t_first) : 0;
             // a lane has one token's scale: a load beside each result's store would wait for it
@@ -711,10 +746,16 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
             // A negative scale: the token holds an infinity or a NaN (xprep_row).  `main` has its results' signs, W_lo * inf in `small` would be NaN
             // wherever W_lo is zero.
             const uint32_t wild = __ballot_sync(0xffffffffu, scale < 0.f);
-            if (ok && own > 0) add_columns(kColSmall, wild);  // complete: the last unit's d_full followed every product
+            if (ok && own > 0) {  // complete: the last unit's d_full followed every product
+                const uint32_t col = two ? (uint32_t)N : kColSmall, also = two && nv > 1 ? (uint32_t)(4 * N) : kNone;
+                if (wild) add_columns(col, also, wild);
+                else add_columns(col, also, 0u);
+            }
+            // what `main` lost on average (see the header)
+            const float back = down * (1.0f + (halves || two ? 0x1p-23f : 0x1p-22f));
             // two multiplications: the product of the powers may leave f32's range where the result does not
 #pragma unroll
-            for (int t = 0; t < kOwn; t++) y[t] = (y[t] * down) * fabsf(__shfl_sync(0xffffffffu, scale, t));
+            for (int t = 0; t < kOwn; t++) y[t] = (y[t] * back) * fabsf(__shfl_sync(0xffffffffu, scale, t));
             if (p.partial) {
                 float* dst = p.partial + ((size_t)(blockIdx.z * (pair ? 2 : 1) + mat) * p.T + t_first) * p.n + grow;
 #pragma unroll

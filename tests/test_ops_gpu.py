@@ -247,6 +247,25 @@ def test_many_token_product_beside_a_large_activation(gpu, typ, m):
     assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / bound).max()
 
 
+@pytest.mark.parametrize("typ,m,runs", [(2, 5, 8), (8, 5, 8), (14, 30, 8), (2, 70, 8), (8, 70, 8), (8, 40, 16), (14, 70, 16), (12, 70, 16), (13, 70, 16)])
+def test_many_token_product_is_centred(gpu, typ, m, runs):
+    """The tensor cores cut off toward zero: uncorrected, results are 1.6e-7 (eight additions to a run) or 2.8e-7 (sixteen) too small on average.  Corrected
+    to one or two 2^-23, 5e-8 of that is left; 1e-7 is asked for.  Around the mean an addition is off by a unit's length, 2^-23 or less of its run, divided by
+    the root of twelve: 1e-7 or 1.4e-7 for all of a run, 1e-7 more where up to 16 runs are added: twice that for types without offsets (those are large sums
+    of opposite signs)."""
+    k, n = 2048, 256
+    r = rng(typ + m + 3)
+    w, dense = scaled_blocks(gpu, typ, n, k, np.ones((n, 1)), r)
+    a = r.standard_normal((m, k)).astype(np.float32)
+    got = gpu.qmatmul(typ, a.ravel(), w, m, k, n).reshape(m, n).astype(np.float64)
+    want = a.astype(np.float64) @ dense.T
+    off = got - want
+    mean = (off * want).sum() / (want * want).sum()
+    assert abs(mean) <= 1e-7, mean
+    if typ not in (12, 13):
+        assert np.linalg.norm(off) <= 2 * np.sqrt(runs / 12 + 0.7) * 2.0 ** -23 * np.linalg.norm(want), np.linalg.norm(off) / np.linalg.norm(want)
+
+
 def test_qmatmul_linearity_full_size(gpu, oracle):
     """7B-shape matrices: A(x+y) = Ax + Ay and a sample of rows against the oracle."""
     from leafcutterllm_b200 import synth
