@@ -22,8 +22,11 @@
 // Emptying every 128 costs 8 % of a 7B prompt, where the tensor pipe is the bound, and 0.7 % of the short prompts of a small Q4_0 / Q8_0 model,
 // whose matrix-vector kernels add in f32: those have it.  Up to 32 tokens tensor memory has room for two sums of 128 elements each, at no cost.
 //
-// Q4_K / Q5_K weights are d * sc * q - dmin * m: the first part is the weight above, the second joins as more k: -dmin * m (17
-// bits, two f16) of a sub-block against the sum of the activations over it, 16 values per 256-element unit, behind the last unit.
+// Q4_K / Q5_K weights are d * sc * q - dmin * m = d * sc * (q - c) + (c * d * sc - dmin * m), c the middle of q's range (8 or 16): the first part is the
+// weight above, the second joins as more k: two f16 of a sub-block against the sum of the activations over it, 16 values per 256-element unit, behind
+// the last unit.  About the middle, because with q itself both parts are large and of opposite signs, and the cut-off sums' error with them:
+// 7.0e-7 of the result for normal activations and 7.3e-5 for positive ones at k = 2048, 2.3e-7 and 1.4e-6 about the middle (qgemm_umma.cu's kernel,
+// integers and a drain per unit: 5.5e-7 and 3.2e-5).
 //
 // One CTA owns 128 weight rows (the M of tcgen05.mma; for gate/up 64 rows of each, so that SiLU(gate) * up happens here) and up to 128
 // tokens, and walks k in chunks of 32 elements:
@@ -177,8 +180,9 @@ __device__ __forceinline__ void split_product(uint32_t s, uint32_t q, uint32_t& 
     lo = h2_fma(s, q, h2_neg(hi));
 }
 // Elements 32 j ... 32 j + 31 of a row's unit times `up`, as f16 pairs: column c holds elements 2 c and 2 c + 1.
-// Q4_K (mod.rs:66-98): sub-block j has the low (even j) or high nibbles of bytes 32 (j / 2) ... under scale sc[j];
-// (1024 + q) sc - 1024 sc is one fused multiply-add with the exact result sc q <= 945.  Q5_K (mod.rs:101-142): a fifth bit, <= 1953.
+// Q4_K (mod.rs:66-98): sub-block j has the low (even j) or high nibbles of bytes 32 (j / 2) ... under scale sc[j]; the nibbles are brought up to
+// 16 q, and (1024 + 16 q) (sc / 16) - 1152 (sc / 16) is one fused multiply-add with the exact result sc (q - 8): 1152 = 9 * 2^7 and a scale of six bits
+// make a constant that f16 holds, 1032 would not.  Q5_K (mod.rs:101-142): a fifth bit; 8 q and 1152 (sc / 8) likewise.
 struct UnitHead { float d; uint32_t sc_lo, sc_hi; };  // d times `up`, the eight scales (of the types that have them)
 template <uint32_t TYPE>
 __device__ __forceinline__ UnitHead load_head(const unsigned char* rp, float up) {
@@ -196,27 +200,25 @@ __device__ __forceinline__ UnitHead load_head(const unsigned char* rp, float up)
 template <uint32_t TYPE>
 __device__ __forceinline__ void unpack_chunk(const unsigned char* rp, const UnitHead& head, int j, float up, uint32_t (&hi)[16], uint32_t (&lo)[16]) {
     if constexpr (kHasMin<TYPE>) {
-        // high nibbles stay where they are: (1024 + 16 q) (sc / 16) - 1024 (sc / 16)
-        const float sub = (float)(((j < 4 ? head.sc_lo : head.sc_hi) >> (8 * (j & 3))) & 0xFFu);
         constexpr bool fifth = TYPE == LC_TYPE_Q5_K;
-        const float fs = (j & 1) && !fifth ? sub * 0.0625f : sub;
-        const uint32_t mask = (j & 1) && !fifth ? 0xF0F0F0F0u : 0x0F0F0F0Fu;
-        const uint32_t d = h2_pair(head.d), sc = h2_pair(fs), bias = h2_pair(-1024.0f * fs);
-        const uint4* q = reinterpret_cast<const uint4*>(rp + (TYPE == LC_TYPE_Q5_K ? 48 : 16) + 32 * (j >> 1));
-        const int sh = (j & 1) * 4;
+        const float fs = (float)(((j < 4 ? head.sc_lo : head.sc_hi) >> (8 * (j & 3))) & 0xFFu) * (fifth ? 0.125f : 0.0625f);
+        const uint32_t d = h2_pair(head.d), sc = h2_pair(fs), bias = h2_pair(-1152.0f * fs);
+        const uint4* q = reinterpret_cast<const uint4*>(rp + (fifth ? 48 : 16) + 32 * (j >> 1));
+        // the nibbles to bits 4 - 7 of their bytes, with a fifth bit to 3 - 6 (what the rotation brings from other bytes is masked out)
+        const uint32_t rot = fifth ? (j & 1 ? 31 : 3) : (j & 1 ? 0 : 4);
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const uint4 v = q[h];
             const uint32_t vv[4] = {v.x, v.y, v.z, v.w};
             uint32_t hb[4] = {0u, 0u, 0u, 0u};
-            if constexpr (TYPE == LC_TYPE_Q5_K) {
+            if constexpr (fifth) {
                 const uint4 hq = *reinterpret_cast<const uint4*>(rp + 16 + 16 * h);
                 hb[0] = hq.x; hb[1] = hq.y; hb[2] = hq.z; hb[3] = hq.w;
             }
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                uint32_t b = (fifth ? vv[i] >> sh : vv[i]) & mask;
-                if constexpr (TYPE == LC_TYPE_Q5_K) b |= ((hb[i] >> j) & 0x01010101u) << 4;
+                uint32_t b = __funnelshift_l(vv[i], vv[i], rot) & (fifth ? 0x78787878u : 0xF0F0F0F0u);
+                if constexpr (fifth) b |= (hb[i] << (7 - j)) & 0x80808080u;
                 const int c = h * 8 + i * 2;
                 split_product(d, h2_fma(bias_pair(b, 0), sc, bias), hi[c], lo[c]);
                 split_product(d, h2_fma(bias_pair(b, 1), sc, bias), hi[c + 1], lo[c + 1]);
@@ -281,20 +283,21 @@ __device__ __forceinline__ void unpack_chunk(const unsigned char* rp, const Unit
         }
     }
 }
-// The offset operand of a unit: p[i] = -dmin * m[i] has at most 17 significant bits, so hi = f16(p) and lo = f16(p - hi)
-// carry it exactly.  Columns 0-3: the eight hi as pairs (k' = 0..7), columns 4-7: the eight lo (k' = 8..15); the sums tile holds
-// each sub-block sum at k' and k' + 8.
+// The offset operand of a unit: p[i] = c * d * sc[i] - dmin * m[i], hi = f16(p) and lo = f16(p - hi).  Columns 0-3: the eight hi
+// as pairs (k' = 0..7), columns 4-7: the eight lo (k' = 8..15); the sums tile holds each sub-block sum at k' and k' + 8.
+template <uint32_t TYPE>
 __device__ __forceinline__ void unpack_mins(uint4 w, float up, uint32_t* col) {
     uint32_t sc_lo, sc_hi, mn_lo, mn_hi;
     unpack_scales_k4(w.y, w.z, w.w, &sc_lo, &sc_hi, &mn_lo, &mn_hi);
-    const float dmin = h2f((uint16_t)(w.x >> 16)) * up;
+    const float dmin = h2f((uint16_t)(w.x >> 16)) * up, mid = h2f((uint16_t)(w.x & 0xFFFFu)) * up * (TYPE == LC_TYPE_Q5_K ? 16.f : 8.f);
 #pragma unroll
     for (int j2 = 0; j2 < 4; j2++) {
         __half hi[2], lo[2];
 #pragma unroll
         for (int e = 0; e < 2; e++) {
             const int i = 2 * j2 + e;
-            const float pr = -dmin * (float)(((i < 4 ? mn_lo : mn_hi) >> (8 * (i & 3))) & 0xFFu);
+            const uint32_t sh = 8 * (i & 3), sc = ((i < 4 ? sc_lo : sc_hi) >> sh) & 0xFFu, mn = ((i < 4 ? mn_lo : mn_hi) >> sh) & 0xFFu;
+            const float pr = fmaf(mid, (float)sc, -dmin * (float)mn);  // both products are exact, so this rounds once
             hi[e] = __float2half_rn(pr);
             lo[e] = __float2half_rn(pr - __half2float(hi[e]));
         }
@@ -326,7 +329,7 @@ __global__ void __launch_bounds__(256) row_scale_kernel(uint32_t typ, const unsi
             const float sm = (float)max(max(s & 0xFFu, (s >> 8) & 0xFFu), max((s >> 16) & 0xFFu, s >> 24));
             const float mm = (float)max(max(m & 0xFFu, (m >> 8) & 0xFFu), max((m >> 16) & 0xFFu, m >> 24));
             const float d = fabsf(h2f((uint16_t)(h.x & 0xFFFFu))), dm = fabsf(h2f((uint16_t)(h.x >> 16)));
-            v = fmaxf(d * fmaxf(sm, 1.f) * (typ == LC_TYPE_Q4_K ? 15.f : 31.f), dm * fmaxf(mm, 1.f));
+            v = d * fmaxf(sm, 1.f) * (typ == LC_TYPE_Q4_K ? 8.f : 16.f) + dm * fmaxf(mm, 1.f);  // not below either part of a weight
         } else if (typ == LC_TYPE_Q4_0) {
             v = 8.f * fabsf(h2f((uint16_t)f16_at(rp + (size_t)b * 18)));
         } else if (typ == LC_TYPE_Q8_0) {
@@ -726,7 +729,7 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
                     for (int e = 0; e < 2; e++) {
                         uint4 hd = make_uint4(0u, 0u, 0u, 0u);
                         if (live && u + e < u_begin + nu) hd = *reinterpret_cast<const uint4*>(wrow + (size_t)(u + e) * kPitch);
-                        unpack_mins(hd, up, col + 8 * e);
+                        unpack_mins<TYPE>(hd, up, col + 8 * e);
                     }
                     tmem_st16(a_stage + (WIDE ? 0 : jj * 32), col);
                     if (WIDE || jj == 1) {
