@@ -5,8 +5,9 @@
 //   y[t, r] = sum_k x[t, k] * w[r, k]
 //
 // Weights stay as raw GGUF blocks in HBM; nothing dequantised is ever written back.  Both factors enter the tensor cores as sums
-// of two f16: a weight, times a power of two of its row, is hi + lo with 22 bits (every type but Q6_K has at most 21, so it is
-// exact), an activation, times a power of two of its token, is hi + lo with 22 bits.  Three of the four products count
+// of two f16: a weight, times a power of two of its row, is hi + lo with 22 bits and nothing below 2^-24 (every type but Q6_K has at most 21 bits, so
+// it is exact unless it is smaller than 2^-17 of its row's largest, and off by 2^-38 of that at most), an activation, times a power of two
+// of its token, is hi + lo with 22 bits.  Three of the four products count
 // (lo * lo is 2^-22 of the result): per 16 elements of k
 //
 //   main  += W_hi * X_hi                       one tcgen05.mma with N = 2 * tokens over [X_hi | X_lo] forms the first two,
@@ -148,11 +149,6 @@ __device__ __forceinline__ uint32_t h2_mul(uint32_t a, uint32_t b) {
     asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
     return d;
 }
-__device__ __forceinline__ uint32_t h2_add(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-}
 __device__ __forceinline__ uint32_t h2_neg(uint32_t a) { return a ^ 0x80008000u; }
 __device__ __forceinline__ uint32_t h2_pair(float v) {  // (v, v) as f16x2
     const __half2 h = __float2half2_rn(v);
@@ -179,11 +175,13 @@ __device__ __forceinline__ void split_product(uint32_t s, uint32_t q, uint32_t& 
     hi = h2_mul(s, q);
     lo = h2_fma(s, q, h2_neg(hi));
 }
-// Elements 32 j ... 32 j + 31 of a row's unit times `up`, as f16 pairs: column c holds elements 2 c and 2 c + 1.
+// Elements 32 j ... 32 j + 31 of a row's unit times `up`, as f16 pairs: column c holds elements 2 c and 2 c + 1.  The integer's factor is a power of two
+// that brings it to about 1 and the scale's the inverse: the scale, rounded to f16 before the product, then keeps its bits down to 2^-28 of the row's
+// largest (with whole integers to 2^-18 in Q4_K, and an error there that counted 945 times).
 // Q4_K (mod.rs:66-98): sub-block j has the low (even j) or high nibbles of bytes 32 (j / 2) ... under scale sc[j]; the nibbles are brought up to
-// 16 q, and (1024 + 16 q) (sc / 16) - 1152 (sc / 16) is one fused multiply-add with the exact result sc (q - 8): 1152 = 9 * 2^7 and a scale of six bits
-// make a constant that f16 holds, 1032 would not.  Q5_K (mod.rs:101-142): a fifth bit; 8 q and 1152 (sc / 8) likewise.
-struct UnitHead { float d; uint32_t sc_lo, sc_hi; };  // d times `up`, the eight scales (of the types that have them)
+// 16 q, and (1024 + 16 q) (sc / 2^14) - 1152 (sc / 2^14) is one fused multiply-add with the exact result sc (q - 8) / 2^10: 1152 = 9 * 2^7 and a scale of
+// six bits make a constant that f16 holds, 1032 would not.  Q5_K (mod.rs:101-142): a fifth bit; 8 q and sc / 2^13 likewise.
+struct UnitHead { float d; uint32_t sc_lo, sc_hi; };  // d times `up` and the integer's factor, the eight scales (of the types that have them)
 template <uint32_t TYPE>
 __device__ __forceinline__ UnitHead load_head(const unsigned char* rp, float up) {
     UnitHead h{0.f, 0u, 0u};
@@ -191,9 +189,9 @@ __device__ __forceinline__ UnitHead load_head(const unsigned char* rp, float up)
         const uint4 w = *reinterpret_cast<const uint4*>(rp);  // d, dmin, 12 scale bytes
         uint32_t mn_lo, mn_hi;
         unpack_scales_k4(w.y, w.z, w.w, &h.sc_lo, &h.sc_hi, &mn_lo, &mn_hi);
-        h.d = h2f((uint16_t)(w.x & 0xFFFFu)) * up;
+        h.d = h2f((uint16_t)(w.x & 0xFFFFu)) * up * 1024.f;
     } else if constexpr (TYPE == LC_TYPE_Q6_K) {
-        h.d = h2f((uint16_t)f16_at(rp + 208)) * up;
+        h.d = h2f((uint16_t)f16_at(rp + 208)) * up * 32.f;
     }
     return h;
 }
@@ -201,7 +199,7 @@ template <uint32_t TYPE>
 __device__ __forceinline__ void unpack_chunk(const unsigned char* rp, const UnitHead& head, int j, float up, uint32_t (&hi)[16], uint32_t (&lo)[16]) {
     if constexpr (kHasMin<TYPE>) {
         constexpr bool fifth = TYPE == LC_TYPE_Q5_K;
-        const float fs = (float)(((j < 4 ? head.sc_lo : head.sc_hi) >> (8 * (j & 3))) & 0xFFu) * (fifth ? 0.125f : 0.0625f);
+        const float fs = (float)(((j < 4 ? head.sc_lo : head.sc_hi) >> (8 * (j & 3))) & 0xFFu) * (fifth ? 0x1p-13f : 0x1p-14f);
         const uint32_t d = h2_pair(head.d), sc = h2_pair(fs), bias = h2_pair(-1152.0f * fs);
         const uint4* q = reinterpret_cast<const uint4*>(rp + (fifth ? 48 : 16) + 32 * (j >> 1));
         // the nibbles to bits 4 - 7 of their bytes, with a fifth bit to 3 - 6 (what the rotation brings from other bytes is masked out)
@@ -230,15 +228,15 @@ __device__ __forceinline__ void unpack_chunk(const unsigned char* rp, const Unit
         const uint4 a = p[0], b = p[1];  // j <= 7: the block ends within two pieces (at most byte 14 + 18 of them)
         uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}, o[5];
         shift_words(w, at & 15, o);
-        const uint32_t d = h2_pair(h2f((uint16_t)(o[0] & 0xFFFFu)) * up), m8 = 0xE408E408u;  // -1032
+        const uint32_t d = h2_pair(h2f((uint16_t)(o[0] & 0xFFFFu)) * up * 8.f), f = 0x30003000u, m = 0xD808D808u;  // 2^-3; -129 = -1032 / 8
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const uint32_t v = __funnelshift_r(o[i], o[i + 1], 16);
             const uint32_t bl = v & 0x0F0F0F0Fu, bh = (v >> 4) & 0x0F0F0F0Fu;
-            split_product(d, h2_add(bias_pair(bl, 0), m8), hi[2 * i], lo[2 * i]);
-            split_product(d, h2_add(bias_pair(bl, 1), m8), hi[2 * i + 1], lo[2 * i + 1]);
-            split_product(d, h2_add(bias_pair(bh, 0), m8), hi[8 + 2 * i], lo[8 + 2 * i]);
-            split_product(d, h2_add(bias_pair(bh, 1), m8), hi[9 + 2 * i], lo[9 + 2 * i]);
+            split_product(d, h2_fma(bias_pair(bl, 0), f, m), hi[2 * i], lo[2 * i]);
+            split_product(d, h2_fma(bias_pair(bl, 1), f, m), hi[2 * i + 1], lo[2 * i + 1]);
+            split_product(d, h2_fma(bias_pair(bh, 0), f, m), hi[8 + 2 * i], lo[8 + 2 * i]);
+            split_product(d, h2_fma(bias_pair(bh, 1), f, m), hi[9 + 2 * i], lo[9 + 2 * i]);
         }
     } else if constexpr (TYPE == LC_TYPE_Q8_0) {  // mod.rs:37-51: 34 bytes: scale, 32 signed bytes
         const int at = 34 * j;
@@ -246,12 +244,12 @@ __device__ __forceinline__ void unpack_chunk(const unsigned char* rp, const Unit
         const uint4 a = p[0], b = p[1], e = p[2];  // ends at most at byte 14 + 34 of the three pieces
         uint32_t w[12] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, e.x, e.y, e.z, e.w}, o[9];
         shift_words(w, at & 15, o);
-        const uint32_t d = h2_pair(h2f((uint16_t)(o[0] & 0xFFFFu)) * up), m = 0xE480E480u;  // -1152 = -(1024 + 128)
+        const uint32_t d = h2_pair(h2f((uint16_t)(o[0] & 0xFFFFu)) * up * 128.f), f = 0x20002000u, m = 0xC880C880u;  // 2^-7; -9 = -(1024 + 128) / 128
 #pragma unroll
         for (int i = 0; i < 8; i++) {
             const uint32_t v = __funnelshift_r(o[i], o[i + 1], 16) ^ 0x80808080u;  // byte + 128
-            split_product(d, h2_add(bias_pair(v, 0), m), hi[2 * i], lo[2 * i]);
-            split_product(d, h2_add(bias_pair(v, 1), m), hi[2 * i + 1], lo[2 * i + 1]);
+            split_product(d, h2_fma(bias_pair(v, 0), f, m), hi[2 * i], lo[2 * i]);
+            split_product(d, h2_fma(bias_pair(v, 1), f, m), hi[2 * i + 1], lo[2 * i + 1]);
         }
     } else {  // Q6_K, mod.rs:145-180; rp: the block's first byte, on an even address
         const int n = j >> 2, quad = j & 3;
@@ -275,7 +273,7 @@ __device__ __forceinline__ void unpack_chunk(const unsigned char* rp, const Unit
             const uint32_t b = ((vl >> (4 * (quad >> 1))) & 0x0F0F0F0Fu) | (((vh >> (2 * quad)) & 0x03030303u) << 4);
 #pragma unroll
             for (int k = 0; k < 2; k++) {
-                const uint32_t q = h2_add(bias_pair(b, k), 0xE420E420u);  // -1056 = -(1024 + 32)
+                const uint32_t q = h2_fma(bias_pair(b, k), 0x28002800u, 0xD020D020u);  // 2^-5; -33 = -(1024 + 32) / 32
                 const int c = 2 * i + k;
                 split_product(sh[i >> 2], q, hi[c], lo[c]);
                 lo[c] = h2_fma(sl[i >> 2], q, lo[c]);
@@ -308,8 +306,8 @@ __device__ __forceinline__ void unpack_mins(uint4 w, float up, uint32_t* col) {
 }
 
 // ---- row scales ----------------------------------------------------------------------------------------------------------
-// A power of two per row that brings its weights up to 2^13 ... 2^14: the low half of a weight then keeps its bits above
-// 2^-24, f16's smallest step, unless it is 2^-17 of the row's largest.  One warp per row; down[r] = 2^-s.
+// A power of two per row that brings its weights up to 2^13 ... 2^14 (Q4_K and Q5_K rows whose largest scales belong to blocks of small sc: less): the low
+// half of a weight then keeps its bits above 2^-24, f16's smallest step, unless it is 2^-17 of the row's largest.  One warp per row; down[r] = 2^-s.
 __global__ void __launch_bounds__(256) row_scale_kernel(uint32_t typ, const unsigned char* __restrict__ w, size_t row_bytes, int n, int k, float* __restrict__ down) {
     pdl_wait();
     pdl_launch_dependents();
@@ -329,7 +327,8 @@ __global__ void __launch_bounds__(256) row_scale_kernel(uint32_t typ, const unsi
             const float sm = (float)max(max(s & 0xFFu, (s >> 8) & 0xFFu), max((s >> 16) & 0xFFu, s >> 24));
             const float mm = (float)max(max(m & 0xFFu, (m >> 8) & 0xFFu), max((m >> 16) & 0xFFu, m >> 24));
             const float d = fabsf(h2f((uint16_t)(h.x & 0xFFFFu))), dm = fabsf(h2f((uint16_t)(h.x >> 16)));
-            v = d * fmaxf(sm, 1.f) * (typ == LC_TYPE_Q4_K ? 8.f : 16.f) + dm * fmaxf(mm, 1.f);  // not below either part of a weight
+            v = d * fmaxf(sm, 1.f) * (typ == LC_TYPE_Q4_K ? 8.f : 16.f) + dm * fmaxf(mm, 1.f);  // not below either part of a weight,
+            v = fmaxf(v, 512.f * d);                                                            // and 2^10 d comes below 2^15
         } else if (typ == LC_TYPE_Q4_0) {
             v = 8.f * fabsf(h2f((uint16_t)f16_at(rp + (size_t)b * 18)));
         } else if (typ == LC_TYPE_Q8_0) {

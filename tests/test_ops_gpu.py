@@ -280,6 +280,25 @@ def test_many_token_product_of_positive_activations(gpu, typ, k):
     assert np.linalg.norm(got - want) <= 4e-7 * (1 + 0.16 * np.sqrt(k)) * np.linalg.norm(want), np.linalg.norm(got - want) / np.linalg.norm(want)
 
 
+@pytest.mark.parametrize("m", [5, 70])
+@pytest.mark.parametrize("typ", [2, 8, 12, 13, 14])
+def test_many_token_product_of_small_blocks_beside_large_ones(gpu, typ, m):
+    """Rows in which every other block is 2^20 times smaller, and no activations but over those: a weight is off by 2^-25 beside a row's largest of
+    2^13 and more, i.e. by 2^-38 of that at most (uniformly, so results by its share of the activations' root of squares: four times that, seven
+    deviations, is asked for), beside what every result is off by."""
+    k, n = 2048, 70
+    r = rng(typ + m + 4)
+    be = gpu.QUANT_GEOMETRY[typ][0]
+    small = np.arange(k // be) % 2 == 1
+    # block scales of 2^6 ... 2^7 and 2^-14 ... 2^-13, where f16 still has all its bits
+    w, dense = scaled_blocks(gpu, typ, n, k, {2: 8, 8: 128, 12: 945, 13: 1953, 14: 4064}[typ] * np.exp2(r.uniform(6, 7, (n, k // be)) - 20.0 * small), r)
+    a = (r.standard_normal((m, k)) * np.repeat(small, be)).astype(np.float32)
+    got = gpu.qmatmul(typ, a.ravel(), w, m, k, n).reshape(m, n)
+    want = a.astype(np.float64) @ dense.T
+    bound = 2e-5 * np.sqrt((a.astype(np.float64) ** 2) @ (dense.T ** 2)) + 4 * 2.0 ** -38 * np.linalg.norm(a.astype(np.float64), axis=1)[:, None] * np.abs(dense).max(1)
+    assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / bound).max()
+
+
 def test_qmatmul_linearity_full_size(gpu, oracle):
     """7B-shape matrices: A(x+y) = Ax + Ay and a sample of rows against the oracle."""
     from leafcutterllm_b200 import synth
