@@ -143,8 +143,11 @@ int32_t launch_row_scales(const QWeight& w, float* down, cudaStream_t s);
 // true when launch_qgemm implements these arguments for T tokens (T at least LC_GEMM_MIN_TOKENS, default 5: up to four tokens the
 // matrix-vector kernels are faster, from five on they would run their 8-token form, which this product beats)
 bool qgemm_applies(const GemvArgs& a, int T, const GemmWorkspace& ws);
+// true when the summing kernel, which takes four outputs a thread, can write this product's result: k may be split
+bool qgemm_sum_ok(const GemvArgs& a);
 // a.m = number of tokens; queues two kernels (activation preparation, product), three when k is split (reduction)
-int32_t launch_qgemm(const GemvArgs& a, GemmWorkspace& ws, cudaStream_t s, int* launches = nullptr);// Tensor map over f16 activations [2 halves][rows][k] with a box of 64 elements x box_rows rows x both halves, 128-byte swizzle.
+int32_t launch_qgemm(const GemvArgs& a, GemmWorkspace& ws, cudaStream_t s, int* launches = nullptr);
+// Tensor map over f16 activations [2 halves][rows][k] with a box of 64 elements x box_rows rows x both halves, 128-byte swizzle.
 bool make_act_tmap(void* out128, const void* base, uint64_t k, uint64_t rows, uint32_t box_rows);
 bool make_act_tmap_chunks(void* out128, const void* base, uint64_t k, uint64_t rows, uint32_t box_rows, uint32_t box_chunks);
 // ---- qgemm_split.cu ----

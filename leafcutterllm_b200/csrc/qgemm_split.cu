@@ -871,7 +871,7 @@ int32_t launch_type(const GemvArgs& a, const GemmWorkspace& ws, GemmParams& p, c
     double best = 0;
     for (int c = 1; c <= (group ? 1 : std::min(8, nquads)); c++) {
         const size_t bytes = (size_t)c * nmat * p.T * p.n * sizeof(float);
-        if (c > 1 && (bytes > ws.partial_bytes || p.n % 4 != 0)) break;
+        if (c > 1 && (bytes > ws.partial_bytes || !qgemm_sum_ok(a))) break;
         const long waves = ((long)tiles * ttiles * c + sm_count() - 1) / sm_count();
         const double cost = (double)waves * (std::min((nquads + c - 1) / c * 4, p.k / kUnitElems) * unit_cycles(g.N) + 6000) + (c > 1 ? 4000 + 2.0 * bytes / 3000 : 0);
         if (c == 1 || cost < best) { best = cost; ks = c; }

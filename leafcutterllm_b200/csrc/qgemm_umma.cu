@@ -901,6 +901,10 @@ bool qgemm_applies(const GemvArgs& a, int T, const GemmWorkspace& ws) {
     return true;
 }
 
+bool qgemm_sum_ok(const GemvArgs& a) {
+    return a.w->n % 4 == 0 && (uintptr_t)a.out % 16 == 0 && (a.epi != EPI_ADD_RESIDUAL || (uintptr_t)a.residual % 16 == 0);
+}
+
 // The product of prepared activations through the kernel above.  *slices > 0: the shares (or gate's and up's sums) are in ws.partial.
 static int32_t launch_qgemm_tile(const GemvArgs& a, GemmWorkspace& ws, int* slices, cudaStream_t s) {
     const int T = a.m, K = a.w->k, n = a.w->n;
@@ -946,7 +950,7 @@ static int32_t launch_qgemm_tile(const GemvArgs& a, GemmWorkspace& ws, int* slic
         long best = -1;
         for (int c = 1; c <= std::min(8, nquads); c++) {
             if (c > 1 && (size_t)c * nmat * T * n * sizeof(float) > ws.partial_bytes) break;
-            if (c > 1 && (n % 4 != 0 || T > 2 * kMaxTok)) break;
+            if (c > 1 && (!qgemm_sum_ok(a) || T > 2 * kMaxTok)) break;
             const long waves = ((long)tiles * nmat * ttiles * c + sms - 1) / sms;
             const long cost = waves * (((nquads + c - 1) / c) * 4 + 4) + (c > 1 ? 3 : 0);
             if (best < 0 || cost < best) { best = cost; ks = c; }
@@ -959,10 +963,10 @@ static int32_t launch_qgemm_tile(const GemvArgs& a, GemmWorkspace& ws, int* slic
             snprintf(name, sizeof(name), "LC_GEMM_KS_%d_%d", n, K);
             if (const char* v = getenv(name)) f = atoi(v);
         }
-        if (f > 0 && f <= nquads && (f == 1 || (n % 4 == 0 && (size_t)f * nmat * T * n * sizeof(float) <= ws.partial_bytes))) ks = f;
+        if (f > 0 && f <= nquads && (f == 1 || (qgemm_sum_ok(a) && (size_t)f * nmat * T * n * sizeof(float) <= ws.partial_bytes))) ks = f;
     }
     const bool summed = ks > 1 || nmat == 2;
-    if (summed) LC_CHECK((size_t)ks * nmat * T * n * sizeof(float) <= ws.partial_bytes && n % 4 == 0, LC_ERR_UNSUPPORTED, "qgemm: sums buffer too small");
+    if (summed) LC_CHECK((size_t)ks * nmat * T * n * sizeof(float) <= ws.partial_bytes && qgemm_sum_ok(a), LC_ERR_UNSUPPORTED, "qgemm: sums buffer too small or output unaligned");
     p.ksplit = ks;
     p.tiles = tiles; p.nmat = nmat;
     p.partial = summed ? ws.partial : nullptr;

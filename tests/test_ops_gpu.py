@@ -299,6 +299,34 @@ def test_many_token_product_of_small_blocks_beside_large_ones(gpu, typ, m):
     assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / bound).max()
 
 
+@pytest.mark.parametrize("m", [5, 70])
+@pytest.mark.parametrize("typ", [2, 8, 12, 13, 14])
+def test_many_token_product_into_an_unaligned_output(gpu, typ, m):
+    """Two row tiles over a long k, which several CTAs share where the summing kernel may write four results at once: an output on a word boundary takes the
+    way without it, to the same results but for the order of the sums."""
+    import ctypes as C
+    lib, chk = gpu.load(), gpu._capi.check
+    k, n = 4096, 256
+    r = rng(typ + m + 5)
+    w, dense = scaled_blocks(gpu, typ, n, k, np.ones((n, 1)), r)
+    a = r.standard_normal((m, k)).astype(np.float32)
+    ptr = [C.c_void_p() for _ in range(3)]
+    for p, size in zip(ptr, (a.nbytes, w.nbytes, 4 * m * n + 16)):
+        chk(lib.lc_dev_alloc(size, C.byref(p)))
+    chk(lib.lc_dev_upload(ptr[0], a.ctypes.data_as(C.c_void_p), a.nbytes))
+    chk(lib.lc_dev_upload(ptr[1], w.ctypes.data_as(C.c_void_p), w.nbytes))
+    want = a.astype(np.float64) @ dense.T
+    bound = 2e-5 * np.sqrt((a.astype(np.float64) ** 2) @ (dense.T ** 2))
+    for off in (0, 4, 8):
+        out = C.c_void_p(ptr[2].value + off)
+        got = np.empty((m, n), np.float32)
+        chk(lib.lc_qmatmul_dev(typ, ptr[0], ptr[1], m, k, n, out))
+        chk(lib.lc_dev_download(got.ctypes.data_as(C.c_void_p), out, got.nbytes))
+        assert (np.abs(got - want) <= bound).all(), (off, (np.abs(got - want) / bound).max())
+    for p in ptr:
+        lib.lc_dev_free(p)
+
+
 def test_qmatmul_linearity_full_size(gpu, oracle):
     """7B-shape matrices: A(x+y) = Ax + Ay and a sample of rows against the oracle."""
     from leafcutterllm_b200 import synth
