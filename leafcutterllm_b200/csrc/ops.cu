@@ -438,7 +438,7 @@ static int32_t qmatmul_rows(const QWeight& w, const float* a_dev, size_t m, floa
     probe.x = a_dev;
     probe.out = c_dev;
     const int chunk = 512;
-    if (qgemm_split_weight_ok(w) && m >= 5) {
+    if (qgemm_split_weight_ok(w) && m >= 5 && qgemm_row_fits(w.k)) {
         if (!ws.xh || ws.k_max < w.k) {
             qgemm_workspace_free(&ws);
             LC_TRY(qgemm_workspace_alloc(&ws, chunk, w.k));

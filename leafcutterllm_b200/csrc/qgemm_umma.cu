@@ -893,10 +893,11 @@ static int gemm_min_tokens() {
     static const int v = getenv("LC_GEMM_MIN_TOKENS") ? atoi(getenv("LC_GEMM_MIN_TOKENS")) : 5;
     return v;
 }
+bool qgemm_row_fits(int k) { return (size_t)k * sizeof(float) + 64 * sizeof(float) <= kMaxSmem; }  // 58,048 elements
 bool qgemm_applies(const GemvArgs& a, int T, const GemmWorkspace& ws) {
     if (!a.w || !ws.xh || a.group || !qgemm_split_weight_ok(*a.w)) return false;
     if (a.epi == EPI_SILU_MUL && (!a.w2 || a.w2->typ != a.w->typ || !qgemm_split_weight_ok(*a.w2))) return false;
-    if (T < gemm_min_tokens() || T > ws.t_cap || a.w->k > ws.k_max) return false;
+    if (T < gemm_min_tokens() || T > ws.t_cap || a.w->k > ws.k_max || !qgemm_row_fits(a.w->k)) return false;
     if (((uintptr_t)a.x % 16) != 0 || (a.norm_w && ((uintptr_t)a.norm_w % 16) != 0)) return false;
     return true;
 }
@@ -1022,7 +1023,7 @@ int32_t launch_qgemm(const GemvArgs& a, GemmWorkspace& ws, cudaStream_t s, int* 
     if (slices) {
         count += 1;
         const size_t plane = (size_t)T * n;
-        if (a.prep_next && n % kUnitElems == 0 && n <= ws.k_max) {
+        if (a.prep_next && n % kUnitElems == 0 && n <= ws.k_max && qgemm_row_fits(n)) {
             // one CTA per token sums the shares and prepares the row for the next product, whose k is this n
             const size_t rsmem = (size_t)n * sizeof(float);
             if (rsmem > 48 * 1024) LC_CUDA(ensure_smem_limit((const void*)qgemm_reduce_prep_kernel, rsmem));
@@ -1041,7 +1042,7 @@ int32_t launch_qgemm(const GemvArgs& a, GemmWorkspace& ws, cudaStream_t s, int* 
 
 int32_t launch_qgemm_group(const GemvArgs& a, GemmWorkspace& ws, const GemmGroup& group, const int32_t* rows, int div, cudaStream_t s, int* launches) {
     const int K = a.w->k;
-    LC_CHECK(a.m >= 1 && a.m <= ws.t_cap && K <= ws.k_max && qgemm_split_weight_ok(*a.w) && group.offsets && group.n_experts >= 1 && group.typical >= 1,
+    LC_CHECK(a.m >= 1 && a.m <= ws.t_cap && K <= ws.k_max && qgemm_row_fits(K) && qgemm_split_weight_ok(*a.w) && group.offsets && group.n_experts >= 1 && group.typical >= 1,
              LC_ERR_INVALID, "grouped qgemm: %d rows of %d elements do not fit", a.m, K);
     ws.prep_x = nullptr;
     const size_t smem = (size_t)K * sizeof(float);

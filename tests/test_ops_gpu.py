@@ -327,6 +327,21 @@ def test_many_token_product_into_an_unaligned_output(gpu, typ, m):
         lib.lc_dev_free(p)
 
 
+@pytest.mark.parametrize("k", [57856, 58112, 65536])  # the longest row but one unit that the preparation holds in shared memory; the first past it; far past it
+@pytest.mark.parametrize("typ", [2, 8, 12, 13, 14])
+def test_rows_past_the_many_token_product(gpu, typ, k):
+    """Five tokens of rows too long for its preparation take the matrix-vector kernels.  A sum of k f32 products in any order is off by sqrt(k) 2^-24
+    of the products' root of squares at most on average: 2e-5 is more than that."""
+    m, n = 5, 12
+    r = rng(typ + k)
+    w, dense = scaled_blocks(gpu, typ, n, k, np.ones((n, 1)), r)
+    a = r.standard_normal((m, k)).astype(np.float32)
+    got = gpu.qmatmul(typ, a.ravel(), w, m, k, n).reshape(m, n)
+    want = a.astype(np.float64) @ dense.T
+    bound = 2e-5 * np.sqrt((a.astype(np.float64) ** 2) @ (dense.T ** 2))
+    assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / bound).max()
+
+
 def test_qmatmul_linearity_full_size(gpu, oracle):
     """7B-shape matrices: A(x+y) = Ax + Ay and a sample of rows against the oracle."""
     from leafcutterllm_b200 import synth
