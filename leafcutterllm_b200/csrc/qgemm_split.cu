@@ -463,6 +463,10 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
         // ---------------------------------------------------------------- producer of the raw units
         // the weights do not depend on the kernel ahead of this one, so this stream starts before the wait for it
         if (lane == 0) {
+            if (p.offsets) {
+                tmap_acquire(map0);
+                if (pair) tmap_acquire(map1);
+            }
             int sr = 0, in_flight = 0;
             uint32_t phase = 1;
             {

@@ -62,6 +62,19 @@ def test_moe_product_of_experts(gpu, oracle, n_experts, top_k, tokens):
     eng.close()
 
 
+def test_moe_handles_one_after_the_other(gpu, oracle):
+    """Models of different shapes, each closed before the next is opened, so that one's tensor maps come to lie where another's lay: both grouped forms
+    (more than nine rows per expert, and few) see their own."""
+    from leafcutterllm_b200 import synth
+    for hidden, ffn in ((256, 512), (512, 256), (256, 1024), (256, 512)):
+        spec = moe_spec(layers=1, hidden=hidden, heads=hidden // 128, kv=hidden // 128, ffn=ffn, n_experts=4, top_k=2)
+        eng, om = make_pair(gpu, oracle, spec, max_seq_len=64)
+        prompt = synth.prompt_tokens(40, spec.vocab_size, hidden + ffn)
+        assert_close(eng.forward(prompt), om.forward(prompt), LOGIT_ABS, LOGIT_REL, f"{hidden} x {ffn}, 40 tokens")
+        assert_close(eng.forward([5]), om.forward([5]), LOGIT_ABS, LOGIT_REL, f"{hidden} x {ffn}, decode after it")
+        eng.close()
+
+
 def test_moe_batched_decode(gpu, oracle):
     """Twelve sequences decode together: the grouped launch runs two passes per expert where an expert received more than
     eight tokens; tokens must equal the oracle's sequence by sequence."""
