@@ -333,17 +333,22 @@ int32_t moe_block(lc_model* m, int l, const float* x, const float* norm_w, int T
         m->launches_in_call += launches;
         return LC_OK;
     }
-    for (int e = 0; e < El; e++) {
-        GemvArgs g;
-        g.w = &w.egate[e]; g.w2 = &w.eup[e]; g.x = x; g.norm_w = norm_w; g.eps = m->cfg.rms_eps; g.out = m->d_ffn; g.epi = EPI_SILU_MUL;
-        g.prep_next = true;  // the expert's down projection reads d_ffn next, without a norm
-        LC_TRY(gemv_tiled(m, g, T, m->F, m->H));
-        GemvArgs d;
-        d.w = &w.edown[e]; d.x = m->d_ffn; d.out = m->d_moe_yall + (size_t)e * m->t_cap * m->H;
-        LC_TRY(gemv_tiled(m, d, T, m->H, m->F));
+    for (int t0 = 0; t0 < T; t0 += kMoeSlice) {
+        const int n = std::min(kMoeSlice, T - t0);
+        const size_t row0 = (size_t)t0 * m->H;
+        for (int e = 0; e < El; e++) {
+            GemvArgs g;
+            g.w = &w.egate[e]; g.w2 = &w.eup[e]; g.x = x + row0; g.norm_w = norm_w; g.eps = m->cfg.rms_eps; g.out = m->d_ffn; g.epi = EPI_SILU_MUL;
+            g.prep_next = true;  // the expert's down projection reads d_ffn next, without a norm
+            LC_TRY(gemv_tiled(m, g, n, m->F, m->H));
+            GemvArgs d;
+            d.w = &w.edown[e]; d.x = m->d_ffn; d.out = m->d_moe_yall + (size_t)e * kMoeSlice * m->H;
+            LC_TRY(gemv_tiled(m, d, n, m->H, m->F));
+        }
+        LC_TRY(launch_moe_combine(m->d_moe_yall, m->d_moe_sel + (size_t)t0 * K, m->d_moe_w + (size_t)t0 * K, K, m->H, n, 1, (size_t)kMoeSlice, e0, El,
+                                  residual ? residual + row0 : nullptr, out + row0, m->stream));
+        m->launches_in_call += 1;
     }
-    LC_TRY(launch_moe_combine(m->d_moe_yall, m->d_moe_sel, m->d_moe_w, K, m->H, T, 1, (size_t)m->t_cap, e0, El, residual, out, m->stream));
-    m->launches_in_call += 1;
     return LC_OK;
 }
 
@@ -955,20 +960,20 @@ static int32_t alloc_block_buffers(lc_model* m) {
     LC_TRY(dalloc(&m->d_qkv, (size_t)T * m->nqkv)); LC_TRY(dalloc(&m->d_attn, (size_t)T * nq));
     bool dense = m->cfg.n_experts == 0;  // some layer runs a feed-forward or every expert on every token
     for (const LayerW& w : m->layers) dense = dense || !w.grouped_ok;
-    if (dense) LC_TRY(dalloc(&m->d_ffn, (size_t)T * F));
-    LC_TRY(qgemm_workspace_alloc(&m->gemm_ws, m->cfg.n_experts > 0 ? T * m->cfg.top_k : T, std::max(std::max(H, F), nq)));  // rows: a token's, once per expert it goes to
+    if (dense) LC_TRY(dalloc(&m->d_ffn, (size_t)(m->cfg.n_experts > 0 ? std::min(T, kMoeSlice) : T) * F));
+    bool any = false, all = true;  // layers whose experts have the grouped forms
+    for (const LayerW& w : m->layers) { any = any || w.grouped_ok; all = all && w.grouped_ok; }
+    LC_TRY(qgemm_workspace_alloc(&m->gemm_ws, any ? T * m->cfg.top_k : T, std::max(std::max(H, F), nq)));  // rows: a token's, once per expert it goes to
     if (m->any_unfused_qkv) LC_TRY(dalloc(&m->d_qkv_parts, (size_t)T * m->nqkv));
     if (m->cfg.n_experts > 0) {
         const int E = m->cfg.n_experts, K = m->cfg.top_k;
         LC_TRY(dalloc(&m->d_moe_sel, (size_t)T * K)); LC_TRY(dalloc(&m->d_moe_w, (size_t)T * K));
         LC_TRY(dalloc(&m->d_moe_cnt, (size_t)E + 1)); LC_TRY(dalloc(&m->d_moe_lists, (size_t)E * kMoeGroupedTokens));
         LC_CUDA(cudaMemsetAsync(m->d_moe_cnt, 0, ((size_t)E + 1) * sizeof(int32_t), m->stream));  // the word behind the counts is the router's ticket
-        bool any = false, all = true;  // layers whose experts have the grouped forms
-        for (const LayerW& w : m->layers) { any = any || w.grouped_ok; all = all && w.grouped_ok; }
         const size_t slots = (size_t)(any ? std::max(T, kMoeGroupedTokens) : kMoeGroupedTokens) * K;
         LC_TRY(dalloc(&m->d_moe_h, slots * F)); LC_TRY(dalloc(&m->d_moe_y, slots * H));
         LC_TRY(dalloc(&m->d_moe_off, (size_t)m->El + 1)); LC_TRY(dalloc(&m->d_moe_rows, slots));
-        if (!all) LC_TRY(dalloc(&m->d_moe_yall, (size_t)E * T * H));
+        if (!all) LC_TRY(dalloc(&m->d_moe_yall, (size_t)E * std::min(T, kMoeSlice) * H));
         auto planes_alloc = [&](GemvPlanes* pl, size_t rows, int k) -> int32_t {
             const size_t units = rows * (size_t)(k / 256);
             if (units == 0) return LC_OK;

@@ -43,6 +43,7 @@ constexpr int kPrefillChunk = 2048;
 // Tokens per tile from which prompts attend tile by tile where the tensor-core kernel does not apply; shorter runs would leave most warps of a
 // tile idle while one of them walks the whole context, which the split-context kernel shares out.
 constexpr int kRowsRun = 8;
+constexpr int kMoeSlice = 512;           // tokens that run through every expert together (their outputs are kept for the sum: experts x tokens x hidden floats)
 constexpr int kAttnSlice = 512;          // tokens per launch of the attention kernels that split a context (their scratch grows with both)
 constexpr int kTileRun = 16;             // runs of fewer tokens attend token by token
 constexpr int kChunkRun = 32;            // runs of fewer tokens walk the gated delta rule token by token

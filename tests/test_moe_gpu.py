@@ -75,6 +75,34 @@ def test_moe_handles_one_after_the_other(gpu, oracle):
         eng.close()
 
 
+def test_moe_every_expert_in_slices(gpu, oracle):
+    """Experts without a grouped form: 1,100 tokens run through every expert 512 at a time, the last 76 of them, and are summed in their own rows."""
+    from leafcutterllm_b200 import synth
+    spec = moe_spec(layer_type=2, layers=1, n_experts=3, top_k=2)
+    eng, om = make_pair(gpu, oracle, spec, max_seq_len=1104)
+    x = np.random.default_rng(4).standard_normal((1100, spec.hidden_size)).astype(np.float32)
+    got, want = eng.probe_ffn(0, x), om.ffn(0, x)
+    # as for the dense feed-forward: SiLU(gate) * up of two many-token products (2e-5 of the largest each, tested with the product), then a third
+    assert_close(got, want, 1e-4 * np.abs(want).max(), 1e-4, "1100 rows")
+    eng.close()
+
+
+def test_moe_every_expert_memory_does_not_grow_with_the_pass(gpu):
+    """32 experts' outputs of 2,048 tokens would be 32 * 2,048 * 512 floats = 128 MiB, three quarters of it past the 512 that they are kept for.  A pass's other
+    buffers for 1,536 more tokens (hidden rows, q k v, attention, slots, prepared rows: about ten rows of 512 to 1,024 floats each) are below 64 MiB."""
+    import torch
+    from leafcutterllm_b200 import synth
+    spec = moe_spec(layer_type=2, layers=1, hidden=512, heads=4, kv=4, ffn=512, n_experts=32, top_k=2)
+    torch.cuda.init()
+    used = []
+    for capacity in (512, 512, 2048):  # the first one pays for what the library sets up once
+        before = torch.cuda.mem_get_info()[0]
+        eng = synth.build_engine(spec, capacity, kv_pool_tokens=2048)
+        used.append(before - torch.cuda.mem_get_info()[0])
+        eng.close()
+    assert used[2] - used[1] < 64 << 20, used
+
+
 def test_moe_batched_decode(gpu, oracle):
     """Twelve sequences decode together: the grouped launch runs two passes per expert where an expert received more than
     eight tokens; tokens must equal the oracle's sequence by sequence."""
