@@ -142,8 +142,7 @@ bool qgemm_split_weight_ok(const QWeight& w);
 int32_t launch_row_scales(const QWeight& w, float* down, cudaStream_t s);
 // true when the preparation, which holds a token's row in shared memory, takes rows of k elements; longer ones stay with the matrix-vector kernels
 bool qgemm_row_fits(int k);
-// true when launch_qgemm implements these arguments for T tokens (T at least LC_GEMM_MIN_TOKENS, default 5: up to four tokens the
-// matrix-vector kernels are faster, from five on they would run their 8-token form, which this product beats)
+// true when launch_qgemm implements these arguments for T tokens and is the faster way (from LC_GEMM_MIN_TOKENS on where that is set)
 bool qgemm_applies(const GemvArgs& a, int T, const GemmWorkspace& ws);
 // true when the summing kernel, which takes four outputs a thread, can write this product's result: k may be split
 bool qgemm_sum_ok(const GemvArgs& a);

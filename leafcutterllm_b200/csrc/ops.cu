@@ -430,7 +430,7 @@ int32_t lc_dequantize_dev(uint32_t typ, const void* bytes_dev, size_t n_elems, f
 }
 
 // Rows of `a` against a quantised matrix: token tiles of at most 8 rows per pass of the matrix-vector kernels, or -- for
-// five rows and more of the types it knows -- chunks of up to 512 rows through the tensor-core product (qgemm_umma.cu).
+// where it is faster, from 5 to 13 rows on -- chunks of up to 512 rows through the tensor-core product (qgemm_umma.cu).
 static int32_t qmatmul_rows(const QWeight& w, const float* a_dev, size_t m, float* c_dev) {
     static GemmWorkspace ws;  // callers are serialised (L1 mutex / single library stream)
     GemvArgs probe;

@@ -889,15 +889,22 @@ void qgemm_workspace_free(GemmWorkspace* ws) {
     ws->tok_scale = nullptr;
 }
 
-static int gemm_min_tokens() {
-    static const int v = getenv("LC_GEMM_MIN_TOKENS") ? atoi(getenv("LC_GEMM_MIN_TOKENS")) : 5;
-    return v;
+// Fewest tokens for this product; below, the matrix-vector kernels are faster.  Steps of an engine (7B shape, four layers of one type, us), matrix-vector / product:
+// Q4_0 five tokens 1426 / 756, Q8_0 1126 / 808, Q6_K five 1088 / 1210, six 1228 / 1210, eight 1285 / 1210.  A matrix without row scales (a call of
+// lc_qmatmul) is read once more for them, where its type needs them (us): Q8_0 [4096 -> 11008] eight tokens 34 / 40, nine 44 / 40; Q6_K eight 38 / 66, 16 tokens
+// 74 / 67, [4096 -> 4096] eight 21 / 26, nine 27 / 26, [2048 -> 2048] 16 tokens 22 / 23; Q4_0 five 49 / 36, 28 / 18, 15 / 15.
+static int gemm_min_tokens(const QWeight& w) {
+    static const char* const v = getenv("LC_GEMM_MIN_TOKENS");
+    if (v) return atoi(v);
+    if (w.typ == LC_TYPE_Q6_K) return w.row_down ? 6 : 13;
+    if (w.typ == LC_TYPE_Q8_0) return w.row_down ? 5 : 9;
+    return 5;
 }
 bool qgemm_row_fits(int k) { return (size_t)k * sizeof(float) + 64 * sizeof(float) <= kMaxSmem; }  // 58,048 elements
 bool qgemm_applies(const GemvArgs& a, int T, const GemmWorkspace& ws) {
     if (!a.w || !ws.xh || a.group || !qgemm_split_weight_ok(*a.w)) return false;
     if (a.epi == EPI_SILU_MUL && (!a.w2 || a.w2->typ != a.w->typ || !qgemm_split_weight_ok(*a.w2))) return false;
-    if (T < gemm_min_tokens() || T > ws.t_cap || a.w->k > ws.k_max || !qgemm_row_fits(a.w->k)) return false;
+    if (T < gemm_min_tokens(*a.w) || T > ws.t_cap || a.w->k > ws.k_max || !qgemm_row_fits(a.w->k)) return false;
     if (((uintptr_t)a.x % 16) != 0 || (a.norm_w && ((uintptr_t)a.norm_w % 16) != 0)) return false;
     return true;
 }

@@ -192,7 +192,7 @@ def scaled_blocks(gpu, typ, n, k, size, r):
     return w, gpu.dequantize(typ, w, n * k).reshape(n, k).astype(np.float64)
 
 
-@pytest.mark.parametrize("m", [5, 70])  # the tiles of up to 64 tokens and of more
+@pytest.mark.parametrize("m", [16, 70])  # the tiles of up to 64 tokens and of more
 @pytest.mark.parametrize("typ", [2, 8, 12, 13, 14])
 def test_many_token_product_at_the_ends_of_f32(gpu, typ, m):
     """Tokens whose largest element is a denormal, just above 2^-126, or just below f32's end: the power of two that brings them to f16's range has
@@ -210,7 +210,7 @@ def test_many_token_product_at_the_ends_of_f32(gpu, typ, m):
     assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / bound).max(1)
 
 
-@pytest.mark.parametrize("m", [5, 70])
+@pytest.mark.parametrize("m", [16, 70])
 @pytest.mark.parametrize("typ", [2, 8, 14])
 def test_many_token_product_of_infinities(gpu, typ, m):
     """A token with one infinity gives infinities of the weights' signs (NaN where the weight is zero), one with a NaN gives NaN, the others what they always give."""
@@ -231,7 +231,7 @@ def test_many_token_product_of_infinities(gpu, typ, m):
     assert (np.abs(got[rest] - want) <= 2e-5 * np.sqrt((a[rest].astype(np.float64) ** 2) @ (dense.T ** 2))).all()
 
 
-@pytest.mark.parametrize("m", [5, 70])
+@pytest.mark.parametrize("m", [16, 70])
 @pytest.mark.parametrize("typ", [2, 8, 12, 13, 14])
 def test_many_token_product_beside_a_large_activation(gpu, typ, m):
     """One element 2^12 times the size of the others, over blocks of zeros: the others keep their 22 bits, and results the bound that they have without it."""
@@ -247,7 +247,7 @@ def test_many_token_product_beside_a_large_activation(gpu, typ, m):
     assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / bound).max()
 
 
-@pytest.mark.parametrize("typ,m,runs", [(2, 5, 8), (8, 5, 8), (14, 30, 8), (2, 70, 8), (8, 70, 8), (8, 40, 16), (14, 70, 16), (12, 70, 16), (13, 70, 16)])
+@pytest.mark.parametrize("typ,m,runs", [(2, 5, 8), (8, 16, 8), (14, 30, 8), (2, 70, 8), (8, 70, 8), (8, 40, 16), (14, 70, 16), (12, 70, 16), (13, 70, 16)])
 def test_many_token_product_is_centred(gpu, typ, m, runs):
     """The tensor cores cut off toward zero: uncorrected, results are 1.6e-7 (eight additions to a run) or 2.8e-7 (sixteen) too small on average.  Corrected
     to one or two 2^-23, 5e-8 of that is left; 1e-7 is asked for.  Around the mean an addition is off by a unit's length, 2^-23 or less of its run, divided by
@@ -280,7 +280,7 @@ def test_many_token_product_of_positive_activations(gpu, typ, k):
     assert np.linalg.norm(got - want) <= 4e-7 * (1 + 0.16 * np.sqrt(k)) * np.linalg.norm(want), np.linalg.norm(got - want) / np.linalg.norm(want)
 
 
-@pytest.mark.parametrize("m", [5, 70])
+@pytest.mark.parametrize("m", [16, 70])
 @pytest.mark.parametrize("typ", [2, 8, 12, 13, 14])
 def test_many_token_product_of_small_blocks_beside_large_ones(gpu, typ, m):
     """Rows in which every other block is 2^20 times smaller, and no activations but over those: a weight is off by 2^-25 beside a row's largest of
@@ -299,7 +299,7 @@ def test_many_token_product_of_small_blocks_beside_large_ones(gpu, typ, m):
     assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / bound).max()
 
 
-@pytest.mark.parametrize("m", [5, 70])
+@pytest.mark.parametrize("m", [16, 70])
 @pytest.mark.parametrize("typ", [2, 8, 12, 13, 14])
 def test_many_token_product_into_an_unaligned_output(gpu, typ, m):
     """Two row tiles over a long k, which several CTAs share where the summing kernel may write four results at once: an output on a word boundary takes the
@@ -330,15 +330,28 @@ def test_many_token_product_into_an_unaligned_output(gpu, typ, m):
 @pytest.mark.parametrize("k", [57856, 58112, 65536])  # the longest row but one unit that the preparation holds in shared memory; the first past it; far past it
 @pytest.mark.parametrize("typ", [2, 8, 12, 13, 14])
 def test_rows_past_the_many_token_product(gpu, typ, k):
-    """Five tokens of rows too long for its preparation take the matrix-vector kernels.  A sum of k f32 products in any order is off by sqrt(k) 2^-24
+    """Tokens whose rows are too long for its preparation take the matrix-vector kernels.  A sum of k f32 products in any order is off by sqrt(k) 2^-24
     of the products' root of squares at most on average: 2e-5 is more than that."""
-    m, n = 5, 12
+    m, n = 16, 12
     r = rng(typ + k)
     w, dense = scaled_blocks(gpu, typ, n, k, np.ones((n, 1)), r)
     a = r.standard_normal((m, k)).astype(np.float32)
     got = gpu.qmatmul(typ, a.ravel(), w, m, k, n).reshape(m, n)
     want = a.astype(np.float64) @ dense.T
     bound = 2e-5 * np.sqrt((a.astype(np.float64) ** 2) @ (dense.T ** 2))
+    assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / bound).max()
+
+
+@pytest.mark.parametrize("m", [4, 5, 8, 9, 12, 13, 516, 521])  # both sides of where either type changes from the matrix-vector kernels, alone and behind 512 rows
+@pytest.mark.parametrize("typ", [8, 14])
+def test_few_rows_on_both_sides_of_the_switch(gpu, typ, m):
+    k, n = 768, 130
+    r = rng(typ + m + 6)
+    w, dense = scaled_blocks(gpu, typ, n, k, np.ones((n, 1)), r)
+    a = r.standard_normal((m, k)).astype(np.float32)
+    got = gpu.qmatmul(typ, a.ravel(), w, m, k, n).reshape(m, n)
+    want = a.astype(np.float64) @ dense.T
+    bound = 2e-5 * np.sqrt((a.astype(np.float64) ** 2) @ (dense.T ** 2))  # either way's rounding, as above
     assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / bound).max()
 
 
