@@ -1,6 +1,7 @@
 // Operator-level kernels: one per method of the reference's `trait Backend`
 // (rust/src/backend/mod.rs:18-46) plus RoPE, argmax and the shard-order
 // quantised GEMMs, and the host-pointer C entry points built on them.
+#include <map>
 #include <mutex>
 #include <algorithm>
 #include "lc_kernels.h"
@@ -432,7 +433,13 @@ int32_t lc_dequantize_dev(uint32_t typ, const void* bytes_dev, size_t n_elems, f
 // Rows of `a` against a quantised matrix: token tiles of at most 8 rows per pass of the matrix-vector kernels, or -- for
 // where it is faster, from 5 to 13 rows on -- chunks of up to 512 rows through the tensor-core product (qgemm_umma.cu).
 static int32_t qmatmul_rows(const QWeight& w, const float* a_dev, size_t m, float* c_dev) {
-    static GemmWorkspace ws;  // callers are serialised (L1 mutex / single library stream)
+    // One workspace per device, whose calls follow one another on the library's stream there; one caller at a time queues its kernels and grows it.
+    static std::mutex ws_mutex;
+    static std::map<int, GemmWorkspace> ws_of;
+    int dev = 0;
+    LC_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(ws_mutex);
+    GemmWorkspace& ws = ws_of[dev];
     GemvArgs probe;
     probe.w = &w;
     probe.x = a_dev;

@@ -865,9 +865,9 @@ int32_t qgemm_workspace_alloc(GemmWorkspace* ws, int t_cap, int k_max) {
     ws->k_max = k_max;
     const size_t bytes = (size_t)2 * ws->t_cap * k_max * sizeof(__half);
     LC_CUDA(cudaMalloc(&ws->xh, bytes));
-    LC_CUDA(cudaMemset(ws->xh, 0, bytes));  // rows past the tokens of a call are multiplied too (and dropped): keep them finite
+    LC_CUDA(cudaMemsetAsync(ws->xh, 0, bytes, stream()));  // in order with the kernels that write it.  Rows past the tokens of a call are multiplied too (and dropped): keep them finite
     LC_CUDA(cudaMalloc(&ws->sx, bytes / 16));
-    LC_CUDA(cudaMemset(ws->sx, 0, bytes / 16));
+    LC_CUDA(cudaMemsetAsync(ws->sx, 0, bytes / 16, stream()));
     LC_CUDA(cudaMalloc((void**)&ws->tok_scale, (size_t)ws->t_cap * sizeof(float)));
     // shares of k of the batched decode step, and the two matrices of gate/up of one token tile
     ws->partial_bytes = std::max((size_t)64 << 20, (size_t)2 * kMaxTok * k_max * sizeof(float));

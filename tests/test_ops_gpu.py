@@ -355,6 +355,49 @@ def test_few_rows_on_both_sides_of_the_switch(gpu, typ, m):
     assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / bound).max()
 
 
+def test_many_token_products_from_several_threads(gpu):
+    """Four threads queue products of different types, row lengths and token counts on device buffers of their own: each finds its own results, to the bit,
+    whatever the others' need of the workspace that they share."""
+    import ctypes as C
+    import threading
+    lib, chk = gpu.load(), gpu._capi.check
+    jobs = []
+    for i, (typ, m, k, n) in enumerate([(2, 16, 2048, 256), (8, 70, 4352, 384), (14, 40, 1024, 130), (12, 100, 8192, 256)]):
+        r = rng(typ + m + 7)
+        w, _ = scaled_blocks(gpu, typ, n, k, np.ones((n, 1)), r)
+        a = r.standard_normal((m, k)).astype(np.float32)
+        ptr = [C.c_void_p() for _ in range(3)]
+        for p, size in zip(ptr, (a.nbytes, w.nbytes, 4 * m * n)):
+            chk(lib.lc_dev_alloc(size, C.byref(p)))
+        chk(lib.lc_dev_upload(ptr[0], a.ctypes.data_as(C.c_void_p), a.nbytes))
+        chk(lib.lc_dev_upload(ptr[1], w.ctypes.data_as(C.c_void_p), w.nbytes))
+        jobs.append((typ, m, k, n, ptr))
+
+    def run(job):
+        typ, m, k, n, ptr = job
+        chk(lib.lc_qmatmul_dev(typ, ptr[0], ptr[1], m, k, n, ptr[2]))
+        out = np.empty((m, n), np.float32)
+        chk(lib.lc_dev_download(out.ctypes.data_as(C.c_void_p), ptr[2], out.nbytes))
+        return out
+    alone = [run(j) for j in jobs]
+    wrong = []
+
+    def work(i):
+        chk(lib.lc_dev_sync())  # brings the device's context to this thread: without it tensor maps cannot be encoded, and the first call takes another kernel
+        for _ in range(60):
+            if not np.array_equal(run(jobs[i]), alone[i]):
+                wrong.append(i)
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(jobs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for *_, ptr in jobs:
+        for p in ptr:
+            lib.lc_dev_free(p)
+    assert not wrong
+
+
 def test_qmatmul_linearity_full_size(gpu, oracle):
     """7B-shape matrices: A(x+y) = Ax + Ay and a sample of rows against the oracle."""
     from leafcutterllm_b200 import synth
