@@ -238,9 +238,11 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_staged_kernel(AttnP
 #pragma unroll 4
             for (int s2 = 0; s2 < live; s2++) {  // no branch: the pieces' loads are in flight together
                 const float* ps = pp + (size_t)s2 * (HD + 2);
-                const float scl = expf(__ldcg(ps) - mm);
-                ll += __ldcg(ps + 1) * scl;
-                a += __ldcg(ps + 2 + tid) * scl;
+                const float ms = __ldcg(ps), ls = __ldcg(ps + 1), as = __ldcg(ps + 2 + tid);
+                const bool none = ms == -INFINITY;  // every score of the piece fell below f32's range: no weight, and sums that are NaN
+                const float scl = expf(ms - mm);
+                ll += none ? 0.f : ls * scl;
+                a += none ? 0.f : as * scl;
             }
             p.out[(size_t)item * HD + tid] = a / ll;
             if (tid == 0) p.counters[item] = 0;

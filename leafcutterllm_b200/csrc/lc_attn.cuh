@@ -307,11 +307,13 @@ __device__ __forceinline__ void attention_item(const AttnParams& p, int item, in
     for (int d = tid; d < HD; d += kAttnWarps * 32) {
         float ll = 0.f, a = 0.f;
 #pragma unroll 4
-        for (int s = 0; s < live; s++) {  // every one of them has a key; no branch: the pieces' loads are in flight together
+        for (int s = 0; s < live; s++) {  // no branch: the pieces' loads are in flight together
             const float* ps = pp + (size_t)s * (HD + 2);
-            const float sc = expf(__ldcg(ps) - mm);
-            ll += __ldcg(ps + 1) * sc;
-            a += __ldcg(ps + 2 + d) * sc;
+            const float ms = __ldcg(ps), ls = __ldcg(ps + 1), as = __ldcg(ps + 2 + d);
+            const bool none = ms == -INFINITY;  // every score of the piece fell below f32's range: no weight, and sums that are NaN
+            const float sc = expf(ms - mm);
+            ll += none ? 0.f : ls * sc;
+            a += none ? 0.f : as * sc;
         }
         p.out[(size_t)item * HD + d] = a / ll;
     }

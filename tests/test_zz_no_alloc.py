@@ -113,6 +113,32 @@ def test_static_scratch_rejects_what_does_not_fit(gpu):
         d.close()
 
 
+@pytest.mark.parametrize("n_heads,n_kv,hd", [(8, 8, 128), (32, 4, 64)])  # the kernel with shared-memory staging, the split-context kernel
+def test_a_piece_whose_scores_are_all_minus_infinity_has_no_weight(gpu, n_heads, n_kv, hd):
+    """The first half of the context, whole pieces of it, has scores below f32's range: the softmax over the others is what it would be without."""
+    lib, page_tokens, ctx = gpu.load(), 16, 4096
+    n_pages = ctx // page_tokens
+    r = np.random.default_rng(hd)
+    K = (0.1 * r.standard_normal((n_pages, n_kv, page_tokens, hd))).astype(np.float16)
+    K[..., 0] = 0
+    K[: n_pages // 2, ..., 0] = -60000
+    V = r.standard_normal((n_pages, n_kv, page_tokens, hd)).astype(np.float16)
+    q = r.standard_normal((n_heads, hd)).astype(np.float32)
+    q[:, 0] = 3e38
+    d = Dev(gpu)
+    try:
+        kd, vd, td, qd = d.put(K), d.put(V), d.put(np.arange(n_pages, dtype=np.int32)), d.put(q)
+        out = d.empty(n_heads * hd * 4)
+        gpu._capi.check(lib.lc_attention_decode_dev(qd, kd, vd, td, n_pages, ctx, n_heads, n_kv, hd, page_tokens, 0, out))
+        gpu._capi.check(lib.lc_dev_sync())
+        got = d.get(out, (n_heads, hd))
+        half = np.arange(n_pages // 2, n_pages, dtype=np.int32)
+        want = reference(q, K, V, half, ctx // 2, n_heads, n_kv, hd, page_tokens)
+        assert np.abs(got - want).max() <= 1e-4 + 1e-3 * np.abs(want).max()
+    finally:
+        d.close()
+
+
 @pytest.mark.parametrize("ctx,accepted", [(7936, True), (7937, False)])
 def test_static_scratch_size_rule_at_its_edge(gpu, ctx, accepted):
     """32 heads of 128 dims: 62 pieces of 128 keys are the most whose partials fit the array, so a context of 7936 is
