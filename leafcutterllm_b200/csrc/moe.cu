@@ -101,7 +101,7 @@ moe_route_kernel(const float* __restrict__ x, const float* __restrict__ norm_w, 
             j++;
         }
     }
-    if (lists == nullptr) return;   // many-token calls run every expert on every token and only need sel / wsel
+    if (lists == nullptr) return;   // many-token calls only need sel / wsel (moe_order_kernel, or every expert on every token)
     if (threadIdx.x == 0) {
         __threadfence();  // this token's choices are in global memory before the ticket is
         last_s = atomicAdd(ticket, 1u) == (unsigned)(T - 1) ? 1 : 0;

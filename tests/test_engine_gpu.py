@@ -81,7 +81,7 @@ def test_switches(gpu, oracle, kw):
 
 
 def test_chunked_prefill_matches(gpu, oracle):
-    """A prompt longer than the engine's prefill chunk (512 tokens) keeps call-relative RoPE indices."""
+    """700 tokens in one pass, eleven tiles of prompt attention, call-relative RoPE indices (longer than a pass: test_prompt_longer_than_a_pass)."""
     from leafcutterllm_b200 import synth
     spec = small_spec(12, 12, 12, layers=1, hidden=256, heads=4, kv=4, ffn=256, vocab=500)
     eng, om = make_pair(gpu, oracle, spec, max_seq_len=800)
@@ -107,12 +107,28 @@ def test_prompt_attention_in_tiles(gpu, oracle, hd, kv_dtype, page, rows):
 
 @pytest.mark.parametrize("types,heads", [((12, 12, 12), 2), ((2, 8, 8), 8)])
 def test_prompt_longer_than_a_pass(gpu, oracle, types, heads):
-    """2,100 tokens: a full pass of 2,048 and a short one behind it; heads of 128 (tiled prefill attention) and of 32 (in slices of 512 tokens)."""
+    """2,100 tokens: a full pass of 2,048 and a short one behind it; heads of 128 (tiles on the tensor cores) and of 32 (tiles in f32)."""
     from leafcutterllm_b200 import synth
     spec = small_spec(*types, layers=1, hidden=256, heads=heads, kv=heads, ffn=256, vocab=300)
     eng, om = make_pair(gpu, oracle, spec, max_seq_len=2112)
     prompt = synth.prompt_tokens(2100, spec.vocab_size, 1)
     assert_close(eng.forward(prompt), om.forward(prompt), LOGIT_ABS, LOGIT_REL, "2100-token prefill")
+    eng.close()
+
+
+def test_many_short_runs_attend_in_slices(gpu, oracle):
+    """130 sequences of five tokens are 650 tokens in tiles of five, too few for tiled attention: the split-context kernel takes 512 tokens and then 138
+    (sequence 102 lies on the border), with one scratch and one set of counters for both.  Then five more tokens each, behind the first."""
+    from leafcutterllm_b200 import synth
+    spec = small_spec(2, 8, 8, layers=2, hidden=256, heads=8, kv=8, ffn=256, vocab=300)
+    eng, om = make_pair(gpu, oracle, spec, max_seq_len=16, max_seqs=130)
+    ids = list(range(130))
+    calls = [[synth.prompt_tokens(5, spec.vocab_size, 1000 * c + i).tolist() for i in ids] for c in range(2)]
+    got = [eng.forward_batch(ids, parts)[0] for parts in calls]
+    for i in (0, 1, 50, 101, 102, 103, 128, 129):
+        om.kv_clear()
+        for c in range(2):
+            assert_close(got[c][i], om.forward(calls[c][i]), LOGIT_ABS, LOGIT_REL, f"sequence {i}, call {c}")
     eng.close()
 
 

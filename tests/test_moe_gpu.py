@@ -3,7 +3,7 @@
 The reference has no mixture-of-experts code, so the oracle's `moe_forward` is this project's own definition (router
 logits in f32, top-k with equal logits going to the higher expert index, softmax over the chosen logits, chosen experts
 summed in ascending index): parity here is unpinned by the reference.  What the tests pin is that the CUDA path -- the
-router kernel, the one-launch grouped expert products, the every-expert path of long calls, the weighted sum -- computes
+router kernel, the one-launch grouped expert products, the every-expert path of other types, the weighted sum -- computes
 that definition on the same bytes."""
 import numpy as np
 import pytest
@@ -37,11 +37,12 @@ def test_moe_prefill_decode_and_tokens(gpu, oracle, n_experts, top_k):
     eng.close()
 
 
-def test_moe_long_call_runs_every_expert(gpu, oracle):
-    """A 150-token prefill is past the grouped launch's 64 tokens: every expert runs on every token through the
-    many-token product and the sum keeps the chosen ones."""
+@pytest.mark.parametrize("layer_type", [12, 2])
+def test_moe_long_call(gpu, oracle, layer_type):
+    """A 150-token prefill is past the grouped matrix-vector launch's 64 tokens.  Q4_K experts run their own rows as one many-token product; Q4_0 experts have
+    no grouped form, so every expert runs on every token and the sum keeps the chosen ones."""
     from leafcutterllm_b200 import synth
-    spec = moe_spec(layers=1, n_experts=4, top_k=2)
+    spec = moe_spec(layer_type=layer_type, layers=1, n_experts=4, top_k=2)
     eng, om = make_pair(gpu, oracle, spec, max_seq_len=192)
     prompt = synth.prompt_tokens(150, spec.vocab_size, 5)
     assert_close(eng.forward(prompt), om.forward(prompt), LOGIT_ABS, LOGIT_REL, "150-token prefill")

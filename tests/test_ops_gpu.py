@@ -131,9 +131,9 @@ def test_qmatmul_vs_oracle(gpu, oracle, typ, m, k, n):
 @pytest.mark.parametrize("typ", [12, 13])
 @pytest.mark.parametrize("m,k,n", [(9, 256, 128), (16, 512, 128), (64, 4096, 512), (40, 2816, 300), (130, 1024, 256), (200, 11008, 128)])
 def test_qmatmul_q4k_many_tokens_tensor_core_gemm(gpu, oracle, monkeypatch, typ, m, k, n):
-    """Q4_K and Q5_K (the same unit with a fifth bit per element).  Nine tokens and more go through the tcgen05 product (weights dequantised into tensor memory as f16 high/low halves,
-    activations as swizzled f16 high/low tiles): one k unit, token counts that are not a multiple of 16 or of the
-    64-token tile, rows that are not a multiple of 128, a long k.  Activations carry a wide dynamic range so that the
+    """Q4_K and Q5_K (the same unit with a fifth bit per element).  Five tokens and more go through a tcgen05 product (up to 64: integers in tensor memory, drained
+    per unit; more: weights as f16 high/low halves; activations as swizzled f16 high/low tiles): one k unit, token counts that are not a multiple of 16 or of
+    the token tiles, rows that are not a multiple of 128, a long k.  Activations carry a wide dynamic range so that the
     per-token power-of-two scale matters."""
     from leafcutterllm_b200 import synth
     w = synth.host_tensor(typ, 43, f"gemm_{k}_{n}", n * k)
@@ -143,6 +143,8 @@ def test_qmatmul_q4k_many_tokens_tensor_core_gemm(gpu, oracle, monkeypatch, typ,
     want = oracle.qmatmul(typ, a, w, m, k, n).reshape(m, n)
     for t in range(m):  # per token: its own scale
         assert_close(got[t], want[t], 2e-5 * np.abs(want[t]).max(), 1e-4, f"gemm {m}x{k}x{n} token {t}")
+    if m > 64:  # another kernel, which has no such form
+        return
     monkeypatch.setenv("LC_GEMM_TERMS", "1")  # plain f16 operands: 2^-11 per factor
     fast = gpu.qmatmul(typ, a, w, m, k, n).reshape(m, n)
     for t in range(m):
@@ -155,8 +157,8 @@ def test_qmatmul_q4k_many_tokens_tensor_core_gemm(gpu, oracle, monkeypatch, typ,
 @pytest.mark.parametrize("typ", [2, 8, 12, 13, 14])
 def test_many_token_product_vs_oracle(gpu, oracle, typ, m, k, n):
     """Weights of both signs whose block scales differ by 2^12 inside a row and by 2^24 between rows, tokens that differ by e^12.
-    A weight keeps 22 bits beside its row's largest (2^-23), an activation 22 beside its token's, and 256 products are added with
-    truncation before each rounded sum (measured 3.5e-7 of the sum of squares' root): 2e-5 of the largest result leaves ten times that."""
+    A weight and an activation keep 22 bits each, and 256 products are added with truncation before each rounded sum (measured 3.5e-7 of the
+    sum of squares' root before its mean is corrected): 2e-5 of that root for every single result leaves fifty times that."""
     r = rng(typ * 1000 + k + n + m)
     be, bb = gpu.QUANT_GEOMETRY[typ]
     w = r.integers(0, 256, n * k // be * bb, dtype=np.uint8).reshape(n, -1, bb)
