@@ -134,10 +134,9 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_staged_kernel(AttnP
     const int n = t_end - t_begin, live = (pos + p.chunk) / p.chunk;  // pieces that hold a key of this token; the grid has room for the longest context
     if (n <= 0) return;
     __syncthreads();  // barrier initialised
-    bool ok = true;
-    if (n > 0) ok = mbar_wait(&bar, 0);
+    const bool ok = mbar_wait(&bar, 0);
     const int rp = fused ? p.tok_rope[tok] : 0;
-    if (n > 0 && fused && pos >= t_begin && pos < t_end) {
+    if (fused && pos >= t_begin && pos < t_end) {
         // the token of this step replaces the (stale) staged slot: rotate, round through f16, keep in the cache
         const int row = pos - t_begin;
         float kr[1], vr;
@@ -167,56 +166,53 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_staged_kernel(AttnP
     for (int hq = 0; hq < gsz; hq++) {
         const int h = kvh * gsz + hq, item = tok * n_heads + h;
         float* pout = p.partial + ((size_t)item * p.n_splits + split) * (HD + 2);
-        float m = -INFINITY, l = 0.f, a_out = 0.f;
-        if (n > 0) {
-            {
-                float qv[1];
-                load_rotated<1, HD>(p.q + (size_t)tok * p.q_stride + h * HD, tid, rp, p.theta, qv);
-                __syncthreads();  // the previous head is done with q_s / p_s / acc_s
-                q_s[tid] = qv[0];
-            }
-            __syncthreads();
-            float sc = -INFINITY;
-            if (tid < n) {
-                float d0 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;
-                const __half* krow = K_s + (size_t)tid * HD;
-#pragma unroll
-                for (int j = 0; j < 16; j++) {
-                    const int c = (j + tid) & 15;
-                    const uint4 kq = *reinterpret_cast<const uint4*>(krow + c * 8);
-                    const float4 qa = *reinterpret_cast<const float4*>(q_s + c * 8);
-                    const float4 qb = *reinterpret_cast<const float4*>(q_s + c * 8 + 4);
-                    const __half2* h2 = reinterpret_cast<const __half2*>(&kq);
-                    const float2 k0 = __half22float2(h2[0]), k1 = __half22float2(h2[1]), k2 = __half22float2(h2[2]), k3 = __half22float2(h2[3]);
-                    d0 = fmaf(qa.x, k0.x, d0); d1 = fmaf(qa.y, k0.y, d1); d2 = fmaf(qa.z, k1.x, d2); d3 = fmaf(qa.w, k1.y, d3);
-                    d0 = fmaf(qb.x, k2.x, d0); d1 = fmaf(qb.y, k2.y, d1); d2 = fmaf(qb.z, k3.x, d2); d3 = fmaf(qb.w, k3.y, d3);
-                }
-                sc = ((d0 + d1) + (d2 + d3)) / inv_div;
-            }
-            const float wm = warp_max(sc);
-            if (lane == 0) red_s[warp] = wm;
-            __syncthreads();
-            m = fmaxf(fmaxf(red_s[0], red_s[1]), fmaxf(red_s[2], red_s[3]));
-            const float pe = (tid < n) ? expf(sc - m) : 0.f;
-            p_s[tid] = pe;
-            const float ws = warp_sum(pe);
-            if (lane == 0) red_s[4 + warp] = ws;
-            __syncthreads();
-            l = ((red_s[4] + red_s[5]) + red_s[6]) + red_s[7];
-            float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-            const int kend = min(n, 32 * warp + 32);
-#pragma unroll 4
-            for (int k = 32 * warp; k < kend; k++) {
-                const float pk = p_s[k];
-                const uint2 vq = *reinterpret_cast<const uint2*>(V_s + (size_t)k * HD + 4 * lane);
-                const __half2* h2 = reinterpret_cast<const __half2*>(&vq);
-                const float2 v0 = __half22float2(h2[0]), v1 = __half22float2(h2[1]);
-                a0 = fmaf(pk, v0.x, a0); a1 = fmaf(pk, v0.y, a1); a2 = fmaf(pk, v1.x, a2); a3 = fmaf(pk, v1.y, a3);
-            }
-            *reinterpret_cast<float4*>(acc_s + warp * HD + 4 * lane) = make_float4(a0, a1, a2, a3);
-            __syncthreads();
-            a_out = ((acc_s[tid] + acc_s[HD + tid]) + acc_s[2 * HD + tid]) + acc_s[3 * HD + tid];
+        {
+            float qv[1];
+            load_rotated<1, HD>(p.q + (size_t)tok * p.q_stride + h * HD, tid, rp, p.theta, qv);
+            __syncthreads();  // the previous head is done with q_s / p_s / acc_s
+            q_s[tid] = qv[0];
         }
+        __syncthreads();
+        float sc = -INFINITY;
+        if (tid < n) {
+            float d0 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;
+            const __half* krow = K_s + (size_t)tid * HD;
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
+                const int c = (j + tid) & 15;
+                const uint4 kq = *reinterpret_cast<const uint4*>(krow + c * 8);
+                const float4 qa = *reinterpret_cast<const float4*>(q_s + c * 8);
+                const float4 qb = *reinterpret_cast<const float4*>(q_s + c * 8 + 4);
+                const __half2* h2 = reinterpret_cast<const __half2*>(&kq);
+                const float2 k0 = __half22float2(h2[0]), k1 = __half22float2(h2[1]), k2 = __half22float2(h2[2]), k3 = __half22float2(h2[3]);
+                d0 = fmaf(qa.x, k0.x, d0); d1 = fmaf(qa.y, k0.y, d1); d2 = fmaf(qa.z, k1.x, d2); d3 = fmaf(qa.w, k1.y, d3);
+                d0 = fmaf(qb.x, k2.x, d0); d1 = fmaf(qb.y, k2.y, d1); d2 = fmaf(qb.z, k3.x, d2); d3 = fmaf(qb.w, k3.y, d3);
+            }
+            sc = ((d0 + d1) + (d2 + d3)) / inv_div;
+        }
+        const float wm = warp_max(sc);
+        if (lane == 0) red_s[warp] = wm;
+        __syncthreads();
+        const float m = fmaxf(fmaxf(red_s[0], red_s[1]), fmaxf(red_s[2], red_s[3]));
+        const float pe = (tid < n) ? expf(sc - m) : 0.f;
+        p_s[tid] = pe;
+        const float ws = warp_sum(pe);
+        if (lane == 0) red_s[4 + warp] = ws;
+        __syncthreads();
+        const float l = ((red_s[4] + red_s[5]) + red_s[6]) + red_s[7];
+        float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+        const int kend = min(n, 32 * warp + 32);
+#pragma unroll 4
+        for (int k = 32 * warp; k < kend; k++) {
+            const float pk = p_s[k];
+            const uint2 vq = *reinterpret_cast<const uint2*>(V_s + (size_t)k * HD + 4 * lane);
+            const __half2* h2 = reinterpret_cast<const __half2*>(&vq);
+            const float2 v0 = __half22float2(h2[0]), v1 = __half22float2(h2[1]);
+            a0 = fmaf(pk, v0.x, a0); a1 = fmaf(pk, v0.y, a1); a2 = fmaf(pk, v1.x, a2); a3 = fmaf(pk, v1.y, a3);
+        }
+        *reinterpret_cast<float4*>(acc_s + warp * HD + 4 * lane) = make_float4(a0, a1, a2, a3);
+        __syncthreads();
+        const float a_out = ((acc_s[tid] + acc_s[HD + tid]) + acc_s[2 * HD + tid]) + acc_s[3 * HD + tid];
         if (live == 1) {
             p.out[(size_t)item * HD + tid] = a_out / l;
             continue;

@@ -1,5 +1,7 @@
-// tcgen05 wrappers: operand descriptors, the product with both operands in shared memory, tensor-memory allocation and reads.
+// tcgen05 wrappers: operand descriptors, the products with both operands in shared memory or the first in tensor memory, tensor-memory allocation, reads and
+// stores; f16 pairs out of bytes.
 #pragma once
+#include <cuda_fp16.h>
 #include "lc_tma.cuh"
 
 namespace lc {
@@ -26,6 +28,25 @@ __device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t da, uint64
         "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// f32 accumulate, f16 x f16, both K-major, M = 128
+__host__ __device__ constexpr uint32_t idesc_f16(int n_tok) {
+    return (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(n_tok >> 3) << 17) | (128u >> 4 << 24);
+}
+// D[tmem] (+)= A[tmem] * B[smem]^T
+__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(db), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+        "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -48,6 +69,18 @@ __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t cols) {
 }
 __device__ __forceinline__ void tmem_free(uint32_t tmem, uint32_t cols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
+}
+
+// bytes b0, b1 (or b2, b3) of v as the f16 pair (1024 + b0, 1024 + b1): 0x64 is the high byte of 1024.0
+__device__ __forceinline__ uint32_t bias_pair(uint32_t v, int upper) { return __byte_perm(v, 0x64646464u, upper ? 0x5342u : 0x5140u); }
+__device__ __forceinline__ uint32_t h2_fma(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+__device__ __forceinline__ uint32_t h2_pair(float v) {  // (v, v) as f16x2
+    const __half2 h = __float2half2_rn(v);
+    return *reinterpret_cast<const uint32_t*>(&h);
 }
 
 // qgemv.cu: bf16 tensor map of (d0 contiguous elements, d1, d2) with the strides of d1 and d2 in elements, 128-byte swizzle,

@@ -109,25 +109,6 @@ struct GemmParams {
 };
 
 // ---- tcgen05 wrappers -------------------------------------------------------------------------------------------------
-// f32 accumulate, f16 x f16, both K-major, M = 128
-__host__ __device__ constexpr uint32_t idesc_f16(int n_tok) {
-    return (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(n_tok >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
-}
-// D[tmem] (+)= A[tmem] * B[smem]^T
-__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(db), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
-        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
-        "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-        : "memory");
-}
 __device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t* r) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
 }
@@ -137,23 +118,12 @@ __device__ __forceinline__ bool elect_one() {
     return r != 0;
 }
 // ---- unpacking ---------------------------------------------------------------------------------------------------------
-// bytes b0, b1 (or b2, b3) of v as the f16 pair (1024 + b0, 1024 + b1): 0x64 is the high byte of 1024.0
-__device__ __forceinline__ uint32_t bias_pair(uint32_t v, int upper) { return __byte_perm(v, 0x64646464u, upper ? 0x5342u : 0x5140u); }
-__device__ __forceinline__ uint32_t h2_fma(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
 __device__ __forceinline__ uint32_t h2_mul(uint32_t a, uint32_t b) {
     uint32_t d;
     asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
     return d;
 }
 __device__ __forceinline__ uint32_t h2_neg(uint32_t a) { return a ^ 0x80008000u; }
-__device__ __forceinline__ uint32_t h2_pair(float v) {  // (v, v) as f16x2
-    const __half2 h = __float2half2_rn(v);
-    return *reinterpret_cast<const uint32_t*>(&h);
-}
 __device__ __forceinline__ uint32_t f16_at(const unsigned char* p) { return *reinterpret_cast<const uint16_t*>(p); }
 // words [0, OUT) of the bytes that begin `shift` (even, below 16) bytes into w; `shift` is the same for the whole warp
 template <int IN, int OUT>
@@ -436,21 +406,19 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
             pdl_wait();
             int sb = 0, in_flight = 0;
             uint32_t phase = 1;
-            {
-                for (int v = 0; v < nv && ok; v++) {
-                    const int nc = chunks_of(v);
-                    for (int c = 0; c < nc; c++) {
-                        if (!mbar_wait(&b_empty[sb], phase)) { ok = false; break; }
-                        const CUtensorMap* m = v < nu ? &tmx : &tms;
-                        const int x = v < nu ? (u_begin + v) * kUnitElems + c * 64 : (u_begin / 4 + (v - nu) * 4 + c) * 64;
-                        unsigned char* const tile = bt + (size_t)sb * 2 * b_half;
-                        const int odd = swapped(v, c);
-                        mbar_expect_tx(&b_full[sb], 2 * b_half);
-                        tma_load_3d(tile + odd * b_half, m, x, tok0, 0, &b_full[sb]);
-                        tma_load_3d(tile + (1 - odd) * b_half, m, x, tok0, 1, &b_full[sb]);
-                        in_flight = min(in_flight + 1, BS);
-                        if (++sb == BS) { sb = 0; phase ^= 1; }
-                    }
+            for (int v = 0; v < nv && ok; v++) {
+                const int nc = chunks_of(v);
+                for (int c = 0; c < nc; c++) {
+                    if (!mbar_wait(&b_empty[sb], phase)) { ok = false; break; }
+                    const CUtensorMap* m = v < nu ? &tmx : &tms;
+                    const int x = v < nu ? (u_begin + v) * kUnitElems + c * 64 : (u_begin / 4 + (v - nu) * 4 + c) * 64;
+                    unsigned char* const tile = bt + (size_t)sb * 2 * b_half;
+                    const int odd = swapped(v, c);
+                    mbar_expect_tx(&b_full[sb], 2 * b_half);
+                    tma_load_3d(tile + odd * b_half, m, x, tok0, 0, &b_full[sb]);
+                    tma_load_3d(tile + (1 - odd) * b_half, m, x, tok0, 1, &b_full[sb]);
+                    in_flight = min(in_flight + 1, BS);
+                    if (++sb == BS) { sb = 0; phase ^= 1; }
                 }
             }
             if (!ok)  // copies in flight land first: the newest of each stage (phase: that of `empty` for stage sb)
@@ -469,17 +437,15 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
             }
             int sr = 0, in_flight = 0;
             uint32_t phase = 1;
-            {
-                for (int v = 0; v < nu; v++) {
-                    if (!mbar_wait(&raw_empty[sr], phase)) { ok = false; break; }
-                    mbar_expect_tx(&raw_full[sr], raw_bytes);
+            for (int v = 0; v < nu; v++) {
+                if (!mbar_wait(&raw_empty[sr], phase)) { ok = false; break; }
+                mbar_expect_tx(&raw_full[sr], raw_bytes);
 #pragma unroll
-                    for (int b = 0; b < 4; b++)
-                        tma_load_2d(raw + (size_t)sr * raw_bytes + b * 32 * kPitch, pair && b >= 2 ? map1 : map0, (u_begin + v) * (kPitch / 4),
-                                    row0 + (pair ? b & 1 : b) * 32, &raw_full[sr]);
-                    in_flight = min(in_flight + 1, RS);
-                    if (++sr == RS) { sr = 0; phase ^= 1; }
-                }
+                for (int b = 0; b < 4; b++)
+                    tma_load_2d(raw + (size_t)sr * raw_bytes + b * 32 * kPitch, pair && b >= 2 ? map1 : map0, (u_begin + v) * (kPitch / 4),
+                                row0 + (pair ? b & 1 : b) * 32, &raw_full[sr]);
+                in_flight = min(in_flight + 1, RS);
+                if (++sr == RS) { sr = 0; phase ^= 1; }
             }
             if (!ok)
                 for (int i = 0; i < in_flight; i++) {
@@ -491,31 +457,29 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
         // ---------------------------------------------------------------- the same by words: a warp per row, every other row
         int sr = 0;
         uint32_t phase = 1;
-        {
-            for (int v = 0; v < nu; v++) {
-                ok = __all_sync(0xffffffffu, mbar_wait(&raw_empty[sr], phase));
-                if (!ok) break;
-                uint32_t dst = smem_u32(raw + (size_t)sr * raw_bytes + (warp - 2) * kPitch) + lane * 4;
+        for (int v = 0; v < nu; v++) {
+            ok = __all_sync(0xffffffffu, mbar_wait(&raw_empty[sr], phase));
+            if (!ok) break;
+            uint32_t dst = smem_u32(raw + (size_t)sr * raw_bytes + (warp - 2) * kPitch) + lane * 4;
 #pragma unroll 1
-                for (int half = 0; half < 2; half++) {  // rows 0 .. 63, 64 .. 127 (pair: of the second matrix)
-                    const int first = row0 + (pair ? 0 : half * 64) + warp - 2;
-                    const unsigned char* src = (pair && half ? ref1.w : ref0.w) + (size_t)(u_begin + v) * 210;
-                    const size_t step = 2 * p.row_bytes;
-                    const int live = min(32, (p.n - first + 1) / 2);  // rows past the end: any data, dropped at the end
-                    const unsigned char* row = src + (size_t)first * p.row_bytes;
+            for (int half = 0; half < 2; half++) {  // rows 0 .. 63, 64 .. 127 (pair: of the second matrix)
+                const int first = row0 + (pair ? 0 : half * 64) + warp - 2;
+                const unsigned char* src = (pair && half ? ref1.w : ref0.w) + (size_t)(u_begin + v) * 210;
+                const size_t step = 2 * p.row_bytes;
+                const int live = min(32, (p.n - first + 1) / 2);  // rows past the end: any data, dropped at the end
+                const unsigned char* row = src + (size_t)first * p.row_bytes;
 #pragma unroll 4
-                    for (int r = 0; r < live; r++, row += step, dst += 2 * kPitch) {
-                        const unsigned char* base = reinterpret_cast<const unsigned char*>((uintptr_t)row & ~(uintptr_t)2) + lane * 4;
-                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(base) : "memory");
-                        // words 32 ... 52; of the last one only two bytes where the block began on a word
-                        const uint32_t take = lane < 20 ? 4u : 2u + ((uint32_t)(uintptr_t)row & 2u);
-                        if (lane < 21) asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + 128), "l"(base + 128), "r"(take) : "memory");
-                    }
-                    dst += (32 - max(live, 0)) * 2 * kPitch;
+                for (int r = 0; r < live; r++, row += step, dst += 2 * kPitch) {
+                    const unsigned char* base = reinterpret_cast<const unsigned char*>((uintptr_t)row & ~(uintptr_t)2) + lane * 4;
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(base) : "memory");
+                    // words 32 ... 52; of the last one only two bytes where the block began on a word
+                    const uint32_t take = lane < 20 ? 4u : 2u + ((uint32_t)(uintptr_t)row & 2u);
+                    if (lane < 21) asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + 128), "l"(base + 128), "r"(take) : "memory");
                 }
-                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&raw_full[sr])) : "memory");
-                if (++sr == RS) { sr = 0; phase ^= 1; }
+                dst += (32 - max(live, 0)) * 2 * kPitch;
             }
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&raw_full[sr])) : "memory");
+            if (++sr == RS) { sr = 0; phase ^= 1; }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
     } else if (warp == 1) {
@@ -664,149 +628,147 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
         int sr = 0;
         uint32_t raw_phase = 0, a_phase = 1;
         if (p.row_dynamic) pdl_wait();
-        {
-            const int grow = row0 + (pair ? row & 63 : row);
-            const bool live = grow < p.n;
-            const unsigned char* const wrow = weights + (size_t)min(grow, p.n - 1) * p.row_bytes;
-            const float down = live ? (mat ? ref1.down : ref0.down)[grow] : 1.0f, up = live ? 1.0f / down : 0.0f;
+        const int grow = row0 + (pair ? row & 63 : row);
+        const bool live = grow < p.n;
+        const unsigned char* const wrow = weights + (size_t)min(grow, p.n - 1) * p.row_bytes;
+        const float down = live ? (mat ? ref1.down : ref0.down)[grow] : 1.0f, up = live ? 1.0f / down : 0.0f;
 #pragma unroll
-            for (int t = 0; t < kOwn; t++) y[t] = 0.f;
-            for (int v = 0; v < nu && ok; v++) {
-                ok = wait_all(&raw_full[sr], raw_phase);
-                if (!ok) break;
-                const unsigned char* rp = raw + (size_t)sr * raw_bytes + (size_t)row * kPitch;
-                if constexpr (kWords) rp += (uint32_t)(uintptr_t)(wrow + (size_t)(u_begin + v) * 210) & 2u;
-                const UnitHead head = load_head<TYPE>(rp, up);
+        for (int t = 0; t < kOwn; t++) y[t] = 0.f;
+        for (int v = 0; v < nu && ok; v++) {
+            ok = wait_all(&raw_full[sr], raw_phase);
+            if (!ok) break;
+            const unsigned char* rp = raw + (size_t)sr * raw_bytes + (size_t)row * kPitch;
+            if constexpr (kWords) rp += (uint32_t)(uintptr_t)(wrow + (size_t)(u_begin + v) * 210) & 2u;
+            const UnitHead head = load_head<TYPE>(rp, up);
 #pragma unroll 1
-                for (int jj = 0; jj < 2; jj++) {
-                    if (!WIDE && jj == 0) {  // the products of the stage's use before are complete
-                        ok = wait_all(&a_empty[g], a_phase);
-                        if (!ok) break;
-                        a_phase ^= 1;
-                        tc_fence_after();
-                    }
-                    uint32_t hi[16], lo[16];
-                    unpack_chunk<TYPE>(rp, head, WIDE ? g + 4 * jj : 2 * g + jj, up, hi, lo);
-                    if (jj == 1) {
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(&raw_empty[sr]);
-                    }
-                    if (WIDE) {
-                        ok = wait_all(&a_empty[g], a_phase);
-                        if (!ok) break;
-                        a_phase ^= 1;
-                        tc_fence_after();
-                    }
-                    tmem_st16(a_stage + (WIDE ? 0 : jj * 32), hi);
-                    tmem_st16(a_stage + (WIDE ? 0 : jj * 32) + 16, lo);
-                    if (WIDE || jj == 1) {
-                        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(&a_full[g]);
-                    }
-                    if (halves && (jj || v > 0)) {  // the run before
-                        drain(2 * v + jj - 1);
-                        if (!ok) break;
-                    }
+            for (int jj = 0; jj < 2; jj++) {
+                if (!WIDE && jj == 0) {  // the products of the stage's use before are complete
+                    ok = wait_all(&a_empty[g], a_phase);
+                    if (!ok) break;
+                    a_phase ^= 1;
+                    tc_fence_after();
                 }
-                if (!halves && ok && v > 0) drain(v - 1);
-                if (++sr == RS) { sr = 0; raw_phase ^= 1; }
+                uint32_t hi[16], lo[16];
+                unpack_chunk<TYPE>(rp, head, WIDE ? g + 4 * jj : 2 * g + jj, up, hi, lo);
+                if (jj == 1) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&raw_empty[sr]);
+                }
+                if (WIDE) {
+                    ok = wait_all(&a_empty[g], a_phase);
+                    if (!ok) break;
+                    a_phase ^= 1;
+                    tc_fence_after();
+                }
+                tmem_st16(a_stage + (WIDE ? 0 : jj * 32), hi);
+                tmem_st16(a_stage + (WIDE ? 0 : jj * 32) + 16, lo);
+                if (WIDE || jj == 1) {
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&a_full[g]);
+                }
+                if (halves && (jj || v > 0)) {  // the run before
+                    drain(2 * v + jj - 1);
+                    if (!ok) break;
+                }
             }
-            for (int v = nu; kHasMin<TYPE> && v < nv && ok; v++) {
-                // the offset operand: two units' sixteen values per sub-chunk, from their headers in global memory (L2: the units passed through it)
-                const int last_j = 2 * chunks_of(v);
+            if (!halves && ok && v > 0) drain(v - 1);
+            if (++sr == RS) { sr = 0; raw_phase ^= 1; }
+        }
+        for (int v = nu; kHasMin<TYPE> && v < nv && ok; v++) {
+            // the offset operand: two units' sixteen values per sub-chunk, from their headers in global memory (L2: the units passed through it)
+            const int last_j = 2 * chunks_of(v);
 #pragma unroll 1
-                for (int jj = 0; jj < 2; jj++) {
-                    const int j = WIDE ? g + 4 * jj : 2 * g + jj;
-                    if (j >= last_j) break;
-                    if (WIDE || jj == 0) {
-                        ok = wait_all(&a_empty[g], a_phase);
-                        if (!ok) break;
-                        a_phase ^= 1;
-                        tc_fence_after();
-                    }
-                    const int u = u_begin + ((v - nu) * 4 + (j >> 1)) * 4 + (j & 1) * 2;
-                    uint32_t col[16];
-#pragma unroll
-                    for (int e = 0; e < 2; e++) {
-                        uint4 hd = make_uint4(0u, 0u, 0u, 0u);
-                        if (live && u + e < u_begin + nu) hd = *reinterpret_cast<const uint4*>(wrow + (size_t)(u + e) * kPitch);
-                        unpack_mins<TYPE>(hd, up, col + 8 * e);
-                    }
-                    tmem_st16(a_stage + (WIDE ? 0 : jj * 32), col);
-                    if (WIDE || jj == 1) {
-                        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(&a_full[g]);
-                    }
+            for (int jj = 0; jj < 2; jj++) {
+                const int j = WIDE ? g + 4 * jj : 2 * g + jj;
+                if (j >= last_j) break;
+                if (WIDE || jj == 0) {
+                    ok = wait_all(&a_empty[g], a_phase);
+                    if (!ok) break;
+                    a_phase ^= 1;
+                    tc_fence_after();
                 }
-                if (ok) drain(v - 1);
-            }
-            if (ok) drain(run_of(nv - 1, 3));
-            pdl_wait();
-            const int t_first = tok0 + tbase, mine = ok ? min(own, tok_end - t_first) : 0;
-            // a lane has one token's scale: a load beside each result's store would wait for it
-            const float scale = lane < mine ? __ldg(p.tok_scale + t_first + lane) : 0.f;
-            // A negative scale: the token holds an infinity or a NaN (xprep_row).  `main` has its results' signs, W_lo * inf in `small` would be NaN
-            // wherever W_lo is zero.
-            const uint32_t wild = __ballot_sync(0xffffffffu, scale < 0.f);
-            if (ok && own > 0) {  // complete: the last unit's d_full followed every product
-                const uint32_t col = two ? (uint32_t)N : kColSmall, also = two && nv > 1 ? (uint32_t)(4 * N) : kNone;
-                if (wild) add_columns(col, also, wild);
-                else add_columns(col, also, 0u);
-            }
-            // what `main` lost on average (see the header)
-            const float back = down * (1.0f + (halves || two ? 0x1p-23f : 0x1p-22f));
-            // two multiplications: the product of the powers may leave f32's range where the result does not
+                const int u = u_begin + ((v - nu) * 4 + (j >> 1)) * 4 + (j & 1) * 2;
+                uint32_t col[16];
 #pragma unroll
-            for (int t = 0; t < kOwn; t++) y[t] = (y[t] * back) * fabsf(__shfl_sync(0xffffffffu, scale, t));
-            if (p.partial) {
-                float* dst = p.partial + ((size_t)(blockIdx.z * (pair ? 2 : 1) + mat) * p.T + t_first) * p.n + grow;
+                for (int e = 0; e < 2; e++) {
+                    uint4 hd = make_uint4(0u, 0u, 0u, 0u);
+                    if (live && u + e < u_begin + nu) hd = *reinterpret_cast<const uint4*>(wrow + (size_t)(u + e) * kPitch);
+                    unpack_mins<TYPE>(hd, up, col + 8 * e);
+                }
+                tmem_st16(a_stage + (WIDE ? 0 : jj * 32), col);
+                if (WIDE || jj == 1) {
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&a_full[g]);
+                }
+            }
+            if (ok) drain(v - 1);
+        }
+        if (ok) drain(run_of(nv - 1, 3));
+        pdl_wait();
+        const int t_first = tok0 + tbase, mine = ok ? min(own, tok_end - t_first) : 0;
+        // a lane has one token's scale: a load beside each result's store would wait for it
+        const float scale = lane < mine ? __ldg(p.tok_scale + t_first + lane) : 0.f;
+        // A negative scale: the token holds an infinity or a NaN (xprep_row).  `main` has its results' signs, W_lo * inf in `small` would be NaN
+        // wherever W_lo is zero.
+        const uint32_t wild = __ballot_sync(0xffffffffu, scale < 0.f);
+        if (ok && own > 0) {  // complete: the last unit's d_full followed every product
+            const uint32_t col = two ? (uint32_t)N : kColSmall, also = two && nv > 1 ? (uint32_t)(4 * N) : kNone;
+            if (wild) add_columns(col, also, wild);
+            else add_columns(col, also, 0u);
+        }
+        // what `main` lost on average (see the header)
+        const float back = down * (1.0f + (halves || two ? 0x1p-23f : 0x1p-22f));
+        // two multiplications: the product of the powers may leave f32's range where the result does not
+#pragma unroll
+        for (int t = 0; t < kOwn; t++) y[t] = (y[t] * back) * fabsf(__shfl_sync(0xffffffffu, scale, t));
+        if (p.partial) {
+            float* dst = p.partial + ((size_t)(blockIdx.z * (pair ? 2 : 1) + mat) * p.T + t_first) * p.n + grow;
+#pragma unroll
+            for (int t = 0; t < kOwn; t++)
+                if (live && t < mine) dst[(size_t)t * p.n] = y[t];
+        } else if (pair) {
+            // rows 0 .. 63 of the tile are gate, 64 .. 127 up: the halves meet in the activation stages, which nothing uses any more
+            float* const ex = reinterpret_cast<float*>(bt) + (size_t)tbase * 64 + (row & 63);
+            float* const dst = p.out + (size_t)t_first * p.n + grow;
+            if (mat == 0) {
 #pragma unroll
                 for (int t = 0; t < kOwn; t++)
-                    if (live && t < mine) dst[(size_t)t * p.n] = y[t];
-            } else if (pair) {
-                // rows 0 .. 63 of the tile are gate, 64 .. 127 up: the halves meet in the activation stages, which nothing uses any more
-                float* const ex = reinterpret_cast<float*>(bt) + (size_t)tbase * 64 + (row & 63);
-                float* const dst = p.out + (size_t)t_first * p.n + grow;
-                if (mat == 0) {
-#pragma unroll
-                    for (int t = 0; t < kOwn; t++)
-                        if (t < mine) ex[t * 64] = silu_f(y[t]);
-                }
-                asm volatile("bar.sync %0, 128;" ::"r"(1 + g) : "memory");  // all of the group's warps come here, whatever their waits gave
-                if (mat == 1) {
-#pragma unroll
-                    for (int t = 0; t < kOwn; t++)
-                        if (live && t < mine) dst[(size_t)t * p.n] = __fmul_rn(ex[t * 64], y[t]);
-                }
-            } else if (p.row_map) {
-                const int to = lane < mine ? __ldg(p.row_map + t_first + lane) : 0;
-#pragma unroll
-                for (int t = 0; t < kOwn; t++) {
-                    const int r = __shfl_sync(0xffffffffu, to, t);
-                    if (live && t < mine) p.out[(size_t)r * p.n + grow] = y[t];
-                }
-            } else {
-                const size_t o = (size_t)t_first * p.n + grow;
-                if (p.epi == EPI_ADD_RESIDUAL) {
-                    // the loads of sixteen tokens together (`residual` may be `out`): one beside each store takes a trip to L2 for each,
-                    // 244 us against 197 without a residual for 2,048 tokens x [4096 -> 4096]
-#pragma unroll
-                    for (int t0 = 0; t0 < kOwn; t0 += 16) {
-                        float r[16];
-#pragma unroll
-                        for (int t = 0; t < 16; t++) r[t] = live && t0 + t < mine ? p.residual[o + (size_t)(t0 + t) * p.n] : 0.f;
-#pragma unroll
-                        for (int t = 0; t < 16; t++) y[t0 + t] = __fadd_rn(r[t], y[t0 + t]);
-                    }
-                }
+                    if (t < mine) ex[t * 64] = silu_f(y[t]);
+            }
+            asm volatile("bar.sync %0, 128;" ::"r"(1 + g) : "memory");  // all of the group's warps come here, whatever their waits gave
+            if (mat == 1) {
 #pragma unroll
                 for (int t = 0; t < kOwn; t++)
-                    if (live && t < mine) p.out[o + (size_t)t * p.n] = y[t];
+                    if (live && t < mine) dst[(size_t)t * p.n] = __fmul_rn(ex[t * 64], y[t]);
             }
+        } else if (p.row_map) {
+            const int to = lane < mine ? __ldg(p.row_map + t_first + lane) : 0;
+#pragma unroll
+            for (int t = 0; t < kOwn; t++) {
+                const int r = __shfl_sync(0xffffffffu, to, t);
+                if (live && t < mine) p.out[(size_t)r * p.n + grow] = y[t];
+            }
+        } else {
+            const size_t o = (size_t)t_first * p.n + grow;
+            if (p.epi == EPI_ADD_RESIDUAL) {
+                // the loads of sixteen tokens together (`residual` may be `out`): one beside each store takes a trip to L2 for each,
+                // 244 us against 197 without a residual for 2,048 tokens x [4096 -> 4096]
+#pragma unroll
+                for (int t0 = 0; t0 < kOwn; t0 += 16) {
+                    float r[16];
+#pragma unroll
+                    for (int t = 0; t < 16; t++) r[t] = live && t0 + t < mine ? p.residual[o + (size_t)(t0 + t) * p.n] : 0.f;
+#pragma unroll
+                    for (int t = 0; t < 16; t++) y[t0 + t] = __fadd_rn(r[t], y[t0 + t]);
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < kOwn; t++)
+                if (live && t < mine) p.out[o + (size_t)t * p.n] = y[t];
         }
     }
     if (!ok && p.error_flag) atomicCAS(p.error_flag, 0, 3);

@@ -83,25 +83,6 @@ struct GemmParams {
 };
 
 // ---- tcgen05 wrappers -------------------------------------------------------------------------------------------------
-// f32 accumulate, f16 x f16, both K-major, M = 128
-__host__ __device__ constexpr uint32_t idesc_f16(int n_tok) {
-    return (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(n_tok >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
-}
-// D[tmem] (+)= A[tmem] * B[smem]^T
-__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(db), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
-        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
-        "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-        : "memory");
-}
 // ---- unpacking ---------------------------------------------------------------------------------------------------------
 struct HdrQ4K { float d, dmin; uint32_t sc_lo, sc_hi, mn_lo, mn_hi; };
 __device__ __forceinline__ void load_hdr(const unsigned char* rp, HdrQ4K& h) {
@@ -109,17 +90,6 @@ __device__ __forceinline__ void load_hdr(const unsigned char* rp, HdrQ4K& h) {
     h.d = h2f((uint16_t)(w.x & 0xFFFFu));
     h.dmin = h2f((uint16_t)(w.x >> 16));
     unpack_scales_k4(w.y, w.z, w.w, &h.sc_lo, &h.sc_hi, &h.mn_lo, &h.mn_hi);
-}
-// bytes b0, b1 (or b2, b3) of v, each < 64, as the f16 pair (1024 + b0, 1024 + b1): 0x64 is the high byte of 1024.0
-__device__ __forceinline__ uint32_t bias_pair(uint32_t v, int upper) { return __byte_perm(v, 0x64646464u, upper ? 0x5342u : 0x5140u); }
-__device__ __forceinline__ uint32_t h2_fma(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-__device__ __forceinline__ uint32_t h2_pair(float v) {  // (v, v) as f16x2; v is a small integer
-    const __half2 h = __float2half2_rn(v);
-    return *reinterpret_cast<const uint32_t*>(&h);
 }
 // Chunk c of a unit = group c of mod.rs:77-96: 32 bytes whose low nibbles are elements 0..31 under sc[2c] and whose high
 // nibbles are elements 32..63 under sc[2c + 1].  Column j of `col` holds (sc q) of elements 2j, 2j + 1, exact in f16:
@@ -287,7 +257,7 @@ xprep_kernel(const float* __restrict__ x, const int32_t* __restrict__ rows, int 
     xprep_row(row, acc, amax, norm_w, eps, K, t, xh, lo_offset, sx, sx_lo_offset, tok_scale, sh);
 }
 
-// grid = (row tiles x matrices, token tiles, shares of k).  tmw0 / tmw1: raw blocks of the matrix (and of `up` for
+// grid = (row tiles x matrices, 1, shares of k).  tmw0 / tmw1: raw blocks of the matrix (and of `up` for
 // EPI_SILU_MUL: CTAs past the first matrix's tiles work on the second), box = one unit x 128 rows.  tmx: the prepared
 // activations [2 halves][t_cap rows][k] f16 seen in four dimensions (element, row, half, 64-element chunk), box = 64 elements
 // x N rows x both halves x two chunks, 128-byte swizzle; tms: the sub-block sums [2][t_cap rows][k / 16], box = 64 x N x both halves.
@@ -313,7 +283,7 @@ qgemm_umma_q4k_kernel(const __grid_constant__ CUtensorMap tmw0, const __grid_con
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int mat = (int)blockIdx.x >= p.tiles ? 1 : 0, tile = (int)blockIdx.x - mat * p.tiles, tok0 = blockIdx.y * kMaxTok;
+    const int mat = (int)blockIdx.x >= p.tiles ? 1 : 0, tile = (int)blockIdx.x - mat * p.tiles;
     const int N = p.N;
     // this CTA's share of k: whole groups of four units (one tile of sub-block sums), so that only its last tile can be short
     const int nquads = (p.k / kUnitElems + 3) / 4;
@@ -375,7 +345,7 @@ qgemm_umma_q4k_kernel(const __grid_constant__ CUtensorMap tmw0, const __grid_con
     // the call behind the main loop the 64-sequence step was 0.06 ms per layer slower (the attention grid started late).
     bool ok = true;
     // diagnostics: cycles spent in each kind of wait (slot), and in the role's whole loop (slot 7)
-    const bool tracing = p.trace && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
+    const bool tracing = p.trace && blockIdx.x == 0 && blockIdx.z == 0;
     unsigned wacc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     const unsigned t_role0 = (unsigned)clock64();
     auto twait = [&](uint64_t* bar, uint32_t parity, int slot) -> bool {
@@ -408,10 +378,10 @@ qgemm_umma_q4k_kernel(const __grid_constant__ CUtensorMap tmw0, const __grid_con
                     const int q = b_next >> 3, ss = q & 1;
                     if (!twait(&s_empty[ss], ((q >> 1) & 1) ^ 1, 1)) { ok = false; break; }
                     mbar_expect_tx(&s_full[ss], b_bytes);
-                    tma_load_3d(st + (size_t)ss * b_bytes, &tms, (u_begin / 4 + q) * 64, tok0, 0, &s_full[ss]);
+                    tma_load_3d(st + (size_t)ss * b_bytes, &tms, (u_begin / 4 + q) * 64, 0, 0, &s_full[ss]);
                 }
                 mbar_expect_tx(&b_full[sb], 2 * b_bytes);
-                tma_load_4d(bt + (size_t)sb * 2 * b_bytes, &tmx, 0, tok0, 0, u_begin * 4 + b_next * 2, &b_full[sb]);
+                tma_load_4d(bt + (size_t)sb * 2 * b_bytes, &tmx, 0, 0, 0, u_begin * 4 + b_next * 2, &b_full[sb]);
             }
             trace_out(0);
         }
@@ -604,13 +574,13 @@ qgemm_umma_q4k_kernel(const __grid_constant__ CUtensorMap tmw0, const __grid_con
                 float* dst = p.partial + ((size_t)(blockIdx.z * p.nmat + mat) * p.T) * p.n;
 #pragma unroll
                 for (int t = 0; t < kTokD; t++) {
-                    const int tok = tok0 + tbase + t;
+                    const int tok = tbase + t;
                     if (tbase + t < N && tok < p.T) dst[(size_t)tok * p.n + grow] = y[t] * fabsf(__ldg(p.tok_scale + tok));
                 }
             } else {
 #pragma unroll
                 for (int t = 0; t < kTokD; t++) {
-                    const int tok = tok0 + tbase + t;
+                    const int tok = tbase + t;
                     if (tbase + t < N && tok < p.T) {
                         const size_t o = (size_t)tok * p.n + grow;
                         float v = y[t] * fabsf(__ldg(p.tok_scale + tok));
@@ -913,7 +883,7 @@ bool qgemm_sum_ok(const GemvArgs& a) {
     return a.w->n % 4 == 0 && (uintptr_t)a.out % 16 == 0 && (a.epi != EPI_ADD_RESIDUAL || (uintptr_t)a.residual % 16 == 0);
 }
 
-// The product of prepared activations through the kernel above.  *slices > 0: the shares (or gate's and up's sums) are in ws.partial.
+// The product of prepared activations of up to kMaxTok tokens through the kernel above.  *slices > 0: the shares (or gate's and up's sums) are in ws.partial.
 static int32_t launch_qgemm_tile(const GemvArgs& a, GemmWorkspace& ws, int* slices, cudaStream_t s) {
     const int T = a.m, K = a.w->k, n = a.w->n;
     const int terms = (getenv("LC_GEMM_TERMS") && atoi(getenv("LC_GEMM_TERMS")) == 1) ? 1 : 3;  // read per call so that a test can switch it
@@ -951,15 +921,15 @@ static int32_t launch_qgemm_tile(const GemvArgs& a, GemmWorkspace& ws, int* slic
     // Few tiles (a batched decode step on the square matrices): split k over several CTAs so that all SMs work; the
     // shares are summed, in a fixed order, by a small second kernel.  Cost model: waves x units per CTA, plus four
     // units' worth of prologue and epilogue per wave.  The two matrices of gate/up always meet in that kernel.
-    const int tiles = (n + kRows - 1) / kRows, ttiles = (T + kMaxTok - 1) / kMaxTok, nquads = (K / kUnitElems + 3) / 4;
+    const int tiles = (n + kRows - 1) / kRows, nquads = (K / kUnitElems + 3) / 4;
     int ks = 1;
     {
         const int sms = sm_count();
         long best = -1;
         for (int c = 1; c <= std::min(8, nquads); c++) {
             if (c > 1 && (size_t)c * nmat * T * n * sizeof(float) > ws.partial_bytes) break;
-            if (c > 1 && (!qgemm_sum_ok(a) || T > 2 * kMaxTok)) break;
-            const long waves = ((long)tiles * nmat * ttiles * c + sms - 1) / sms;
+            if (c > 1 && !qgemm_sum_ok(a)) break;
+            const long waves = ((long)tiles * nmat * c + sms - 1) / sms;
             const long cost = waves * (((nquads + c - 1) / c) * 4 + 4) + (c > 1 ? 3 : 0);
             if (best < 0 || cost < best) { best = cost; ks = c; }
         }
@@ -978,7 +948,7 @@ static int32_t launch_qgemm_tile(const GemvArgs& a, GemmWorkspace& ws, int* slic
     p.ksplit = ks;
     p.tiles = tiles; p.nmat = nmat;
     p.partial = summed ? ws.partial : nullptr;
-    dim3 grid((unsigned)(tiles * nmat), (unsigned)ttiles, (unsigned)ks);
+    dim3 grid((unsigned)(tiles * nmat), 1, (unsigned)ks);
     LC_CUDA(launch_pdl(kern, grid, dim3(kThreads), smem, s, *t0, *t1, tmx, tms, p));
     *slices = summed ? nmat * ks : 0;
     if (want_trace) {
