@@ -287,8 +287,9 @@ attention_rows_kernel(const float* __restrict__ q, int q_stride, float* __restri
 #pragma unroll
         for (int r = 0; r < kRowsPer; r++) {
             const float z = t0 + lane <= tl.pos0 + r0 + r ? s[r] / root : -INFINITY;
-            const float mn = fmaxf(m[r], warp_max(z));  // finite from the first tile on: every row sees position 0
-            const float alpha = expf(m[r] - mn), w = expf(z - mn);
+            const float mn = fmaxf(m[r], warp_max(z));
+            const float ref = mn == -INFINITY ? 0.f : mn;  // every score so far fell below f32's range: no weight, and no inf - inf
+            const float alpha = expf(m[r] - ref), w = expf(z - ref);
             m[r] = mn;
             l[r] = fmaf(l[r], alpha, w);
 #pragma unroll
