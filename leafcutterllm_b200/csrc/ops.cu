@@ -430,8 +430,8 @@ int32_t lc_dequantize_dev(uint32_t typ, const void* bytes_dev, size_t n_elems, f
     return launch_dequant(typ, bytes_dev, n_elems, out_dev, stream());
 }
 
-// Rows of `a` against a quantised matrix: token tiles of at most 8 rows per pass of the matrix-vector kernels, or -- for
-// where it is faster, from 5 to 13 rows on -- chunks of up to 512 rows through the tensor-core product (qgemm_umma.cu).
+// Rows of `a` against a quantised matrix: token tiles of at most 8 rows per pass of the matrix-vector kernels, or --
+// where it is faster, from five to thirteen rows on -- chunks of up to 512 rows through the tensor-core product (qgemm_umma.cu).
 static int32_t qmatmul_rows(const QWeight& w, const float* a_dev, size_t m, float* c_dev) {
     // One workspace per device, whose calls follow one another on the library's stream there; one caller at a time queues its kernels and grows it.
     static std::mutex ws_mutex;
@@ -448,7 +448,10 @@ static int32_t qmatmul_rows(const QWeight& w, const float* a_dev, size_t m, floa
     if (qgemm_split_weight_ok(w) && m >= 5 && qgemm_row_fits(w.k)) {
         if (!ws.xh || ws.k_max < w.k) {
             qgemm_workspace_free(&ws);
-            LC_TRY(qgemm_workspace_alloc(&ws, chunk, w.k));
+            if (qgemm_workspace_alloc(&ws, chunk, w.k) != LC_OK) {  // no room: the matrix-vector kernels need none
+                qgemm_workspace_free(&ws);
+                (void)cudaGetLastError();
+            }
         }
     }
     for (size_t m0 = 0; m0 < m;) {

@@ -400,6 +400,44 @@ def test_many_token_products_from_several_threads(gpu):
     assert not wrong
 
 
+NO_ROOM = """
+import ctypes, sys
+sys.path.insert(0, {root!r})
+import numpy as np
+import leafcutterllm_b200 as gpu
+from leafcutterllm_b200 import synth
+lib, typ, m, k, n = gpu.load(), {typ}, 16, 4096, 64
+w = synth.host_tensor(typ, 5, "room", n * k)
+a = np.random.default_rng(2).standard_normal((m, k)).astype(np.float32)
+gpu.qmatmul(typ, np.zeros((4, 4 * k), np.float32), synth.host_tensor(typ, 6, "more", 16 * n * k), 4, 4 * k, 4 * n)  # room for the call's own inputs
+held, size, at = [], 16 << 30, ctypes.c_void_p()
+while size >= 32 << 20:
+    if lib.lc_dev_alloc(size, ctypes.byref(at)) == 0:
+        held.append(at.value)
+    else:
+        size >>= 1
+full = gpu.qmatmul(typ, a, w, m, k, n).reshape(m, n)
+for p in held:
+    lib.lc_dev_free(ctypes.c_void_p(p))
+free = gpu.qmatmul(typ, a, w, m, k, n).reshape(m, n)
+want = a.astype(np.float64) @ gpu.dequantize(typ, w, n * k).reshape(n, k).T.astype(np.float64)
+for got in (full, free):  # 4096 products in f32 or better
+    assert np.abs(got - want).max() <= 2e-5 * np.abs(want).max(), np.abs(got - want).max()
+"""
+
+
+@pytest.mark.parametrize("typ", [2, 14])
+def test_qmatmul_without_room_for_the_many_token_product(gpu, typ):
+    """Sixteen rows while the device has no memory left for the product's workspace (64 MB and more) run through the matrix-vector kernels; afterwards, with
+    room again, through the product.  In a process of its own, whose workspace no other test has made."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", NO_ROOM.format(root=root, typ=typ)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
 def test_qmatmul_linearity_full_size(gpu, oracle):
     """7B-shape matrices: A(x+y) = Ax + Ay and a sample of rows against the oracle."""
     from leafcutterllm_b200 import synth
