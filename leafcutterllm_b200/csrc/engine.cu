@@ -196,6 +196,14 @@ void try_push(lc_model* m, GemvArgs* a, int T) {
     m->pending_pushed = true;
 }
 
+// Tiles of 64 queries against the kernel that splits contexts (see kRowsWork).  LC_ATTN_ROWS=1 / 0: always / never; read per call so that a test can switch it.
+static bool attention_by_rows(const lc_model* m, int T) {
+    if (T < 16 || m->n_tiles <= 0) return false;
+    if (const char* v = getenv("LC_ATTN_ROWS")) return atoi(v) != 0;
+    return T * m->kv_elt >= kRowsBytes * m->n_tiles &&
+           m->tile_keys * m->nh * m->kv_elt >= kRowsWork * (m->tile_rows + 44) * m->tile_longest;
+}
+
 // attention_forward (attention.rs:37-118) for layer `l` on T tokens whose (normalised or raw) input is `x`.
 int32_t attention_block(lc_model* m, int l, const float* x, const float* norm_w, int T, const float* residual, float* out,
                         bool decode_step) {
@@ -247,7 +255,7 @@ int32_t attention_block(lc_model* m, int l, const float* x, const float* norm_w,
         static const bool no_tc = getenv("LC_PREFILL_FMA") != nullptr;  // diagnostics: the one-CTA-per-(token, head) kernel for every call
         if (T >= 16 && m->n_tiles > 0 && !no_tc && attention_prefill_applies(kv, m->nh))  // a prefill chunk: tiles of 64 queries on the tensor cores
             LC_TRY(launch_attention_prefill(q, m->nqkv, m->d_attn, m->nh, kv, m->d_tiles, m->n_tiles, m->d_page_table, m->pages_per_seq, m->stream));
-        else if (T >= 16 && m->n_tiles > 0 && T >= kRowsRun * m->n_tiles && !no_tc && attention_rows_applies(kv, m->nh, q, m->nqkv))
+        else if (!no_tc && attention_by_rows(m, T) && attention_rows_applies(kv, m->nh, q, m->nqkv))
             LC_TRY(launch_attention_rows(q, m->nqkv, m->d_attn, m->nh, kv, m->d_tiles, m->n_tiles, m->d_page_table, m->pages_per_seq, m->stream));
         else
             for (int t0 = 0; t0 < T; t0 += kAttnSlice) {
@@ -514,6 +522,13 @@ int32_t upload_meta(lc_model* m, const std::vector<int64_t>& tok, const std::vec
     }
     if (m->stack) LC_TRY(stack_upload_runs(m, seq, pos));
     m->n_tiles = (int)tiles.size();
+    m->tile_rows = m->tile_longest = 0;
+    m->tile_keys = 0;
+    for (const PrefillTile& t : tiles) {
+        m->tile_rows = std::max(m->tile_rows, (int)t.n);
+        m->tile_longest = std::max(m->tile_longest, t.pos0 + t.n);
+        m->tile_keys += t.n * (t.pos0 + 0.5 * t.n + 200.0);
+    }
     if (!tiles.empty()) LC_CUDA(cudaMemcpyAsync(m->d_tiles, tiles.data(), tiles.size() * sizeof(PrefillTile), cudaMemcpyHostToDevice, m->stream));
     // the copies read pageable host vectors that die with the caller's frame
     LC_CUDA(cudaStreamSynchronize(m->stream));

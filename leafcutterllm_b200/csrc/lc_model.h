@@ -40,9 +40,15 @@ struct LayerW {
 // Tokens per pass.  The experts of a mixture receive a share of them each, and the fuller their tiles the better (Mixtral shape, 4 layers,
 // 1,600 tokens: 36.9 ms in passes of 1,024, 33.1 in one); the step buffers grow with it.
 constexpr int kPrefillChunk = 2048;
-// Tokens per tile from which prompts attend tile by tile where the tensor-core kernel does not apply; shorter runs would leave most warps of a
-// tile idle while one of them walks the whole context, which the split-context kernel shares out.
-constexpr int kRowsRun = 8;
+// Prompts attend tile by tile, where the tensor-core kernel does not apply, if that is the faster way (attention_by_rows).  Measured, four layers, us per call of
+// [sequences x new tokens @ tokens before them], tiles / split-context kernel:
+//   heads of 64, f32 cache, 32 heads: 1x16@0 304 / 320, 1x16@1000 712 / 472, 1x64@1000 1291 / 1126, 1x128@1000 1545 / 2225, 4x16@1000 862 / 1060, 16x8@1000 1367 / 1861
+//   the same, f16 cache:              1x16@0 313 / 304, 1x128@0 453 / 495, 1x128@1000 1528 / 1146, 4x16@0 331 / 375, 16x8@1000 1357 / 1033
+//   heads of 128, f32, 32 heads:      1x16@3500 3971 / 1327, 1x128@3500 6381 / 8551, 4x16@3500 4028 / 4224;  heads of 256, f16, 8 heads: 1x128@3500 6277 / 1993
+// A tile walks its context alone, (rows + 44) * 0.93 ns * head_dim per 32 keys; the split-context kernel takes 2.5e-4 ns per (token, head, key) and byte of a key's head and,
+// whatever the context, as long as 200 keys for each.  In these units the line lies at kRowsWork; tiles with few rows are bound by their copies.
+constexpr double kRowsWork = 12500.0 / 108.0;
+constexpr int kRowsBytes = 32;  // fewest new tokens per tile, times the bytes of a cached value
 constexpr int kMoeSlice = 512;           // tokens that run through every expert together (their outputs are kept for the sum: experts x tokens x hidden floats)
 constexpr int kAttnSlice = 512;          // tokens per launch of the attention kernels that split a context (their scratch grows with both)
 constexpr int kTileRun = 16;             // runs of fewer tokens attend token by token
@@ -52,7 +58,7 @@ constexpr int kTokTile = 8;
 constexpr int kMoeGroupedTokens = 64;  // most tokens of a call whose experts run as one grouped matrix-vector launch
 // Rows per expert beyond which the experts run as a grouped many-token product instead: the matrix-vector kernel reads the experts again for
 // every four rows.  Mixtral shape, us per step of two layers, matrix-vector / product: 24 sequences (6 rows per expert) 1761 / 2169, 32 (8)
-// 2143 / 2263, 48 (12) 2899 / 2563, 64 (16) 3656 / 3028.
+// 2143 / 2263, 48 (12) 2899 / 2563, 64 (16) 3656 / 3028.  They meet between 8 and 12 rows (a straight line through both puts it at 9); one shape measured.
 constexpr int kMoeProductRows = 9;
 
 }  // namespace lc
@@ -84,7 +90,8 @@ struct lc_model {
     long long* d_key_max = nullptr;
     float* d_logits_all = nullptr;       // dist: the ranks' logit slices gathered for the host
     PrefillTile* d_tiles = nullptr;      // the call's tokens as runs of up to 64 consecutive positions of one sequence
-    int n_tiles = 0;
+    int n_tiles = 0, tile_rows = 0, tile_longest = 0;  // tiles of this pass; the most new tokens of one, the longest context
+    double tile_keys = 0;                              // keys that all tokens see together, and 200 more for each token
     float* pending_dst = nullptr;        // where the next sum over the ranks has to land
     bool pending_pushed = false;         // ... and whether the product already sent its rows to the ranks
     GemvPush push_desc;

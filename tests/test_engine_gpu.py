@@ -92,10 +92,11 @@ def test_chunked_prefill_matches(gpu, oracle):
 
 @pytest.mark.parametrize("rows", [16, 63, 65, 130])  # one tile with idle warps, a row short of a tile, one more, two full ones and a short one
 @pytest.mark.parametrize("hd,kv_dtype,page", [(32, "f16", 16), (32, "f32", 5), (64, "f32", 16), (64, "f16", 32), (128, "f32", 16), (128, "f16", 8), (256, "f16", 16), (256, "f32", 16)])
-def test_prompt_attention_in_tiles(gpu, oracle, hd, kv_dtype, page, rows):
+def test_prompt_attention_in_tiles(gpu, oracle, monkeypatch, hd, kv_dtype, page, rows):
     """Head sizes, cache types and page sizes that the tensor-core prompt attention does not take; a second run of rows behind the first,
     so that tiles begin past position 0.  The host's and the device's powf differ by an ulp or two, which is 260 * 2^-22 = 6e-5 of an angle at the
     last position and of the scores' order: 2e-4 of the largest output; an f16 cache may round a key or value the other way (2^-11 of it): 1e-3."""
+    monkeypatch.setenv("LC_ATTN_ROWS", "1")  # these few heads are faster through the kernel that splits contexts
     spec = small_spec(12, 12, 12, layers=1, hidden=512, heads=512 // hd, kv=max(1, 256 // hd), ffn=256, vocab=64)
     eng, om = make_pair(gpu, oracle, spec, max_seq_len=2 * rows, kv_dtype=kv_dtype, kv_page_tokens=page, rope_mode="absolute")
     x = np.random.default_rng(hd + rows).standard_normal((2 * rows, 512)).astype(np.float32)
@@ -105,10 +106,38 @@ def test_prompt_attention_in_tiles(gpu, oracle, hd, kv_dtype, page, rows):
     eng.close()
 
 
-def test_prompt_attention_where_the_first_keys_score_minus_infinity(gpu, oracle):
+@pytest.mark.parametrize("rows,tiles", [(16, False), (128, True)])
+def test_prompt_attention_takes_the_faster_kernel(gpu, monkeypatch, rows, tiles):
+    """Behind 1,000 tokens: 16 rows of 32 heads are faster with the context split (a tile would walk it alone), 128 rows in two tiles.  The kernels add in different
+    orders, so their outputs tell which one ran; sums of 1,128 weights and 2,048 products in f32 differ by 1e-5 of the largest output at most."""
+    from leafcutterllm_b200 import synth
+    spec = small_spec(12, 12, 12, layers=1, hidden=2048, heads=32, kv=4, ffn=256, vocab=64)
+    eng = synth.build_engine(spec, 1200, on_device=True, kv_dtype="f32", rope_mode="absolute")
+    x = np.random.default_rng(rows).standard_normal((1000 + rows, 2048)).astype(np.float32)
+
+    def run():
+        eng.kv_clear()
+        eng.probe_attention(0, x[:500])
+        eng.probe_attention(0, x[500:1000])
+        return eng.probe_attention(0, x[1000:])
+
+    got = run()
+    monkeypatch.setenv("LC_ATTN_ROWS", "1")
+    by_rows = run()
+    monkeypatch.setenv("LC_ATTN_ROWS", "0")
+    split = run()
+    assert not np.array_equal(by_rows, split)
+    assert_close(by_rows, split, 1e-5 * np.abs(split).max(), 0, "the two kernels")
+    assert np.array_equal(got, by_rows if tiles else split)
+    eng.close()
+
+
+@pytest.mark.parametrize("tiles", ["1", "0"])
+def test_prompt_attention_where_the_first_keys_score_minus_infinity(gpu, oracle, monkeypatch, tiles):
     """The last 20 rows' scores with keys 0 ... 63 fall below f32's range: the softmax over the other keys is what it would be without them.  One head of
     256 whose 100th dim is not rotated (theta^-200/256); there the first rows' keys have -1e34 and the last rows' queries 1e6, elsewhere both next to nothing.  The
     bound is test_prompt_attention_in_tiles's, row by row."""
+    monkeypatch.setenv("LC_ATTN_ROWS", tiles)
     from dataclasses import replace
     from leafcutterllm_b200 import synth
     spec = replace(small_spec(12, 12, 12, layers=1, hidden=256, heads=1, kv=1, ffn=256, vocab=64), rope_theta=1e30)
@@ -137,7 +166,8 @@ def test_prompt_attention_where_the_first_keys_score_minus_infinity(gpu, oracle)
 
 @pytest.mark.parametrize("types,heads", [((12, 12, 12), 2), ((2, 8, 8), 8)])
 def test_prompt_longer_than_a_pass(gpu, oracle, types, heads):
-    """2,100 tokens: a full pass of 2,048 and a short one behind it; heads of 128 (tiles on the tensor cores) and of 32 (tiles in f32)."""
+    """2,100 tokens: a full pass of 2,048 and a short one behind it; heads of 128 (tiles on the tensor cores) and of 32 (tiles in f32, then the kernel that
+    splits contexts)."""
     from leafcutterllm_b200 import synth
     spec = small_spec(*types, layers=1, hidden=256, heads=heads, kv=heads, ffn=256, vocab=300)
     eng, om = make_pair(gpu, oracle, spec, max_seq_len=2112)
