@@ -46,6 +46,7 @@
 // 128 / 64 / 32 / 13 cycles at N = 256 / 128 / 64 / 16), i.e. a third of the f16 rate.  ncu, 2,048 tokens, Q4_K: tensor pipe active 71 % of the
 // cycles for [4096 -> 12288] (505 us), 68 % for gate and up of 11008 (911 us); issue slots 65 %, two thirds of them unpacking (2.4 instructions per
 // weight, Q6_K five).  512 tokens x [4096 -> 12288]: 138 us, where two products per weight and 64 tokens per CTA (qgemm_umma.cu) took 203.
+// (Before the offsets and fractions of the unpacking above; a 7B prompt takes 0.6 % longer with them.)
 #include <algorithm>
 #include <cstdlib>
 #include <cuda_fp16.h>
@@ -811,7 +812,8 @@ GemmShape shape_for(int T) {
     g.smem = fixed + g.b_stages * b + g.raw_stages * raw;
     return g;
 }
-// cycles of the tensor pipe per 256-element unit
+// Cycles per 256-element unit, 16 pairs of products: the tensor pipe's N / 2 and N, but no less than about 45 each, the pace at which products are issued
+// (57 by a lone lane, see the issuing loop; the pipe itself would take 13 at N = 16).  An estimate, like the fixed costs below: it ranks the shares of k.
 long unit_cycles(int N) {
     const long one = std::max(45, N / 2), two = std::max(45, N);
     return 16 * (one + two);
@@ -832,7 +834,7 @@ int32_t launch_type(const GemvArgs& a, const GemmWorkspace& ws, GemmParams& p, c
     const int tiles = (p.n * nmat + kRows - 1) / kRows, ttiles = group ? p.T / g.N + group->n_experts : (p.T + g.N - 1) / g.N, nquads = (p.k / kUnitElems + 3) / 4;
     // Few tiles (a batched decode step, a short prompt): k is cut over several CTAs so that all SMs work, and a second kernel adds
     // the shares in a fixed order.  Cost in cycles: waves of units plus a fixed part (launch, first unit, drain) per wave, and the
-    // shares' trip through L2 at 3000 bytes per cycle.
+    // shares' trip through L2 at 3000 bytes per cycle.  6000, 4000 and 3000 are estimates too (3 us and 2 us; 5.7 TB/s), not fitted one by one.
     int ks = 1;
     double best = 0;
     for (int c = 1; c <= (group ? 1 : std::min(8, nquads)); c++) {

@@ -1,4 +1,5 @@
-// Q4_K (and Q5_K: the kernel's UB = 176 form) weights times MANY tokens (prefill chunks, batched decode steps of five or more sequences) on the
+// Q4_K (and Q5_K: the kernel's UB = 176 form) weights times 5 to 64 tokens (batched decode steps, short prompts; more tokens and the other types:
+// qgemm_split.cu, whose activation preparation, sums and dispatch are here too) on the
 // 5th-generation tensor cores: the dense contraction of the path (Tensor::matmul with m > 1, rust/src/tensor.rs:107-135,
 // over weights that the reference dequantises per call, rust/src/model/loader.rs:213-224).
 //
@@ -31,7 +32,7 @@
 //              tile for the summing kernel (shares of k; SiLU(gate) * up).
 //
 // Activations are prepared by xprep_kernel: optional RMS norm (rust/src/backend/cpu.rs:49-60), a power-of-two scale per
-// token that brings its largest magnitude into [0.5, 1) (so neither half leaves the f16 range), the hi/lo split, and
+// token that brings its largest magnitude into [2^9, 2^10) (see xprep_row), the hi/lo split, and
 // the sub-block sums.  Every accumulator is written by one thread's products, in program order, and the drain adds the
 // units in k order: results are deterministic.
 //
