@@ -25,7 +25,7 @@ __global__ void sanity_kernel(uint32_t typ, const uint8_t* __restrict__ w, size_
 }
 
 __global__ void __launch_bounds__(1024) embed_kernel(uint32_t typ, const uint8_t* __restrict__ w, size_t rows, size_t cols,
-                                                     const int64_t* __restrict__ ids, float* __restrict__ out) {
+                                                     const int64_t* __restrict__ ids, float* __restrict__ out, EmbedTurns turn) {
     pdl_launch_dependents();
     pdl_wait();  // the token ids may come from the kernel ahead (a decode step's advance), and `out` may still be read by it
     int t = blockIdx.x;
@@ -33,6 +33,13 @@ __global__ void __launch_bounds__(1024) embed_kernel(uint32_t typ, const uint8_t
     bool ok = id >= 0 && (size_t)id < rows;
     for (size_t c = threadIdx.x; c < cols; c += blockDim.x)
         out[(size_t)t * cols + c] = ok ? dequant_elem(typ, w, (size_t)id * cols + c) : 0.0f;
+    if (turn.rot) {
+        for (int d = threadIdx.x; d < turn.half; d += blockDim.x) {
+            const float freq = __fdiv_rn(1.0f, powf(turn.theta, __fdiv_rn(__fmul_rn(2.0f, (float)d), (float)(2 * turn.half))));
+            const float angle = __fmul_rn((float)turn.tok_rope[t], freq);
+            static_cast<float2*>(turn.rot)[(size_t)t * turn.half + d] = make_float2(cosf(angle), sinf(angle));
+        }
+    }
 }
 
 static int grid_for(size_t n, int block) {
@@ -60,10 +67,11 @@ int32_t launch_sanity_scan(uint32_t typ, const void* w, size_t n, unsigned long 
 }
 
 int32_t launch_embed(uint32_t typ, const void* w, size_t rows, size_t cols, const int64_t* ids, int n, float* out,
-                     cudaStream_t s) {
+                     const EmbedTurns* turn, cudaStream_t s) {
     if (n <= 0) return LC_OK;
     // a row is a few thousand elements, each decoded on its own: many threads, a few elements each
-    LC_CUDA(launch_pdl(embed_kernel, dim3((unsigned)n), dim3(cols >= 2048 ? 1024 : 256), 0, s, typ, (const uint8_t*)w, rows, cols, ids, out));
+    LC_CUDA(launch_pdl(embed_kernel, dim3((unsigned)n), dim3(cols >= 2048 ? 1024 : 256), 0, s, typ, (const uint8_t*)w, rows, cols, ids, out,
+                       turn ? *turn : EmbedTurns{}));
     return LC_OK;
 }
 

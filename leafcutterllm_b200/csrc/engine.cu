@@ -246,6 +246,7 @@ int32_t attention_block(lc_model* m, int l, const float* x, const float* norm_w,
         AttnFusion fz{k, v, m->d_tok_rope, m->cfg.rope_theta};
         fz.positions_settled = l > 0;  // the first layer of a step may run while the previous step still advances the positions
         fz.stream_slots = m->d_stream_slots;
+        fz.rot = m->d_rot;
         LC_TRY(launch_attention(q, m->nqkv, m->d_attn, T, m->nh, kv, m->d_tok_seq, m->d_tok_pos, m->d_page_table, m->pages_per_seq,
                                 m->cfg.max_seq_len, m->d_attn_scratch, m->d_attn_counters, &fz, m->stream));
         m->launches_in_call += 1;
@@ -419,7 +420,9 @@ int32_t run_layers(lc_model* lead, int T, bool decode_step) {
     if (lead->stack) return stack_run_layers(lead, T, decode_step);
     std::vector<lc_model*> R = ranks_of(lead);
     for (lc_model* m : R) {
-        LC_TRY(launch_embed(m->embed->typ, m->embed->view, m->embed->rows, m->embed->cols, m->d_tokens, T, m->d_hidden, m->stream));
+        const EmbedTurns turn{m->d_tok_rope, m->cfg.rope_theta, m->hd / 2, m->d_rot};
+        LC_TRY(launch_embed(m->embed->typ, m->embed->view, m->embed->rows, m->embed->cols, m->d_tokens, T, m->d_hidden,
+                            decode_step && T > 1 && m->d_rot ? &turn : nullptr, m->stream));
         m->launches_in_call += 1;
     }
     const size_t count = (size_t)T * lead->H;
@@ -965,6 +968,7 @@ static int32_t alloc_block_pools(lc_model* m) {
             LC_TRY(dalloc((uint8_t**)&m->d_stream_slots, slot_bytes));
             LC_CUDA(cudaMemsetAsync(m->d_stream_slots, 0, slot_bytes, m->stream));
         }
+        LC_TRY(dalloc((float2**)&m->d_rot, (size_t)m->max_seqs * (m->hd / 2)));
     }
     return LC_OK;
 }
@@ -1002,6 +1006,7 @@ static int32_t alloc_block_buffers(lc_model* m) {
     }
     size_t sc = 16;
     for (int t = 1; t <= std::max(kAttnSlice, m->max_seqs); t++) sc = std::max(sc, attention_scratch_bytes(t, m->nh, m->hd, m->cfg.max_seq_len));
+    if (m->d_rot) sc = std::max(sc, attention_batch_scratch_bytes(m->nh, m->nkv, m->hd));
     m->attn_scratch_bytes = sc;
     LC_TRY(dalloc((uint8_t**)&m->d_attn_scratch, sc));
     LC_TRY(dalloc(&m->d_attn_counters, (size_t)T * m->nh));
@@ -1094,7 +1099,7 @@ int32_t lc_model_destroy(lc_model* m) {
                     m->moe_planes_x.planes, m->moe_planes_x.sxf, m->moe_planes_x.inv2s, m->moe_planes_h.planes, m->moe_planes_h.sxf, m->moe_planes_h.inv2s,
                     m->d_stream_slots, m->d_page_table, m->d_tokens, m->d_tok_seq, m->d_tok_pos, m->d_tok_rope, m->d_last_idx, m->d_hidden, m->d_hidden2,
                     m->d_qkv, m->d_attn, m->d_ffn, m->d_last, m->d_logits, m->d_next, m->d_out_tokens, m->d_step_ctr,
-                    m->d_attn_scratch, m->d_attn_counters, m->d_sanity, m->d_qkv_parts};
+                    m->d_attn_scratch, m->d_attn_counters, m->d_sanity, m->d_qkv_parts, m->d_rot};
     for (void* p : bufs) if (p) cudaFree(p);
     qgemm_workspace_free(&m->gemm_ws);
     if (m->pin_tokens) cudaFreeHost(m->pin_tokens);

@@ -37,6 +37,10 @@ bool attention_stream_applies(const AttnParams& a, int n_tok);
 // slots: attention_stream_slot_bytes(n_heads, n_kv) bytes of zeroed device memory owned by the caller (left zeroed)
 int32_t launch_attention_stream(const AttnParams& a, unsigned long long* slots, cudaStream_t s);
 
+// attention_batch.cu: one new token for each of two or more sequences, the same heads and caches, as one stream over all of them
+bool attention_batch_applies(const AttnParams& a, int n_tok);
+int32_t launch_attention_batch(const AttnParams& a, const void* rot, int n_tok, cudaStream_t s);
+
 template <int DPL, bool F32>
 __device__ __forceinline__ void load_slice(const void* pool, size_t elem_off, float (&out)[DPL]) {
     if (F32) {

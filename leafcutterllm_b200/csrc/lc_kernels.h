@@ -21,8 +21,10 @@ int32_t launch_scan_scales(uint32_t typ, const void* raw_dev, size_t n_blocks, u
 int32_t launch_sanity_scan(uint32_t typ, const void* w, size_t n_elems, unsigned long long* count, cudaStream_t s);
 // One f32 row of a quantised [rows, cols] tensor per token id (embedding gather,
 // rust/src/inference/engine.rs:134-144; id outside [0, rows) -> zero row).
+// turn (a decode step's; may be null): also the cosine and sine of token t's rotation of pair d, rot[t * half + d]; attention.rs:16-20
+struct EmbedTurns { const int32_t* tok_rope; float theta; int half; void* rot; };
 int32_t launch_embed(uint32_t typ, const void* w, size_t rows, size_t cols, const int64_t* ids, int n, float* out,
-                     cudaStream_t s);
+                     const EmbedTurns* turn, cudaStream_t s);
 
 // ---- ops.cu ----
 int32_t launch_vec_add(const float* a, const float* b, size_t n, float* o, cudaStream_t s);
@@ -189,6 +191,7 @@ int32_t launch_rope_kv_append(float* q, float* k, const float* v, int row_stride
 // tok_pos[i] is the cache position of token i (it attends to positions 0..tok_pos[i]).
 // scratch: split-KV partials, sized by attention_scratch_bytes().
 size_t attention_scratch_bytes(int n_tok, int n_heads, int hd, int max_ctx);
+size_t attention_batch_scratch_bytes(int n_heads, int n_kv, int hd);  // ... and of a handle whose steps pass `rot`
 // counters: n_tok*n_heads ints, zero before the first launch (the kernel leaves them zero).
 // fuse (decode steps only, every token the single new token of its sequence): q is rotated on load and the new
 // key/value are taken from k_new/v_new (rows q_stride floats apart), rotated, and stored into the cache by this kernel,
@@ -202,6 +205,7 @@ struct AttnFusion {
     // first launch; the kernel leaves them zero).  They belong to the caller -- one set per model -- because a captured
     // decode step keeps the pointer.
     unsigned long long* stream_slots = nullptr;
+    const void* rot = nullptr;  // float2 [tokens][hd / 2]: cosine and sine of the step's rotations (launch_embed), for the kernel of batches
 };
 int32_t launch_attention(const float* q, int q_stride, float* out, int n_tok, int n_heads, const KvLayout& kv,
                          const int32_t* tok_seq, const int32_t* tok_pos, const int32_t* page_table, int pages_per_seq, int max_ctx,

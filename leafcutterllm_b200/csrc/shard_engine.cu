@@ -395,7 +395,7 @@ extern "C" int32_t lc_shard_engine_forward(lc_shard_engine* e, const int64_t* to
         LC_CUDA(cudaMemcpyAsync(e->d_pos, pos.data(), (size_t)T * 4, cudaMemcpyHostToDevice, s));
         LC_CUDA(cudaMemcpyAsync(e->d_rope, rope.data(), (size_t)T * 4, cudaMemcpyHostToDevice, s));
         LC_CUDA(cudaStreamSynchronize(s));  // the host vectors die with this iteration
-        LC_TRY(launch_embed(LC_TYPE_F32, e->embed, (size_t)e->V, (size_t)H, e->d_tokens, T, e->d_hidden, s));
+        LC_TRY(launch_embed(LC_TYPE_F32, e->embed, (size_t)e->V, (size_t)H, e->d_tokens, T, e->d_hidden, nullptr, s));
         for (int l = 0; l < e->L; l++) {
             lc_shard_engine::Layer& w = e->layers[l];
             KvLayout kv;

@@ -273,6 +273,30 @@ def test_batched_decode_attention_over_several_context_pieces(gpu, oracle):
     eng.close()
 
 
+@pytest.mark.parametrize("heads,kv", [(4, 4), (4, 2), (4, 1), (8, 1)])
+def test_batched_decode_attention_as_one_stream(gpu, oracle, heads, kv):
+    """The (token, kv head, page) items of a decode step cut into one run per warp: contexts on both sides of a page's edge, a first token, one that many runs
+    share (38 pages), for 1, 2, 4 and 8 query heads per kv head, with rotation by position.  Against the oracle: keys and values of both are
+    rounded to f16 (2^-11 at most), so results that differ by more than four times that (2-norm) are wrong."""
+    from leafcutterllm_b200 import synth
+    spec = small_spec(12, 12, 12, layers=1, hidden=128 * heads, heads=heads, kv=kv, ffn=512, vocab=512)
+    lens = [15, 16, 600, 1, 31, 33, 128]
+    ids = list(range(len(lens)))
+    eng, om = make_pair(gpu, oracle, spec, max_seq_len=640, max_seqs=len(lens), rope_mode="absolute")
+    prompts = [synth.prompt_tokens(n, spec.vocab_size, 400 + i).tolist() for i, n in enumerate(lens)]
+    fed = np.random.default_rng(heads + kv).integers(0, spec.vocab_size, (3, len(lens)))
+    eng.forward_batch(ids, prompts, want_logits=False)
+    got = [eng.forward_batch(ids, [[int(t)] for t in row])[0].copy() for row in fed]
+    eng.close()
+    for i, p in enumerate(prompts):
+        om.kv_clear()
+        om.forward(p)
+        for step, row in enumerate(fed):
+            want = np.asarray(om.forward([int(row[i])]), np.float64)
+            err = np.linalg.norm(got[step][i] - want) / np.linalg.norm(want)
+            assert err < 4 * 2.0 ** -11, (i, step, err)
+
+
 def test_prefill_attention_on_tensor_cores_ragged(gpu, oracle):
     """head_dim 128, f16 cache: calls of 16 tokens and more run the tiled tensor-core prefill attention.  Four sequences of
     70, 16, 129 and 33 tokens in ONE call (tiles end where a sequence ends; 129 = two full tiles and a one-token tile), then a
