@@ -13,6 +13,14 @@
 //   main  += W_hi * X_hi                       one tcgen05.mma with N = 2 * tokens over [X_hi | X_lo] forms the first two,
 //   small += W_hi * X_lo,  small += W_lo * X_hi    a second with N = tokens the third.
 //
+// Q4_K and Q5_K need two: within a 256-element unit, over which `main` runs, a weight's first part (below) is d times the integer sc (q - c) of at most
+// ten bits, which one f16 holds; `main` takes the integers, and the thread that empties it multiplies by d.  Beside X_lo, 2^-11 of X, the weight
+// may be rounded to f16:
+//
+//   main += I * X_hi,  small += f16(d I) * X_lo.
+//
+// (2,048 tokens, 7B shape: 87.5 -> 75.5 ms a prompt with this in place of three products; distance from 64 bits 6.5e-4 -> 4.0e-4, most of it the cache's f16.)
+//
 // The tensor cores truncate when they add to an f32 accumulator: the error grows with the number of additions (measured on
 // N(0,1) products: 3.5e-7 of the result after 256 elements of k, 1.2e-6 after 1024, 9.6e-6 after 8192; 3 terms into one accumulator
 // 1.0e-6 after 256).  So `main`, 2^11 times larger than `small`, is emptied into registers every 128 or 256 elements and those sums are
@@ -35,18 +43,17 @@
 //   producers  one thread requests the activation tiles (64 elements x N tokens, hi and lo, 128-byte swizzle), one the raw blocks of a
 //              256-element unit (TMA boxes of 32 rows; Q6_K's 210-byte blocks have no 16-byte alignment: two warps copy them by words);
 //   unpack     sixteen warps in four groups that take the chunks in turn (two at a time up to 64 tokens): thread r owns row r, turns the chunk's 32
-//              elements into f16 integers by byte permutes, hi = d' q and lo = d' q - hi by two f16x2 instructions (exact), and stores both with
+//              elements into f16 integers by byte permutes, hi = d' q and lo = d' q - hi by two f16x2 instructions (exact; Q4_K, Q5_K: I and d' I), and stores both with
 //              tcgen05.st as the A operand in TENSOR MEMORY (lane = row, column = two consecutive k).  A group has a tensor-memory
 //              stage of its own, so every barrier has one waiter that sees all of its phases;
 //   multiply   one warp, whose elected lane issues;
 //   drain      the unpack warps again: when a run is through, group g adds tokens 32 g ... 32 g + 31 of `main` to its registers, one
 //              run behind its unpacking, so it never waits for the products it feeds.  `main` has two places that runs take in turn.
 //
-// What bounds it: the tensor pipe.  192 cycles per 128 rows x 128 tokens x 16 elements (128 + 64 for the two instructions; measured
-// 128 / 64 / 32 / 13 cycles at N = 256 / 128 / 64 / 16), i.e. a third of the f16 rate.  ncu, 2,048 tokens, Q4_K: tensor pipe active 71 % of the
-// cycles for [4096 -> 12288] (505 us), 68 % for gate and up of 11008 (911 us); issue slots 65 %, two thirds of them unpacking (2.4 instructions per
-// weight, Q6_K five).  512 tokens x [4096 -> 12288]: 138 us, where two products per weight and 64 tokens per CTA (qgemm_umma.cu) took 203.
-// (Before the offsets and fractions of the unpacking above; a 7B prompt takes 0.6 % longer with them.)
+// What bounds it: the tensor pipe where three products count, 192 cycles per 128 rows x 128 tokens x 16 elements (128 + 64 for the two instructions; measured
+// 128 / 64 / 32 / 13 cycles at N = 256 / 128 / 64 / 16), i.e. a third of the f16 rate, 68 - 71 % active.  Q4_K with its two products: 54 % active (ncu, 512 tokens x
+// [4096 -> 12288], 123 us; 138 with three); a unit takes 3,600 cycles, 2,048 of them products, the rest the way from a stage's last product over its
+// refilling to its next first one.
 #include <algorithm>
 #include <cstdlib>
 #include <cuda_fp16.h>
@@ -189,8 +196,10 @@ __device__ __forceinline__ void unpack_chunk(const unsigned char* rp, const Unit
                 uint32_t b = __funnelshift_l(vv[i], vv[i], rot) & (fifth ? 0x78787878u : 0xF0F0F0F0u);
                 if constexpr (fifth) b |= (hb[i] << (7 - j)) & 0x80808080u;
                 const int c = h * 8 + i * 2;
-                split_product(d, h2_fma(bias_pair(b, 0), sc, bias), hi[c], lo[c]);
-                split_product(d, h2_fma(bias_pair(b, 1), sc, bias), hi[c + 1], lo[c + 1]);
+                hi[c] = h2_fma(bias_pair(b, 0), sc, bias);
+                hi[c + 1] = h2_fma(bias_pair(b, 1), sc, bias);
+                lo[c] = h2_mul(d, hi[c]);
+                lo[c + 1] = h2_mul(d, hi[c + 1]);
             }
         }
     } else if constexpr (TYPE == LC_TYPE_Q4_0) {  // mod.rs:16-34: 18 bytes: scale, low nibbles = elements 0..15, high = 16..31
@@ -510,7 +519,16 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
                     const uint32_t st = WIDE ? (2 * c + h) & 3 : c, a = a0 + (WIDE ? st * 32 : st * 64 + h * 32);
                     if (WIDE || h == 0) ok = ok && mbar_wait(&a_full[st], (uint32_t)(WIDE ? c >> 1 : v & 1));  // the stage's uses: WIDE 2 v and 2 v + 1, else v
                     tc_fence_after();
-                    if (one && ok) {
+                    if (one && ok && kHasMin<TYPE>) {
+                        const uint64_t bb = b_both + 4 * h;
+                        umma_f16_ts(d_main, a, bb + to_hi, id1, (uint32_t)!(anew && h == 0));
+                        umma_f16_ts(d_small, a + 16, bb + to_lo, id1, (uint32_t)(v > (two ? 1 : 0) || c > 0 || h > 0));
+                        umma_f16_ts(d_main, a + 8, bb + 2 + to_hi, id1, 1u);
+                        umma_f16_ts(d_small, a + 24, bb + 2 + to_lo, id1, 1u);
+                        if (WIDE || h == 1) umma_commit(&a_empty[st]);
+                        if (h == 1) umma_commit(&b_empty[sb]);
+                        if (h == 1 && end) umma_commit(&d_full[run & 1]);
+                    } else if (one && ok) {
                         const uint64_t bb = b_both + 4 * h;
                         if (anew && h == 0) {  // main
                             umma_f16_ts(d_main, a, bb + to_hi, id1, 0u);
@@ -578,8 +596,12 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
         auto wait_all = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); };
         float y[kOwn];
         constexpr uint32_t kNone = ~0u;
-        // skip: a bit for each token that keeps what it has; also: a second column, whose sums are added to the first's (up to 32 tokens, eight a thread)
-        auto add_columns = [&](uint32_t col, uint32_t also, uint32_t skip) {
+        // times: what the sums are multiplied by; skip: a bit for each token that keeps what it has; also: a second column, whose sums are added to the
+        // first's (up to 32 tokens, eight a thread)
+        auto add_columns = [&](uint32_t col, uint32_t also, float times, uint32_t skip) {
+            auto add = [&](float& to, uint32_t a, uint32_t bit) {
+                if (!((skip >> bit) & 1u)) to = kHasMin<TYPE> ? fmaf(times, __uint_as_float(a), to) : to + __uint_as_float(a);
+            };
             const uint32_t base = lane_base + tbase;
             if constexpr (WIDE) {
 #pragma unroll
@@ -589,7 +611,7 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
                         tmem_ld16(base + col + t0, a);
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                        for (int t = 0; t < 16; t++) y[t0 + t] += (skip >> (t0 + t)) & 1u ? 0.f : __uint_as_float(a[t]);
+                        for (int t = 0; t < 16; t++) add(y[t0 + t], a[t], t0 + t);
                     }
             } else {
                 uint32_t a[16];
@@ -610,18 +632,18 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
                 for (int t0 = 0; t0 < 16; t0 += 4)
                     if (t0 < own) {
 #pragma unroll
-                        for (int t = t0; t < t0 + 4; t++) y[t] += (skip >> t) & 1u ? 0.f : __uint_as_float(a[t]);
+                        for (int t = t0; t < t0 + 4; t++) add(y[t], a[t], t);
                     }
             }
         };
-        auto drain = [&](int q) {  // run q
+        auto drain = [&](int q, float times) {  // run q
             if (own <= 0) return;
             const int place = q & 1;
             ok = wait_all(&d_full[place], (q >> 1) & 1);
             if (!ok) return;
             tc_fence_after();
-            if (two) add_columns((uint32_t)(3 * place * N), chunks_of(q) > 2 ? (uint32_t)((3 * place + 2) * N) : kNone, 0u);
-            else add_columns(place ? kColSmall + (uint32_t)N : kColSmall - (uint32_t)N, kNone, 0u);
+            if (two) add_columns((uint32_t)(3 * place * N), chunks_of(q) > 2 ? (uint32_t)((3 * place + 2) * N) : kNone, times, 0u);
+            else add_columns(place ? kColSmall + (uint32_t)N : kColSmall - (uint32_t)N, kNone, times, 0u);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&d_empty[place]);
@@ -635,6 +657,7 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
         const float down = live ? (mat ? ref1.down : ref0.down)[grow] : 1.0f, up = live ? 1.0f / down : 0.0f;
 #pragma unroll
         for (int t = 0; t < kOwn; t++) y[t] = 0.f;
+        float d_of_run = 1.0f;  // Q4_K, Q5_K: what the unit before is still to be multiplied by
         for (int v = 0; v < nu && ok; v++) {
             ok = wait_all(&raw_full[sr], raw_phase);
             if (!ok) break;
@@ -670,11 +693,12 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
                     if (lane == 0) mbar_arrive(&a_full[g]);
                 }
                 if (halves && (jj || v > 0)) {  // the run before
-                    drain(2 * v + jj - 1);
+                    drain(2 * v + jj - 1, 1.0f);
                     if (!ok) break;
                 }
             }
-            if (!halves && ok && v > 0) drain(v - 1);
+            if (!halves && ok && v > 0) drain(v - 1, d_of_run);
+            d_of_run = head.d;
             if (++sr == RS) { sr = 0; raw_phase ^= 1; }
         }
         for (int v = nu; kHasMin<TYPE> && v < nv && ok; v++) {
@@ -706,9 +730,9 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
                     if (lane == 0) mbar_arrive(&a_full[g]);
                 }
             }
-            if (ok) drain(v - 1);
+            if (ok) drain(v - 1, v == nu ? d_of_run : 1.0f);
         }
-        if (ok) drain(run_of(nv - 1, 3));
+        if (ok) drain(run_of(nv - 1, 3), 1.0f);  // of Q4_K and Q5_K: offsets
         pdl_wait();
         const int t_first = tok0 + tbase, mine = ok ? min(own, tok_end - t_first) : 0;
         // a lane has one token's scale: a load beside each result's store would wait for it
@@ -718,8 +742,8 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
         const uint32_t wild = __ballot_sync(0xffffffffu, scale < 0.f);
         if (ok && own > 0) {  // complete: the last unit's d_full followed every product
             const uint32_t col = two ? (uint32_t)N : kColSmall, also = two && nv > 1 ? (uint32_t)(4 * N) : kNone;
-            if (wild) add_columns(col, also, wild);
-            else add_columns(col, also, 0u);
+            if (wild) add_columns(col, also, 1.0f, wild);
+            else add_columns(col, also, 1.0f, 0u);
         }
         // what `main` lost on average (see the header)
         const float back = down * (1.0f + (halves || two ? 0x1p-23f : 0x1p-22f));
