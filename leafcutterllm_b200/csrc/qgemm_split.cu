@@ -1,4 +1,4 @@
-// Quantised weights (Q4_K, Q5_K, Q6_K, Q4_0, Q8_0) times MANY tokens (prompts, batched decode steps) on the 5th-generation tensor
+// Quantised weights (Q6_K, Q4_0, Q8_0; Q4_K and Q5_K: qgemm_whole.cu) times MANY tokens (prompts, batched decode steps) on the 5th-generation tensor
 // cores: the dense contraction of the path (Tensor::matmul with m > 1, rust/src/tensor.rs:107-135,
 // over weights that the reference dequantises per call, rust/src/model/loader.rs:213-224).
 //
@@ -13,14 +13,6 @@
 //   main  += W_hi * X_hi                       one tcgen05.mma with N = 2 * tokens over [X_hi | X_lo] forms the first two,
 //   small += W_hi * X_lo,  small += W_lo * X_hi    a second with N = tokens the third.
 //
-// Q4_K and Q5_K need two: within a 256-element unit, over which `main` runs, a weight's first part (below) is d times the integer sc (q - c) of at most
-// ten bits, which one f16 holds; `main` takes the integers, and the thread that empties it multiplies by d.  Beside X_lo, 2^-11 of X, the weight
-// may be rounded to f16:
-//
-//   main += I * X_hi,  small += f16(d I) * X_lo.
-//
-// (2,048 tokens, 7B shape: 87.5 -> 75.5 ms a prompt with this in place of three products; distance from 64 bits 6.5e-4 -> 4.0e-4, most of it the cache's f16.)
-//
 // The tensor cores truncate when they add to an f32 accumulator: the error grows with the number of additions (measured on
 // N(0,1) products: 3.5e-7 of the result after 256 elements of k, 1.2e-6 after 1024, 9.6e-6 after 8192; 3 terms into one accumulator
 // 1.0e-6 after 256).  So `main`, 2^11 times larger than `small`, is emptied into registers every 128 or 256 elements and those sums are
@@ -31,106 +23,49 @@
 // Emptying every 128 costs 8 % of a 7B prompt, where the tensor pipe is the bound, and 0.7 % of the short prompts of a small Q4_0 / Q8_0 model,
 // whose matrix-vector kernels add in f32: those have it.  Up to 32 tokens tensor memory has room for two sums of 128 elements each, at no cost.
 //
-// Q4_K / Q5_K weights are d * sc * q - dmin * m = d * sc * (q - c) + (c * d * sc - dmin * m), c the middle of q's range (8 or 16): the first part is the
-// weight above, the second joins as more k: two f16 of a sub-block against the sum of the activations over it, 16 values per 256-element unit, behind
-// the last unit.  About the middle, because with q itself both parts are large and of opposite signs, and the cut-off sums' error with them:
-// 7.0e-7 of the result for normal activations and 7.3e-5 for positive ones at k = 2048, 2.3e-7 and 1.4e-6 about the middle (qgemm_umma.cu's kernel,
-// integers and a drain per unit: 5.5e-7 and 3.2e-5).
-//
 // One CTA owns 128 weight rows (the M of tcgen05.mma; for gate/up 64 rows of each, so that SiLU(gate) * up happens here) and up to 128
 // tokens, and walks k in chunks of 32 elements:
 //
 //   producers  one thread requests the activation tiles (64 elements x N tokens, hi and lo, 128-byte swizzle), one the raw blocks of a
 //              256-element unit (TMA boxes of 32 rows; Q6_K's 210-byte blocks have no 16-byte alignment: two warps copy them by words);
 //   unpack     sixteen warps in four groups that take the chunks in turn (two at a time up to 64 tokens): thread r owns row r, turns the chunk's 32
-//              elements into f16 integers by byte permutes, hi = d' q and lo = d' q - hi by two f16x2 instructions (exact; Q4_K, Q5_K: I and d' I), and stores both with
+//              elements into f16 integers by byte permutes, hi = d' q and lo = d' q - hi by two f16x2 instructions (exact), and stores both with
 //              tcgen05.st as the A operand in TENSOR MEMORY (lane = row, column = two consecutive k).  A group has a tensor-memory
 //              stage of its own, so every barrier has one waiter that sees all of its phases;
 //   multiply   one warp, whose elected lane issues;
 //   drain      the unpack warps again: when a run is through, group g adds tokens 32 g ... 32 g + 31 of `main` to its registers, one
 //              run behind its unpacking, so it never waits for the products it feeds.  `main` has two places that runs take in turn.
 //
-// What bounds it: the tensor pipe where three products count, 192 cycles per 128 rows x 128 tokens x 16 elements (128 + 64 for the two instructions; measured
-// 128 / 64 / 32 / 13 cycles at N = 256 / 128 / 64 / 16), i.e. a third of the f16 rate, 68 - 71 % active.  Q4_K with its two products: 54 % active (ncu, 512 tokens x
-// [4096 -> 12288], 123 us; 138 with three); a unit takes 3,600 cycles, 2,048 of them products, the rest the way from a stage's last product over its
-// refilling to its next first one.
+// What bounds it: the tensor pipe, 192 cycles per 128 rows x 128 tokens x 16 elements (128 + 64 for the two instructions; measured
+// 128 / 64 / 32 / 13 cycles at N = 256 / 128 / 64 / 16), i.e. a third of the f16 rate, 68 - 71 % active, and with few tokens the groups' way around
+// (3,200 cycles a unit).  In qgemm_whole.cu's order (a run's operand behind one barrier) these types are 4 - 7 % slower: their
+// sums are read twice as often.
 #include <algorithm>
 #include <cstdlib>
 #include <cuda_fp16.h>
 #include "lc_kernels.h"
 #include "lc_quant.cuh"
 #include "lc_tma.cuh"
-#include "lc_umma.cuh"
+#include "lc_qgemm.cuh"
 
 namespace lc {
 
 namespace {
 
-constexpr int kRows = 128;       // weight rows per CTA = MMA M
-constexpr int kMaxTok = 128;     // most tokens per CTA
-constexpr int kMaxRaw = 8;       // raw units in flight
 constexpr int kMaxB = 8;         // activation chunks (64 elements) in flight
-constexpr int kGroups = 4;       // unpack groups of four warps
-constexpr int kControl = 4;      // warps ahead of them: activation producer, issuer, raw producer (Q6_K: two)
-constexpr int kThreads = 32 * (kControl + 4 * kGroups);
 // Tensor-memory columns: main of even runs [128 - N, 128), small [128, 128 + N), main of odd runs [128 + N, 128 + 2 N): small borders on
 // both, so that one instruction covers main and small of either (odd runs have their activations as [lo | hi]).  Behind them
 // the A stages, 32 columns each: 16 of W_hi, 16 of W_lo for 32 elements of k; four, or eight where 64 tokens and fewer leave the room.
 constexpr uint32_t kColSmall = 128;
 __host__ __device__ constexpr uint32_t col_a(int N) { return N <= 64 ? 256u : 384u; }
 
-template <uint32_t TYPE> struct RawUnit;  // bytes of a row's unit in shared memory
-template <> struct RawUnit<LC_TYPE_Q4_K> { static constexpr int pitch = 144; };
-template <> struct RawUnit<LC_TYPE_Q5_K> { static constexpr int pitch = 176; };
-template <> struct RawUnit<LC_TYPE_Q4_0> { static constexpr int pitch = 144; };
-template <> struct RawUnit<LC_TYPE_Q8_0> { static constexpr int pitch = 272; };
-template <> struct RawUnit<LC_TYPE_Q6_K> { static constexpr int pitch = 212; };  // 210 from a word boundary on; an odd number of words: no bank conflicts
 // `main` over half a unit at a time (see the header): as runs of their own ...
 template <uint32_t TYPE, bool WIDE> constexpr bool kHalves = WIDE && (TYPE == LC_TYPE_Q4_0 || TYPE == LC_TYPE_Q8_0);
 // ... or, where tensor memory has room, as two sums of one run: then sets of [main of the first half | small | main of the second], for even units
 // from column 0 on and for odd units behind it
 constexpr int kTwoSums = 32;  // most tokens
-template <uint32_t TYPE> constexpr bool kHasMin = TYPE == LC_TYPE_Q4_K || TYPE == LC_TYPE_Q5_K;
 
-struct GemmParams {
-    float* out;             // [T, n]
-    const float* residual;  // or null
-    const float* tok_scale; // [T] power of two that the preparation divided token t by
-    const float* row_down0; // [n] power of two that brings row r's weights back (and of the second matrix)
-    const float* row_down1;
-    const unsigned char *w0, *w1;  // raw blocks
-    size_t row_bytes;
-    int n, k, T;
-    int N;                  // tokens per CTA, a multiple of 16: the box height of the activation tensor maps
-    int epi;                // GemvEpilogue; EPI_SILU_MUL: 64 rows of each matrix per CTA
-    int raw_stages, b_stages;
-    int ksplit;             // CTAs along k per tile (gridDim.z)
-    int row_dynamic;        // row_down comes from a kernel ahead of this one in the stream
-    float* partial;         // [ksplit][matrices][T][n] f32 for the summing kernel, or null: the CTA holds the whole sum and writes `out`
-    // the experts of a mixture layer (see GemmGroup): activation rows in expert order, expert e's from offsets[e] on; null for a plain product
-    const CUtensorMap *maps0, *maps1;
-    const ExpertRef *refs0, *refs1;
-    const int32_t* offsets;
-    const int32_t* row_map; // row of `out` that activation row r's result goes to (null: r)
-    int n_experts;
-    int* error_flag;
-};
-
-// ---- tcgen05 wrappers -------------------------------------------------------------------------------------------------
-__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t* r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
-}
-__device__ __forceinline__ bool elect_one() {
-    uint32_t r;
-    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(r));
-    return r != 0;
-}
 // ---- unpacking ---------------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t h2_mul(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-}
 __device__ __forceinline__ uint32_t h2_neg(uint32_t a) { return a ^ 0x80008000u; }
 __device__ __forceinline__ uint32_t f16_at(const unsigned char* p) { return *reinterpret_cast<const uint16_t*>(p); }
 // words [0, OUT) of the bytes that begin `shift` (even, below 16) bytes into w; `shift` is the same for the whole warp
@@ -156,53 +91,14 @@ __device__ __forceinline__ void split_product(uint32_t s, uint32_t q, uint32_t& 
 // Elements 32 j ... 32 j + 31 of a row's unit times `up`, as f16 pairs: column c holds elements 2 c and 2 c + 1.  The integer's factor is a power of two
 // that brings it to about 1 and the scale's the inverse: the scale, rounded to f16 before the product, then keeps its bits down to 2^-28 of the row's
 // largest (with whole integers to 2^-18 in Q4_K, and an error there that counted 945 times).
-// Q4_K (mod.rs:66-98): sub-block j has the low (even j) or high nibbles of bytes 32 (j / 2) ... under scale sc[j]; the nibbles are brought up to
-// 16 q, and (1024 + 16 q) (sc / 2^14) - 1152 (sc / 2^14) is one fused multiply-add with the exact result sc (q - 8) / 2^10: 1152 = 9 * 2^7 and a scale of
-// six bits make a constant that f16 holds, 1032 would not.  Q5_K (mod.rs:101-142): a fifth bit; 8 q and sc / 2^13 likewise.
-struct UnitHead { float d; uint32_t sc_lo, sc_hi; };  // d times `up` and the integer's factor, the eight scales (of the types that have them)
+// Q6_K: d times `up` and the integer's factor
 template <uint32_t TYPE>
-__device__ __forceinline__ UnitHead load_head(const unsigned char* rp, float up) {
-    UnitHead h{0.f, 0u, 0u};
-    if constexpr (kHasMin<TYPE>) {
-        const uint4 w = *reinterpret_cast<const uint4*>(rp);  // d, dmin, 12 scale bytes
-        uint32_t mn_lo, mn_hi;
-        unpack_scales_k4(w.y, w.z, w.w, &h.sc_lo, &h.sc_hi, &mn_lo, &mn_hi);
-        h.d = h2f((uint16_t)(w.x & 0xFFFFu)) * up * 1024.f;
-    } else if constexpr (TYPE == LC_TYPE_Q6_K) {
-        h.d = h2f((uint16_t)f16_at(rp + 208)) * up * 32.f;
-    }
-    return h;
+__device__ __forceinline__ float load_head(const unsigned char* rp, float up) {
+    return TYPE == LC_TYPE_Q6_K ? h2f((uint16_t)f16_at(rp + 208)) * up * 32.f : 0.f;
 }
 template <uint32_t TYPE>
-__device__ __forceinline__ void unpack_chunk(const unsigned char* rp, const UnitHead& head, int j, float up, uint32_t (&hi)[16], uint32_t (&lo)[16]) {
-    if constexpr (kHasMin<TYPE>) {
-        constexpr bool fifth = TYPE == LC_TYPE_Q5_K;
-        const float fs = (float)(((j < 4 ? head.sc_lo : head.sc_hi) >> (8 * (j & 3))) & 0xFFu) * (fifth ? 0x1p-13f : 0x1p-14f);
-        const uint32_t d = h2_pair(head.d), sc = h2_pair(fs), bias = h2_pair(-1152.0f * fs);
-        const uint4* q = reinterpret_cast<const uint4*>(rp + (fifth ? 48 : 16) + 32 * (j >> 1));
-        // the nibbles to bits 4 - 7 of their bytes, with a fifth bit to 3 - 6 (what the rotation brings from other bytes is masked out)
-        const uint32_t rot = fifth ? (j & 1 ? 31 : 3) : (j & 1 ? 0 : 4);
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const uint4 v = q[h];
-            const uint32_t vv[4] = {v.x, v.y, v.z, v.w};
-            uint32_t hb[4] = {0u, 0u, 0u, 0u};
-            if constexpr (fifth) {
-                const uint4 hq = *reinterpret_cast<const uint4*>(rp + 16 + 16 * h);
-                hb[0] = hq.x; hb[1] = hq.y; hb[2] = hq.z; hb[3] = hq.w;
-            }
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                uint32_t b = __funnelshift_l(vv[i], vv[i], rot) & (fifth ? 0x78787878u : 0xF0F0F0F0u);
-                if constexpr (fifth) b |= (hb[i] << (7 - j)) & 0x80808080u;
-                const int c = h * 8 + i * 2;
-                hi[c] = h2_fma(bias_pair(b, 0), sc, bias);
-                hi[c + 1] = h2_fma(bias_pair(b, 1), sc, bias);
-                lo[c] = h2_mul(d, hi[c]);
-                lo[c + 1] = h2_mul(d, hi[c + 1]);
-            }
-        }
-    } else if constexpr (TYPE == LC_TYPE_Q4_0) {  // mod.rs:16-34: 18 bytes: scale, low nibbles = elements 0..15, high = 16..31
+__device__ __forceinline__ void unpack_chunk(const unsigned char* rp, float head, int j, float up, uint32_t (&hi)[16], uint32_t (&lo)[16]) {
+    if constexpr (TYPE == LC_TYPE_Q4_0) {  // mod.rs:16-34: 18 bytes: scale, low nibbles = elements 0..15, high = 16..31
         const int at = 18 * j;
         const uint4* p = reinterpret_cast<const uint4*>(rp + (at & ~15));
         const uint4 a = p[0], b = p[1];  // j <= 7: the block ends within two pieces (at most byte 14 + 18 of them)
@@ -242,7 +138,7 @@ __device__ __forceinline__ void unpack_chunk(const unsigned char* rp, const Unit
         uint32_t sh[2], sl[2];
 #pragma unroll
         for (int i = 0; i < 2; i++) {  // d sc has 18 bits: two f16
-            const float s = head.d * (float)*reinterpret_cast<const int8_t*>(rp + 192 + 8 * n + 2 * quad + i);
+            const float s = head * (float)*reinterpret_cast<const int8_t*>(rp + 192 + 8 * n + 2 * quad + i);
             const float top = __half2float(__float2half_rn(s));
             sh[i] = h2_pair(s);
             sl[i] = h2_pair(s - top);
@@ -261,30 +157,6 @@ __device__ __forceinline__ void unpack_chunk(const unsigned char* rp, const Unit
         }
     }
 }
-// The offset operand of a unit: p[i] = c * d * sc[i] - dmin * m[i], hi = f16(p) and lo = f16(p - hi).  Columns 0-3: the eight hi
-// as pairs (k' = 0..7), columns 4-7: the eight lo (k' = 8..15); the sums tile holds each sub-block sum at k' and k' + 8.
-template <uint32_t TYPE>
-__device__ __forceinline__ void unpack_mins(uint4 w, float up, uint32_t* col) {
-    uint32_t sc_lo, sc_hi, mn_lo, mn_hi;
-    unpack_scales_k4(w.y, w.z, w.w, &sc_lo, &sc_hi, &mn_lo, &mn_hi);
-    const float dmin = h2f((uint16_t)(w.x >> 16)) * up, mid = h2f((uint16_t)(w.x & 0xFFFFu)) * up * (TYPE == LC_TYPE_Q5_K ? 16.f : 8.f);
-#pragma unroll
-    for (int j2 = 0; j2 < 4; j2++) {
-        __half hi[2], lo[2];
-#pragma unroll
-        for (int e = 0; e < 2; e++) {
-            const int i = 2 * j2 + e;
-            const uint32_t sh = 8 * (i & 3), sc = ((i < 4 ? sc_lo : sc_hi) >> sh) & 0xFFu, mn = ((i < 4 ? mn_lo : mn_hi) >> sh) & 0xFFu;
-            const float pr = fmaf(mid, (float)sc, -dmin * (float)mn);  // both products are exact, so this rounds once
-            hi[e] = __float2half_rn(pr);
-            lo[e] = __float2half_rn(pr - __half2float(hi[e]));
-        }
-        const __half2 a = __halves2half2(hi[0], hi[1]), b = __halves2half2(lo[0], lo[1]);
-        col[j2] = *reinterpret_cast<const uint32_t*>(&a);
-        col[4 + j2] = *reinterpret_cast<const uint32_t*>(&b);
-    }
-}
-
 // ---- row scales ----------------------------------------------------------------------------------------------------------
 // A power of two per row that brings its weights up to 2^13 ... 2^14 (Q4_K and Q5_K rows whose largest scales belong to blocks of small sc: less): the low
 // half of a weight then keeps its bits above 2^-24, f16's smallest step, unless it is 2^-17 of the row's largest.  One warp per row; down[r] = 2^-s.
@@ -331,16 +203,16 @@ __global__ void __launch_bounds__(256) row_scale_kernel(uint32_t typ, const unsi
 
 // grid = (row tiles, token tiles, shares of k).  tm0 / tm1: raw blocks of the
 // matrix (and of `up` for EPI_SILU_MUL), box = one unit x 32 rows.  tmx: the prepared activations [2 halves][t_cap rows][k] f16, box = 64
-// elements x N rows of one half; tms: the sub-block sums [2][t_cap rows][k / 16], the same box.
+// elements x N rows of one half.
 // WIDE: more than 64 tokens.  Sub-chunk j (32 elements) of a unit then belongs to group j & 3, stage by stage; else group g has the 64 elements
 // from 64 g on as one stage, so that the issuer waits half as often for products that are soon over.
 template <uint32_t TYPE, bool WIDE>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kGemmThreads, 1)
 qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1, const __grid_constant__ CUtensorMap tmx,
-                  const __grid_constant__ CUtensorMap tms, GemmParams p) {
+                   GemmParams p) {
     constexpr int kPitch = RawUnit<TYPE>::pitch;
     constexpr bool kWords = TYPE == LC_TYPE_Q6_K;  // raw units copied by words
-    constexpr uint32_t raw_bytes = kPitch * kRows;
+    constexpr uint32_t raw_bytes = kPitch * kGemmRows;
     constexpr int kOwn = WIDE ? 32 : 16;           // tokens whose sums a thread keeps
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -349,7 +221,7 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
     const int N = p.N;
     const int RS = p.raw_stages, BS = p.b_stages;
     const uint32_t b_half = (uint32_t)N * 128u;
-    const int row0 = blockIdx.x * (pair ? kRows / 2 : kRows), nquads = (p.k / kUnitElems + 3) / 4;
+    const int row0 = blockIdx.x * (pair ? kGemmRows / 2 : kGemmRows), nunits = p.k / kUnitElems;
     int tok0 = blockIdx.y * N, tok_end = p.T;
     const CUtensorMap *map0 = &tm0, *map1 = &tm1;
     ExpertRef ref0{p.w0, p.row_down0}, ref1{p.w1, p.row_down1};
@@ -370,9 +242,9 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
     unsigned char* bt = smem;                          // [BS][two tiles of N x 128 B]
     unsigned char* raw = bt + (size_t)BS * 2 * b_half;  // [RS][raw_bytes]
     uint64_t* bars = reinterpret_cast<uint64_t*>(raw + (size_t)RS * raw_bytes);
-    uint64_t* raw_full = bars;                 // [kMaxRaw] producer -> unpack
-    uint64_t* raw_empty = raw_full + kMaxRaw;  // [kMaxRaw] unpack (a warp each) -> producer
-    uint64_t* b_full = raw_empty + kMaxRaw;    // [kMaxB]   producer -> issuer
+    uint64_t* raw_full = bars;                 // [kGemmRaw] producer -> unpack
+    uint64_t* raw_empty = raw_full + kGemmRaw;  // [kGemmRaw] unpack (a warp each) -> producer
+    uint64_t* b_full = raw_empty + kGemmRaw;    // [kMaxB]   producer -> issuer
     uint64_t* b_empty = b_full + kMaxB;        // [kMaxB]   commit -> producer
     uint64_t* a_full = b_empty + kMaxB;        // [4]       a group's four warps -> issuer
     uint64_t* a_empty = a_full + 4;            // [4]       commit -> that group
@@ -381,11 +253,11 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
     uint64_t* wound = d_empty + 2;             // [1]       products in flight when a wait of the issuer ran out
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(wound + 1);
 
-    const int drains = WIDE ? 4 * ((N + 31) / 32) : 4 * kGroups;  // warps that keep sums
+    const int drains = WIDE ? 4 * ((N + 31) / 32) : 4 * kGemmGroups;  // warps that keep sums
     if (warp == 0 && lane == 0) {
-        for (int i = 0; i < kMaxRaw; i++) { mbar_init(&raw_full[i], kWords ? 64 : 1); mbar_init(&raw_empty[i], 4 * kGroups); }
+        for (int i = 0; i < kGemmRaw; i++) { mbar_init(&raw_full[i], kWords ? 64 : 1); mbar_init(&raw_empty[i], 4 * kGemmGroups); }
         for (int i = 0; i < kMaxB; i++) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
-        for (int i = 0; i < kGroups; i++) { mbar_init(&a_full[i], 4); mbar_init(&a_empty[i], 1); }
+        for (int i = 0; i < kGemmGroups; i++) { mbar_init(&a_full[i], 4); mbar_init(&a_empty[i], 1); }
         for (int i = 0; i < 2; i++) { mbar_init(&d_full[i], 1); mbar_init(&d_empty[i], drains); }
         mbar_init(wound, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -398,12 +270,8 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
     const uint32_t tmem = *tmem_slot;
     bool ok = true;
 
-    // this CTA's share of k: whole groups of four units (one chunk of sub-block sums); unit v below is u_begin + v
-    const int u_begin = (int)((long long)blockIdx.z * nquads / p.ksplit) * 4;
-    const int nu = min((int)((long long)(blockIdx.z + 1) * nquads / p.ksplit) * 4, p.k / kUnitElems) - u_begin;
-    const int sum_chunks = kHasMin<TYPE> ? (nu + 3) / 4 : 0;  // chunks of sub-block sums behind the units, four units each,
-    const int nv = nu + (sum_chunks + 3) / 4;                 // as further units of up to four chunks
-    auto chunks_of = [&](int v) { return v < nu ? 4 : min(4, sum_chunks - 4 * (v - nu)); };
+    // this CTA's share of k in units; unit v below is u_begin + v
+    const int u_begin = (int)((long long)blockIdx.z * nunits / p.ksplit), nu = (int)((long long)(blockIdx.z + 1) * nunits / p.ksplit) - u_begin;
     constexpr bool halves = kHalves<TYPE, WIDE>;
     const bool two = !WIDE && N <= kTwoSums;
     auto run_of = [&](int v, int c) { return halves ? 2 * v + (c >> 1) : v; };  // of `main`, which has two places that the runs take in turn
@@ -416,17 +284,15 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
             pdl_wait();
             int sb = 0, in_flight = 0;
             uint32_t phase = 1;
-            for (int v = 0; v < nv && ok; v++) {
-                const int nc = chunks_of(v);
-                for (int c = 0; c < nc; c++) {
+            for (int v = 0; v < nu && ok; v++) {
+                for (int c = 0; c < 4; c++) {
                     if (!mbar_wait(&b_empty[sb], phase)) { ok = false; break; }
-                    const CUtensorMap* m = v < nu ? &tmx : &tms;
-                    const int x = v < nu ? (u_begin + v) * kUnitElems + c * 64 : (u_begin / 4 + (v - nu) * 4 + c) * 64;
+                    const int x = (u_begin + v) * kUnitElems + c * 64;
                     unsigned char* const tile = bt + (size_t)sb * 2 * b_half;
                     const int odd = swapped(v, c);
                     mbar_expect_tx(&b_full[sb], 2 * b_half);
-                    tma_load_3d(tile + odd * b_half, m, x, tok0, 0, &b_full[sb]);
-                    tma_load_3d(tile + (1 - odd) * b_half, m, x, tok0, 1, &b_full[sb]);
+                    tma_load_3d(tile + odd * b_half, &tmx, x, tok0, 0, &b_full[sb]);
+                    tma_load_3d(tile + (1 - odd) * b_half, &tmx, x, tok0, 1, &b_full[sb]);
                     in_flight = min(in_flight + 1, BS);
                     if (++sb == BS) { sb = 0; phase ^= 1; }
                 }
@@ -519,16 +385,7 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
                     const uint32_t st = WIDE ? (2 * c + h) & 3 : c, a = a0 + (WIDE ? st * 32 : st * 64 + h * 32);
                     if (WIDE || h == 0) ok = ok && mbar_wait(&a_full[st], (uint32_t)(WIDE ? c >> 1 : v & 1));  // the stage's uses: WIDE 2 v and 2 v + 1, else v
                     tc_fence_after();
-                    if (one && ok && kHasMin<TYPE>) {
-                        const uint64_t bb = b_both + 4 * h;
-                        umma_f16_ts(d_main, a, bb + to_hi, id1, (uint32_t)!(anew && h == 0));
-                        umma_f16_ts(d_small, a + 16, bb + to_lo, id1, (uint32_t)(v > (two ? 1 : 0) || c > 0 || h > 0));
-                        umma_f16_ts(d_main, a + 8, bb + 2 + to_hi, id1, 1u);
-                        umma_f16_ts(d_small, a + 24, bb + 2 + to_lo, id1, 1u);
-                        if (WIDE || h == 1) umma_commit(&a_empty[st]);
-                        if (h == 1) umma_commit(&b_empty[sb]);
-                        if (h == 1 && end) umma_commit(&d_full[run & 1]);
-                    } else if (one && ok) {
+                    if (one && ok) {
                         const uint64_t bb = b_both + 4 * h;
                         if (anew && h == 0) {  // main
                             umma_f16_ts(d_main, a, bb + to_hi, id1, 0u);
@@ -549,45 +406,14 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
                 if (++sb == BS) { sb = 0; b_phase ^= 1; b_both = b_first; }
             }
         }
-        for (int v = nu; kHasMin<TYPE> && v < nv && ok; v++) {  // the offsets: no low halves beside the high ones
-            const int nc = chunks_of(v);
-            for (int c = 0; c < nc && ok; c++) {
-                const uint32_t d_small = small_of(v), odd = (uint32_t)swapped(v, c);
-                const uint32_t d_both = odd ? d_small : d_small - (uint32_t)N, d_main = odd ? d_small + (uint32_t)N : d_both;
-                if (c == 0 && v >= 2) ok = mbar_wait(&d_empty[v & 1], (v / 2 - 1) & 1);  // these types' runs are units
-                ok = ok && mbar_wait(&b_full[sb], b_phase);
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const uint32_t st = WIDE ? (2 * c + h) & 3 : c, a = a0 + (WIDE ? st * 32 : st * 64 + h * 32);
-                    if (WIDE || h == 0) ok = ok && mbar_wait(&a_full[st], (uint32_t)(WIDE ? c >> 1 : v & 1));
-                    tc_fence_after();
-                    if (one && ok) {
-                        const uint64_t bb = b_both + 4 * h;
-                        if ((c == 0 || (two && c == 2)) && h == 0) {
-                            umma_f16_ts(d_main, a, bb + (odd ? b_tile : 0), id1, 0u);
-                            umma_f16_ts(d_small, a, bb + (odd ? 0 : b_tile), id1, (uint32_t)(v > (two ? 1 : 0) || c > 0));
-                        } else {
-                            umma_f16_ts(d_both, a, bb, id2, 1u);
-                        }
-                        umma_f16_ts(d_both, a + 8, bb + 2, id2, 1u);
-                        if (WIDE || h == 1) umma_commit(&a_empty[st]);
-                        if (h == 1) umma_commit(&b_empty[sb]);
-                        if (h == 1 && c == nc - 1) umma_commit(&d_full[v & 1]);
-                    }
-                    __syncwarp();
-                }
-                b_both += b_step;
-                if (++sb == BS) { sb = 0; b_phase ^= 1; b_both = b_first; }
-            }
-        }
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) {
             if (one) umma_commit(wound);
             mbar_wait(wound, 0);
         }
-    } else if (warp >= kControl) {
+    } else if (warp >= kGemmControl) {
         // ---------------------------------------------------------------- unpack and drain, then the epilogue
-        const int g = (warp - kControl) >> 2, quarter = warp & 3;
+        const int g = (warp - kGemmControl) >> 2, quarter = warp & 3;
         const int row = quarter * 32 + lane;  // of the tile; also the tensor-memory lane
         const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16), a_stage = lane_base + col_a(N) + (uint32_t)g * (WIDE ? 32 : 64);
         const int mat = pair ? quarter >> 1 : 0;
@@ -596,12 +422,8 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
         auto wait_all = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); };
         float y[kOwn];
         constexpr uint32_t kNone = ~0u;
-        // times: what the sums are multiplied by; skip: a bit for each token that keeps what it has; also: a second column, whose sums are added to the
-        // first's (up to 32 tokens, eight a thread)
-        auto add_columns = [&](uint32_t col, uint32_t also, float times, uint32_t skip) {
-            auto add = [&](float& to, uint32_t a, uint32_t bit) {
-                if (!((skip >> bit) & 1u)) to = kHasMin<TYPE> ? fmaf(times, __uint_as_float(a), to) : to + __uint_as_float(a);
-            };
+        // skip: a bit for each token that keeps what it has; also: a second column, whose sums are added to the first's (up to 32 tokens, eight a thread)
+        auto add_columns = [&](uint32_t col, uint32_t also, uint32_t skip) {
             const uint32_t base = lane_base + tbase;
             if constexpr (WIDE) {
 #pragma unroll
@@ -611,7 +433,7 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
                         tmem_ld16(base + col + t0, a);
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                        for (int t = 0; t < 16; t++) add(y[t0 + t], a[t], t0 + t);
+                        for (int t = 0; t < 16; t++) y[t0 + t] += (skip >> (t0 + t)) & 1u ? 0.f : __uint_as_float(a[t]);
                     }
             } else {
                 uint32_t a[16];
@@ -632,18 +454,18 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
                 for (int t0 = 0; t0 < 16; t0 += 4)
                     if (t0 < own) {
 #pragma unroll
-                        for (int t = t0; t < t0 + 4; t++) add(y[t], a[t], t);
+                        for (int t = t0; t < t0 + 4; t++) y[t] += (skip >> t) & 1u ? 0.f : __uint_as_float(a[t]);
                     }
             }
         };
-        auto drain = [&](int q, float times) {  // run q
+        auto drain = [&](int q) {  // run q
             if (own <= 0) return;
             const int place = q & 1;
             ok = wait_all(&d_full[place], (q >> 1) & 1);
             if (!ok) return;
             tc_fence_after();
-            if (two) add_columns((uint32_t)(3 * place * N), chunks_of(q) > 2 ? (uint32_t)((3 * place + 2) * N) : kNone, times, 0u);
-            else add_columns(place ? kColSmall + (uint32_t)N : kColSmall - (uint32_t)N, kNone, times, 0u);
+            if (two) add_columns((uint32_t)(3 * place * N), (uint32_t)((3 * place + 2) * N), 0u);
+            else add_columns(place ? kColSmall + (uint32_t)N : kColSmall - (uint32_t)N, kNone, 0u);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&d_empty[place]);
@@ -657,13 +479,12 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
         const float down = live ? (mat ? ref1.down : ref0.down)[grow] : 1.0f, up = live ? 1.0f / down : 0.0f;
 #pragma unroll
         for (int t = 0; t < kOwn; t++) y[t] = 0.f;
-        float d_of_run = 1.0f;  // Q4_K, Q5_K: what the unit before is still to be multiplied by
         for (int v = 0; v < nu && ok; v++) {
             ok = wait_all(&raw_full[sr], raw_phase);
             if (!ok) break;
             const unsigned char* rp = raw + (size_t)sr * raw_bytes + (size_t)row * kPitch;
             if constexpr (kWords) rp += (uint32_t)(uintptr_t)(wrow + (size_t)(u_begin + v) * 210) & 2u;
-            const UnitHead head = load_head<TYPE>(rp, up);
+            const float head = load_head<TYPE>(rp, up);
 #pragma unroll 1
             for (int jj = 0; jj < 2; jj++) {
                 if (!WIDE && jj == 0) {  // the products of the stage's use before are complete
@@ -693,46 +514,14 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
                     if (lane == 0) mbar_arrive(&a_full[g]);
                 }
                 if (halves && (jj || v > 0)) {  // the run before
-                    drain(2 * v + jj - 1, 1.0f);
+                    drain(2 * v + jj - 1);
                     if (!ok) break;
                 }
             }
-            if (!halves && ok && v > 0) drain(v - 1, d_of_run);
-            d_of_run = head.d;
+            if (!halves && ok && v > 0) drain(v - 1);
             if (++sr == RS) { sr = 0; raw_phase ^= 1; }
         }
-        for (int v = nu; kHasMin<TYPE> && v < nv && ok; v++) {
-            // the offset operand: two units' sixteen values per sub-chunk, from their headers in global memory (L2: the units passed through it)
-            const int last_j = 2 * chunks_of(v);
-#pragma unroll 1
-            for (int jj = 0; jj < 2; jj++) {
-                const int j = WIDE ? g + 4 * jj : 2 * g + jj;
-                if (j >= last_j) break;
-                if (WIDE || jj == 0) {
-                    ok = wait_all(&a_empty[g], a_phase);
-                    if (!ok) break;
-                    a_phase ^= 1;
-                    tc_fence_after();
-                }
-                const int u = u_begin + ((v - nu) * 4 + (j >> 1)) * 4 + (j & 1) * 2;
-                uint32_t col[16];
-#pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    uint4 hd = make_uint4(0u, 0u, 0u, 0u);
-                    if (live && u + e < u_begin + nu) hd = *reinterpret_cast<const uint4*>(wrow + (size_t)(u + e) * kPitch);
-                    unpack_mins<TYPE>(hd, up, col + 8 * e);
-                }
-                tmem_st16(a_stage + (WIDE ? 0 : jj * 32), col);
-                if (WIDE || jj == 1) {
-                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&a_full[g]);
-                }
-            }
-            if (ok) drain(v - 1, v == nu ? d_of_run : 1.0f);
-        }
-        if (ok) drain(run_of(nv - 1, 3), 1.0f);  // of Q4_K and Q5_K: offsets
+        if (ok) drain(run_of(nu - 1, 3));
         pdl_wait();
         const int t_first = tok0 + tbase, mine = ok ? min(own, tok_end - t_first) : 0;
         // a lane has one token's scale: a load beside each result's store would wait for it
@@ -741,60 +530,16 @@ qgemm_split_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
         // wherever W_lo is zero.
         const uint32_t wild = __ballot_sync(0xffffffffu, scale < 0.f);
         if (ok && own > 0) {  // complete: the last unit's d_full followed every product
-            const uint32_t col = two ? (uint32_t)N : kColSmall, also = two && nv > 1 ? (uint32_t)(4 * N) : kNone;
-            if (wild) add_columns(col, also, 1.0f, wild);
-            else add_columns(col, also, 1.0f, 0u);
+            const uint32_t col = two ? (uint32_t)N : kColSmall, also = two && nu > 1 ? (uint32_t)(4 * N) : kNone;
+            if (wild) add_columns(col, also, wild);
+            else add_columns(col, also, 0u);
         }
         // what `main` lost on average (see the header)
         const float back = down * (1.0f + (halves || two ? 0x1p-23f : 0x1p-22f));
         // two multiplications: the product of the powers may leave f32's range where the result does not
 #pragma unroll
         for (int t = 0; t < kOwn; t++) y[t] = (y[t] * back) * fabsf(__shfl_sync(0xffffffffu, scale, t));
-        if (p.partial) {
-            float* dst = p.partial + ((size_t)(blockIdx.z * (pair ? 2 : 1) + mat) * p.T + t_first) * p.n + grow;
-#pragma unroll
-            for (int t = 0; t < kOwn; t++)
-                if (live && t < mine) dst[(size_t)t * p.n] = y[t];
-        } else if (pair) {
-            // rows 0 .. 63 of the tile are gate, 64 .. 127 up: the halves meet in the activation stages, which nothing uses any more
-            float* const ex = reinterpret_cast<float*>(bt) + (size_t)tbase * 64 + (row & 63);
-            float* const dst = p.out + (size_t)t_first * p.n + grow;
-            if (mat == 0) {
-#pragma unroll
-                for (int t = 0; t < kOwn; t++)
-                    if (t < mine) ex[t * 64] = silu_f(y[t]);
-            }
-            asm volatile("bar.sync %0, 128;" ::"r"(1 + g) : "memory");  // all of the group's warps come here, whatever their waits gave
-            if (mat == 1) {
-#pragma unroll
-                for (int t = 0; t < kOwn; t++)
-                    if (live && t < mine) dst[(size_t)t * p.n] = __fmul_rn(ex[t * 64], y[t]);
-            }
-        } else if (p.row_map) {
-            const int to = lane < mine ? __ldg(p.row_map + t_first + lane) : 0;
-#pragma unroll
-            for (int t = 0; t < kOwn; t++) {
-                const int r = __shfl_sync(0xffffffffu, to, t);
-                if (live && t < mine) p.out[(size_t)r * p.n + grow] = y[t];
-            }
-        } else {
-            const size_t o = (size_t)t_first * p.n + grow;
-            if (p.epi == EPI_ADD_RESIDUAL) {
-                // the loads of sixteen tokens together (`residual` may be `out`): one beside each store takes a trip to L2 for each,
-                // 244 us against 197 without a residual for 2,048 tokens x [4096 -> 4096]
-#pragma unroll
-                for (int t0 = 0; t0 < kOwn; t0 += 16) {
-                    float r[16];
-#pragma unroll
-                    for (int t = 0; t < 16; t++) r[t] = live && t0 + t < mine ? p.residual[o + (size_t)(t0 + t) * p.n] : 0.f;
-#pragma unroll
-                    for (int t = 0; t < 16; t++) y[t0 + t] = __fadd_rn(r[t], y[t0 + t]);
-                }
-            }
-#pragma unroll
-            for (int t = 0; t < kOwn; t++)
-                if (live && t < mine) p.out[o + (size_t)t * p.n] = y[t];
-        }
+        store_sums<kOwn>(p, y, bt, pair, mat, g, row, grow, live, t_first, tbase, mine);
     }
     if (!ok && p.error_flag) atomicCAS(p.error_flag, 0, 3);
     tc_fence_before();
@@ -822,58 +567,33 @@ int32_t launch_row_scales(const QWeight& w, float* down, cudaStream_t s) {
 }
 
 namespace {
-struct GemmShape { int N, raw_stages, b_stages; size_t smem; };
-// Tokens per CTA: the fewest tiles, filled evenly.  Stages: five activation chunks (with few tokens eight) and the raw units that fit.
-template <uint32_t TYPE>
-GemmShape shape_for(int T) {
-    GemmShape g;
-    const int tt = (T + kMaxTok - 1) / kMaxTok;
-    g.N = (((T + tt - 1) / tt) + 15) & ~15;
-    const size_t raw = (size_t)RawUnit<TYPE>::pitch * kRows, fixed = 1024 + 512, b = (size_t)2 * g.N * 128;
-    g.b_stages = g.N <= 64 ? kMaxB : 5;
-    while (g.b_stages > 3 && fixed + g.b_stages * b + 3 * raw > kMaxSmem) g.b_stages--;
-    g.raw_stages = std::min<int>(kMaxRaw, (int)((kMaxSmem - fixed - g.b_stages * b) / raw));
-    g.smem = fixed + g.b_stages * b + g.raw_stages * raw;
-    return g;
-}
-// Cycles per 256-element unit, 16 pairs of products: the tensor pipe's N / 2 and N, but no less than about 45 each, the pace at which products are issued
-// (57 by a lone lane, see the issuing loop; the pipe itself would take 13 at N = 16).  An estimate, like the fixed costs below: it ranks the shares of k.
-long unit_cycles(int N) {
-    const long one = std::max(45, N / 2), two = std::max(45, N);
-    return 16 * (one + two);
-}
+// Cycles of a unit (k = 4096, one wave): 3,200 for five tokens, 3,500 for 64, 4,000 for 96, 4,400 for 128, of which products are 16 * 3 N / 2.
+double unit_cycles(int N) { return 2950 + 11.4 * N; }
+constexpr double kFixedCycles = 8000;
 
 template <uint32_t TYPE>
 int32_t launch_type(const GemvArgs& a, const GemmWorkspace& ws, GemmParams& p, const GemmGroup* group, int* summed_slices, cudaStream_t s) {
-    const GemmShape g = shape_for<TYPE>(group ? group->typical : p.T);
-    p.N = g.N; p.raw_stages = g.raw_stages; p.b_stages = g.b_stages;
-    auto kern = g.N <= 64 ? qgemm_split_kernel<TYPE, false> : qgemm_split_kernel<TYPE, true>;
-    LC_CUDA(ensure_smem_limit((const void*)kern, g.smem));
-    alignas(64) CUtensorMap tmx, tms;
+    const int nmat = a.epi == EPI_SILU_MUL ? 2 : 1, tiles = (p.n * nmat + kGemmRows - 1) / kGemmRows;
+    const GemmCut cut = group ? GemmCut{gemm_tokens(group->typical), 1} : gemm_cut(a, ws, p.T, tiles, p.k / kUnitElems, nmat, unit_cycles(gemm_tokens(p.T)), kFixedCycles);
+    // five activation chunks (with few tokens eight) and the raw units that fit
+    const size_t raw = (size_t)RawUnit<TYPE>::pitch * kGemmRows, fixed = 1024 + 512, b = (size_t)2 * cut.N * 128;
+    p.N = cut.N;
+    p.b_stages = cut.N <= 64 ? kMaxB : 5;
+    while (p.b_stages > 3 && fixed + p.b_stages * b + 3 * raw > kMaxSmem) p.b_stages--;
+    p.raw_stages = std::min<int>(kGemmRaw, (int)((kMaxSmem - fixed - p.b_stages * b) / raw));
+    p.ksplit = cut.ks;
+    p.partial = cut.ks > 1 ? ws.partial : nullptr;
+    *summed_slices = cut.ks > 1 ? cut.ks * nmat : 0;
+    const size_t smem = fixed + p.b_stages * b + p.raw_stages * raw;
+    auto kern = cut.N <= 64 ? qgemm_split_kernel<TYPE, false> : qgemm_split_kernel<TYPE, true>;
+    LC_CUDA(ensure_smem_limit((const void*)kern, smem));
+    alignas(64) CUtensorMap tmx;
     const size_t rows = (size_t)ws.t_cap;
-    LC_CHECK(make_bf16_tmap_3d(&tmx, ws.xh, (uint64_t)p.k, rows, 2, (uint64_t)p.k, rows * p.k, 64, (uint32_t)g.N, 1) &&
-                 make_bf16_tmap_3d(&tms, ws.sx, (uint64_t)p.k / 16, rows, 2, (uint64_t)p.k / 16, rows * (p.k / 16), 64, (uint32_t)g.N, 1),
-             LC_ERR_CUDA, "qgemm: activation tensor maps");
-    const int nmat = a.epi == EPI_SILU_MUL ? 2 : 1;
-    const int tiles = (p.n * nmat + kRows - 1) / kRows, ttiles = group ? p.T / g.N + group->n_experts : (p.T + g.N - 1) / g.N, nquads = (p.k / kUnitElems + 3) / 4;
-    // Few tiles (a batched decode step, a short prompt): k is cut over several CTAs so that all SMs work, and a second kernel adds
-    // the shares in a fixed order.  Cost in cycles: waves of units plus a fixed part (launch, first unit, drain) per wave, and the
-    // shares' trip through L2 at 3000 bytes per cycle.  6000, 4000 and 3000 are estimates too (3 us and 2 us; 5.7 TB/s), not fitted one by one.
-    int ks = 1;
-    double best = 0;
-    for (int c = 1; c <= (group ? 1 : std::min(8, nquads)); c++) {
-        const size_t bytes = (size_t)c * nmat * p.T * p.n * sizeof(float);
-        if (c > 1 && (bytes > ws.partial_bytes || !qgemm_sum_ok(a))) break;
-        const long waves = ((long)tiles * ttiles * c + sm_count() - 1) / sm_count();
-        const double cost = (double)waves * (std::min((nquads + c - 1) / c * 4, p.k / kUnitElems) * unit_cycles(g.N) + 6000) + (c > 1 ? 4000 + 2.0 * bytes / 3000 : 0);
-        if (c == 1 || cost < best) { best = cost; ks = c; }
-    }
-    p.ksplit = ks;
-    p.partial = ks > 1 ? ws.partial : nullptr;
-    *summed_slices = ks > 1 ? ks * nmat : 0;
+    LC_CHECK(make_bf16_tmap_3d(&tmx, ws.xh, (uint64_t)p.k, rows, 2, (uint64_t)p.k, rows * p.k, 64, (uint32_t)cut.N, 1), LC_ERR_CUDA, "qgemm: activation tensor map");
     const CUtensorMap* t0 = (const CUtensorMap*)a.w->tmap;
     const CUtensorMap* t1 = a.w2 ? (const CUtensorMap*)a.w2->tmap : t0;
-    LC_CUDA(launch_pdl(kern, dim3((unsigned)tiles, (unsigned)ttiles, (unsigned)ks), dim3(kThreads), g.smem, s, *t0, *t1, tmx, tms, p));
+    const unsigned ttiles = (unsigned)(group ? p.T / cut.N + group->n_experts : (p.T + cut.N - 1) / cut.N);
+    LC_CUDA(launch_pdl(kern, dim3((unsigned)tiles, ttiles, (unsigned)cut.ks), dim3(kGemmThreads), smem, s, *t0, *t1, tmx, p));
     return LC_OK;
 }
 }  // namespace
@@ -903,15 +623,14 @@ int32_t launch_qgemm_split(const GemvArgs& a, GemmWorkspace& ws, const GemmGroup
         p.row_dynamic = 1;
         *launches += pair ? 2 : 1;
     }
-    p.out = a.out; p.residual = a.residual; p.tok_scale = ws.tok_scale;
+    p.out = a.out; p.residual = a.residual; p.xh = (const __half*)ws.xh; p.tok_scale = ws.tok_scale;
     p.w0 = (const unsigned char*)a.w->data; p.w1 = pair ? (const unsigned char*)a.w2->data : p.w0;
     p.row_bytes = a.w->row_bytes;
     p.n = n; p.k = a.w->k; p.T = a.m; p.epi = (int)a.epi;
     p.error_flag = gemv_error_flag_dev();
     *launches += 1;
     switch (a.w->typ) {
-        case LC_TYPE_Q4_K: return launch_type<LC_TYPE_Q4_K>(a, ws, p, group, slices, s);
-        case LC_TYPE_Q5_K: return launch_type<LC_TYPE_Q5_K>(a, ws, p, group, slices, s);
+        case LC_TYPE_Q4_K: case LC_TYPE_Q5_K: return launch_qgemm_whole(a, ws, p, group, slices, s);
         case LC_TYPE_Q4_0: return launch_type<LC_TYPE_Q4_0>(a, ws, p, group, slices, s);
         case LC_TYPE_Q8_0: return launch_type<LC_TYPE_Q8_0>(a, ws, p, group, slices, s);
         default: return launch_type<LC_TYPE_Q6_K>(a, ws, p, group, slices, s);

@@ -233,6 +233,26 @@ def test_many_token_product_of_infinities(gpu, typ, m):
     assert (np.abs(got[rest] - want) <= 2e-5 * np.sqrt((a[rest].astype(np.float64) ** 2) @ (dense.T ** 2))).all()
 
 
+@pytest.mark.parametrize("typ", [12, 13])
+@pytest.mark.parametrize("m,k,n", [(65, 256, 70), (129, 512, 300), (97, 768, 1), (70, 4352, 130), (200, 11008, 64)])
+def test_many_token_product_in_pairs_of_ctas(gpu, typ, m, k, n):
+    """Q4_K and Q5_K: one, two and three units (offsets behind the last, and behind the second), seventeen (two runs of offsets), shares of k that begin at any unit;
+    row counts that leave the second CTA of a pair few rows or none, token counts that leave it few tokens.  One token holds an infinity: its results have the weights' signs."""
+    r = rng(typ + m + k)
+    w, dense = scaled_blocks(gpu, typ, n, k, np.exp2(r.uniform(-1, 0, (n, k // 256))), r)
+    a = r.standard_normal((m, k)).astype(np.float32)
+    a[3, k - 100] = -np.inf
+    got = gpu.qmatmul(typ, a.ravel(), w, m, k, n).reshape(m, n)
+    with np.errstate(invalid="ignore"):
+        assert np.array_equal(got[3], (a[3, k - 100] * dense[:, k - 100]).astype(np.float32), equal_nan=True)
+    rest = [t for t in range(m) if t != 3]
+    want = a[rest].astype(np.float64) @ dense.T
+    assert np.linalg.norm(got[rest] - want) <= 4e-7 * np.linalg.norm(want)
+    # 22 bits of an activation and sums that lose up to 2^-22 of a run, the offsets' as large: 1.7e-7 of the root of the products' squares in a result on average, up to
+    # 2.9e-7 where eight shares of k are added; the largest of ten thousand results is up to eight times that (2.2e-6 measured): the bound of the tests above, 2e-5, leaves room
+    assert (np.abs(got[rest] - want) <= 2e-5 * np.sqrt((a[rest].astype(np.float64) ** 2) @ (dense.T ** 2))).all()
+
+
 @pytest.mark.parametrize("m", [16, 70])
 @pytest.mark.parametrize("typ", [2, 8, 12, 13, 14])
 def test_many_token_product_beside_a_large_activation(gpu, typ, m):
