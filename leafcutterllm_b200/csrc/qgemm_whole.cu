@@ -13,7 +13,8 @@
 // itself both parts are large and of opposite signs, and the cut-off sums' error with them: 7.0e-7 of the result for normal activations and 7.3e-5 for positive ones at k = 2048.)
 //
 // The tensor cores truncate when they add to an f32 accumulator.  A unit's low halves are multiplied first, into an empty accumulator, so that they add little to what is cut
-// off; the rest, 1.2e-7 of a sum on average (integers and f16 have few bits: less than for halves of weights, qgemm_split.cu), is put back by a factor.
+// off; the rest, 2.1e-7 of a sum on average, is put back by a factor (error of a result,
+// k = 4,096: 1.3e-7 - 2.2e-7; with three products of halves 2.0e-7 - 2.4e-7).
 //
 // Two CTAs are a pair (cta_group::2): 128 weight rows each (for gate/up 64 rows of each matrix, so that SiLU(gate) * up happens here), up to 128 tokens, whose
 // activations lie half in one's and half in the other's shared memory.  That is why there are pairs: alone, a CTA's activations take 64 bytes a cycle of
@@ -30,7 +31,7 @@
 // With stages of 32 elements, a barrier for each and a third of each stage's way spent waiting, a unit took 3,600 cycles.  2,048 tokens x [4096 -> 12288]
 // 473 -> 442 us, x [11008 -> 4096] 421 -> 381, 512 tokens 123 -> 113 and 107 -> 96, 128 tokens 48 -> 43.
 // Tried: the sums read while a unit is unpacked (spills: 25 % slower), registers moved from the control warps (spills), one lane of a warp waiting for all
-// (15 % slower), offsets first (the products wait 7,000 cycles for the headers) or last (the tile does, 4,000).
+// (15 % slower), offsets first or last (see below).
 #include <algorithm>
 #include <cstdlib>
 #include <cuda_fp16.h>
@@ -46,7 +47,8 @@ namespace {
 constexpr int kMaxB = 8;         // activation stages (two chunks of 64 elements) in flight
 // Tensor-memory columns, for even and for odd runs each: 128 of sums (N; up to 64 tokens 2 N, those with low halves of activations first), 128 of the A operand.
 constexpr uint32_t kColPlace = 128, kColA = 256;
-constexpr float kCutOff = 1.0f + 0x1p-23f;  // what a run's sums lost on average (see the header)
+// What sums lost on average: put back where a run is multiplied anyway, and the rest (8.9e-8, the mean over k = 4,096 ... 14,336 whole and in eight shares) at the end
+constexpr float kCutOff = 1.0f + 0x1p-23f, kCutOffAll = 0x1.8p-24f;
 
 // ---- tcgen05 wrappers -------------------------------------------------------------------------------------------------
 // the registers go through it: nothing that uses what was loaded may be moved ahead of the wait
@@ -253,9 +255,9 @@ qgemm_whole_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
     // this CTA's share of k in units; unit v below is u_begin + v
     const int u_begin = (int)((long long)blockIdx.z * nunits / p.ksplit);
     const int nu = (int)((long long)(blockIdx.z + 1) * nunits / p.ksplit) - u_begin;
-    // chunks of sub-block sums, four units each, in n_off runs of up to four chunks behind the first two units: the rows' headers are on their way meanwhile (at
-    // the start the products waited for them, 7,000 cycles of a tile of 17 units; at the end the tile did, 4,000)
-    const int sum_chunks = (nu + 3) / 4, n_off = (sum_chunks + 3) / 4, off_at = min(nu, 2);
+    // chunks of sub-block sums, four units each, in n_off runs of up to four chunks ahead of the last unit: the rows' headers have come meanwhile (at the start the products wait
+    // for them, 7,000 cycles of a tile of 17 units; at the end the tile does, 4,000), and hardly any additions are made at the offsets' size, which may be well above the result's
+    const int sum_chunks = (nu + 3) / 4, n_off = (sum_chunks + 3) / 4, off_at = nu - 1;
     const int nq = n_off + nu;
     auto is_unit = [&](int q) { return q < off_at || q >= off_at + n_off; };
     auto chunks_of = [&](int q) { return is_unit(q) ? 4 : min(4, sum_chunks - 4 * (q - off_at)); };
@@ -501,7 +503,6 @@ qgemm_whole_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
             operand_ready(q);
             if (++sr == RS) { sr = 0; raw_phase ^= 1; }
         }
-        if (off_at == nu) for (int q = off_at; q < nq && ok; q++) offsets(q);
         for (int q = max(0, nq - 2); q < nq && ok; q++) drain(q, q == nq - 1 ? d1 : d2);
         pdl_wait();
         const int t_first = tok0 + tbase, mine = ok ? min(own, tok_end - t_first) : 0;
@@ -518,7 +519,7 @@ qgemm_whole_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
         }
         // two multiplications: the product of the powers may leave f32's range where the result does not
 #pragma unroll
-        for (int t = 0; t < kOwn; t++) y[t] = (y[t] * down) * fabsf(__shfl_sync(0xffffffffu, scale, t));
+        for (int t = 0; t < kOwn; t++) y[t] = (fmaf(y[t], kCutOffAll, y[t]) * down) * fabsf(__shfl_sync(0xffffffffu, scale, t));
         store_sums<kOwn>(p, y, bt, pair, mat, g, row, grow, live, t_first, tbase, mine);
     }
     if (!ok && p.error_flag) atomicCAS(p.error_flag, 0, 3);

@@ -236,7 +236,7 @@ def test_many_token_product_of_infinities(gpu, typ, m):
 @pytest.mark.parametrize("typ", [12, 13])
 @pytest.mark.parametrize("m,k,n", [(65, 256, 70), (129, 512, 300), (97, 768, 1), (70, 4352, 130), (200, 11008, 64)])
 def test_many_token_product_in_pairs_of_ctas(gpu, typ, m, k, n):
-    """Q4_K and Q5_K: one, two and three units (offsets behind the last, and behind the second), seventeen (two runs of offsets), shares of k that begin at any unit;
+    """Q4_K and Q5_K: one, two and three units (the offsets come ahead of the last), seventeen (two runs of offsets), shares of k that begin at any unit;
     row counts that leave the second CTA of a pair few rows or none, token counts that leave it few tokens.  One token holds an infinity: its results have the weights' signs."""
     r = rng(typ + m + k)
     w, dense = scaled_blocks(gpu, typ, n, k, np.exp2(r.uniform(-1, 0, (n, k // 256))), r)
