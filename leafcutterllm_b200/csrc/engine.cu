@@ -12,6 +12,7 @@
 #include <algorithm>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 #include "lc_model.h"
@@ -1014,6 +1015,9 @@ static int32_t alloc_block_buffers(lc_model* m) {
     return LC_OK;
 }
 
+static void logits_blocks_alloc(const lc_model* m);
+static void logits_blocks_leave(const lc_model* m);
+
 int32_t lc_model_finalize(lc_model* m) {
     LC_TRY(check_model(m, false));
     LC_CHECK(!m->finalized, LC_ERR_STATE, "model already finalized");
@@ -1070,6 +1074,7 @@ int32_t lc_model_finalize(lc_model* m) {
     LC_CUDA(cudaHostAlloc((void**)&m->pin_tokens, (size_t)m->max_seqs * 8, cudaHostAllocDefault));
     LC_CUDA(cudaHostAlloc((void**)&m->pin_next, ((size_t)m->head_rows + 1) * 8, cudaHostAllocDefault));  // + one word: the device error flag of a call
     LC_CUDA(cudaHostAlloc((void**)&m->pin_logits, (size_t)m->head_rows * m->cfg.vocab_size * 4, cudaHostAllocDefault));
+    logits_blocks_alloc(m);
     LC_TRY(reserve_out_tokens(m, (size_t)1024 * m->max_seqs));
     LC_CUDA(cudaEventCreate(&m->ev0));
     LC_CUDA(cudaEventCreate(&m->ev1));
@@ -1105,6 +1110,7 @@ int32_t lc_model_destroy(lc_model* m) {
     if (m->pin_tokens) cudaFreeHost(m->pin_tokens);
     if (m->pin_next) cudaFreeHost(m->pin_next);
     if (m->pin_logits) cudaFreeHost(m->pin_logits);
+    logits_blocks_leave(m);
     if (m->ev0) cudaEventDestroy(m->ev0);
     if (m->ev1) cudaEventDestroy(m->ev1);
     delete m;
@@ -1187,10 +1193,77 @@ int32_t lc_kv_length(const lc_model* m, int32_t seq_id, int32_t* out) {
     return LC_OK;
 }
 
+// ---- page-locked blocks for logits (lc_logits_take) ----
+// A block outlives its handle while somebody holds it.  What comes back without a handle waits for the next handle that is set up or taken down, which adopts or frees it
+// (freeing here would make whoever drops a result wait for the device), up to kLogitsBlockBytes of them.
+struct LogitsBlock { size_t floats; const lc_model* owner; bool taken; };
+static std::mutex g_blocks_lock;
+static std::map<float*, LogitsBlock> g_blocks;
+constexpr int kLogitsBlocks = 2;                           // of a handle: a result that is read while the next step runs
+constexpr size_t kLogitsBlockBytes = (size_t)64 << 20;     // handles whose results may be larger have none
+
+static void logits_blocks_alloc(const lc_model* m) {
+    const size_t floats = (size_t)m->head_rows * m->cfg.vocab_size;
+    if (m->tp > 1 || floats * 4 > kLogitsBlockBytes) return;
+    for (int i = 0; i < kLogitsBlocks; i++) {
+        float* p = nullptr;
+        {
+            std::lock_guard<std::mutex> g(g_blocks_lock);
+            for (auto& b : g_blocks)
+                if (!p && !b.second.owner && !b.second.taken && b.second.floats >= floats) { p = b.first; b.second.owner = m; }
+        }
+        if (p) continue;
+        if (cudaHostAlloc((void**)&p, floats * 4, cudaHostAllocPortable) != cudaSuccess) { (void)cudaGetLastError(); return; }  // results are copied then
+        std::lock_guard<std::mutex> g(g_blocks_lock);
+        g_blocks[p] = LogitsBlock{floats, m, false};
+    }
+}
+static void logits_blocks_leave(const lc_model* m) {
+    std::lock_guard<std::mutex> g(g_blocks_lock);
+    for (auto it = g_blocks.begin(); it != g_blocks.end();) {
+        if ((it->second.owner == m || !it->second.owner) && !it->second.taken) { cudaFreeHost(it->first); it = g_blocks.erase(it); continue; }
+        if (it->second.owner == m) it->second.owner = nullptr;
+        ++it;
+    }
+}
+static bool in_logits_block(const float* p, size_t floats) {
+    std::lock_guard<std::mutex> g(g_blocks_lock);
+    auto it = g_blocks.upper_bound(const_cast<float*>(p));
+    if (it == g_blocks.begin()) return false;
+    --it;
+    return it->second.taken && p + floats <= it->first + it->second.floats;
+}
+int32_t lc_logits_take(lc_model* m, uint64_t floats, float** out) {
+    LC_TRY(check_model(m, true));
+    LC_CHECK(out, LC_ERR_INVALID, "null output");
+    *out = nullptr;
+    std::lock_guard<std::mutex> g(g_blocks_lock);
+    for (auto& b : g_blocks)
+        if (b.second.owner == m && !b.second.taken && b.second.floats >= floats) { b.second.taken = true; *out = b.first; break; }
+    return LC_OK;
+}
+int32_t lc_logits_give(float* block) {
+    std::lock_guard<std::mutex> g(g_blocks_lock);
+    auto it = g_blocks.find(block);
+    LC_CHECK(it != g_blocks.end() && it->second.taken, LC_ERR_INVALID, "lc_logits_give: not a block that was taken");
+    it->second.taken = false;
+    if (it->second.owner) return LC_OK;
+    size_t waiting = 0;
+    for (auto& b : g_blocks)
+        if (!b.second.owner && !b.second.taken) waiting += b.second.floats * 4;
+    if (waiting > kLogitsBlockBytes) { cudaFreeHost(it->first); g_blocks.erase(it); }
+    return LC_OK;
+}
+
 // The logits rows [0, n_rows) of the whole vocabulary on the host: a whole model copies them; a cut model puts the ranks'
 // vocabulary slices side by side (an all-gather when the ranks are processes).
 static int32_t fetch_logits(lc_model* lead, int n_rows, float* host_out) {
     const int Vfull = lead->cfg.vocab_size, Vl = lead->V;
+    if (lead->tp == 1 && in_logits_block(host_out, (size_t)n_rows * Vfull)) {
+        LC_CUDA(cudaMemcpyAsync(host_out, lead->d_logits, (size_t)n_rows * Vfull * 4, cudaMemcpyDeviceToHost, lead->stream));
+        LC_CUDA(cudaStreamSynchronize(lead->stream));
+        return LC_OK;
+    }
     if (lead->tp == 1) {
         LC_CUDA(cudaMemcpyAsync(lead->pin_logits, lead->d_logits, (size_t)n_rows * Vfull * 4, cudaMemcpyDeviceToHost, lead->stream));
         LC_CUDA(cudaStreamSynchronize(lead->stream));

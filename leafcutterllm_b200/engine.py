@@ -20,6 +20,17 @@ def _p(a: np.ndarray):
     return a.ctypes.data_as(C.c_void_p)
 
 
+class _Block:
+    """A page-locked block that the library lends; goes back when the last array over it is gone."""
+
+    def __init__(self, address: int, shape: tuple):
+        self.address, self._give = address, load().lc_logits_give
+        self.__array_interface__ = {"data": (address, False), "shape": shape, "typestr": "<f4", "version": 3}
+
+    def __del__(self):
+        self._give(self.address)
+
+
 class Engine:
     def __init__(self, hidden_size: int, num_layers: int, num_heads: int, num_kv_heads: int, intermediate_size: int,
                  vocab_size: int, max_seq_len: int = 4096, rope_theta: float = 10000.0, rms_eps: float = 1e-5,
@@ -144,16 +155,22 @@ class Engine:
     # ---- Engine::forward / generate ---------------------------------------
     def forward(self, tokens: Iterable[int]) -> np.ndarray:
         t = np.ascontiguousarray(list(tokens), dtype=np.int64)
-        out = np.empty(self.vocab_size, np.float32)
+        out = self._logits_array(1)[0]
         check(load().lc_forward(self._h, _p(t), t.size, _p(out)))
         return out
+
+    def _logits_array(self, rows: int) -> np.ndarray:
+        """Where a call's logits go: page-locked memory that the device writes into, while the handle has some to lend."""
+        shape, block = (rows, self.vocab_size), C.c_void_p()
+        check(load().lc_logits_take(self._h, rows * self.vocab_size, C.byref(block)))
+        return np.asarray(_Block(block.value, shape)) if block.value else np.empty(shape, np.float32)
 
     def forward_batch(self, seq_ids: Sequence[int], token_lists: Sequence[Sequence[int]], want_logits: bool = True):
         n = len(seq_ids)
         ids = np.ascontiguousarray(seq_ids, dtype=np.int32)
         counts = np.ascontiguousarray([len(t) for t in token_lists], dtype=np.int32)
         flat = np.ascontiguousarray([x for t in token_lists for x in t], dtype=np.int64)
-        logits = np.empty((n, self.vocab_size), np.float32) if want_logits else None
+        logits = self._logits_array(n) if want_logits else None
         nxt = np.empty(n, np.int64)
         check(load().lc_forward_batch(self._h, n, _p(ids), _p(flat), _p(counts), _p(logits) if want_logits else None, _p(nxt)))
         return logits, nxt
@@ -177,7 +194,7 @@ class Engine:
         n_want = np.ascontiguousarray([len(w) for w in want], dtype=np.int32)
         places = np.ascontiguousarray([x for w in want for x in w] + [0], dtype=np.int32)
         rows = int(n_want.sum())
-        logits = np.empty((rows, self.vocab_size), np.float32)
+        logits = self._logits_array(rows)
         nxt = np.empty(rows, np.int64)
         check(load().lc_step(self._h, len(seq_ids), _p(ids), _p(flat), _p(counts), _p(n_want), _p(places), _p(logits), _p(nxt)))
         return logits, nxt

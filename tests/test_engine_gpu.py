@@ -273,6 +273,31 @@ def test_batched_decode_attention_over_several_context_pieces(gpu, oracle):
     eng.close()
 
 
+def test_results_stay_what_they_are_while_somebody_holds_them(gpu, oracle):
+    """Logits lie in blocks that the handle lends.  Four results held at once (more than it has), views of them, and one that outlives its handle keep their
+    values; blocks come back when the last view goes."""
+    from leafcutterllm_b200 import synth
+    spec = small_spec(12, 12, 12, layers=1)
+    eng = synth.build_engine(spec, 64, max_seqs=3)
+    ids, steps = [0, 1, 2], [[[7], [8], [9]], [[1], [2], [3]], [[4], [5], [6]], [[10], [11], [12]]]
+    held = [eng.forward_batch(ids, s)[0] for s in steps]
+    again = synth.build_engine(spec, 64, max_seqs=3)
+    kept = [again.forward_batch(ids, s)[0].copy() for s in steps]
+    for a, b in zip(held, kept):
+        assert np.array_equal(a, b)
+    lent = {a.ctypes.data for a in held}
+    view = held[0][1:, ::2]
+    del held
+    reused = [again.forward_batch(ids, s)[0] for s in steps[:2]] + [eng.forward_batch(ids, s)[0] for s in steps[:1]]
+    assert reused[-1].ctypes.data in lent and np.array_equal(view, kept[0][1:, ::2])
+    last = eng.forward_batch(ids, steps[0])[0]
+    want = last.copy()
+    eng.close()
+    again.forward_batch(ids, steps[1])
+    assert np.array_equal(last, want) and np.array_equal(view, kept[0][1:, ::2])
+    again.close()
+
+
 @pytest.mark.parametrize("heads,kv", [(4, 4), (4, 2), (4, 1), (8, 1)])
 def test_batched_decode_attention_as_one_stream(gpu, oracle, heads, kv):
     """The (token, kv head, page) items of a decode step cut into one run per warp: contexts on both sides of a page's edge, a first token, one that many runs
