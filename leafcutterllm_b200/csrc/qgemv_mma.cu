@@ -130,8 +130,8 @@ qgemv_mma_q4k_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_const
     off += (size_t)2 * WARPS * M * 32 * 4;
     float* gate_vals = reinterpret_cast<float*>(smem + off);     // [M][32]
     off += (size_t)M * 32 * 4;
-    float* scratch = reinterpret_cast<float*>(smem + off);       // [32 + M]
-    off += (size_t)(32 + M) * 4;
+    float* scratch = reinterpret_cast<float*>(smem + off);       // [WARPS][M] sums of squares
+    off += (size_t)WARPS * M * 4;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + ((off + 7) & ~(size_t)7)) + warp * STAGES;
 
     const int units_mine = (nunits > warp) ? (nunits - warp + WARPS - 1) / WARPS : 0;
@@ -163,7 +163,7 @@ qgemv_mma_q4k_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_const
     }
     // One token whose k fits one or two units per warp: each warp reads its own elements ONCE, for the sum of squares and for
     // the planes, and the gains of its first unit (weights: no dependency on the kernel ahead) are already in registers by then.
-    const bool one_pass = !GROUPED && (M == 1) && p.norm_w != nullptr && nunits <= 2 * WARPS;
+    const bool one_pass = !GROUPED && (M == 1) && p.norm_w != nullptr && nunits <= 2 * WARPS;  // longer rows: below
     float nw0[8];
     if (one_pass && warp < nunits) {
         const float4* np = reinterpret_cast<const float4*>(p.norm_w + warp * kUnitElems + 8 * lane);
@@ -204,27 +204,15 @@ qgemv_mma_q4k_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_const
         // No barrier here: the planes are those of x * gain, and the RMS factor -- one scalar for the whole row -- multiplies
         // the finished row sums behind the barrier of the cross-warp reduction, where every warp's part of the sum of
         // squares is visible.  A unit's power-of-two scale follows its own largest magnitude, so it does not care.
-    } else if (!GROUPED && p.norm_w) {
-        for (int tk = 0; tk < M; tk++) {
-            float ss = 0.f;
-            if (tk < m_act) {
-                const float* xr = xrow(tk);
-                for (int i = threadIdx.x; i < p.k; i += blockDim.x) { float v = xr[i]; ss = fmaf(v, v, ss); }
-            }
-            ss = warp_sum(ss);
-            __syncthreads();
-            if (lane == 0) scratch[warp] = ss;
-            __syncthreads();
-            if (warp == 0) {
-                float r = (lane < WARPS) ? scratch[lane] : 0.f;
-                r = warp_sum(r);
-                if (lane == 0) scratch[32 + tk] = 1.0f / sqrtf(r / (float)p.k + p.eps);
-            }
-        }
-        __syncthreads();
     }
 
     // ---- each warp writes the fixed-point planes of its own units ----
+    // Several tokens (or a long row) with a norm: as above, the planes are those of x * gain and the factors come in behind the reduction's barrier, so a row is read once and nothing waits for
+    // its sum of squares (token by token, with scalar loads and three barriers each, four tokens took 6 us of a 20 us launch)
+    const bool late = !GROUPED && !one_pass && p.norm_w != nullptr;
+    float ss_own[M];
+#pragma unroll
+    for (int tk = 0; tk < M; tk++) ss_own[tk] = 0.f;
     for (int ui = 0; ui < (GROUPED ? 0 : units_mine); ui++) {
         const int unit = warp + ui * WARPS;
 #pragma unroll
@@ -247,18 +235,27 @@ qgemv_mma_q4k_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_const
                 float4 u0 = xp[0], u1 = xp[1];
                 v[0] = u0.x; v[1] = u0.y; v[2] = u0.z; v[3] = u0.w; v[4] = u1.x; v[5] = u1.y; v[6] = u1.z; v[7] = u1.w;
                 if (p.norm_w) {
-                    const float sc = scratch[32 + tk];
                     const float4* np = reinterpret_cast<const float4*>(p.norm_w + e0);
-                    float4 n0 = np[0], n1 = np[1];
+                    const float4 n0 = np[0], n1 = np[1];
                     const float nw[8] = {n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, n1.z, n1.w};
 #pragma unroll
-                    for (int j = 0; j < 8; j++) v[j] = (v[j] * sc) * nw[j];
+                    for (int j = 0; j < 8; j++) {
+                        ss_own[tk] = fmaf(v[j], v[j], ss_own[tk]);
+                        v[j] *= nw[j];
+                    }
                 }
             } else {
 #pragma unroll
                 for (int j = 0; j < 8; j++) v[j] = 0.f;
             }
             unit_planes(v, lane, planes + plane_off<M>(unit, 0, tk, 0), M * 96, sxf + (unit * M + tk) * 8, inv2s + unit * M + tk);
+        }
+    }
+    if (late) {
+#pragma unroll
+        for (int tk = 0; tk < M; tk++) {
+            const float ss = warp_sum(ss_own[tk]);
+            if (lane == 0) scratch[warp * M + tk] = ss;
         }
     }
     __syncwarp();
@@ -552,9 +549,9 @@ qgemv_mma_q4k_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_const
 #pragma unroll 4
                 for (int w = 0; w < WARPS; w++) {
                     y += rb[(w * M + tk) * 32 + lane];
-                    if (one_pass) ssq += scratch[w];  // same order in every thread and CTA
+                    if (one_pass || late) ssq += scratch[w * M + tk];  // same order in every thread and CTA
                 }
-                if (one_pass) y *= 1.0f / sqrtf(ssq / (float)p.k + p.eps);  // cpu.rs:52-55
+                if (one_pass || late) y *= 1.0f / sqrtf(ssq / (float)p.k + p.eps);  // cpu.rs:52-55
                 const int row = lane < TR ? tile * TR + lane : p.n;  // lanes past the tile's rows hold nothing
                 bool have = false;
                 if (p.epi == EPI_SILU_MUL) {
@@ -662,7 +659,7 @@ static size_t mma_smem_bytes(int k, bool grouped = false, int unit_bytes = 144) 
     int nunits = grouped ? 0 : k / kUnitElems;
     size_t b = (size_t)WARPS * STAGES * unit_bytes * kTileRows;
     b += (size_t)nunits * 8 * M * 96 + (size_t)nunits * M * 8 * 4 + (size_t)nunits * M * 4;
-    b += (size_t)2 * WARPS * M * 32 * 4 + (size_t)M * 32 * 4 + (size_t)(32 + M) * 4;
+    b += (size_t)2 * WARPS * M * 32 * 4 + (size_t)M * 32 * 4 + (size_t)WARPS * M * 4;
     b = (b + 7) & ~(size_t)7;
     b += (size_t)WARPS * STAGES * 8;
     return b + kGroupedSlots * 4;  // head room for the slot words of the grouped form

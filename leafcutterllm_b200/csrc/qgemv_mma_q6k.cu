@@ -98,7 +98,7 @@ qgemv_mma_q6k_kernel(const unsigned char* __restrict__ w0, const unsigned char* 
     off += (size_t)2 * WARPS * M * kRows * 4;
     float* gate_vals = reinterpret_cast<float*>(smem + off);  // [M][16]
     off += (size_t)M * kRows * 4;
-    float* scratch = reinterpret_cast<float*>(smem + off);    // [32 + M]
+    float* scratch = reinterpret_cast<float*>(smem + off);    // [WARPS][M] sums of squares
 
     const int units_mine = (nunits > warp) ? (nunits - warp + WARPS - 1) / WARPS : 0;
     const int tiles_mine = (ntiles > (int)blockIdx.x) ? (ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
@@ -139,27 +139,12 @@ qgemv_mma_q6k_kernel(const unsigned char* __restrict__ w0, const unsigned char* 
     pdl_launch_dependents();
     pdl_wait();
 
-    // ---- RMS-norm scale per token (cpu.rs:49-60) when fused ----
-    if (p.norm_w) {
-        for (int tk = 0; tk < M; tk++) {
-            float ss = 0.f;
-            if (tk < m_act) {
-                const float* xr = p.x + (size_t)tk * p.k;
-                for (int i = threadIdx.x; i < p.k; i += blockDim.x) { const float v = xr[i]; ss = fmaf(v, v, ss); }
-            }
-            ss = warp_sum(ss);
-            __syncthreads();
-            if (lane == 0) scratch[warp] = ss;
-            __syncthreads();
-            if (warp == 0) {
-                float r = (lane < WARPS) ? scratch[lane] : 0.f;
-                r = warp_sum(r);
-                if (lane == 0) scratch[32 + tk] = 1.0f / sqrtf(r / (float)p.k + p.eps);
-            }
-        }
-        __syncthreads();
-    }
     // ---- each warp writes the fixed-point planes of its own units ----
+    // With a norm (cpu.rs:49-60) the planes are those of x * gain; the row's factor multiplies the finished sums behind the reduction's barrier, where every
+    // warp's part of the sum of squares is visible (qgemv_mma.cu).
+    float ss_own[M];
+#pragma unroll
+    for (int tk = 0; tk < M; tk++) ss_own[tk] = 0.f;
     for (int ui = 0; ui < units_mine; ui++) {
         const int unit = warp + ui * WARPS;
         const int e0 = unit * kUnitElems + 8 * lane;
@@ -171,12 +156,14 @@ qgemv_mma_q6k_kernel(const unsigned char* __restrict__ w0, const unsigned char* 
                 const float4 u0 = xp[0], u1 = xp[1];
                 v[0] = u0.x; v[1] = u0.y; v[2] = u0.z; v[3] = u0.w; v[4] = u1.x; v[5] = u1.y; v[6] = u1.z; v[7] = u1.w;
                 if (p.norm_w) {
-                    const float sc = scratch[32 + tk];
                     const float4* np = reinterpret_cast<const float4*>(p.norm_w + e0);
                     const float4 n0 = np[0], n1 = np[1];
                     const float nw[8] = {n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, n1.z, n1.w};
 #pragma unroll
-                    for (int j = 0; j < 8; j++) v[j] = (v[j] * sc) * nw[j];
+                    for (int j = 0; j < 8; j++) {
+                        ss_own[tk] = fmaf(v[j], v[j], ss_own[tk]);
+                        v[j] *= nw[j];
+                    }
                 }
             } else {
 #pragma unroll
@@ -197,6 +184,13 @@ qgemv_mma_q6k_kernel(const unsigned char* __restrict__ w0, const unsigned char* 
             unsigned char* sp = ssum + (size_t)(unit * NPAIR + (tk >> 1)) * 256 + (3 * (tk & 1) + pl) * 16 + is;
             sp[0] = (unsigned char)lo;
             sp[128] = (unsigned char)hi;
+        }
+    }
+    if (p.norm_w) {
+#pragma unroll
+        for (int tk = 0; tk < M; tk++) {
+            const float ss = warp_sum(ss_own[tk]);
+            if (lane == 0) scratch[warp * M + tk] = ss;
         }
     }
     __syncwarp();
@@ -341,9 +335,13 @@ qgemv_mma_q6k_kernel(const unsigned char* __restrict__ w0, const unsigned char* 
             __syncthreads();
             if (warp < M && lane < kRows) {
                 const int tk = warp;
-                float y = 0.f;
+                float y = 0.f, ssq = 0.f;
 #pragma unroll 4
-                for (int w = 0; w < WARPS; w++) y += rb[(w * M + tk) * kRows + lane];
+                for (int w = 0; w < WARPS; w++) {
+                    y += rb[(w * M + tk) * kRows + lane];
+                    if (p.norm_w) ssq += scratch[w * M + tk];  // same order in every thread and CTA
+                }
+                if (p.norm_w) y *= 1.0f / sqrtf(ssq / (float)p.k + p.eps);
                 const int row = tile * kRows + lane;
                 bool have = false;
                 if (p.epi == EPI_SILU_MUL) {
@@ -369,7 +367,7 @@ size_t q6k_smem_bytes(int k) {
     const int nunits = k / kUnitElems;
     size_t b = (size_t)WARPS * STAGES * kStageBytes;
     b += (size_t)nunits * 8 * M * 96 + (size_t)nunits * ((M + 1) / 2) * 256 + (size_t)nunits * M * 4;
-    b += (size_t)2 * WARPS * M * kRows * 4 + (size_t)M * kRows * 4 + (size_t)(32 + M) * 4;
+    b += (size_t)2 * WARPS * M * kRows * 4 + (size_t)M * kRows * 4 + (size_t)WARPS * M * 4;
     return b;
 }
 
