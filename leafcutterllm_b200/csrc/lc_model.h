@@ -57,9 +57,9 @@ constexpr int kStackChunk = 2048;      // tokens per pass of a checkpoint-direct
 constexpr int kTokTile = 8;
 constexpr int kMoeGroupedTokens = 64;  // most tokens of a call whose experts run as one grouped matrix-vector launch
 // Rows per expert beyond which the experts run as a grouped many-token product instead: the matrix-vector kernel reads the experts again for
-// every four rows.  Mixtral shape, us per step of two layers, matrix-vector / product: 24 sequences (6 rows per expert) 1761 / 2169, 32 (8)
-// 2143 / 2263, 48 (12) 2899 / 2563, 64 (16) 3656 / 3028.  They meet between 8 and 12 rows (a straight line through both puts it at 9); one shape measured.
-constexpr int kMoeProductRows = 9;
+// every four rows.  Mixtral shape, us per step of two layers, matrix-vector / product: 16 sequences (4 rows per expert) 1049 / 1385, 24 (6)
+// 1314 / 1400, 28 (7) 1433 / 1405, 32 (8) 1576 / 1407, 48 (12) 2110 / 1473.  One shape measured.
+constexpr float kMoeProductRows = 6.5f;
 
 }  // namespace lc
 
