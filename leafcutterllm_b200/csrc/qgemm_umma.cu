@@ -985,6 +985,10 @@ static int32_t launch_qgemm_tile(const GemvArgs& a, GemmWorkspace& ws, int* slic
 // 64 tokens [4096 -> 12288] 41 / 44; 512 tokens 212 / 138, gate and up 327 / 237.
 static bool use_split(uint32_t typ, int T) { return T > kMaxTok || (typ != LC_TYPE_Q4_K && typ != LC_TYPE_Q5_K); }
 
+// Threads for a token's row.  Few tokens: its three dependent passes are latency, so many threads with one or a few float4 each (64 sequences, 4 layers: 2.43 / 2.40 / 2.40 ms per step
+// with 256 / 512 / 1024 threads).  Many: CTAs that wait at different barriers fill the SM (2,048 rows of 4096: 15.9 us with 256, 18.8 with 512 or 128, 26.3 with 1024).
+static int xprep_threads(int T, int K) { return K >= 4096 && T < 256 ? 1024 : 256; }
+
 int32_t launch_qgemm(const GemvArgs& a, GemmWorkspace& ws, cudaStream_t s, int* launches) {
     const int T = a.m, K = a.w->k, n = a.w->n;
     LC_CHECK(qgemm_applies(a, T, ws), LC_ERR_INVALID, "qgemm: arguments outside what the kernel implements");
@@ -997,9 +1001,7 @@ int32_t launch_qgemm(const GemvArgs& a, GemmWorkspace& ws, cudaStream_t s, int* 
     if (!prepared) {
         const size_t smem = (size_t)K * sizeof(float);
         if (smem > 48 * 1024) LC_CUDA(ensure_smem_limit((const void*)xprep_kernel, smem));
-        // a token's row is short (16 - 44 KB) and its three passes are latency: many threads, one or a few float4 each
-        // (64 sequences, 4 layers: 2.43 / 2.40 / 2.40 ms per step with 256 / 512 / 1024 threads)
-        LC_CUDA(launch_pdl(xprep_kernel, dim3(T), dim3(K >= 4096 ? 1024 : 256), smem, s, a.x, (const int32_t*)nullptr, 1, (const int32_t*)nullptr, a.norm_w, a.eps, K, (__half*)ws.xh, lo_offset, (__half*)ws.sx,
+        LC_CUDA(launch_pdl(xprep_kernel, dim3(T), dim3(xprep_threads(T, K)), smem, s, a.x, (const int32_t*)nullptr, 1, (const int32_t*)nullptr, a.norm_w, a.eps, K, (__half*)ws.xh, lo_offset, (__half*)ws.sx,
                            sx_lo_offset, ws.tok_scale));
     }
     int slices = 0, count = prepared ? 0 : 1;
@@ -1036,7 +1038,7 @@ int32_t launch_qgemm_group(const GemvArgs& a, GemmWorkspace& ws, const GemmGroup
     ws.prep_x = nullptr;
     const size_t smem = (size_t)K * sizeof(float);
     if (smem > 48 * 1024) LC_CUDA(ensure_smem_limit((const void*)xprep_kernel, smem));
-    LC_CUDA(launch_pdl(xprep_kernel, dim3(a.m), dim3(K >= 4096 ? 1024 : 256), smem, s, a.x, rows, div, group.offsets + group.n_experts, a.norm_w, a.eps, K, (__half*)ws.xh, (size_t)ws.t_cap * K,
+    LC_CUDA(launch_pdl(xprep_kernel, dim3(a.m), dim3(xprep_threads(a.m, K)), smem, s, a.x, rows, div, group.offsets + group.n_experts, a.norm_w, a.eps, K, (__half*)ws.xh, (size_t)ws.t_cap * K,
                        (__half*)ws.sx, (size_t)ws.t_cap * (K / 16), ws.tok_scale));
     int slices = 0;
     *launches += 1;
