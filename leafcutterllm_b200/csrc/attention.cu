@@ -136,11 +136,12 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_staged_kernel(AttnP
     __syncthreads();  // barrier initialised
     const bool ok = mbar_wait(&bar, 0);
     const int rp = fused ? p.tok_rope[tok] : 0;
+    const float2* const rot = p.rot ? p.rot + (size_t)tok * (HD / 2) : nullptr;
     if (fused && pos >= t_begin && pos < t_end) {
         // the token of this step replaces the (stale) staged slot: rotate, round through f16, keep in the cache
         const int row = pos - t_begin;
         float kr[1], vr;
-        load_rotated<1, HD>(p.k_new + (size_t)tok * p.q_stride + kvh * HD, tid, rp, p.theta, kr);
+        load_rotated<1, HD>(p.k_new + (size_t)tok * p.q_stride + kvh * HD, tid, rp, p.theta, rot, kr);
         vr = __ldcg(p.v_new + (size_t)tok * p.q_stride + kvh * HD + tid);
         const __half hk = __float2half_rn(kr[0]), hv = __float2half_rn(vr);  // cache/mod.rs:35-36
         K_s[row * HD + tid] = hk;
@@ -168,7 +169,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_staged_kernel(AttnP
         float* pout = p.partial + ((size_t)item * p.n_splits + split) * (HD + 2);
         {
             float qv[1];
-            load_rotated<1, HD>(p.q + (size_t)tok * p.q_stride + h * HD, tid, rp, p.theta, qv);
+            load_rotated<1, HD>(p.q + (size_t)tok * p.q_stride + h * HD, tid, rp, p.theta, rot, qv);
             __syncthreads();  // the previous head is done with q_s / p_s / acc_s
             q_s[tid] = qv[0];
         }
@@ -351,10 +352,11 @@ int32_t launch_attention(const float* q, int q_stride, float* out, int n_tok, in
     p.counters = counters;
     p.k_new = fuse ? fuse->k_new : nullptr; p.v_new = fuse ? fuse->v_new : nullptr;
     p.tok_rope = fuse ? fuse->tok_rope : nullptr; p.theta = fuse ? fuse->theta : 0.f;
+    p.rot = fuse ? (const float2*)fuse->rot : nullptr;
     p.positions_settled = (fuse && fuse->positions_settled) ? 1 : 0;
     p.error_flag = gemv_error_flag_dev();
     if (fuse && fuse->stream_slots && attention_stream_applies(p, n_tok)) return launch_attention_stream(p, fuse->stream_slots, s);
-    if (fuse && fuse->rot && attention_batch_applies(p, n_tok)) return launch_attention_batch(p, fuse->rot, n_tok, s);
+    if (p.rot && attention_batch_applies(p, n_tok)) return launch_attention_batch(p, n_tok, s);
     switch (kv.hd) {
         case 32: return launch_attention_hd<32>(p, n_tok, max_ctx, s);
         case 64: return launch_attention_hd<64>(p, n_tok, max_ctx, s);

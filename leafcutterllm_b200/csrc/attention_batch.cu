@@ -41,7 +41,6 @@ constexpr float kWeightLog2 = 14.f;          // weights are times 2^14, so that 
 
 struct BatchParams {
     AttnParams a;
-    const float2* rot;  // [n_tok][64] cosine and sine of each pair
     int n_tok;
 };
 
@@ -192,7 +191,7 @@ attention_batch_kernel(const __grid_constant__ CUtensorMap ktm, const __grid_con
                     for (int kt = 0; kt < 4; kt++)
 #pragma unroll
                         for (int r = 0; r < 2; r++)
-                            rotate_pair(x[kt][r], x[kt + 4][r], __ldcg(reinterpret_cast<const float4*>(P.rot + (size_t)tok * (kHD / 2) + kt * 16 + 2 * t4 + 8 * r)));
+                            rotate_pair(x[kt][r], x[kt + 4][r], __ldcg(reinterpret_cast<const float4*>(p.rot + (size_t)tok * (kHD / 2) + kt * 16 + 2 * t4 + 8 * r)));
                 }
                 float big = 0.f;
 #pragma unroll
@@ -228,7 +227,7 @@ attention_batch_kernel(const __grid_constant__ CUtensorMap ktm, const __grid_con
             const int d = 4 * (lane & 15);  // of the pair's first half; lanes 16 - 31 have the second
             float4 a = __ldcg(reinterpret_cast<const float4*>(kn + d)), b = __ldcg(reinterpret_cast<const float4*>(kn + d + kHD / 2));
             if (rp != 0) {
-                const float4* const cs = reinterpret_cast<const float4*>(P.rot + (size_t)tok * (kHD / 2) + d);
+                const float4* const cs = reinterpret_cast<const float4*>(p.rot + (size_t)tok * (kHD / 2) + d);
                 float2 a0 = make_float2(a.x, a.y), a1 = make_float2(a.z, a.w), b0 = make_float2(b.x, b.y), b1 = make_float2(b.z, b.w);
                 rotate_pair(a0, b0, __ldcg(cs));
                 rotate_pair(a1, b1, __ldcg(cs + 1));
@@ -432,13 +431,13 @@ bool attention_batch_applies(const AttnParams& a, int n_tok) {
     // Up to four tokens of models without kv groups go to the staged kernel (attention.cu), which has a CTA per 128 keys and less to do ahead of them: 7B shape, 8 layers, us
     // per step staged / here: 3 sequences of 200 768 / 815, of 1,000 870 / 890, of 4,000 1,280 / 1,100.  With kv groups it serves one query head after the other
     // (Mixtral shape, 4 layers, 3 sequences: 1,018 / 965, 1,041 / 990, 1,236 / 1,030).
-    return n_tok >= 2 && (n_tok > 4 || gsz > 1) && n_tok <= kMaxBatch && a.k_new && a.kv.k_tmap && a.kv.v_tmap && a.kv.hd == kHD && !a.kv.kv_f32 && a.kv.page_tokens == kPage &&
+    return n_tok >= 2 && (n_tok > 4 || gsz > 1) && n_tok <= kMaxBatch && a.k_new && a.rot && a.kv.k_tmap && a.kv.v_tmap && a.kv.hd == kHD && !a.kv.kv_f32 && a.kv.page_tokens == kPage &&
            a.n_heads % a.kv.n_kv == 0 && (gsz == 1 || gsz == 2 || gsz == 4 || gsz == 8) && a.q_stride % 4 == 0;
 }
 
-int32_t launch_attention_batch(const AttnParams& a, const void* rot, int n_tok, cudaStream_t s) {
+int32_t launch_attention_batch(const AttnParams& a, int n_tok, cudaStream_t s) {
     BatchParams P;
-    P.a = a; P.rot = (const float2*)rot; P.n_tok = n_tok;
+    P.a = a; P.n_tok = n_tok;
     switch (a.n_heads / a.kv.n_kv) {
         case 1: return launch_batch<1>(P, s);
         case 2: return launch_batch<2>(P, s);

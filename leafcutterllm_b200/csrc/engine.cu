@@ -421,9 +421,10 @@ int32_t run_layers(lc_model* lead, int T, bool decode_step) {
     if (lead->stack) return stack_run_layers(lead, T, decode_step);
     std::vector<lc_model*> R = ranks_of(lead);
     for (lc_model* m : R) {
+        // (in call-relative mode a decode step's rotations are by nothing)
         const EmbedTurns turn{m->d_tok_rope, m->cfg.rope_theta, m->hd / 2, m->d_rot};
         LC_TRY(launch_embed(m->embed->typ, m->embed->view, m->embed->rows, m->embed->cols, m->d_tokens, T, m->d_hidden,
-                            decode_step && T > 1 && m->d_rot ? &turn : nullptr, m->stream));
+                            decode_step && m->cfg.rope_mode ? &turn : nullptr, m->stream));
         m->launches_in_call += 1;
     }
     const size_t count = (size_t)T * lead->H;
@@ -969,7 +970,6 @@ static int32_t alloc_block_pools(lc_model* m) {
             LC_TRY(dalloc((uint8_t**)&m->d_stream_slots, slot_bytes));
             LC_CUDA(cudaMemsetAsync(m->d_stream_slots, 0, slot_bytes, m->stream));
         }
-        LC_TRY(dalloc((float2**)&m->d_rot, (size_t)m->max_seqs * (m->hd / 2)));
     }
     return LC_OK;
 }
@@ -1007,7 +1007,8 @@ static int32_t alloc_block_buffers(lc_model* m) {
     }
     size_t sc = 16;
     for (int t = 1; t <= std::max(kAttnSlice, m->max_seqs); t++) sc = std::max(sc, attention_scratch_bytes(t, m->nh, m->hd, m->cfg.max_seq_len));
-    if (m->d_rot) sc = std::max(sc, attention_batch_scratch_bytes(m->nh, m->nkv, m->hd));
+    if (m->k_tmaps_ok) sc = std::max(sc, attention_batch_scratch_bytes(m->nh, m->nkv, m->hd));
+    LC_TRY(dalloc((float2**)&m->d_rot, (size_t)m->max_seqs * (m->hd / 2)));
     m->attn_scratch_bytes = sc;
     LC_TRY(dalloc((uint8_t**)&m->d_attn_scratch, sc));
     LC_TRY(dalloc(&m->d_attn_counters, (size_t)T * m->nh));

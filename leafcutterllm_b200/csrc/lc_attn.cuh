@@ -28,6 +28,7 @@ struct AttnParams {
     const float* v_new;
     const int32_t* tok_rope;
     float theta;
+    const float2* rot;     // [n_tok][hd / 2] cosine and sine of each pair's rotation, or null: computed here
     int positions_settled; // decode-step fusion: tok_pos may be read before the grid dependency wait
     int* error_flag;       // set when a bounded wait runs out (may be null)
 };
@@ -39,7 +40,7 @@ int32_t launch_attention_stream(const AttnParams& a, unsigned long long* slots, 
 
 // attention_batch.cu: one new token for each of two or more sequences, the same heads and caches, as one stream over all of them
 bool attention_batch_applies(const AttnParams& a, int n_tok);
-int32_t launch_attention_batch(const AttnParams& a, const void* rot, int n_tok, cudaStream_t s);
+int32_t launch_attention_batch(const AttnParams& a, int n_tok, cudaStream_t s);
 
 template <int DPL, bool F32>
 __device__ __forceinline__ void load_slice(const void* pool, size_t elem_off, float (&out)[DPL]) {
@@ -88,9 +89,10 @@ __device__ __forceinline__ void widen(const RawSlice<DPL, F32>& r, float (&out)[
 }
 
 // Dims d0 .. d0+DPL-1 of a head vector at `base`, rotated by position `rp` (attention.rs:13-34: pairs
-// (d, d + hd/2), freq = 1 / theta^(2d/hd)).  rp == 0 is the identity and skips the trigonometry.
+// (d, d + hd/2), freq = 1 / theta^(2d/hd)).  rp == 0 is the identity and skips the trigonometry.  rot: this token's row of the table that the step's first
+// kernel left (powers, sines and cosines in every CTA cost as much as half of a batch's attention), or null.
 template <int DPL, int HD>
-__device__ __forceinline__ void load_rotated(const float* base, int d0, int rp, float theta, float (&out)[DPL]) {
+__device__ __forceinline__ void load_rotated(const float* base, int d0, int rp, float theta, const float2* rot, float (&out)[DPL]) {
 #pragma unroll
     for (int i = 0; i < DPL; i++) out[i] = __ldcg(base + d0 + i);  // written by another CTA of a persistent kernel: read through L2
     if (rp == 0) return;
@@ -98,9 +100,15 @@ __device__ __forceinline__ void load_rotated(const float* base, int d0, int rp, 
 #pragma unroll
     for (int i = 0; i < DPL; i++) {
         const int d = d0 + i, dd = d < HALF ? d : d - HALF;
-        const float freq = __fdiv_rn(1.0f, powf(theta, __fdiv_rn(__fmul_rn(2.0f, (float)dd), (float)HD)));
-        const float angle = __fmul_rn((float)rp, freq);
-        const float ca = cosf(angle), sa = sinf(angle);
+        float2 cs;
+        if (rot) {
+            cs = __ldcg(rot + dd);
+        } else {
+            const float freq = __fdiv_rn(1.0f, powf(theta, __fdiv_rn(__fmul_rn(2.0f, (float)dd), (float)HD)));
+            const float angle = __fmul_rn((float)rp, freq);
+            cs = make_float2(cosf(angle), sinf(angle));
+        }
+        const float ca = cs.x, sa = cs.y;
         if (d < HALF) out[i] = __fsub_rn(__fmul_rn(__ldcg(base + d), ca), __fmul_rn(__ldcg(base + d + HALF), sa));
         else out[i] = __fadd_rn(__fmul_rn(__ldcg(base + d - HALF), sa), __fmul_rn(__ldcg(base + d), ca));
     }
@@ -166,8 +174,9 @@ __device__ __forceinline__ void attention_item(const AttnParams& p, int item, in
         const int32_t* pt = p.page_table + (size_t)p.tok_seq[tok] * p.pages_per_seq;
         const float inv_div = sqrtf((float)HD);   // attention.rs:93: dot / sqrt(head_dim)
         const int rp = p.k_new ? p.tok_rope[tok] : 0;
+        const float2* const rot = p.rot ? p.rot + (size_t)tok * (HD / 2) : nullptr;
         float qr[DPL];
-        load_rotated<DPL, HD>(p.q + (size_t)tok * p.q_stride + h * HD, sub * DPL, rp, p.theta, qr);
+        load_rotated<DPL, HD>(p.q + (size_t)tok * p.q_stride + h * HD, sub * DPL, rp, p.theta, rot, qr);
 
         auto key_addr = [&](int t) -> size_t {
             int page = pt[t / kv.page_tokens];
@@ -237,7 +246,7 @@ __device__ __forceinline__ void attention_item(const AttnParams& p, int item, in
         if (has_new) {
             // the token of this step: rotate, round through the cache type, and (one head per kv group) store
             float kr[DPL], vr[DPL];
-            load_rotated<DPL, HD>(p.k_new + (size_t)tok * p.q_stride + kvh * HD, sub * DPL, rp, p.theta, kr);
+            load_rotated<DPL, HD>(p.k_new + (size_t)tok * p.q_stride + kvh * HD, sub * DPL, rp, p.theta, rot, kr);
             const float* vp = p.v_new + (size_t)tok * p.q_stride + kvh * HD + sub * DPL;
 #pragma unroll
             for (int i = 0; i < DPL; i++) vr[i] = __ldcg(vp + i);

@@ -205,7 +205,7 @@ struct AttnFusion {
     // first launch; the kernel leaves them zero).  They belong to the caller -- one set per model -- because a captured
     // decode step keeps the pointer.
     unsigned long long* stream_slots = nullptr;
-    const void* rot = nullptr;  // float2 [tokens][hd / 2]: cosine and sine of the step's rotations (launch_embed), for the kernel of batches
+    const void* rot = nullptr;  // float2 [tokens][hd / 2]: cosine and sine of the step's rotations (launch_embed)
 };
 int32_t launch_attention(const float* q, int q_stride, float* out, int n_tok, int n_heads, const KvLayout& kv,
                          const int32_t* tok_seq, const int32_t* tok_pos, const int32_t* page_table, int pages_per_seq, int max_ctx,

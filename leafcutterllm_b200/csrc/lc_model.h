@@ -124,7 +124,7 @@ struct lc_model {
     size_t out_tokens_cap = 0;
     int32_t* d_step_ctr = nullptr;
     unsigned long long* d_stream_slots = nullptr;  // cross-CTA merge slots of the single-token attention kernel (zero between launches)
-    void* d_rot = nullptr;                         // float2 [max_seqs][hd / 2]: cosines and sines of a decode step's rotations (f16 pools of 128-dim heads)
+    void* d_rot = nullptr;                         // float2 [max_seqs][hd / 2]: cosines and sines of a decode step's rotations
     // mixture-of-experts scratch: the router's picks and weights per token, per-expert slot counts and lists, the slots'
     // FFN hidden rows and outputs, every expert's output plane (experts that have no grouped form)
     int32_t *d_moe_sel = nullptr, *d_moe_cnt = nullptr, *d_moe_lists = nullptr;
