@@ -249,26 +249,49 @@ attention_rows_kernel(const float* __restrict__ q, int q_stride, float* __restri
         for (int d = 0; d < DPL; d++) acc[r][d] = 0.f;
     }
     const float root = sqrtf((float)HD);  // attention.rs:93: dot / sqrt(head_dim)
+    // Piece i of the keys and values from t0 on: a float4 of each, zeros past the end (weight zero, and zero times what lies there would not be)
+    auto fetch = [&](int t0, int i, float4& k4, float4& v4) {
+        const int t = i / (HD / 4), c = i % (HD / 4) * 4, pos = t0 + t;
+        k4 = v4 = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (pos >= ctx_end) return;
+        const size_t at = (((size_t)pt[pos / kv.page_tokens] * kv.n_kv + kvh) * kv.page_tokens + pos % kv.page_tokens) * HD + c;
+        if constexpr (F32) {
+            k4 = *reinterpret_cast<const float4*>((const float*)kv.k_pool + at);
+            v4 = *reinterpret_cast<const float4*>((const float*)kv.v_pool + at);
+        } else {
+            const uint2 kh = *reinterpret_cast<const uint2*>((const __half*)kv.k_pool + at), vh = *reinterpret_cast<const uint2*>((const __half*)kv.v_pool + at);
+            const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&kh.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&kh.y));
+            const float2 e = __half22float2(*reinterpret_cast<const __half2*>(&vh.x)), f = __half22float2(*reinterpret_cast<const __half2*>(&vh.y));
+            k4 = make_float4(a.x, a.y, b.x, b.y);
+            v4 = make_float4(e.x, e.y, f.x, f.y);
+        }
+    };
+    // Heads of up to 64: a thread's pieces of the next 32 keys wait in registers while these are worked on (a page-table entry and a row, one after the other, took a third of
+    // a step); wider heads have no registers for them.
+    constexpr int kPieces = kRowsK * (HD / 4) / (32 * kRowsWarps);
+    constexpr bool kAhead = HD <= 64;
+    static_assert(kRowsK * (HD / 4) % (32 * kRowsWarps) == 0, "");
+    float4 nk[kAhead ? kPieces : 1], nv[kAhead ? kPieces : 1];
+    if constexpr (kAhead) {
+#pragma unroll
+        for (int j = 0; j < kPieces; j++) fetch(0, tid + j * 32 * kRowsWarps, nk[j], nv[j]);
+    }
     for (int t0 = 0; t0 < ctx_end; t0 += kRowsK) {
         __syncthreads();  // the tile before has been read
-        for (int i = tid; i < kRowsK * (HD / 4); i += blockDim.x) {
-            const int t = i / (HD / 4), c = i % (HD / 4) * 4, pos = t0 + t;
-            float4 k4 = make_float4(0.f, 0.f, 0.f, 0.f), v4 = k4;  // past the end: weight zero, and zero times what lies there would not be
-            if (pos < ctx_end) {
-                const size_t at = (((size_t)pt[pos / kv.page_tokens] * kv.n_kv + kvh) * kv.page_tokens + pos % kv.page_tokens) * HD + c;
-                if constexpr (F32) {
-                    k4 = *reinterpret_cast<const float4*>((const float*)kv.k_pool + at);
-                    v4 = *reinterpret_cast<const float4*>((const float*)kv.v_pool + at);
-                } else {
-                    const uint2 kh = *reinterpret_cast<const uint2*>((const __half*)kv.k_pool + at), vh = *reinterpret_cast<const uint2*>((const __half*)kv.v_pool + at);
-                    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&kh.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&kh.y));
-                    const float2 e = __half22float2(*reinterpret_cast<const __half2*>(&vh.x)), f = __half22float2(*reinterpret_cast<const __half2*>(&vh.y));
-                    k4 = make_float4(a.x, a.y, b.x, b.y);
-                    v4 = make_float4(e.x, e.y, f.x, f.y);
-                }
-            }
+#pragma unroll
+        for (int j = 0; j < kPieces; j++) {
+            const int i = tid + j * 32 * kRowsWarps, t = i / (HD / 4), c = i % (HD / 4) * 4;
+            float4 k4, v4;
+            if constexpr (kAhead) { k4 = nk[j]; v4 = nv[j]; }
+            else fetch(t0, i, k4, v4);
             *reinterpret_cast<float4*>(sk + t * (HD + 4) + c) = k4;
             *reinterpret_cast<float4*>(sv + t * HD + c) = v4;
+        }
+        if constexpr (kAhead) {
+            if (t0 + kRowsK < ctx_end) {
+#pragma unroll
+                for (int j = 0; j < kPieces; j++) fetch(t0 + kRowsK, tid + j * 32 * kRowsWarps, nk[j], nv[j]);
+            }
         }
         __syncthreads();
         if (mine <= 0 || t0 > last) continue;
