@@ -16,7 +16,7 @@ namespace lc {
 
 // One thread has a pair (d, d + hd / 2) of one token and takes it through several heads: the angle's power, sine and cosine are the same for all of
 // them and cost more than the rotation (a thread per pair and head: 27 us for 512 tokens of 32 + 32 heads, against 8 us of memory traffic).
-__global__ void rope_kv_append_kernel(float* __restrict__ q, float* __restrict__ k, const float* __restrict__ v, int row_stride,
+__global__ void rope_kv_append_kernel(float* __restrict__ q, float* __restrict__ k, const float* __restrict__ v, int row_stride, int kv_stride,
                                       int n_heads, KvLayout kv, const int32_t* __restrict__ tok_seq,
                                       const int32_t* __restrict__ tok_pos, const int32_t* __restrict__ tok_rope,
                                       const int32_t* __restrict__ page_table, int pages_per_seq, float theta) {
@@ -39,8 +39,8 @@ __global__ void rope_kv_append_kernel(float* __restrict__ q, float* __restrict__
             p[d + half] = __fadd_rn(__fmul_rn(x1, sa), __fmul_rn(x2, ca));
         } else {
             const int kh = h - n_heads;
-            float* p = k + (size_t)tok * row_stride + kh * hd;
-            const float* pv = v + (size_t)tok * row_stride + kh * hd;
+            float* p = k + (size_t)tok * kv_stride + kh * hd;
+            const float* pv = v + (size_t)tok * kv_stride + kh * hd;
             const float x1 = p[d], x2 = p[d + half];
             const float r1 = __fsub_rn(__fmul_rn(x1, ca), __fmul_rn(x2, sa));
             const float r2 = __fadd_rn(__fmul_rn(x1, sa), __fmul_rn(x2, ca));
@@ -141,8 +141,8 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_staged_kernel(AttnP
         // the token of this step replaces the (stale) staged slot: rotate, round through f16, keep in the cache
         const int row = pos - t_begin;
         float kr[1], vr;
-        load_rotated<1, HD>(p.k_new + (size_t)tok * p.q_stride + kvh * HD, tid, rp, p.theta, rot, kr);
-        vr = __ldcg(p.v_new + (size_t)tok * p.q_stride + kvh * HD + tid);
+        load_rotated<1, HD>(p.k_new + (size_t)tok * p.kv_stride + kvh * HD, tid, rp, p.theta, rot, kr);
+        vr = __ldcg(p.v_new + (size_t)tok * p.kv_stride + kvh * HD + tid);
         const __half hk = __float2half_rn(kr[0]), hv = __float2half_rn(vr);  // cache/mod.rs:35-36
         K_s[row * HD + tid] = hk;
         V_s[row * HD + tid] = hv;
@@ -265,7 +265,7 @@ static cudaError_t launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, cudaS
     return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
 
-int32_t launch_rope_kv_append(float* q, float* k, const float* v, int row_stride, int n_tok, int n_heads, const KvLayout& kv,
+int32_t launch_rope_kv_append(float* q, float* k, const float* v, int row_stride, int kv_stride, int n_tok, int n_heads, const KvLayout& kv,
                               const int32_t* tok_seq, const int32_t* tok_pos, const int32_t* tok_rope,
                               const int32_t* page_table, int pages_per_seq, float theta, cudaStream_t s) {
     if (n_tok <= 0) return LC_OK;
@@ -273,7 +273,7 @@ int32_t launch_rope_kv_append(float* q, float* k, const float* v, int row_stride
     LC_CHECK(half >= 1 && half * lanes <= 1024, LC_ERR_UNSUPPORTED, "rope: head_dim %d", kv.hd);
     // few tokens: the heads over several CTAs, down to one head per thread
     const int parts = std::min((heads + lanes - 1) / lanes, std::max(1, 8 * sm_count() / n_tok));
-    LC_CUDA(launch_k(rope_kv_append_kernel, dim3((unsigned)n_tok, (unsigned)parts), dim3((unsigned)(half * lanes)), s, q, k, v, row_stride, n_heads, kv, tok_seq,
+    LC_CUDA(launch_k(rope_kv_append_kernel, dim3((unsigned)n_tok, (unsigned)parts), dim3((unsigned)(half * lanes)), s, q, k, v, row_stride, kv_stride, n_heads, kv, tok_seq,
                      tok_pos, tok_rope, page_table, pages_per_seq, theta));
     return LC_OK;
 }
@@ -288,8 +288,8 @@ static void split_plan(int n_tok, int n_heads, int max_ctx, int* chunk, int* n_s
     if (splits < 1) splits = 1;
     int ch = (max_ctx + splits - 1) / splits;
     ch = (ch + 63) / 64 * 64;
-    // A batched decode step (up to 256 tokens, each over its own long context): contexts differ widely, and the CTA of the
-    // longest one would run on alone at the end; 1024-key pieces keep the tail short (64 sequences: 2.66 -> 2.49 ms for 4 layers).
+    // A batched decode step (up to 256 tokens, each over its own long context; caches and heads that attention_batch.cu does not take): contexts differ widely, and the CTA of
+    // the longest one would run on alone at the end; 1024-key pieces keep the tail short (64 sequences: 2.66 -> 2.49 ms for 4 layers).
     if (n_tok <= 256 && ch > 1024) ch = 1024;
     *chunk = ch;
     *n_splits = (max_ctx + ch - 1) / ch;
@@ -306,10 +306,9 @@ size_t attention_scratch_bytes(int n_tok, int n_heads, int hd, int max_ctx) {
 }
 
 static bool staged_applies(const AttnParams& p, int n_tok) {
-    // few tokens (decode): the split-context kernel with shared-memory staging; many tokens (prefill) keep one CTA per (token, head)
-    // Up to four tokens; from eight on the pipelined split-context kernel is faster (7B shape, 8 layers, 1024 keys of context, ms per
-    // step staged / split: 4 sequences 0.95 / 0.97, 8 sequences 1.47 / 1.41, 16 sequences 1.77 / 1.55; Mixtral shape, 16 sequences:
-    // 17.9 / 17.1 ms per step).
+    // Few tokens (decode): the split-context kernel with shared-memory staging; many tokens (prefill) keep one CTA per (token, head).  Up to four tokens, against the pipelined
+    // split-context kernel (7B shape, 8 layers, 1024 keys of context, ms per step staged / split: 4 sequences 0.95 / 0.97, 8 sequences 1.47 / 1.41), where
+    // attention_batch.cu leaves them here (attention_batch_applies has the figures).
     static const int lim = getenv("LC_ATTN_STAGED_TOKENS") ? atoi(getenv("LC_ATTN_STAGED_TOKENS")) : 4;
     return p.kv.hd == 128 && !p.kv.kv_f32 && p.kv.page_tokens == 16 && n_tok * p.n_heads <= staged_pair_limit() && n_tok <= lim;
 }
@@ -353,6 +352,7 @@ int32_t launch_attention(const float* q, int q_stride, float* out, int n_tok, in
     p.k_new = fuse ? fuse->k_new : nullptr; p.v_new = fuse ? fuse->v_new : nullptr;
     p.tok_rope = fuse ? fuse->tok_rope : nullptr; p.theta = fuse ? fuse->theta : 0.f;
     p.rot = fuse ? (const float2*)fuse->rot : nullptr;
+    p.kv_stride = fuse ? fuse->kv_stride : 0;
     p.positions_settled = (fuse && fuse->positions_settled) ? 1 : 0;
     p.error_flag = gemv_error_flag_dev();
     if (fuse && fuse->stream_slots && attention_stream_applies(p, n_tok)) return launch_attention_stream(p, fuse->stream_slots, s);

@@ -223,7 +223,7 @@ attention_batch_kernel(const __grid_constant__ CUtensorMap ktm, const __grid_con
             // this step's token replaces the stale staged row: rotate, round through f16 (cache/mod.rs:35-36), keep in the cache
             const int pos = p.tok_pos[tok], r = pos % kPage, rp = p.tok_rope[tok];
             nvalid = r + 1;
-            const float* const kn = p.k_new + (size_t)tok * p.q_stride + (size_t)kvh * kHD;
+            const float* const kn = p.k_new + (size_t)tok * p.kv_stride + (size_t)kvh * kHD;
             const int d = 4 * (lane & 15);  // of the pair's first half; lanes 16 - 31 have the second
             float4 a = __ldcg(reinterpret_cast<const float4*>(kn + d)), b = __ldcg(reinterpret_cast<const float4*>(kn + d + kHD / 2));
             if (rp != 0) {
@@ -235,7 +235,7 @@ attention_batch_kernel(const __grid_constant__ CUtensorMap ktm, const __grid_con
                 b = make_float4(b0.x, b0.y, b1.x, b1.y);
             }
             const float4 kr = lane < 16 ? a : b;
-            const float4 vr = __ldcg(reinterpret_cast<const float4*>(p.v_new + (size_t)tok * p.q_stride + (size_t)kvh * kHD + 4 * lane));
+            const float4 vr = __ldcg(reinterpret_cast<const float4*>(p.v_new + (size_t)tok * p.kv_stride + (size_t)kvh * kHD + 4 * lane));
             const uint2 kw = make_uint2(half_pair(kr.x, kr.y), half_pair(kr.z, kr.w)), vw = make_uint2(half_pair(vr.x, vr.y), half_pair(vr.z, vr.w));
             // dims 4 lane ..: box lane / 16, chunk (lane % 16) / 2 (swizzled by the row), 8 bytes into it for odd lanes
             const int off = (lane >> 4) * kKHalf + r * 128 + ((((lane & 15) >> 1) ^ (r & 7)) << 4) + (lane & 1) * 8;
@@ -432,7 +432,7 @@ bool attention_batch_applies(const AttnParams& a, int n_tok) {
     // per step staged / here: 3 sequences of 200 768 / 815, of 1,000 870 / 890, of 4,000 1,280 / 1,100.  With kv groups it serves one query head after the other
     // (Mixtral shape, 4 layers, 3 sequences: 1,018 / 965, 1,041 / 990, 1,236 / 1,030).
     return n_tok >= 2 && (n_tok > 4 || gsz > 1) && n_tok <= kMaxBatch && a.k_new && a.rot && a.kv.k_tmap && a.kv.v_tmap && a.kv.hd == kHD && !a.kv.kv_f32 && a.kv.page_tokens == kPage &&
-           a.n_heads % a.kv.n_kv == 0 && (gsz == 1 || gsz == 2 || gsz == 4 || gsz == 8) && a.q_stride % 4 == 0;
+           a.n_heads % a.kv.n_kv == 0 && (gsz == 1 || gsz == 2 || gsz == 4 || gsz == 8) && a.q_stride % 4 == 0 && a.kv_stride % 4 == 0;
 }
 
 int32_t launch_attention_batch(const AttnParams& a, int n_tok, cudaStream_t s) {

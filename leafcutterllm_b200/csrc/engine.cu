@@ -213,55 +213,52 @@ int32_t attention_block(lc_model* m, int l, const float* x, const float* norm_w,
     g.x = x;
     g.norm_w = norm_w;
     g.eps = m->cfg.rms_eps;
+    float* qkv = m->d_qkv;
+    int q_stride = m->nqkv, kv_stride = m->nqkv;
     if (w.fused_qkv) {
         g.w = &w.qkv;
         g.out = m->d_qkv;
         // the fused output is [T, nqkv] only when every token tile writes rows of nqkv floats
         LC_TRY(gemv_tiled(m, g, T, m->nqkv, m->H));
     } else {
-        // q/k/v of different types: three products.  One token writes straight into its row of d_qkv; several tokens go
-        // through contiguous parts and are interleaved into the [T][nq + 2 nkv hd] rows the attention kernels expect.
+        // q/k/v of different types: three products, three contiguous parts (one token: of its row in d_qkv, which is the same)
         const int nq = m->nh * m->hd, nkvd = m->nkv * m->hd;
         const QWeight* ws3[3] = {&w.q, &w.k, &w.v};
         const int ns[3] = {nq, nkvd, nkvd};
-        size_t part_off = 0, col_off = 0;
+        qkv = T == 1 ? m->d_qkv : m->d_qkv_parts;
+        q_stride = nq; kv_stride = nkvd;
+        size_t off = 0;
         for (int i = 0; i < 3; i++) {
             g.w = ws3[i];
-            g.out = T == 1 ? m->d_qkv + col_off : m->d_qkv_parts + part_off;
+            g.out = qkv + off;
             LC_TRY(gemv_tiled(m, g, T, ns[i], m->H));
-            if (T > 1) {
-                LC_CUDA(cudaMemcpy2DAsync(m->d_qkv + col_off, (size_t)m->nqkv * 4, g.out, (size_t)ns[i] * 4, (size_t)ns[i] * 4, (size_t)T,
-                                          cudaMemcpyDeviceToDevice, m->stream));
-                m->launches_in_call += 1;
-            }
-            part_off += (size_t)T * ns[i];
-            col_off += ns[i];
+            off += (size_t)T * ns[i];
         }
     }
     KvLayout kv = kv_layout(m, l);
-    float* q = m->d_qkv;
-    float* k = m->d_qkv + (size_t)m->nh * m->hd;
-    float* v = k + (size_t)m->nkv * m->hd;
+    float* q = qkv;
+    float* k = qkv + (w.fused_qkv ? (size_t)1 : (size_t)T) * m->nh * m->hd;
+    float* v = k + (w.fused_qkv ? (size_t)1 : (size_t)T) * m->nkv * m->hd;
     if (decode_step) {
         // one new token per sequence: rotation and the cache append ride inside the attention kernel
-        AttnFusion fz{k, v, m->d_tok_rope, m->cfg.rope_theta};
+        AttnFusion fz{k, v, kv_stride, m->d_tok_rope, m->cfg.rope_theta};
         fz.positions_settled = l > 0;  // the first layer of a step may run while the previous step still advances the positions
         fz.stream_slots = m->d_stream_slots;
         fz.rot = m->d_rot;
-        LC_TRY(launch_attention(q, m->nqkv, m->d_attn, T, m->nh, kv, m->d_tok_seq, m->d_tok_pos, m->d_page_table, m->pages_per_seq,
+        LC_TRY(launch_attention(q, q_stride, m->d_attn, T, m->nh, kv, m->d_tok_seq, m->d_tok_pos, m->d_page_table, m->pages_per_seq,
                                 m->cfg.max_seq_len, m->d_attn_scratch, m->d_attn_counters, &fz, m->stream));
         m->launches_in_call += 1;
     } else {
-        LC_TRY(launch_rope_kv_append(q, k, v, m->nqkv, T, m->nh, kv, m->d_tok_seq, m->d_tok_pos, m->d_tok_rope, m->d_page_table,
+        LC_TRY(launch_rope_kv_append(q, k, v, q_stride, kv_stride, T, m->nh, kv, m->d_tok_seq, m->d_tok_pos, m->d_tok_rope, m->d_page_table,
                                      m->pages_per_seq, m->cfg.rope_theta, m->stream));
         static const bool no_tc = getenv("LC_PREFILL_FMA") != nullptr;  // diagnostics: the one-CTA-per-(token, head) kernel for every call
         if (T >= 16 && m->n_tiles > 0 && !no_tc && attention_prefill_applies(kv, m->nh))  // a prefill chunk: tiles of 64 queries on the tensor cores
-            LC_TRY(launch_attention_prefill(q, m->nqkv, m->d_attn, m->nh, kv, m->d_tiles, m->n_tiles, m->d_page_table, m->pages_per_seq, m->stream));
-        else if (!no_tc && attention_by_rows(m, T) && attention_rows_applies(kv, m->nh, q, m->nqkv))
-            LC_TRY(launch_attention_rows(q, m->nqkv, m->d_attn, m->nh, kv, m->d_tiles, m->n_tiles, m->d_page_table, m->pages_per_seq, m->stream));
+            LC_TRY(launch_attention_prefill(q, q_stride, m->d_attn, m->nh, kv, m->d_tiles, m->n_tiles, m->d_page_table, m->pages_per_seq, m->stream));
+        else if (!no_tc && attention_by_rows(m, T) && attention_rows_applies(kv, m->nh, q, q_stride))
+            LC_TRY(launch_attention_rows(q, q_stride, m->d_attn, m->nh, kv, m->d_tiles, m->n_tiles, m->d_page_table, m->pages_per_seq, m->stream));
         else
             for (int t0 = 0; t0 < T; t0 += kAttnSlice) {
-                LC_TRY(launch_attention(q + (size_t)t0 * m->nqkv, m->nqkv, m->d_attn + (size_t)t0 * m->nh * m->hd, std::min(kAttnSlice, T - t0), m->nh, kv,
+                LC_TRY(launch_attention(q + (size_t)t0 * q_stride, q_stride, m->d_attn + (size_t)t0 * m->nh * m->hd, std::min(kAttnSlice, T - t0), m->nh, kv,
                                         m->d_tok_seq + t0, m->d_tok_pos + t0, m->d_page_table, m->pages_per_seq, m->cfg.max_seq_len, m->d_attn_scratch,
                                         m->d_attn_counters, nullptr, m->stream));
                 if (t0 > 0) m->launches_in_call += 1;

@@ -11,6 +11,7 @@ constexpr int kAttnWarps = 4;
 struct AttnParams {
     const float* q;        // [n_tok, q_stride]: head h at q + tok*q_stride + h*hd
     int q_stride;
+    int kv_stride;         // of k_new and v_new: kv head h of token t at t * kv_stride + h * hd
     float* out;            // [n_tok, n_heads*hd]
     int n_heads;
     KvLayout kv;
@@ -246,8 +247,8 @@ __device__ __forceinline__ void attention_item(const AttnParams& p, int item, in
         if (has_new) {
             // the token of this step: rotate, round through the cache type, and (one head per kv group) store
             float kr[DPL], vr[DPL];
-            load_rotated<DPL, HD>(p.k_new + (size_t)tok * p.q_stride + kvh * HD, sub * DPL, rp, p.theta, rot, kr);
-            const float* vp = p.v_new + (size_t)tok * p.q_stride + kvh * HD + sub * DPL;
+            load_rotated<DPL, HD>(p.k_new + (size_t)tok * p.kv_stride + kvh * HD, sub * DPL, rp, p.theta, rot, kr);
+            const float* vp = p.v_new + (size_t)tok * p.kv_stride + kvh * HD + sub * DPL;
 #pragma unroll
             for (int i = 0; i < DPL; i++) vr[i] = __ldcg(vp + i);
             if (h % gsz == 0 && warp == 0 && grp == 0) {

@@ -184,7 +184,7 @@ bool make_key_pool_tmap(void* out128, const void* pool, uint64_t rows);
 // position tok_pos[i], with rotary position tok_rope[i]): rotate q and k in place
 // (rust/src/inference/attention.rs:13-34; q, k, v rows are row_stride floats apart) and store k, v into the paged cache
 // (rust/src/cache/mod.rs:33-61: f32 -> f16 round to nearest even).
-int32_t launch_rope_kv_append(float* q, float* k, const float* v, int row_stride, int n_tok, int n_heads, const KvLayout& kv,
+int32_t launch_rope_kv_append(float* q, float* k, const float* v, int row_stride, int kv_stride, int n_tok, int n_heads, const KvLayout& kv,
                               const int32_t* tok_seq, const int32_t* tok_pos, const int32_t* tok_rope,
                               const int32_t* page_table, int pages_per_seq, float theta, cudaStream_t s);
 // Causal GQA attention of every new token over its sequence's cache (attention.rs:69-113).
@@ -200,7 +200,7 @@ size_t attention_batch_scratch_bytes(int n_heads, int n_kv, int hd);  // ... and
 // step on; false for the first layer, whose positions the end of the previous step may still be writing), so the
 // kernel may read it, and start fetching cached pages, before it waits for the kernel ahead of it.
 struct AttnFusion {
-    const float* k_new; const float* v_new; const int32_t* tok_rope; float theta; bool positions_settled = false;
+    const float* k_new; const float* v_new; int kv_stride; const int32_t* tok_rope; float theta; bool positions_settled = false;
     // Cross-CTA merge slots of the single-token streaming kernel (attention_stream_slot_bytes of them, all zero before the
     // first launch; the kernel leaves them zero).  They belong to the caller -- one set per model -- because a captured
     // decode step keeps the pointer.

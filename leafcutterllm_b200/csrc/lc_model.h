@@ -137,7 +137,7 @@ struct lc_model {
     void* d_attn_scratch = nullptr;
     GemmWorkspace gemm_ws;  // f16 activation halves for the many-token tensor-core product
     bool any_unfused_qkv = false;  // some layer's q/k/v differ in type
-    float* d_qkv_parts = nullptr;  // then: [T][nq] | [T][nkv hd] | [T][nkv hd] before they are interleaved into d_qkv
+    float* d_qkv_parts = nullptr;  // then: [T][nq] | [T][nkv hd] | [T][nkv hd]
     int* d_attn_counters = nullptr;
     size_t attn_scratch_bytes = 0;
     unsigned long long* d_sanity = nullptr;

@@ -979,10 +979,10 @@ static int32_t launch_qgemm_tile(const GemvArgs& a, GemmWorkspace& ws, int* slic
     return LC_OK;
 }
 
-// One token tile of Q4_K / Q5_K stays with the kernel above: it multiplies twice per weight where qgemm_split.cu does three times, and up to
-// 64 tokens its instructions are too short for that to be free.  Measured with the activation preparation, us here / there:
-// 16 tokens [4096 -> 12288] 30.6 / 38.5, [4096 -> 4096] 14.5 / 16.8, [11008 -> 4096] 26.6 / 32.2, gate and up 53 / 78;
-// 64 tokens [4096 -> 12288] 41 / 44; 512 tokens 212 / 138, gate and up 327 / 237.
+// Up to 64 tokens of Q4_K / Q5_K stay with the kernel above, whose CTAs need not wait for one another: a pair of qgemm_whole.cu's is longer on its way to its first product and
+// its epilogue.  Measured with the activation preparation, us here / there: 16 tokens [4096 -> 12288] 30.5 / 35.3, [4096 -> 4096] 14.2 / 18.7,
+// [11008 -> 4096] 26.1 / 30.9, [2048 -> 2048] 13.1 / 14.4; 64 tokens 35.2 / 39.4, 17.2 / 21.0, 31.3 / 35.6, 14.3 / 15.8; 65 tokens there 39.7, 21.4, 36.4, 16.0;
+// 512 tokens [4096 -> 12288] 212 / 113.
 static bool use_split(uint32_t typ, int T) { return T > kMaxTok || (typ != LC_TYPE_Q4_K && typ != LC_TYPE_Q5_K); }
 
 // Threads for a token's row.  Few tokens: its three dependent passes are latency, so many threads with one or a few float4 each (64 sequences, 4 layers: 2.43 / 2.40 / 2.40 ms per step

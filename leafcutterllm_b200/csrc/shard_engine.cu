@@ -406,7 +406,7 @@ extern "C" int32_t lc_shard_engine_forward(lc_shard_engine* e, const int64_t* to
             float* q = e->d_qkv;
             float* k = q + nq;
             float* v = k + e->nkv * e->hd;
-            LC_TRY(launch_rope_kv_append(q, k, v, e->nqkv, T, e->nh, kv, e->d_seq, e->d_pos, e->d_rope, e->d_page_table, e->pages, e->theta, s));
+            LC_TRY(launch_rope_kv_append(q, k, v, e->nqkv, e->nqkv, T, e->nh, kv, e->d_seq, e->d_pos, e->d_rope, e->d_page_table, e->pages, e->theta, s));
             LC_TRY(launch_attention(q, e->nqkv, e->d_attn, T, e->nh, kv, e->d_seq, e->d_pos, e->d_page_table, e->pages, e->max_seq, e->d_scratch,
                                     e->d_counters, nullptr, s));
             LC_TRY(matmul(e, w.o, e->d_attn, T, e->d_o));
