@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_staged_kernel(AttnP
         if (lane == 0) red_s[warp] = wm;
         __syncthreads();
         const float m = fmaxf(fmaxf(red_s[0], red_s[1]), fmaxf(red_s[2], red_s[3]));
-        const float pe = (tid < n) ? expf(sc - m) : 0.f;
+        const float pe = sc == -INFINITY ? 0.f : expf(sc - m);  // lanes without a key, and keys that fell below f32's range, whatever the maximum is
         p_s[tid] = pe;
         const float ws = warp_sum(pe);
         if (lane == 0) red_s[4 + warp] = ws;

@@ -206,7 +206,7 @@ __device__ __forceinline__ void attention_item(const AttnParams& p, int item, in
                     for (int i = 0; i < DPL; i++) acc[i] *= alpha;
                     m = s;
                 }
-                const float pexp = expf(s - m);
+                const float pexp = s == -INFINITY ? 0.f : expf(s - m);  // also as the first key of all, where m is minus infinity too
                 l += pexp;
 #pragma unroll
                 for (int i = 0; i < DPL; i++) acc[i] = fmaf(pexp, vr[i], acc[i]);

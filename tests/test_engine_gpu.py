@@ -164,6 +164,34 @@ def test_prompt_attention_where_the_first_keys_score_minus_infinity(gpu, oracle,
     eng.close()
 
 
+def test_a_piece_that_begins_with_scores_of_minus_infinity(gpu, oracle, monkeypatch):
+    """As above, but only keys 0, 1 and 2 of a piece fall below f32's range, the first that three groups of lanes meet: the other keys of the piece keep their weights."""
+    monkeypatch.setenv("LC_ATTN_ROWS", "0")
+    from dataclasses import replace
+    from leafcutterllm_b200 import synth
+    spec = replace(small_spec(12, 12, 12, layers=1, hidden=256, heads=1, kv=1, ffn=256, vocab=64), rope_theta=1e30)
+    eng, om = make_pair(gpu, oracle, spec, max_seq_len=160, kv_dtype="f32", rope_mode="absolute")
+    names = {name: (typ, dims, kind) for name, typ, dims, kind in spec.tensors()}
+
+    def input_for(which, value):
+        name = f"blk.0.attn_{which}.weight"
+        typ, dims, kind = names[name]
+        w = oracle.dequantize(typ, synth.tensor_bytes(spec, name, typ, dims, kind, 1234), 256 * 256).reshape(256, 256)
+        return np.linalg.solve(w.astype(np.float64), value * np.eye(256)[100])
+
+    r = np.random.default_rng(4)
+    first = np.concatenate([input_for("k", -1e34) * (1 + r.random((3, 1))), 1e-6 * r.standard_normal((61, 256))]).astype(np.float32)
+    last = (input_for("q", 1e6) * (1 + r.random((20, 1)))).astype(np.float32)
+    om.attention(0, first)
+    want = om.attention(0, last)
+    assert np.isfinite(want).all()
+    eng.probe_attention(0, first)
+    got = eng.probe_attention(0, last)
+    for i in range(20):
+        assert_close(got[i], want[i], 2e-4 * np.abs(want[i]).max(), 0, f"row {i}")
+    eng.close()
+
+
 @pytest.mark.parametrize("types,heads", [((12, 12, 12), 2), ((2, 8, 8), 8)])
 def test_prompt_longer_than_a_pass(gpu, oracle, types, heads):
     """2,100 tokens: a full pass of 2,048 and a short one behind it; heads of 128 (tiles on the tensor cores) and of 32 (tiles in f32, then the kernel that
