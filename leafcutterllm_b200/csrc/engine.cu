@@ -1071,8 +1071,8 @@ int32_t lc_model_finalize(lc_model* m) {
     }
     LC_CUDA(cudaHostAlloc((void**)&m->pin_tokens, (size_t)m->max_seqs * 8, cudaHostAllocDefault));
     LC_CUDA(cudaHostAlloc((void**)&m->pin_next, ((size_t)m->head_rows + 1) * 8, cudaHostAllocDefault));  // + one word: the device error flag of a call
-    LC_CUDA(cudaHostAlloc((void**)&m->pin_logits, (size_t)m->head_rows * m->cfg.vocab_size * 4, cudaHostAllocDefault));
     logits_blocks_alloc(m);
+    if (m->tp > 1) LC_CUDA(cudaHostAlloc((void**)&m->pin_logits, (size_t)m->head_rows * m->cfg.vocab_size * 4, cudaHostAllocDefault));
     LC_TRY(reserve_out_tokens(m, (size_t)1024 * m->max_seqs));
     LC_CUDA(cudaEventCreate(&m->ev0));
     LC_CUDA(cudaEventCreate(&m->ev1));
@@ -1192,64 +1192,75 @@ int32_t lc_kv_length(const lc_model* m, int32_t seq_id, int32_t* out) {
 }
 
 // ---- page-locked blocks for logits (lc_logits_take) ----
-// A block outlives its handle while somebody holds it.  What comes back without a handle waits for the next handle that is set up or taken down, which adopts or frees it
-// (freeing here would make whoever drops a result wait for the device), up to kLogitsBlockBytes of them.
-struct LogitsBlock { size_t floats; const lc_model* owner; bool taken; };
-static std::mutex g_blocks_lock;
-static std::map<float*, LogitsBlock> g_blocks;
-constexpr int kLogitsBlocks = 2;                           // of a handle: a result that is read while the next step runs
-constexpr size_t kLogitsBlockBytes = (size_t)64 << 20;     // handles whose results may be larger have none
+// Two blocks of a handle lie side by side in one allocation, by its address: a result that is read while the next step runs.  A region outlives its handle while somebody holds one of
+// its blocks; when that comes back it waits for the next handle that is set up or taken down, which adopts or frees it (freeing it here would make whoever drops
+// a result wait for the device), up to kLogitsBytes of them.
+constexpr int kLogitsBlocks = 2;
+constexpr size_t kLogitsBytes = (size_t)128 << 20;  // handles whose blocks would be larger have none
+struct LogitsRegion {
+    size_t floats;  // of a block
+    const lc_model* owner;
+    bool taken[kLogitsBlocks];
+    bool in_use() const { return taken[0] || taken[1]; }
+    size_t bytes() const { return kLogitsBlocks * floats * sizeof(float); }
+};
+static std::mutex g_logits_lock;
+static std::map<float*, LogitsRegion> g_logits;
 
 static void logits_blocks_alloc(const lc_model* m) {
-    const size_t floats = (size_t)m->head_rows * m->cfg.vocab_size;
-    if (m->tp > 1 || floats * 4 > kLogitsBlockBytes) return;
-    for (int i = 0; i < kLogitsBlocks; i++) {
-        float* p = nullptr;
-        {
-            std::lock_guard<std::mutex> g(g_blocks_lock);
-            for (auto& b : g_blocks)
-                if (!p && !b.second.owner && !b.second.taken && b.second.floats >= floats) { p = b.first; b.second.owner = m; }
-        }
-        if (p) continue;
-        if (cudaHostAlloc((void**)&p, floats * 4, cudaHostAllocPortable) != cudaSuccess) { (void)cudaGetLastError(); return; }  // results are copied then
-        std::lock_guard<std::mutex> g(g_blocks_lock);
-        g_blocks[p] = LogitsBlock{floats, m, false};
-    }
+    const LogitsRegion r{(size_t)m->head_rows * m->cfg.vocab_size, m, {}};
+    if (m->tp > 1 || r.bytes() > kLogitsBytes) return;
+    std::lock_guard<std::mutex> g(g_logits_lock);
+    for (auto& o : g_logits)
+        if (!o.second.owner && !o.second.in_use() && o.second.floats >= r.floats) { o.second.owner = m; return; }
+    float* p = nullptr;
+    if (cudaHostAlloc((void**)&p, r.bytes(), cudaHostAllocPortable) == cudaSuccess) g_logits[p] = r;
+    else (void)cudaGetLastError();  // results are copied then
 }
 static void logits_blocks_leave(const lc_model* m) {
-    std::lock_guard<std::mutex> g(g_blocks_lock);
-    for (auto it = g_blocks.begin(); it != g_blocks.end();) {
-        if ((it->second.owner == m || !it->second.owner) && !it->second.taken) { cudaFreeHost(it->first); it = g_blocks.erase(it); continue; }
+    std::lock_guard<std::mutex> g(g_logits_lock);
+    for (auto it = g_logits.begin(); it != g_logits.end();) {
         if (it->second.owner == m) it->second.owner = nullptr;
-        ++it;
+        if (!it->second.owner && !it->second.in_use()) { cudaFreeHost(it->first); it = g_logits.erase(it); }
+        else ++it;
     }
 }
-static bool in_logits_block(const float* p, size_t floats) {
-    std::lock_guard<std::mutex> g(g_blocks_lock);
-    auto it = g_blocks.upper_bound(const_cast<float*>(p));
-    if (it == g_blocks.begin()) return false;
+// the region that p lies in; the lock is held
+static std::map<float*, LogitsRegion>::iterator logits_region(const float* p) {
+    auto it = g_logits.upper_bound(const_cast<float*>(p));
+    if (it == g_logits.begin()) return g_logits.end();
     --it;
-    return it->second.taken && p + floats <= it->first + it->second.floats;
+    return p < it->first + kLogitsBlocks * it->second.floats ? it : g_logits.end();
+}
+static bool in_logits_block(const float* p, size_t floats) {
+    std::lock_guard<std::mutex> g(g_logits_lock);
+    auto it = logits_region(p);
+    if (it == g_logits.end()) return false;
+    const size_t at = (size_t)(p - it->first), b = at / it->second.floats;
+    return it->second.taken[b] && at + floats <= (b + 1) * it->second.floats;
 }
 int32_t lc_logits_take(lc_model* m, uint64_t floats, float** out) {
     LC_TRY(check_model(m, true));
     LC_CHECK(out, LC_ERR_INVALID, "null output");
     *out = nullptr;
-    std::lock_guard<std::mutex> g(g_blocks_lock);
-    for (auto& b : g_blocks)
-        if (b.second.owner == m && !b.second.taken && b.second.floats >= floats) { b.second.taken = true; *out = b.first; break; }
+    std::lock_guard<std::mutex> g(g_logits_lock);
+    for (auto& r : g_logits)
+        if (r.second.owner == m && r.second.floats >= floats)
+            for (int b = 0; b < kLogitsBlocks && !*out; b++)
+                if (!r.second.taken[b]) { r.second.taken[b] = true; *out = r.first + b * r.second.floats; }
     return LC_OK;
 }
 int32_t lc_logits_give(float* block) {
-    std::lock_guard<std::mutex> g(g_blocks_lock);
-    auto it = g_blocks.find(block);
-    LC_CHECK(it != g_blocks.end() && it->second.taken, LC_ERR_INVALID, "lc_logits_give: not a block that was taken");
-    it->second.taken = false;
-    if (it->second.owner) return LC_OK;
+    std::lock_guard<std::mutex> g(g_logits_lock);
+    auto it = logits_region(block);
+    const size_t at = it == g_logits.end() ? 0 : (size_t)(block - it->first);
+    LC_CHECK(it != g_logits.end() && at % it->second.floats == 0 && it->second.taken[at / it->second.floats], LC_ERR_INVALID, "lc_logits_give: not a block that was taken");
+    it->second.taken[at / it->second.floats] = false;
+    if (it->second.owner || it->second.in_use()) return LC_OK;
     size_t waiting = 0;
-    for (auto& b : g_blocks)
-        if (!b.second.owner && !b.second.taken) waiting += b.second.floats * 4;
-    if (waiting > kLogitsBlockBytes) { cudaFreeHost(it->first); g_blocks.erase(it); }
+    for (auto& r : g_logits)
+        if (!r.second.owner && !r.second.in_use()) waiting += r.second.bytes();
+    if (waiting > kLogitsBytes) { cudaFreeHost(it->first); g_logits.erase(it); }
     return LC_OK;
 }
 
@@ -1262,10 +1273,18 @@ static int32_t fetch_logits(lc_model* lead, int n_rows, float* host_out) {
         LC_CUDA(cudaStreamSynchronize(lead->stream));
         return LC_OK;
     }
-    if (lead->tp == 1) {
-        LC_CUDA(cudaMemcpyAsync(lead->pin_logits, lead->d_logits, (size_t)n_rows * Vfull * 4, cudaMemcpyDeviceToHost, lead->stream));
-        LC_CUDA(cudaStreamSynchronize(lead->stream));
-        memcpy(host_out, lead->pin_logits, (size_t)n_rows * Vfull * 4);
+    if (lead->tp == 1) {  // the caller's own memory: by way of a block, or, while all are held, of one that is kept from the first such call on
+        const size_t floats = (size_t)n_rows * Vfull;
+        float* stage = nullptr;
+        LC_TRY(lc_logits_take(lead, floats, &stage));
+        const bool lent = stage != nullptr;
+        if (!stage && !lead->pin_logits) LC_CUDA(cudaHostAlloc((void**)&lead->pin_logits, (size_t)lead->head_rows * Vfull * 4, cudaHostAllocDefault));
+        if (!stage) stage = lead->pin_logits;
+        cudaError_t e = cudaMemcpyAsync(stage, lead->d_logits, floats * 4, cudaMemcpyDeviceToHost, lead->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(lead->stream);
+        if (e == cudaSuccess) memcpy(host_out, stage, floats * 4);
+        if (lent) LC_TRY(lc_logits_give(stage));
+        LC_CUDA(e);
         return LC_OK;
     }
     if (lead->use_dist) {
