@@ -481,7 +481,7 @@ def gemm_microbench(lc, tokens=(64, 512), small: bool = False, shapes=None) -> d
             us = ms.value * 1e3 / (reps * copies)
             rows.append({"tokens": m, "k": k, "n": n, "weight_MB": round(nb / 1e6, 2), "us_per_launch": round(us, 1),
                          "weight_GBps": round(nb / us / 1e3, 1), "TFLOPs": round(2.0 * m * k * n / us / 1e6, 1)})
-    return {"kernel": "qgemm_umma_q4k_kernel (up to 64 tokens), qgemm_split_kernel (more); tcgen05 kind::f16",
+    return {"kernel": "qgemm_umma_q4k_kernel (up to 64 tokens), qgemm_whole_kernel (more); tcgen05 kind::f16",
             "rows": rows}
 
 
