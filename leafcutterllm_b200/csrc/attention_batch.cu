@@ -14,9 +14,9 @@
 //            one of its two places (a run has a first and a last shared segment, no more) and takes a ticket; the last one adds all in worker order.
 //            At most kMostShares warps share a segment.
 //
-// Bound: HBM.  The kernel that had a CTA per (token, head, 1,024 keys), f32 FMAs and the rotation's powers, sines and cosines in each CTA took 592 us for
-// 2.19 GB (64 sequences of 128 - 4,096 tokens, 32 heads) and 84 us for 67 MB (16 of 1,024, 8 kv heads for 32 heads).
-// Now 380 us (5.8 TB/s of measured 6.4) and 38 us.  Runs of whole pieces per CTA would leave the longest sequence's CTA alone at the end.
+// Bound: HBM.  The kernel that had a CTA per (token, head, 1,024 keys), f32 FMAs and the rotation's powers, sines and cosines in each CTA took 594 us for
+// 2.19 GB (64 sequences of 128 - 4,096 tokens, 32 heads) and 88 us for 67 MB (16 of 1,024, 8 kv heads for 32 heads).
+// Now 388 us (5.6 TB/s of measured 6.4) and 29 us; where a step rotates by nothing and there are no kv groups both take 330 - 337 us for 1.98 GB.  Runs of whole pieces per CTA would leave the longest sequence's CTA alone at the end.
 // The rotation's sines and cosines come from a table that the step's first kernel leaves (`rot`).
 #include <algorithm>
 #include <cstring>
