@@ -19,6 +19,7 @@
 // Now 388 us (5.6 TB/s of measured 6.4) and 29 us; where a step rotates by nothing and there are no kv groups both take 330 - 337 us for 1.98 GB.  Runs of whole pieces per CTA would leave the longest sequence's CTA alone at the end.
 // The rotation's sines and cosines come from a table that the step's first kernel leaves (`rot`).
 #include <algorithm>
+#include <cstdlib>
 #include <cstring>
 #include "lc_kernels.h"
 #include "lc_attn.cuh"
@@ -42,6 +43,7 @@ constexpr float kWeightLog2 = 14.f;          // weights are times 2^14, so that 
 struct BatchParams {
     AttnParams a;
     int n_tok;
+    uint32_t wait_limit;  // of the waits for pages
 };
 
 __device__ __forceinline__ uint32_t half_pair(float a, float b) {
@@ -170,7 +172,36 @@ attention_batch_kernel(const __grid_constant__ CUtensorMap ktm, const __grid_con
     int first_page = 0, st = 0;
     uint32_t parity = 0;
 
-    for (int il = 0; il < n_items; il++) {
+    auto next_item = [&] {
+        if (++page == np) {
+            page = 0;
+            if (++kvh == n_kv) {
+                kvh = 0;
+                if (++tok < P.n_tok) np = pre[tok + 1] - pre[tok];
+            }
+        }
+    };
+    auto segment_ends = [&](int il) { return page == np - 1 || il + 1 == n_items; };  // the segment, or the run
+    auto segment_whole = [&] { return first_page == 0 && page == np - 1; };
+    // A ticket of a segment that several warps have a share of; the last one finds the segment's first warp and its number of shares in w_first and shares
+    int w_first = 0, shares = 0;
+    auto last_of_segment = [&] {
+        const long long s_begin = (long long)n_kv * pre[tok] + (long long)kvh * np;
+        w_first = (int)(((s_begin + 1) * G - 1) / W);
+        shares = (int)(((s_begin + np) * G - 1) / W) - w_first + 1;
+        __threadfence();
+        __syncwarp();
+        int last = 0;
+        if (lane == 0) {
+            last = atomicAdd(&p.counters[tok * n_kv + kvh], 1) == shares - 1;
+            if (last) p.counters[tok * n_kv + kvh] = 0;  // ready for the next launch
+        }
+        last = __shfl_sync(0xffffffffu, last, 0);
+        if (last) __threadfence();
+        return last != 0;
+    };
+
+    for (int il = 0; il < n_items; il++, next_item()) {
         if (!begun) {
             begun = true;
             first_page = page;
@@ -214,8 +245,22 @@ attention_batch_kernel(const __grid_constant__ CUtensorMap ktm, const __grid_con
                 for (int mt = 0; mt < 8; mt++) acc[nt][mt][0] = acc[nt][mt][1] = acc[nt][mt][2] = acc[nt][mt][3] = 0.f;
             }
         }
-        ok = mbar_wait(&full[st], parity) && ok;
+        if (ok && !__all_sync(0xffffffffu, mbar_wait(&full[st], parity, P.wait_limit))) {
+            // The copies under way get their time once more to land in this CTA's memory, and no more are requested: a barrier may not be armed again while its phase is open
+            ok = false;
+            for (int i = 0; i < kStages && il + i < n_items; i++) {
+                mbar_wait(&full[st], parity);
+                if (++st == kStages) { st = 0; parity ^= 1; }
+            }
+        }
         __syncwarp();
+        if (!ok) {  // the rest of the run is only counted: tickets come out as for the other warps, and the counters are left at zero
+            if (segment_ends(il)) {
+                if (!segment_whole()) last_of_segment();
+                begun = false;
+            }
+            continue;
+        }
         unsigned char* const K_b = ring + st * kStageBytes;
         unsigned char* const V_b = K_b + 2 * kKHalf;
         int nvalid = kPage;
@@ -318,8 +363,8 @@ attention_batch_kernel(const __grid_constant__ CUtensorMap ktm, const __grid_con
         if (il + kStages < n_items) copy_next(st);
         if (++st == kStages) { st = 0; parity ^= 1; }
 
-        if (page == np - 1 || il + 1 == n_items) {  // the segment's end, or the run's
-            const bool whole = first_page == 0 && page == np - 1;
+        if (segment_ends(il)) {
+            const bool whole = segment_whole();
             const int slot = first_page > 0 ? 0 : 1;
             float* const mine = p.partial + ((size_t)worker * 2 + slot) * GSZ * kStateWords;
             float* const out = p.out + ((size_t)tok * p.n_heads + (size_t)kvh * GSZ) * kHD;
@@ -341,67 +386,50 @@ attention_batch_kernel(const __grid_constant__ CUtensorMap ktm, const __grid_con
                     dst[mt * 16 + 8] = whole ? v1 / l_own[nt] : v1;
                 }
             }
-            if (!whole) {
-                const long long s_begin = (long long)n_kv * pre[tok] + (long long)kvh * np;
-                const int w_first = (int)(((s_begin + 1) * G - 1) / W), shares = (int)(((s_begin + np) * G - 1) / W) - w_first + 1;
-                __threadfence();
-                __syncwarp();
-                int ticket = 0;
-                if (lane == 0) ticket = atomicAdd(&p.counters[tok * n_kv + kvh], 1);
-                if (__shfl_sync(0xffffffffu, ticket, 0) == shares - 1) {
-                    __threadfence();
-                    const int w = w_first + min(lane, shares - 1);
-                    const float* const theirs = p.partial + ((size_t)w * 2 + (s_begin < w * W / G ? 0 : 1)) * GSZ * kStateWords;
-                    const size_t place = (size_t)(theirs - p.partial);
-                    float e[GSZ], sum[GSZ];  // every load of a round is in flight before the first is used
+            if (!whole && last_of_segment()) {
+                const int w = w_first + min(lane, shares - 1);
+                const float* const theirs = p.partial + ((size_t)w * 2 + ((long long)n_kv * pre[tok] + (long long)kvh * np < w * W / G ? 0 : 1)) * GSZ * kStateWords;
+                const size_t place = (size_t)(theirs - p.partial);
+                float e[GSZ], sum[GSZ];  // every load of a round is in flight before the first is used
 #pragma unroll
-                    for (int h = 0; h < GSZ; h++) {
-                        e[h] = lane < shares ? __ldcg(theirs + h * kStateWords) : -INFINITY;
-                        sum[h] = lane < shares ? __ldcg(theirs + h * kStateWords + 1) : 0.f;
-                    }
-#pragma unroll
-                    for (int h = 0; h < GSZ; h++) {
-                        const float most = warp_max(e[h]);
-                        e[h] = e[h] == -INFINITY ? 0.f : exp2f(e[h] - most);
-                        sum[h] = warp_sum(sum[h] * e[h]);
-                    }
-                    constexpr int kRound = GSZ >= 4 ? 16 / GSZ : 8;
-                    float4 v[GSZ];
-#pragma unroll
-                    for (int h = 0; h < GSZ; h++) v[h] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    for (int s0 = 0; s0 < shares; s0 += kRound) {  // in worker order; past the last share: that one again, not added
-                        float4 u[kRound][GSZ];
-#pragma unroll
-                        for (int i = 0; i < kRound; i++) {
-                            const size_t at = __shfl_sync(0xffffffffu, (unsigned long long)place, min(s0 + i, shares - 1));
-#pragma unroll
-                            for (int h = 0; h < GSZ; h++) u[i][h] = __ldcg(reinterpret_cast<const float4*>(p.partial + at + (size_t)h * kStateWords + 4) + lane);
-                        }
-#pragma unroll
-                        for (int i = 0; i < kRound; i++) {
-                            if (s0 + i >= shares) break;
-#pragma unroll
-                            for (int h = 0; h < GSZ; h++) {
-                                const float es = __shfl_sync(0xffffffffu, e[h], s0 + i);
-                                v[h].x = fmaf(u[i][h].x, es, v[h].x); v[h].y = fmaf(u[i][h].y, es, v[h].y);
-                                v[h].z = fmaf(u[i][h].z, es, v[h].z); v[h].w = fmaf(u[i][h].w, es, v[h].w);
-                            }
-                        }
-                    }
-#pragma unroll
-                    for (int h = 0; h < GSZ; h++)
-                        reinterpret_cast<float4*>(out + h * kHD)[lane] = make_float4(v[h].x / sum[h], v[h].y / sum[h], v[h].z / sum[h], v[h].w / sum[h]);
-                    if (lane == 0) p.counters[tok * n_kv + kvh] = 0;  // ready for the next launch
+                for (int h = 0; h < GSZ; h++) {
+                    e[h] = lane < shares ? __ldcg(theirs + h * kStateWords) : -INFINITY;
+                    sum[h] = lane < shares ? __ldcg(theirs + h * kStateWords + 1) : 0.f;
                 }
+#pragma unroll
+                for (int h = 0; h < GSZ; h++) {
+                    const float most = warp_max(e[h]);
+                    e[h] = e[h] == -INFINITY ? 0.f : exp2f(e[h] - most);
+                    sum[h] = warp_sum(sum[h] * e[h]);
+                }
+                constexpr int kRound = GSZ >= 4 ? 16 / GSZ : 8;
+                float4 v[GSZ];
+#pragma unroll
+                for (int h = 0; h < GSZ; h++) v[h] = make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int s0 = 0; s0 < shares; s0 += kRound) {  // in worker order; past the last share: that one again, not added
+                    float4 u[kRound][GSZ];
+#pragma unroll
+                    for (int i = 0; i < kRound; i++) {
+                        const size_t at = __shfl_sync(0xffffffffu, (unsigned long long)place, min(s0 + i, shares - 1));
+#pragma unroll
+                        for (int h = 0; h < GSZ; h++) u[i][h] = __ldcg(reinterpret_cast<const float4*>(p.partial + at + (size_t)h * kStateWords + 4) + lane);
+                    }
+#pragma unroll
+                    for (int i = 0; i < kRound; i++) {
+                        if (s0 + i >= shares) break;
+#pragma unroll
+                        for (int h = 0; h < GSZ; h++) {
+                            const float es = __shfl_sync(0xffffffffu, e[h], s0 + i);
+                            v[h].x = fmaf(u[i][h].x, es, v[h].x); v[h].y = fmaf(u[i][h].y, es, v[h].y);
+                            v[h].z = fmaf(u[i][h].z, es, v[h].z); v[h].w = fmaf(u[i][h].w, es, v[h].w);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int h = 0; h < GSZ; h++)
+                    reinterpret_cast<float4*>(out + h * kHD)[lane] = make_float4(v[h].x / sum[h], v[h].y / sum[h], v[h].z / sum[h], v[h].w / sum[h]);
             }
             begun = false;
-        }
-        if (++page == np) {
-            page = 0;
-            if (++kvh == n_kv) {
-                kvh = 0;
-                if (++tok < P.n_tok) np = pre[tok + 1] - pre[tok];
-            }
         }
     }
     if (!ok && lane == 0 && p.error_flag) atomicCAS(p.error_flag, 0, 1);
@@ -438,6 +466,8 @@ bool attention_batch_applies(const AttnParams& a, int n_tok) {
 int32_t launch_attention_batch(const AttnParams& a, int n_tok, cudaStream_t s) {
     BatchParams P;
     P.a = a; P.n_tok = n_tok;
+    const char* const limit = getenv("LC_ATTN_WAITS");  // read per launch so that a test can make the waits run out: 0, before they look
+    P.wait_limit = limit ? (uint32_t)atoi(limit) : 1u << 22;
     switch (a.n_heads / a.kv.n_kv) {
         case 1: return launch_batch<1>(P, s);
         case 2: return launch_batch<2>(P, s);

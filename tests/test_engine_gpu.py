@@ -350,6 +350,32 @@ def test_batched_decode_attention_as_one_stream(gpu, oracle, heads, kv):
             assert err < 4 * 2.0 ** -11, (i, step, err)
 
 
+def test_batched_decode_attention_whose_waits_run_out(gpu, monkeypatch):
+    """Every wait for a page gives up before it looks (LC_ATTN_WAITS=0, a step's launches are made anew for another number of sequences): the call ends with an error, and
+    the handle is usable: the tickets of segments that several warps share are back at zero, so the next steps give what a handle gives that never failed."""
+    from leafcutterllm_b200 import synth
+    spec = small_spec(12, 12, 12, layers=2, hidden=512, heads=4, kv=1, ffn=512, vocab=512)
+    lens = [600, 16, 300, 1, 128, 33]
+    prompts = [synth.prompt_tokens(n, spec.vocab_size, 500 + i).tolist() for i, n in enumerate(lens)]
+
+    def steps(eng, n):
+        eng.kv_clear()
+        eng.forward_batch(list(range(n)), prompts[:n], want_logits=False)
+        return [eng.forward_batch(list(range(n)), [[7 + i] for i in range(n)])[0].copy() for _ in range(2)]
+
+    eng = synth.build_engine(spec, 640, max_seqs=len(lens), rope_mode="absolute")
+    want = steps(eng, 5)
+    eng.close()
+    eng = synth.build_engine(spec, 640, max_seqs=len(lens), rope_mode="absolute")
+    monkeypatch.setenv("LC_ATTN_WAITS", "0")
+    with pytest.raises(gpu.LeafcutterError, match="a bounded wait ran out"):
+        steps(eng, 6)
+    monkeypatch.delenv("LC_ATTN_WAITS")
+    for a, b in zip(steps(eng, 5), want):
+        assert np.array_equal(a, b)
+    eng.close()
+
+
 def test_prefill_attention_on_tensor_cores_ragged(gpu, oracle):
     """head_dim 128, f16 cache: calls of 16 tokens and more run the tiled tensor-core prefill attention.  Four sequences of
     70, 16, 129 and 33 tokens in ONE call (tiles end where a sequence ends; 129 = two full tiles and a one-token tile), then a
