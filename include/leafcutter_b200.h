@@ -346,10 +346,6 @@ int32_t lc_forward(lc_model* m, const int64_t* tokens, int32_t n, float* logits_
 int32_t lc_forward_batch(lc_model* m, int32_t n_seqs, const int32_t* seq_ids, const int64_t* tokens,
                          const int32_t* n_tokens, float* logits_out, int64_t* next_out);
 
-/* A page-locked block of this handle for `floats` logits; *out = NULL when none is free or large enough.  Calls that return logits write straight into one (elsewhere
- * they copy once more).  It stays valid, also past lc_model_destroy, until lc_logits_give.  Any thread may take and give. */
-int32_t lc_logits_take(lc_model* m, uint64_t floats, float** out);
-int32_t lc_logits_give(float* block);
 /* lc_forward_batch with a choice of rows: sequence i wants the logits of n_want[i] places (0-based among its tokens of this
  * call, ascending; possibly none), listed in `want` one sequence after the other.  logits_out is [sum of n_want, vocab],
  * next_out the greedy picks of the same rows (both may be NULL). */

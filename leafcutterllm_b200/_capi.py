@@ -124,8 +124,6 @@ SIGNATURES = {
     "lc_kv_memory_bytes": (_i32, [_vp, C.POINTER(_u64)]),
     "lc_kv_length": (_i32, [_vp, _i32, C.POINTER(_i32)]),
     "lc_forward": (_i32, [_vp, _vp, _i32, _vp]),
-    "lc_logits_take": (_i32, [_vp, C.c_uint64, C.POINTER(_vp)]),
-    "lc_logits_give": (_i32, [_vp]),
     "lc_forward_batch": (_i32, [_vp, _i32, _vp, _vp, _vp, _vp, _vp]),
     "lc_generate": (_i32, [_vp, _vp, _i32, _i32, C.c_float, C.c_float, _i32, _vp, C.POINTER(_i32), TOKEN_CB, _vp]),
     "lc_decode_loop": (_i32, [_vp, _i32, _vp, _vp, _i32, _vp, _f]),

@@ -12,7 +12,6 @@
 #include <algorithm>
 #include <cstring>
 #include <map>
-#include <mutex>
 #include <string>
 #include <vector>
 #include "lc_model.h"
@@ -1013,9 +1012,6 @@ static int32_t alloc_block_buffers(lc_model* m) {
     return LC_OK;
 }
 
-static void logits_blocks_alloc(const lc_model* m);
-static void logits_blocks_leave(const lc_model* m);
-
 int32_t lc_model_finalize(lc_model* m) {
     LC_TRY(check_model(m, false));
     LC_CHECK(!m->finalized, LC_ERR_STATE, "model already finalized");
@@ -1071,11 +1067,11 @@ int32_t lc_model_finalize(lc_model* m) {
     }
     LC_CUDA(cudaHostAlloc((void**)&m->pin_tokens, (size_t)m->max_seqs * 8, cudaHostAllocDefault));
     LC_CUDA(cudaHostAlloc((void**)&m->pin_next, ((size_t)m->head_rows + 1) * 8, cudaHostAllocDefault));  // + one word: the device error flag of a call
-    logits_blocks_alloc(m);
-    if (m->tp > 1) LC_CUDA(cudaHostAlloc((void**)&m->pin_logits, (size_t)m->head_rows * m->cfg.vocab_size * 4, cudaHostAllocDefault));
+    LC_CUDA(cudaHostAlloc((void**)&m->pin_logits, (size_t)m->head_rows * m->cfg.vocab_size * 4, cudaHostAllocDefault));
     LC_TRY(reserve_out_tokens(m, (size_t)1024 * m->max_seqs));
     LC_CUDA(cudaEventCreate(&m->ev0));
     LC_CUDA(cudaEventCreate(&m->ev1));
+    for (cudaEvent_t& e : m->ev_logits) LC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     LC_CUDA(cudaStreamSynchronize(m->stream));
     m->finalized = true;
     return LC_OK;
@@ -1108,7 +1104,7 @@ int32_t lc_model_destroy(lc_model* m) {
     if (m->pin_tokens) cudaFreeHost(m->pin_tokens);
     if (m->pin_next) cudaFreeHost(m->pin_next);
     if (m->pin_logits) cudaFreeHost(m->pin_logits);
-    logits_blocks_leave(m);
+    for (cudaEvent_t e : m->ev_logits) if (e) cudaEventDestroy(e);
     if (m->ev0) cudaEventDestroy(m->ev0);
     if (m->ev1) cudaEventDestroy(m->ev1);
     delete m;
@@ -1191,100 +1187,23 @@ int32_t lc_kv_length(const lc_model* m, int32_t seq_id, int32_t* out) {
     return LC_OK;
 }
 
-// ---- page-locked blocks for logits (lc_logits_take) ----
-// Two blocks of a handle lie side by side in one allocation, by its address: a result that is read while the next step runs.  A region outlives its handle while somebody holds one of
-// its blocks; when that comes back it waits for the next handle that is set up or taken down, which adopts or frees it (freeing it here would make whoever drops
-// a result wait for the device), up to kLogitsBytes of them.
-constexpr int kLogitsBlocks = 2;
-constexpr size_t kLogitsBytes = (size_t)128 << 20;  // handles whose blocks would be larger have none
-struct LogitsRegion {
-    size_t floats;  // of a block
-    const lc_model* owner;
-    bool taken[kLogitsBlocks];
-    bool in_use() const { return taken[0] || taken[1]; }
-    size_t bytes() const { return kLogitsBlocks * floats * sizeof(float); }
-};
-static std::mutex g_logits_lock;
-static std::map<float*, LogitsRegion> g_logits;
-
-static void logits_blocks_alloc(const lc_model* m) {
-    const LogitsRegion r{(size_t)m->head_rows * m->cfg.vocab_size, m, {}};
-    if (m->tp > 1 || r.bytes() > kLogitsBytes) return;
-    std::lock_guard<std::mutex> g(g_logits_lock);
-    for (auto& o : g_logits)
-        if (!o.second.owner && !o.second.in_use() && o.second.floats >= r.floats) { o.second.owner = m; return; }
-    float* p = nullptr;
-    if (cudaHostAlloc((void**)&p, r.bytes(), cudaHostAllocPortable) == cudaSuccess) g_logits[p] = r;
-    else (void)cudaGetLastError();  // results are copied then
-}
-static void logits_blocks_leave(const lc_model* m) {
-    std::lock_guard<std::mutex> g(g_logits_lock);
-    for (auto it = g_logits.begin(); it != g_logits.end();) {
-        if (it->second.owner == m) it->second.owner = nullptr;
-        if (!it->second.owner && !it->second.in_use()) { cudaFreeHost(it->first); it = g_logits.erase(it); }
-        else ++it;
-    }
-}
-// the region that p lies in; the lock is held
-static std::map<float*, LogitsRegion>::iterator logits_region(const float* p) {
-    auto it = g_logits.upper_bound(const_cast<float*>(p));
-    if (it == g_logits.begin()) return g_logits.end();
-    --it;
-    return p < it->first + kLogitsBlocks * it->second.floats ? it : g_logits.end();
-}
-static bool in_logits_block(const float* p, size_t floats) {
-    std::lock_guard<std::mutex> g(g_logits_lock);
-    auto it = logits_region(p);
-    if (it == g_logits.end()) return false;
-    const size_t at = (size_t)(p - it->first), b = at / it->second.floats;
-    return it->second.taken[b] && at + floats <= (b + 1) * it->second.floats;
-}
-int32_t lc_logits_take(lc_model* m, uint64_t floats, float** out) {
-    LC_TRY(check_model(m, true));
-    LC_CHECK(out, LC_ERR_INVALID, "null output");
-    *out = nullptr;
-    std::lock_guard<std::mutex> g(g_logits_lock);
-    for (auto& r : g_logits)
-        if (r.second.owner == m && r.second.floats >= floats)
-            for (int b = 0; b < kLogitsBlocks && !*out; b++)
-                if (!r.second.taken[b]) { r.second.taken[b] = true; *out = r.first + b * r.second.floats; }
-    return LC_OK;
-}
-int32_t lc_logits_give(float* block) {
-    std::lock_guard<std::mutex> g(g_logits_lock);
-    auto it = logits_region(block);
-    const size_t at = it == g_logits.end() ? 0 : (size_t)(block - it->first);
-    LC_CHECK(it != g_logits.end() && at % it->second.floats == 0 && it->second.taken[at / it->second.floats], LC_ERR_INVALID, "lc_logits_give: not a block that was taken");
-    it->second.taken[at / it->second.floats] = false;
-    if (it->second.owner || it->second.in_use()) return LC_OK;
-    size_t waiting = 0;
-    for (auto& r : g_logits)
-        if (!r.second.owner && !r.second.in_use()) waiting += r.second.bytes();
-    if (waiting > kLogitsBytes) { cudaFreeHost(it->first); g_logits.erase(it); }
-    return LC_OK;
-}
-
 // The logits rows [0, n_rows) of the whole vocabulary on the host: a whole model copies them; a cut model puts the ranks'
 // vocabulary slices side by side (an all-gather when the ranks are processes).
 static int32_t fetch_logits(lc_model* lead, int n_rows, float* host_out) {
     const int Vfull = lead->cfg.vocab_size, Vl = lead->V;
-    if (lead->tp == 1 && in_logits_block(host_out, (size_t)n_rows * Vfull)) {
-        LC_CUDA(cudaMemcpyAsync(host_out, lead->d_logits, (size_t)n_rows * Vfull * 4, cudaMemcpyDeviceToHost, lead->stream));
-        LC_CUDA(cudaStreamSynchronize(lead->stream));
-        return LC_OK;
-    }
-    if (lead->tp == 1) {  // the caller's own memory: by way of a block, or, while all are held, of one that is kept from the first such call on
-        const size_t floats = (size_t)n_rows * Vfull;
-        float* stage = nullptr;
-        LC_TRY(lc_logits_take(lead, floats, &stage));
-        const bool lent = stage != nullptr;
-        if (!stage && !lead->pin_logits) LC_CUDA(cudaHostAlloc((void**)&lead->pin_logits, (size_t)lead->head_rows * Vfull * 4, cudaHostAllocDefault));
-        if (!stage) stage = lead->pin_logits;
-        cudaError_t e = cudaMemcpyAsync(stage, lead->d_logits, floats * 4, cudaMemcpyDeviceToHost, lead->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(lead->stream);
-        if (e == cudaSuccess) memcpy(host_out, stage, floats * 4);
-        if (lent) LC_TRY(lc_logits_give(stage));
-        LC_CUDA(e);
+    if (lead->tp == 1) {
+        // The caller's memory is written by this thread alone (a copy that the caller began from it is staged when it returns, as from any pageable memory), piece by piece while
+        // the next pieces come: 64 rows of 32,000 493 us, in one piece 610; 16 rows 140 / 160.
+        const size_t bytes = (size_t)n_rows * Vfull * 4, piece = std::max((size_t)1 << 20, (bytes / kLogitsPieces + 255) & ~(size_t)255);
+        char *const to = reinterpret_cast<char*>(host_out), *const pin = reinterpret_cast<char*>(lead->pin_logits);
+        for (size_t at = 0, i = 0; at < bytes; at += piece, i++) {
+            LC_CUDA(cudaMemcpyAsync(pin + at, reinterpret_cast<const char*>(lead->d_logits) + at, std::min(piece, bytes - at), cudaMemcpyDeviceToHost, lead->stream));
+            LC_CUDA(cudaEventRecord(lead->ev_logits[i], lead->stream));
+        }
+        for (size_t at = 0, i = 0; at < bytes; at += piece, i++) {
+            LC_CUDA(cudaEventSynchronize(lead->ev_logits[i]));
+            memcpy(to + at, pin + at, std::min(piece, bytes - at));
+        }
         return LC_OK;
     }
     if (lead->use_dist) {

@@ -54,6 +54,7 @@ constexpr int kAttnSlice = 512;          // tokens per launch of the attention k
 constexpr int kTileRun = 16;             // runs of fewer tokens attend token by token
 constexpr int kChunkRun = 32;            // runs of fewer tokens walk the gated delta rule token by token
 constexpr int kStackChunk = 2048;      // tokens per pass of a checkpoint-directory design
+constexpr int kLogitsPieces = 16;      // most pieces in which logits come to the host
 constexpr int kTokTile = 8;
 constexpr int kMoeGroupedTokens = 64;  // most tokens of a call whose experts run as one grouped matrix-vector launch
 // Rows per expert beyond which the experts run as a grouped many-token product instead: the matrix-vector kernel reads the experts again for
@@ -145,6 +146,7 @@ struct lc_model {
     std::map<int, cudaGraphExec_t> decode_graphs;
     int graph_nodes = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t ev_logits[kLogitsPieces] = {};  // a piece of the logits is in pin_logits
 
     lc_counters ctr{};
     uint64_t launches_in_call = 0;

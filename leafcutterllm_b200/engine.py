@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes as C
 import json
+from collections import deque
 from typing import Callable, Iterable, Optional, Sequence
 
 import numpy as np
@@ -20,15 +21,14 @@ def _p(a: np.ndarray):
     return a.ctypes.data_as(C.c_void_p)
 
 
-class _Block:
-    """A page-locked block that the library lends; goes back when the last array over it is gone."""
+class _Memory:
+    """Ordinary memory of a result; when the last array over it is gone, its engine has it for a later result of the same shape."""
 
-    def __init__(self, address: int, shape: tuple):
-        self.address, self._give = address, load().lc_logits_give
-        self.__array_interface__ = {"data": (address, False), "shape": shape, "typestr": "<f4", "version": 3}
+    def __init__(self, spare: deque, memory: np.ndarray):
+        self._spare, self._memory, self.__array_interface__ = spare, memory, memory.__array_interface__
 
     def __del__(self):
-        self._give(self.address)
+        self._spare.append(self._memory)
 
 
 class Engine:
@@ -46,6 +46,7 @@ class Engine:
         cfg.rope_mode = {"call_relative": 0, "absolute": 1}[rope_mode]
         cfg.max_seqs, cfg.kv_page_tokens, cfg.kv_pool_tokens, cfg.device = max_seqs, kv_page_tokens, kv_pool_tokens, device
         self.cfg = cfg
+        self._spare = deque(maxlen=2)  # memory of results that are gone
         self._h = C.c_void_p()
         check(load().lc_model_create(C.byref(cfg), C.byref(self._h)))
         self.vocab_size = vocab_size
@@ -62,6 +63,7 @@ class Engine:
         over.rope_mode = {"call_relative": 0, "absolute": 1}[rope_mode]
         over.max_seqs, over.kv_page_tokens, over.kv_pool_tokens, over.device = max_seqs, kv_page_tokens, kv_pool_tokens, device
         self = cls.__new__(cls)
+        self._spare = deque(maxlen=2)
         self._h = C.c_void_p()
         check(load().lc_model_load_gguf(str(path).encode(), C.byref(over), C.byref(self._h)))
         cfg = ModelConfig()
@@ -74,6 +76,7 @@ class Engine:
     @classmethod
     def _adopt(cls, handle, max_seqs: int) -> "Engine":
         self = cls.__new__(cls)
+        self._spare = deque(maxlen=2)
         self._h = handle
         cfg = ModelConfig()
         check(load().lc_model_get_config(handle, C.byref(cfg)))
@@ -160,10 +163,15 @@ class Engine:
         return out
 
     def _logits_array(self, rows: int) -> np.ndarray:
-        """Where a call's logits go: page-locked memory that the device writes into, while the handle has some to lend."""
-        shape, block = (rows, self.vocab_size), C.c_void_p()
-        check(load().lc_logits_take(self._h, rows * self.vocab_size, C.byref(block)))
-        return np.asarray(_Block(block.value, shape)) if block.value else np.empty(shape, np.float32)
+        """Where a call's logits go: memory of an earlier result, where there is some (the first write to 8 MB of new pages takes 2 ms, and malloc gives 32 MB and more back)."""
+        shape = (rows, self.vocab_size)
+        try:
+            memory = self._spare.pop()
+        except IndexError:
+            memory = None
+        if memory is None or memory.shape != shape:
+            memory = np.empty(shape, np.float32)
+        return np.asarray(_Memory(self._spare, memory))
 
     def forward_batch(self, seq_ids: Sequence[int], token_lists: Sequence[Sequence[int]], want_logits: bool = True):
         n = len(seq_ids)
@@ -248,6 +256,7 @@ class Engine:
         if self._h:
             load().lc_model_destroy(self._h)
             self._h = C.c_void_p()
+            self._spare = deque(maxlen=0)
 
     def __del__(self):
         try:

@@ -326,6 +326,29 @@ def test_results_stay_what_they_are_while_somebody_holds_them(gpu, oracle):
     again.close()
 
 
+@pytest.mark.parametrize("rows,vocab", [(3, 512), (9, 32000)])
+def test_a_copy_that_begins_before_a_result_is_dropped(gpu, rows, vocab):
+    """A caller starts asynchronous copies of results to the GPU behind work that takes a while, and drops the results; the calls that follow leave what is copied alone."""
+    import torch
+    from leafcutterllm_b200 import synth
+    eng = synth.build_engine(small_spec(12, 12, 12, layers=1, vocab=vocab), 64, max_seqs=rows)
+    ids, steps = list(range(rows)), [[[7 * i + j] for j in range(rows)] for i in range(6)]
+    side, want, got = torch.cuda.Stream(), [], []
+    for s in steps[:3]:
+        logits = eng.forward_batch(ids, s)[0]
+        want.append(logits.copy())
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(200_000_000)
+            got.append(torch.from_numpy(logits).to("cuda", non_blocking=True))
+        del logits
+    for s in steps[3:]:
+        eng.forward_batch(ids, s)
+    torch.cuda.synchronize()
+    eng.close()
+    for a, b in zip(got, want):
+        assert np.array_equal(a.cpu().numpy(), b)
+
+
 @pytest.mark.parametrize("heads,kv", [(4, 4), (4, 2), (4, 1), (8, 1)])
 def test_batched_decode_attention_as_one_stream(gpu, oracle, heads, kv):
     """The (token, kv head, page) items of a decode step cut into one run per warp: contexts on both sides of a page's edge, a first token, one that many runs
