@@ -9,7 +9,8 @@
 //            its input (cached pages belong to earlier steps); page-table entries are read 32 at a time, one per lane;
 //   scores   ldmatrix + mma.sync m16n8k16 against the query heads of the kv group, which are columns of f16 high and low halves
 //            (times a power of two per head, so that 22 bits are kept whatever their size);
-//   sums     online softmax in log2 units, weights times 2^14 as high and low halves against the transposed values;
+//   sums     online softmax in log2 units, weights times 2^14 as high and low halves against the transposed values.  The matrix unit truncates when it adds, so it adds up
+//            a page and no more (a score: 16 dims); the pages are added in f32, and what those roundings lose is kept beside the low halves' sums;
 //   merge    a (token, kv head) that lies within one run is finished by its warp.  Else each of its warps leaves maximum, sum and weighted values in
 //            one of its two places (a run has a first and a last shared segment, no more) and takes a ticket; the last one adds all in worker order.
 //            At most kMostShares warps share a segment.
@@ -38,7 +39,9 @@ constexpr int kMaxBatch = 1024;              // tokens whose page counts a CTA a
 constexpr int kStateWords = 4 + kHD;         // maximum, sum, two pad words, weighted values
 constexpr int kMostShares = 32;              // a lane for each when they are added
 constexpr int kLeastPages = 8;               // of a run: a page costs a warp less than a share costs the warp that adds them (16 sequences of 1,000 and less; 4 and 10: 0 - 2 % slower)
-constexpr float kWeightLog2 = 14.f;          // weights are times 2^14, so that their low halves keep their bits
+constexpr int kChains = 8;                   // of products in a page's scores
+constexpr float kCutOff = 2.7e-8f;           // what a page's weighted values lose on average
+constexpr float kWeightScale = 16384.f;      // weights are times 2^14, so that their low halves keep their bits
 
 struct BatchParams {
     AttnParams a;
@@ -71,6 +74,13 @@ __device__ __forceinline__ void rotate_pair(float2& x, float2& y, float4 cs) {  
     x.y = __fsub_rn(__fmul_rn(u.y, cs.z), __fmul_rn(v.y, cs.w));
     y.x = __fadd_rn(__fmul_rn(u.x, cs.y), __fmul_rn(v.x, cs.x));
     y.y = __fadd_rn(__fmul_rn(u.y, cs.w), __fmul_rn(v.y, cs.z));
+}
+
+// sum += x; what the addition's rounding lost goes to `low` (of a smaller sum than x: a part of it)
+__device__ __forceinline__ void add_keeping(float& sum, float& low, float x) {
+    const float s = sum + x;
+    low += x - (s - sum);
+    sum = s;
 }
 
 template <int GSZ>
@@ -166,7 +176,7 @@ attention_batch_kernel(const __grid_constant__ CUtensorMap ktm, const __grid_con
     const float sc_log2e = 1.4426950408889634f / sqrtf((float)kHD);
     const int col = lane >> 2, t4 = lane & 3;
     float acc[NT][8][4];         // D[16 dims x 8 columns] per m tile: this lane has dims lane / 4 (+ 8), high and low column of head 4 nt + t4
-    float m_own[NT], l_own[NT], fac[NT];  // of head 4 nt + t4: running maximum, this lane's part of the sum, factor from products to scores
+    float m_own[NT], l_own[NT], l_low[NT], fac[NT];  // of head 4 nt + t4: running maximum, this lane's part of the sum and what its roundings lost, factor from products to scores
     uint32_t qf[NT][8][2];
     bool ok = true, begun = false;
     int first_page = 0, st = 0;
@@ -240,7 +250,7 @@ attention_batch_kernel(const __grid_constant__ CUtensorMap ktm, const __grid_con
                     for (int r = 0; r < 2; r++) qf[nt][kt][r] = split_pair(x[kt][r].x * up, x[kt][r].y * up, col & 1);
                 fac[nt] = __shfl_sync(0xffffffffu, down * sc_log2e, 8 * t4);
                 m_own[nt] = -INFINITY;
-                l_own[nt] = 0.f;
+                l_own[nt] = l_low[nt] = 0.f;
 #pragma unroll
                 for (int mt = 0; mt < 8; mt++) acc[nt][mt][0] = acc[nt][mt][1] = acc[nt][mt][2] = acc[nt][mt][3] = 0.f;
             }
@@ -299,11 +309,11 @@ attention_batch_kernel(const __grid_constant__ CUtensorMap ktm, const __grid_con
             __syncwarp();
         }
         {
-            float c[NT][4], c2[NT][4];  // two chains of products
+            float c[NT][kChains][4];
 #pragma unroll
             for (int nt = 0; nt < NT; nt++)
 #pragma unroll
-                for (int i = 0; i < 4; i++) c[nt][i] = c2[nt][i] = 0.f;
+                for (int i = 0; i < kChains; i++) c[nt][i][0] = c[nt][i][1] = c[nt][i][2] = c[nt][i][3] = 0.f;
             const int lrow = (lane & 7) + ((lane >> 3) & 1) * 8;  // the row this lane addresses for ldmatrix
             const uint32_t lm_row = smem_u32(K_b) + (uint32_t)(lrow * 128);
 #pragma unroll
@@ -312,30 +322,38 @@ attention_batch_kernel(const __grid_constant__ CUtensorMap ktm, const __grid_con
                 uint32_t a[4];
                 ldm4(lm_row + (kt >> 2) * kKHalf + ((j ^ (lrow & 7)) << 4), a);
 #pragma unroll
-                for (int nt = 0; nt < NT; nt++) mma_f16(kt & 1 ? c2[nt] : c[nt], a, qf[nt][kt][0], qf[nt][kt][1]);
+                for (int nt = 0; nt < NT; nt++) mma_f16(c[nt][kt & (kChains - 1)], a, qf[nt][kt][0], qf[nt][kt][1]);
             }
             // this lane: keys lane / 4 and lane / 4 + 8 of head 4 nt + t4 (high + low columns)
             float pe[NT][2];
 #pragma unroll
             for (int nt = 0; nt < NT; nt++) {
-                const float s0 = col < nvalid ? ((c[nt][0] + c2[nt][0]) + (c[nt][1] + c2[nt][1])) * fac[nt] : -INFINITY;
-                const float s1 = col + 8 < nvalid ? ((c[nt][2] + c2[nt][2]) + (c[nt][3] + c2[nt][3])) * fac[nt] : -INFINITY;
+#pragma unroll
+                for (int o = kChains / 2; o > 0; o >>= 1)
+#pragma unroll
+                    for (int i = 0; i < o; i++)
+#pragma unroll
+                        for (int r = 0; r < 4; r++) c[nt][i][r] += c[nt][i + o][r];
+                const float s0 = col < nvalid ? (c[nt][0][0] + c[nt][0][1]) * fac[nt] : -INFINITY;
+                const float s1 = col + 8 < nvalid ? (c[nt][0][2] + c[nt][0][3]) * fac[nt] : -INFINITY;
                 float mx = fmaxf(s0, s1);
 #pragma unroll
                 for (int o = 4; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
                 const float m_new = fmaxf(m_own[nt], mx);
                 const float m_sub = m_new == -INFINITY ? 0.f : m_new;  // nothing but scores of minus infinity so far: no weight, not NaN
                 const float corr = exp2f(m_own[nt] - m_sub);
-                pe[nt][0] = exp2f(s0 - m_sub + kWeightLog2);
-                pe[nt][1] = exp2f(s1 - m_sub + kWeightLog2);
-                l_own[nt] = l_own[nt] * corr + (pe[nt][0] + pe[nt][1]);
+                pe[nt][0] = exp2f(s0 - m_sub) * kWeightScale;
+                pe[nt][1] = exp2f(s1 - m_sub) * kWeightScale;
                 m_own[nt] = m_new;
                 if (__any_sync(0xffffffffu, corr != 1.f)) {
+                    l_own[nt] *= corr;
+                    l_low[nt] *= corr;
 #pragma unroll
                     for (int mt = 0; mt < 8; mt++)
 #pragma unroll
                         for (int i = 0; i < 4; i++) acc[nt][mt][i] *= corr;
                 }
+                add_keeping(l_own[nt], l_low[nt], pe[nt][0] + pe[nt][1]);
             }
             // D[16 dims x 8 columns] += V^T[16 dims x 16 keys] . P[16 keys x 8 columns]
             uint32_t pf[NT][2];
@@ -356,7 +374,15 @@ attention_batch_kernel(const __grid_constant__ CUtensorMap ktm, const __grid_con
                 uint32_t a[4];
                 ldm4t(lv_row + (mt >> 2) * kKHalf + ((j ^ (vkey & 7)) << 4), a);
 #pragma unroll
-                for (int nt = 0; nt < NT; nt++) mma_f16(acc[nt][mt], a, pf[nt][0], pf[nt][1]);
+                for (int nt = 0; nt < NT; nt++) {
+                    float d[4] = {};
+                    mma_f16(d, a, pf[nt][0], pf[nt][1]);
+#pragma unroll
+                    for (int i = 0; i < 4; i += 2) {
+                        acc[nt][mt][i + 1] += d[i + 1];
+                        add_keeping(acc[nt][mt][i], acc[nt][mt][i + 1], d[i]);
+                    }
+                }
             }
         }
         __syncwarp();
@@ -370,6 +396,7 @@ attention_batch_kernel(const __grid_constant__ CUtensorMap ktm, const __grid_con
             float* const out = p.out + ((size_t)tok * p.n_heads + (size_t)kvh * GSZ) * kHD;
 #pragma unroll
             for (int nt = 0; nt < NT; nt++) {
+                l_own[nt] += l_low[nt];
 #pragma unroll
                 for (int o = 4; o < 32; o <<= 1) l_own[nt] += __shfl_xor_sync(0xffffffffu, l_own[nt], o);
                 const int h = 4 * nt + t4;
@@ -381,7 +408,7 @@ attention_batch_kernel(const __grid_constant__ CUtensorMap ktm, const __grid_con
                 float* const dst = whole ? out + h * kHD + col : mine + h * kStateWords + 4 + col;
 #pragma unroll
                 for (int mt = 0; mt < 8; mt++) {
-                    const float v0 = acc[nt][mt][0] + acc[nt][mt][1], v1 = acc[nt][mt][2] + acc[nt][mt][3];
+                    const float v0 = acc[nt][mt][0] + fmaf(acc[nt][mt][0], kCutOff, acc[nt][mt][1]), v1 = acc[nt][mt][2] + fmaf(acc[nt][mt][2], kCutOff, acc[nt][mt][3]);
                     dst[mt * 16] = whole ? v0 / l_own[nt] : v0;
                     dst[mt * 16 + 8] = whole ? v1 / l_own[nt] : v1;
                 }

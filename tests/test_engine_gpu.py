@@ -373,6 +373,42 @@ def test_batched_decode_attention_as_one_stream(gpu, oracle, heads, kv):
             assert err < 4 * 2.0 ** -11, (i, step, err)
 
 
+def test_batched_decode_attention_adds_in_32_bits(gpu):
+    """16 sequences of 3,700 random tokens, small queries: the weights are nearly equal, but not to 2^-11, and values positive, so that an error of the sums adds up.  Keys and values
+    are f16 numbers (permutations of one row, so that one gain brings the norm back to the row itself; keys in dims that do not turn at this theta); the output projection adds
+    the even dims alone to the residual, so the last norm does not hide a common factor.  f32 sums, and the head's 4,096 products, leave 1.9e-7 -
+    2.9e-7 of the logits (the kernel that adds with f32 FMAs the same); sums in the matrix unit's accumulators, which truncate, 1.6e-6 - 2.6e-6.  6e-7 lies between."""
+    from leafcutterllm_b200.synth import ModelSpec
+    H, heads, F, V, n, ctx = 4096, 32, 256, 64, 16, 3700
+    r = np.random.default_rng(5)
+    base = np.exp2(r.uniform(-4, 1, H)).astype(np.float16).astype(np.float32)
+    embed = np.stack([r.permutation(base) for _ in range(V)])
+    gain = np.float32(np.sqrt((base.astype(np.float64) ** 2).mean() + 1e-5))
+    even, still = np.arange(H) % 2 == 0, np.arange(H) % 64 >= 32
+    head = r.standard_normal((V, H)).astype(np.float32)
+    made = {"token_embd": embed, "output": head, "attn_q": np.diag(np.where(still, 0.02, 0)).astype(np.float32), "attn_k": np.diag(still.astype(np.float32)), "attn_v": np.eye(H, dtype=np.float32),
+            "attn_output": np.diag(even.astype(np.float32)),
+            "attn_norm": np.full(H, gain, np.float32), "ffn_norm": np.ones(H, np.float32), "output_norm": np.ones(H, np.float32)}
+    spec = ModelSpec("flat", 1, H, heads, heads, F, V, 10000.0, 0, 0, 0)
+    eng = gpu.Engine(H, 1, heads, heads, F, V, max_seq_len=ctx + 16, rope_theta=1e30, max_seqs=n, kv_pool_tokens=n * (ctx + 32), rope_mode="absolute")
+    for name, typ, dims, _ in spec.tensors():
+        eng.set_tensor(name, typ, dims, made.get(name.split(".")[-2], np.zeros(int(np.prod(dims)), np.float32)))
+    eng.finalize()
+    ids = list(range(n))
+    tokens = r.integers(0, V, (n, ctx + 3))
+    eng.forward_batch(ids, tokens[:, :ctx].tolist(), want_logits=False)
+    for step in range(ctx, ctx + 3):
+        got = eng.forward_batch(ids, tokens[:, step:step + 1].tolist())[0]
+        for i in ids:
+            of = embed.astype(np.float64).reshape(V, heads, 128)
+            q = np.where(still, np.float32(0.02), 0) * of[tokens[i, step]].ravel()
+            w = np.bincount(tokens[i, :step + 1], minlength=V) * np.exp(np.einsum("hd,vhd->hv", q.reshape(heads, 128), of) / np.sqrt(128))
+            h = embed[tokens[i, step]] + np.where(even, np.einsum("hv,vhd->hd", w / w.sum(1, keepdims=True), of).ravel(), 0.0)
+            want = head.astype(np.float64) @ (h / np.sqrt((h * h).mean() + 1e-5))
+            assert np.linalg.norm(got[i] - want) < 6e-7 * np.linalg.norm(want), np.linalg.norm(got[i] - want) / np.linalg.norm(want)
+    eng.close()
+
+
 def test_batched_decode_attention_whose_waits_run_out(gpu, monkeypatch):
     """Every wait for a page gives up before it looks (LC_ATTN_WAITS=0, a step's launches are made anew for another number of sequences): the call ends with an error, and
     the handle is usable: the tickets of segments that several warps share are back at zero, so the next steps give what a handle gives that never failed."""
