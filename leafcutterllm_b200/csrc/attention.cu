@@ -356,7 +356,7 @@ int32_t launch_attention(const float* q, int q_stride, float* out, int n_tok, in
     p.positions_settled = (fuse && fuse->positions_settled) ? 1 : 0;
     p.error_flag = gemv_error_flag_dev();
     if (fuse && fuse->stream_slots && attention_stream_applies(p, n_tok)) return launch_attention_stream(p, fuse->stream_slots, s);
-    if (p.rot && attention_batch_applies(p, n_tok)) return launch_attention_batch(p, n_tok, s);
+    if (p.rot && attention_batch_applies(p, n_tok, fuse->turns)) return launch_attention_batch(p, n_tok, s);
     switch (kv.hd) {
         case 32: return launch_attention_hd<32>(p, n_tok, max_ctx, s);
         case 64: return launch_attention_hd<64>(p, n_tok, max_ctx, s);

@@ -481,12 +481,18 @@ size_t attention_batch_scratch_bytes(int n_heads, int n_kv, int hd) {
     return (size_t)sm_count() * kWarps * 2 * (n_heads / n_kv) * kStateWords * sizeof(float);
 }
 
-bool attention_batch_applies(const AttnParams& a, int n_tok) {
+bool attention_batch_applies(const AttnParams& a, int n_tok, bool turns) {
     const int gsz = a.kv.n_kv > 0 ? a.n_heads / a.kv.n_kv : 0;
-    // Up to four tokens of models without kv groups go to the staged kernel (attention.cu), which has a CTA per 128 keys and less to do ahead of them: 7B shape, 8 layers, us
-    // per step staged / here: 3 sequences of 200 768 / 815, of 1,000 870 / 890, of 4,000 1,280 / 1,100.  With kv groups it serves one query head after the other
-    // (Mixtral shape, 4 layers, 3 sequences: 1,018 / 965, 1,041 / 990, 1,236 / 1,030).
-    return n_tok >= 2 && (n_tok > 4 || gsz > 1) && n_tok <= kMaxBatch && a.k_new && a.rot && a.kv.k_tmap && a.kv.v_tmap && a.kv.hd == kHD && !a.kv.kv_f32 && a.kv.page_tokens == kPage &&
+    // Where a step turns queries and keys, the kernels of attention.cu were slower for all sizes while they computed the powers, sines and cosines themselves.  Up to four tokens of
+    // models without kv groups go to the staged kernel, which has a CTA per 128 keys and less to do ahead of them: 7B shape, 8 layers, us per step staged / here: 3 sequences
+    // of 200 768 / 815, of 1,000 870 / 890, of 4,000 1,280 / 1,100.  With kv groups it serves one query head after the other (Mixtral shape, 4 layers, 3 sequences: 1,018 / 965,
+    // 1,041 / 990, 1,236 / 1,030).
+    // Where nothing turns, the line lies where this kernel is not slower for any context, since a captured step does not know them.  us per layer of a small model, contexts of 60
+    // and 1,000, attention.cu / here: up to four sequences, 32 heads on 8, 3 sequences 58.3 / 51.5 and 66.9 / 55.7, but 32 on 16 48.9 / 52.4 and 57.3 / 56.0; more, 32 heads on
+    // 8, 6 sequences 68.6 / 75.2 and 80.0 / 79.6, 24 86.3 / 83.1 and 140 / 103, 8 heads on 1, 48 sequences 76.0 / 87.1 and 110 / 94, 128 74.9 / 75.4 and 138 / 88; without
+    // groups, 8 heads, 24 sequences 71.2 / 75.5 and 95.8 / 99.6, 128 83.3 / 84.7 and 162 / 162.
+    const bool faster = turns ? n_tok > 4 || gsz > 1 : n_tok > 4 ? gsz > 1 && n_tok * a.n_heads >= 1024 : gsz >= 4;
+    return n_tok >= 2 && faster && n_tok <= kMaxBatch && a.k_new && a.rot && a.kv.k_tmap && a.kv.v_tmap && a.kv.hd == kHD && !a.kv.kv_f32 && a.kv.page_tokens == kPage &&
            a.n_heads % a.kv.n_kv == 0 && (gsz == 1 || gsz == 2 || gsz == 4 || gsz == 8) && a.q_stride % 4 == 0 && a.kv_stride % 4 == 0;
 }
 

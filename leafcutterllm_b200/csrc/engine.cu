@@ -244,6 +244,7 @@ int32_t attention_block(lc_model* m, int l, const float* x, const float* norm_w,
         fz.positions_settled = l > 0;  // the first layer of a step may run while the previous step still advances the positions
         fz.stream_slots = m->d_stream_slots;
         fz.rot = m->d_rot;
+        fz.turns = m->cfg.rope_mode != 0;
         LC_TRY(launch_attention(q, q_stride, m->d_attn, T, m->nh, kv, m->d_tok_seq, m->d_tok_pos, m->d_page_table, m->pages_per_seq,
                                 m->cfg.max_seq_len, m->d_attn_scratch, m->d_attn_counters, &fz, m->stream));
         m->launches_in_call += 1;

@@ -40,7 +40,8 @@ bool attention_stream_applies(const AttnParams& a, int n_tok);
 int32_t launch_attention_stream(const AttnParams& a, unsigned long long* slots, cudaStream_t s);
 
 // attention_batch.cu: one new token for each of two or more sequences, the same heads and caches, as one stream over all of them
-bool attention_batch_applies(const AttnParams& a, int n_tok);
+// turns: some token's rotation is not by nothing
+bool attention_batch_applies(const AttnParams& a, int n_tok, bool turns);
 int32_t launch_attention_batch(const AttnParams& a, int n_tok, cudaStream_t s);
 
 template <int DPL, bool F32>

@@ -206,6 +206,7 @@ struct AttnFusion {
     // decode step keeps the pointer.
     unsigned long long* stream_slots = nullptr;
     const void* rot = nullptr;  // float2 [tokens][hd / 2]: cosine and sine of the step's rotations (launch_embed)
+    bool turns = false;         // not all of them are by nothing
 };
 int32_t launch_attention(const float* q, int q_stride, float* out, int n_tok, int n_heads, const KvLayout& kv,
                          const int32_t* tok_seq, const int32_t* tok_pos, const int32_t* page_table, int pages_per_seq, int max_ctx,

@@ -373,6 +373,27 @@ def test_batched_decode_attention_as_one_stream(gpu, oracle, heads, kv):
             assert err < 4 * 2.0 ** -11, (i, step, err)
 
 
+@pytest.mark.parametrize("heads,kv,n", [(8, 2, 128), (8, 2, 127), (8, 2, 5), (8, 2, 4), (8, 4, 4), (4, 4, 9)])
+def test_batched_decode_attention_without_rotation(gpu, oracle, heads, kv, n):
+    """Steps that rotate by nothing, on both sides of the lines between the kernels (1,024 heads of all sequences; up to four sequences, four heads per kv head; no kv groups).
+    Bound as in the test above."""
+    from leafcutterllm_b200 import synth
+    spec = small_spec(12, 12, 12, layers=2, hidden=128 * heads, heads=heads, kv=kv, ffn=256, vocab=256)
+    eng, om = make_pair(gpu, oracle, spec, max_seq_len=80, max_seqs=n)
+    prompts = [synth.prompt_tokens(1 + (7 * i) % 40, spec.vocab_size, 600 + i).tolist() for i in range(n)]
+    fed = np.random.default_rng(n).integers(0, spec.vocab_size, (2, n))
+    eng.forward_batch(list(range(n)), prompts, want_logits=False)
+    got = [eng.forward_batch(list(range(n)), [[int(t)] for t in row])[0].copy() for row in fed]
+    eng.close()
+    for i in range(0, n, 1 if n < 16 else 13):
+        om.kv_clear()
+        om.forward(prompts[i])
+        for step, row in enumerate(fed):
+            want = np.asarray(om.forward([int(row[i])]), np.float64)
+            err = np.linalg.norm(got[step][i] - want) / np.linalg.norm(want)
+            assert err < 4 * 2.0 ** -11, (i, step, err)
+
+
 def test_batched_decode_attention_adds_in_32_bits(gpu):
     """16 sequences of 3,700 random tokens, small queries: the weights are nearly equal, but not to 2^-11, and values positive, so that an error of the sums adds up.  Keys and values
     are f16 numbers (permutations of one row, so that one gain brings the norm back to the row itself; keys in dims that do not turn at this theta); the output projection adds
