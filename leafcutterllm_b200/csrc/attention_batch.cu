@@ -58,6 +58,10 @@ __device__ __forceinline__ uint32_t split_pair(float a, float b, bool low) {
     const __half2 h = __floats2half2_rn(a, b);
     return low ? half_pair(a - __low2float(h), b - __high2float(h)) : *reinterpret_cast<const uint32_t*>(&h);
 }
+__device__ __forceinline__ float4 widened(uint2 w) {
+    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&w.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&w.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
 __device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
@@ -76,6 +80,48 @@ __device__ __forceinline__ void rotate_pair(float2& x, float2& y, float4 cs) {  
     y.y = __fadd_rn(__fmul_rn(u.y, cs.w), __fmul_rn(v.y, cs.z));
 }
 
+// Dims 4 lane ... of a head's vector, turned by its token's row of the table
+__device__ __forceinline__ float4 rotated(const float* vec, const float2* row, bool turns, int lane) {
+    const int d = 4 * (lane & 15);  // of the pairs' first half; lanes 16 - 31 have the second
+    float4 a = __ldcg(reinterpret_cast<const float4*>(vec + d)), b = __ldcg(reinterpret_cast<const float4*>(vec + d + kHD / 2));
+    if (turns) {
+        const float4* const cs = reinterpret_cast<const float4*>(row + d);
+        float2 a0 = make_float2(a.x, a.y), a1 = make_float2(a.z, a.w), b0 = make_float2(b.x, b.y), b1 = make_float2(b.z, b.w);
+        rotate_pair(a0, b0, __ldcg(cs));
+        rotate_pair(a1, b1, __ldcg(cs + 1));
+        a = make_float4(a0.x, a0.y, a1.x, a1.y);
+        b = make_float4(b0.x, b0.y, b1.x, b1.y);
+    }
+    return lane < 16 ? a : b;
+}
+
+// A segment of query head `h` once more, keys [first, end), in f32: where a key or a value of the cache is infinite (beyond f16's range), its product with one half of the query or
+// of the weight is NaN or of the other sign, and the score's or the sum's is not.  A lane has dims 4 lane ...
+struct SegmentState { float most, sum; float4 v; };
+__device__ __noinline__ SegmentState plain_segment(const AttnParams& p, int tok, int h, int first, int end, int lane) {
+    const KvLayout& kv = p.kv;
+    const int kvh = h / (p.n_heads / kv.n_kv);
+    const float4 q = rotated(p.q + (size_t)tok * p.q_stride + (size_t)h * kHD, p.rot + (size_t)tok * (kHD / 2), p.tok_rope[tok] != 0, lane);
+    const int32_t* const pages = p.page_table + (size_t)p.tok_seq[tok] * p.pages_per_seq;
+    const float sc_log2e = 1.4426950408889634f / sqrtf((float)kHD);
+    SegmentState s{-INFINITY, 0.f, make_float4(0.f, 0.f, 0.f, 0.f)};
+    for (int t = first; t < end; t++) {
+        const size_t at = (((size_t)pages[t / kPage] * kv.n_kv + kvh) * kPage + t % kPage) * kHD + 4 * lane;
+        const float4 k = widened(*reinterpret_cast<const uint2*>((const __half*)kv.k_pool + at)), v = widened(*reinterpret_cast<const uint2*>((const __half*)kv.v_pool + at));
+        const float score = warp_sum(fmaf(q.w, k.w, fmaf(q.z, k.z, fmaf(q.y, k.y, q.x * k.x)))) * sc_log2e;
+        if (score > s.most) {
+            const float corr = exp2f(s.most - score);
+            s.most = score;
+            s.sum *= corr;
+            s.v = make_float4(s.v.x * corr, s.v.y * corr, s.v.z * corr, s.v.w * corr);
+        }
+        const float w = score == -INFINITY ? 0.f : exp2f(score - s.most) * kWeightScale;
+        s.sum += w;
+        s.v = make_float4(fmaf(w, v.x, s.v.x), fmaf(w, v.y, s.v.y), fmaf(w, v.z, s.v.z), fmaf(w, v.w, s.v.w));
+    }
+    return s;
+}
+
 // sum += x; what the addition's rounding lost goes to `low` (of a smaller sum than x: a part of it)
 __device__ __forceinline__ void add_keeping(float& sum, float& low, float x) {
     const float s = sum + x;
@@ -85,7 +131,7 @@ __device__ __forceinline__ void add_keeping(float& sum, float& low, float x) {
 
 template <int GSZ>
 __global__ void __launch_bounds__(kWarps * 32, 1)
-attention_batch_kernel(const __grid_constant__ CUtensorMap ktm, const __grid_constant__ CUtensorMap vtm, BatchParams P) {
+attention_batch_kernel(const __grid_constant__ CUtensorMap ktm, const __grid_constant__ CUtensorMap vtm, const __grid_constant__ BatchParams P) {
     constexpr int NT = (2 * GSZ + 7) / 8;  // n tiles of 8 columns: four heads as (high, low)
     extern __shared__ unsigned char smem_raw[];
     unsigned char* const smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -279,17 +325,7 @@ attention_batch_kernel(const __grid_constant__ CUtensorMap ktm, const __grid_con
             const int pos = p.tok_pos[tok], r = pos % kPage, rp = p.tok_rope[tok];
             nvalid = r + 1;
             const float* const kn = p.k_new + (size_t)tok * p.kv_stride + (size_t)kvh * kHD;
-            const int d = 4 * (lane & 15);  // of the pair's first half; lanes 16 - 31 have the second
-            float4 a = __ldcg(reinterpret_cast<const float4*>(kn + d)), b = __ldcg(reinterpret_cast<const float4*>(kn + d + kHD / 2));
-            if (rp != 0) {
-                const float4* const cs = reinterpret_cast<const float4*>(p.rot + (size_t)tok * (kHD / 2) + d);
-                float2 a0 = make_float2(a.x, a.y), a1 = make_float2(a.z, a.w), b0 = make_float2(b.x, b.y), b1 = make_float2(b.z, b.w);
-                rotate_pair(a0, b0, __ldcg(cs));
-                rotate_pair(a1, b1, __ldcg(cs + 1));
-                a = make_float4(a0.x, a0.y, a1.x, a1.y);
-                b = make_float4(b0.x, b0.y, b1.x, b1.y);
-            }
-            const float4 kr = lane < 16 ? a : b;
+            const float4 kr = rotated(kn, p.rot + (size_t)tok * (kHD / 2), rp != 0, lane);
             const float4 vr = __ldcg(reinterpret_cast<const float4*>(p.v_new + (size_t)tok * p.kv_stride + (size_t)kvh * kHD + 4 * lane));
             const uint2 kw = make_uint2(half_pair(kr.x, kr.y), half_pair(kr.z, kr.w)), vw = make_uint2(half_pair(vr.x, vr.y), half_pair(vr.z, vr.w));
             // dims 4 lane ..: box lane / 16, chunk (lane % 16) / 2 (swizzled by the row), 8 bytes into it for odd lanes
@@ -394,6 +430,18 @@ attention_batch_kernel(const __grid_constant__ CUtensorMap ktm, const __grid_con
             const int slot = first_page > 0 ? 0 : 1;
             float* const mine = p.partial + ((size_t)worker * 2 + slot) * GSZ * kStateWords;
             float* const out = p.out + ((size_t)tok * p.n_heads + (size_t)kvh * GSZ) * kHD;
+            uint32_t wild = 0u;  // a bit for each of the group's heads whose sums are infinite or NaN
+#pragma unroll
+            for (int nt = 0; nt < NT; nt++) {
+                float zero = 0.f * (l_own[nt] + l_low[nt]);
+#pragma unroll
+                for (int mt = 0; mt < 8; mt++)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) zero = fmaf(0.f, acc[nt][mt][i], zero);
+                const uint32_t lanes = __ballot_sync(0xffffffffu, zero != 0.f);
+#pragma unroll
+                for (int t = 0; t < 4; t++) wild |= (lanes & (0x11111111u << t)) ? 1u << (4 * nt + t) : 0u;
+            }
 #pragma unroll
             for (int nt = 0; nt < NT; nt++) {
                 l_own[nt] += l_low[nt];
@@ -411,6 +459,17 @@ attention_batch_kernel(const __grid_constant__ CUtensorMap ktm, const __grid_con
                     const float v0 = acc[nt][mt][0] + fmaf(acc[nt][mt][0], kCutOff, acc[nt][mt][1]), v1 = acc[nt][mt][2] + fmaf(acc[nt][mt][2], kCutOff, acc[nt][mt][3]);
                     dst[mt * 16] = whole ? v0 / l_own[nt] : v0;
                     dst[mt * 16 + 8] = whole ? v1 / l_own[nt] : v1;
+                }
+            }
+            for (wild &= (1u << GSZ) - 1u; wild; wild &= wild - 1) {
+                const int h = __ffs(wild) - 1;
+                const SegmentState s = plain_segment(p, tok, kvh * GSZ + h, first_page * kPage, min((page + 1) * kPage, p.tok_pos[tok] + 1), lane);
+                __syncwarp();
+                if (whole) {
+                    reinterpret_cast<float4*>(out + h * kHD)[lane] = make_float4(s.v.x / s.sum, s.v.y / s.sum, s.v.z / s.sum, s.v.w / s.sum);
+                } else {
+                    if (lane == 0) { mine[h * kStateWords] = s.most; mine[h * kStateWords + 1] = s.sum; }
+                    reinterpret_cast<float4*>(mine + h * kStateWords + 4)[lane] = s.v;
                 }
             }
             if (!whole && last_of_segment()) {

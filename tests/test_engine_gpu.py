@@ -430,6 +430,51 @@ def test_batched_decode_attention_adds_in_32_bits(gpu):
     eng.close()
 
 
+@pytest.mark.parametrize("heads,kv", [(4, 4), (4, 1)])
+def test_batched_decode_attention_of_keys_beyond_f16(gpu, oracle, heads, kv):
+    """One token's keys have an element beyond f16's range: minus or plus infinity in the cache.  Queries that give them scores of minus infinity give them no weight, whatever the signs
+    of the halves that queries are cut into; the others' results are NaN in the oracle too.  Bound as in the test above it."""
+    from leafcutterllm_b200.synth import ModelSpec
+    H, V, n, at = 128 * heads, 256, 7, 40  # dim 40 of a head does not turn at this theta
+    r = np.random.default_rng(heads + kv)
+    embed = r.standard_normal((V, H)).astype(np.float32)
+    embed[:, at::128] = 0.0
+    embed[5, at::128] = 90.0  # token 5's keys are infinite there (weights beyond 100 count as zero, so it takes three factors) ...
+    gain = np.ones(H, np.float32)
+    gain[at] = 100.0
+    wq = (r.standard_normal((H, H)) / np.sqrt(H)).astype(np.float32)
+    wk, wv, wo = [(r.standard_normal(s) / np.sqrt(H)).astype(np.float32) for s in ((128 * kv, H), (128 * kv, H), (H, H))]
+    wq[:, at::128] = wk[:, at::128] = 0.0
+    for h in range(kv):
+        wk[128 * h + at, at] = 100.0
+    made = {"token_embd": embed, "output": r.standard_normal((V, H)).astype(np.float32), "attn_q": wq, "attn_k": wk, "attn_v": wv, "attn_output": wo,
+            "attn_norm": gain, "ffn_norm": np.ones(H, np.float32), "output_norm": np.ones(H, np.float32)}
+    spec = ModelSpec("wild", 1, H, heads, kv, 256, V, 1e30, 0, 0, 0)
+    eng = gpu.Engine(H, 1, heads, kv, 256, V, max_seq_len=256, rope_theta=1e30, max_seqs=n, rope_mode="absolute")
+    om = oracle.OracleModel(H, 1, heads, kv, 256, V, max_seq_len=256, rope_theta=1e30, rope_absolute=True)
+    for name, typ, dims, _ in spec.tensors():
+        w = made.get(name.split(".")[-2], np.zeros(int(np.prod(dims)), np.float32))
+        eng.set_tensor(name, typ, dims, w)
+        om.set_tensor(name, typ, dims, np.ascontiguousarray(w).view(np.uint8).ravel())
+    eng.finalize()
+    prompts = [[5 if j % 37 == i else int(t) for j, t in enumerate(r.integers(6, V, 3 + 33 * i))] for i in range(n)]
+    # ... and these queries have there what makes all scores with them minus infinity: tokens whose q is negative there for every head
+    scores = (embed @ wq.T)[:, at::128]
+    fed = [int(t) for t in np.flatnonzero((scores < 0).all(1)) if t > 5][:3]
+    assert len(fed) == 3
+    eng.forward_batch(list(range(n)), prompts, want_logits=False)
+    got = [eng.forward_batch(list(range(n)), [[t]] * n)[0].copy() for t in fed]
+    eng.close()
+    for i in range(n):
+        om.kv_clear()
+        om.forward(prompts[i])
+        for step, t in enumerate(fed):
+            want = np.asarray(om.forward([t]), np.float64)
+            assert np.isfinite(want).all()
+            err = np.linalg.norm(got[step][i] - want) / np.linalg.norm(want)
+            assert err < 4 * 2.0 ** -11, (i, step, err)
+
+
 def test_batched_decode_attention_whose_waits_run_out(gpu, monkeypatch):
     """Every wait for a page gives up before it looks (LC_ATTN_WAITS=0, a step's launches are made anew for another number of sequences): the call ends with an error, and
     the handle is usable: the tickets of segments that several warps share are back at zero, so the next steps give what a handle gives that never failed."""
