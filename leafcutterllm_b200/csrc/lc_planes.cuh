@@ -17,7 +17,7 @@ __device__ __forceinline__ void unit_planes(const float (&v)[8], int lane, unsig
     amax = warp_max(amax);
     // amax = f * 2^ex with f in [0.5, 1): ex from the exponent field (zero, denormal and non-finite inputs fall into the clamp)
     const int ex = (int)((__float_as_uint(amax) >> 23) & 0xFFu) - 126;
-    const int s = max(-100, min(100, 22 - ex));  // |x| * 2^s < 2^22
+    const int s = min(120, 22 - ex);  // |x| * 2^s < 2^22; its inverse, and that over 16, are normal numbers
     const float up = __uint_as_float((uint32_t)(127 + s) << 23), dn = __uint_as_float((uint32_t)(127 - s) << 23);
     // The digits are the bytes of X + 0x808080 with their top bits flipped: that sum is b0 + 256 b1 + 65536 b2 with unsigned
     // bytes, so X = (b0 - 128) + 256 (b1 - 128) + 65536 (b2 - 128), and b - 128 as a signed byte is b ^ 0x80.

@@ -551,7 +551,10 @@ qgemv_mma_q4k_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_const
                     y += rb[(w * M + tk) * 32 + lane];
                     if (one_pass || late) ssq += scratch[w * M + tk];  // same order in every thread and CTA
                 }
-                if (one_pass || late) y *= 1.0f / sqrtf(ssq / (float)p.k + p.eps);  // cpu.rs:52-55
+                if (one_pass || late) {
+                    const float f = 1.0f / sqrtf(ssq / (float)p.k + p.eps);  // cpu.rs:52-55
+                    y = f == 0.f ? 0.f : y * f;  // squares beyond f32's range: zero, also where the sum is too
+                }
                 const int row = lane < TR ? tile * TR + lane : p.n;  // lanes past the tile's rows hold nothing
                 bool have = false;
                 if (p.epi == EPI_SILU_MUL) {

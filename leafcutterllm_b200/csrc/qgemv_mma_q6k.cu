@@ -341,7 +341,10 @@ qgemv_mma_q6k_kernel(const unsigned char* __restrict__ w0, const unsigned char* 
                     y += rb[(w * M + tk) * kRows + lane];
                     if (p.norm_w) ssq += scratch[w * M + tk];  // same order in every thread and CTA
                 }
-                if (p.norm_w) y *= 1.0f / sqrtf(ssq / (float)p.k + p.eps);
+                if (p.norm_w) {
+                    const float f = 1.0f / sqrtf(ssq / (float)p.k + p.eps);
+                    y = f == 0.f ? 0.f : y * f;  // as in qgemv_mma.cu
+                }
                 const int row = tile * kRows + lane;
                 bool have = false;
                 if (p.epi == EPI_SILU_MUL) {

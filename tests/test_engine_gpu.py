@@ -373,6 +373,37 @@ def test_batched_decode_attention_as_one_stream(gpu, oracle, heads, kv):
             assert err < 4 * 2.0 ** -11, (i, step, err)
 
 
+@pytest.mark.parametrize("typ", [12, 14])
+@pytest.mark.parametrize("n", [1, 3, 7])
+def test_norm_of_rows_near_the_ends_of_f32(gpu, typ, n):
+    """The matrix-vector kernels multiply by the norm's factor at the end.  Hidden rows of 1e-26 keep their 22 bits on the way there (bound: what f32 sums of 512 products leave, a few
+    1e-7), and rows whose squares leave f32's range have a factor of zero, so that q, k, v and logits are zero and not NaN, though the sums may leave it as well."""
+    from leafcutterllm_b200 import synth
+    from leafcutterllm_b200.synth import ModelSpec
+    H, V = 512, 64
+    spec = ModelSpec("ends", 1, H, 4, 4, 512, V, 10000.0, typ, 0, typ)
+    r = np.random.default_rng(typ + n)
+    embed = (r.standard_normal((V, H)) * np.where(np.arange(V) < 32, 1e-26, 3e37)[:, None]).astype(np.float32)
+    eng = gpu.Engine(H, 1, 4, 4, 512, V, max_seq_len=32, max_seqs=n, kv_dtype="f32")
+    w = {}
+    for name, t, dims, kind in spec.tensors():
+        data = embed if name.startswith("token_embd") else synth.tensor_bytes(spec, name, t, dims, kind, 77)
+        eng.set_tensor(name, t, dims, data)
+        if t == typ:
+            w[name.split(".")[-2]] = gpu.dequantize(typ, data, int(np.prod(dims))).reshape(dims[1], dims[0]).astype(np.float64)
+    eng.finalize()
+    ids = list(range(n))
+    got = eng.forward_batch(ids, [[i] for i in ids])[0]  # the first token of each sequence: the attention's result is its value
+    for i in ids:
+        x = embed[i].astype(np.float64)
+        h = x + w["attn_output"] @ (w["attn_v"] @ (x / np.sqrt(1e-5)))
+        want = w["output"] @ (h / np.sqrt(1e-5))
+        assert np.linalg.norm(got[i] - want) < 2e-6 * np.linalg.norm(want)
+    eng.kv_clear()
+    assert (eng.forward_batch(ids, [[32 + i] for i in ids])[0] == 0).all()
+    eng.close()
+
+
 @pytest.mark.parametrize("heads,kv,n", [(8, 2, 128), (8, 2, 127), (8, 2, 5), (8, 2, 4), (8, 4, 4), (4, 4, 9)])
 def test_batched_decode_attention_without_rotation(gpu, oracle, heads, kv, n):
     """Steps that rotate by nothing, on both sides of the lines between the kernels (1,024 heads of all sequences; up to four sequences, four heads per kv head; no kv groups).
