@@ -532,6 +532,86 @@ def test_batched_decode_attention_whose_waits_run_out(gpu, monkeypatch):
     eng.close()
 
 
+def close_to(got, want, what):
+    """Keys and values of both sides are rounded to f16 (2^-11 at most): results that differ by more than four times that (2-norm) are wrong."""
+    err = np.linalg.norm(got - want) / np.linalg.norm(want)
+    assert err < 4 * 2.0 ** -11, (what, err)
+
+
+@pytest.mark.parametrize("heads,kv", [(4, 4), (4, 1)])
+def test_batched_decode_attention_of_later_layers(gpu, oracle, heads, kv):
+    """Layers behind the first read positions and page tables, and request cached pages, ahead of the kernel before them.  40 sequences, three layers, rotation by position: page
+    counts of more than 32 tokens, page-table entries reloaded every 32 pages, one context of 257 pages that about 30 runs share; contexts that step over a page's edge.
+    Steps alone, then a loop of captured steps, then a step alone again."""
+    from leafcutterllm_b200 import synth
+    spec = small_spec(12, 12, 12, layers=3, hidden=128 * heads, heads=heads, kv=kv, ffn=256, vocab=256)
+    n, looped = 40, 6
+    lens = [600, 1, 15, 511] + [1 + (11 * i) % 60 for i in range(n - 5)] + [4095]
+    ids, checked = list(range(n)), [0, 1, 2, 3, 9, 32, 33, n - 1]
+    eng, om = make_pair(gpu, oracle, spec, max_seq_len=4112, max_seqs=n, kv_pool_tokens=sum(lens) + 32 * n, rope_mode="absolute")
+    prompts = [synth.prompt_tokens(m, spec.vocab_size, 700 + i).tolist() for i, m in enumerate(lens)]
+    fed = np.random.default_rng(heads + kv).integers(0, spec.vocab_size, (4, n))
+    eng.forward_batch(ids, prompts, want_logits=False)
+    got = [eng.forward_batch(ids, [[int(t)] for t in row])[0].copy() for row in fed[:2]]
+    picks, _ = eng.decode_loop(ids, fed[2], looped)
+    last = eng.forward_batch(ids, [[int(t)] for t in fed[3]])[0].copy()
+    eng.close()
+    for i in checked:
+        om.kv_clear()
+        om.forward(prompts[i])
+        for step in range(2):
+            close_to(got[step][i], np.asarray(om.forward([int(fed[step][i])]), np.float64), (i, step))
+        for t, pick in zip([int(fed[2][i])] + picks[:-1, i].tolist(), picks[:, i]):
+            logits = np.asarray(om.forward([t]), np.float64)
+            assert logits.max() - logits[pick] < 8 * 2.0 ** -11 * np.linalg.norm(logits), (i, t, pick)  # the pick's and the largest's errors
+        close_to(last[i], np.asarray(om.forward([int(fed[3][i])]), np.float64), (i, "last"))
+
+
+@pytest.mark.parametrize("n", [3, 7])
+@pytest.mark.parametrize("heads,kv,hidden,cache,mix", [(4, 4, 512, "f16", "q4_k_m"), (4, 2, 512, "f16", "q4_k_m"), (4, 4, 512, "f32", "q4_k_m"), (4, 2, 256, "f16", ""), (8, 4, 256, "f32", "")])
+def test_batched_decode_turned_by_position(gpu, oracle, n, heads, kv, hidden, cache, mix):
+    """Several sequences at unequal positions, each turned by its own row of the step's table, in every kernel that a step of several tokens has: heads of 128 without kv groups
+    (staged at 3, one stream at 7), with them, an f32 cache, heads of 64 and 32 (split contexts).  With a mix of types the last layers' q, k and v are three
+    products, whose rows lie apart by other strides than a fused product's."""
+    from dataclasses import replace
+    from leafcutterllm_b200 import synth
+    spec = replace(small_spec(12, 12, 12, layers=3, hidden=hidden, heads=heads, kv=kv, ffn=512, vocab=512), mix=mix)
+    lens = [37, 5, 130, 1, 16, 64, 250][:n]
+    eng, om = make_pair(gpu, oracle, spec, max_seq_len=272, max_seqs=n, kv_dtype=cache, rope_mode="absolute", on_device=True)
+    prompts = [synth.prompt_tokens(m, spec.vocab_size, 800 + i).tolist() for i, m in enumerate(lens)]
+    fed = np.random.default_rng(heads + n).integers(0, spec.vocab_size, (3, n))
+    eng.forward_batch(list(range(n)), prompts, want_logits=False)
+    got = [eng.forward_batch(list(range(n)), [[int(t)] for t in row])[0].copy() for row in fed]
+    eng.close()
+    for i in range(n):
+        om.kv_clear()
+        om.forward(prompts[i])
+        for step, row in enumerate(fed):
+            close_to(got[step][i], np.asarray(om.forward([int(row[i])]), np.float64), (i, step))
+
+
+@pytest.mark.parametrize("heads,kv,cache", [(8, 2, "f32"), (16, 4, "f16")])
+def test_batched_decode_attention_split_into_pieces(gpu, oracle, heads, kv, cache):
+    """80 sequences over a cache in f32, and with heads of 64: kernels of split contexts.  1,024-key pieces merged through scratch, the new key in one of them,
+    contexts on both sides of their edges, most pieces empty; turned by position."""
+    from leafcutterllm_b200 import synth
+    spec = small_spec(12, 12, 12, layers=2, hidden=1024, heads=heads, kv=kv, ffn=256, vocab=256)
+    n, special = 80, [5, 1022, 1023, 1024, 2047, 2049, 2500, 4090]
+    lens = special + [1 + (13 * i) % 90 for i in range(n - len(special))]
+    ids = list(range(n))
+    eng, om = make_pair(gpu, oracle, spec, max_seq_len=4096, max_seqs=n, kv_pool_tokens=sum(lens) + 32 * n, kv_dtype=cache, rope_mode="absolute")
+    prompts = [synth.prompt_tokens(m, spec.vocab_size, 900 + i).tolist() for i, m in enumerate(lens)]
+    fed = np.random.default_rng(heads).integers(0, spec.vocab_size, (3, n))
+    eng.forward_batch(ids, prompts, want_logits=False)
+    got = [eng.forward_batch(ids, [[int(t)] for t in row])[0].copy() for row in fed]
+    eng.close()
+    for i in list(range(len(special))) + [20, 79]:
+        om.kv_clear()
+        om.forward(prompts[i])
+        for step, row in enumerate(fed):
+            close_to(got[step][i], np.asarray(om.forward([int(row[i])]), np.float64), (i, step))
+
+
 def test_prefill_attention_on_tensor_cores_ragged(gpu, oracle):
     """head_dim 128, f16 cache: calls of 16 tokens and more run the tiled tensor-core prefill attention.  Four sequences of
     70, 16, 129 and 33 tokens in ONE call (tiles end where a sequence ends; 129 = two full tiles and a one-token tile), then a
