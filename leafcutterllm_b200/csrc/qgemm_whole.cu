@@ -49,6 +49,11 @@ constexpr int kMaxB = 8;         // activation stages (two chunks of 64 elements
 constexpr uint32_t kColPlace = 128, kColA = 256;
 // What sums lost on average: put back where a run is multiplied anyway, and the rest (8.9e-8, the mean over k = 4,096 ... 14,336 whole and in eight shares) at the end
 constexpr float kCutOff = 1.0f + 0x1p-23f, kCutOffAll = 0x1.8p-24f;
+// Offsets times positive activations are of one sign, and a run of them loses the more the more units it adds up: 0.6e-7, 1.1e-7, 2.6e-7 and 4.5e-7 for 5, 7, 11 and 16 units;
+// with activations of both signs 0.1e-7, 0.5e-7, 1.0e-7 and 1.9e-7.  This much goes into the operand (a factor of the sums moves in steps of 1.2e-7).  Errors of results with
+// positive activations, three products of halves / one factor for runs of eight units and more / this: shares of 7 units 5.8e-8 / 1.18e-7 / 3.7e-8, of 11 1.27e-7 / 1.54e-7 / 1.24e-7,
+// of 16 3.5e-7 / 3.7e-7 / 2.8e-7; with normal ones 2.0e-7 / 1.6e-7 / 1.6e-7, 2.0e-7 / 1.7e-7 / 1.9e-7, 2.3e-7 / 2.2e-7 / 2.15e-7.
+__device__ __forceinline__ float offsets_loss(int units) { return fminf(1.75e-8f * (float)units, 8.8e-8f + 6.5e-9f * (float)min(units, 16)); }
 
 // ---- tcgen05 wrappers -------------------------------------------------------------------------------------------------
 // the registers go through it: nothing that uses what was loaded may be moved ahead of the wait
@@ -147,12 +152,14 @@ __device__ __forceinline__ void unpack_integers(const unsigned char* rp, const U
     }
 }
 // The offset operand of a unit: p[i] = c * d * sc[i] - dmin * m[i], hi = f16(p) and lo = f16(p - hi).  Columns 0-3: the eight hi
-// as pairs (k' = 0..7), columns 4-7: the eight lo (k' = 8..15); the sums tile holds each sub-block sum at k' and k' + 8.
+// as pairs (k' = 0..7), columns 4-7: the eight lo (k' = 8..15); the sums tile holds each sub-block sum at k' and k' + 8.  loss: what their sums will lose (offsets_loss).
 template <uint32_t TYPE>
-__device__ __forceinline__ void unpack_mins(uint4 w, float up, uint32_t* col) {
+__device__ __forceinline__ void unpack_mins(uint4 w, float up, float loss, uint32_t* col) {
     uint32_t sc_lo, sc_hi, mn_lo, mn_hi;
     unpack_scales_k4(w.y, w.z, w.w, &sc_lo, &sc_hi, &mn_lo, &mn_hi);
-    const float dmin = h2f((uint16_t)(w.x >> 16)) * up, mid = h2f((uint16_t)(w.x & 0xFFFFu)) * up * (TYPE == LC_TYPE_Q5_K ? 16.f : 8.f);
+    float dmin = h2f((uint16_t)(w.x >> 16)) * up, mid = h2f((uint16_t)(w.x & 0xFFFFu)) * up * (TYPE == LC_TYPE_Q5_K ? 16.f : 8.f);
+    dmin = fmaf(dmin, loss, dmin);
+    mid = fmaf(mid, loss, mid);
 #pragma unroll
     for (int j2 = 0; j2 < 4; j2++) {
         __half hi[2], lo[2];
@@ -466,16 +473,18 @@ qgemm_whole_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constan
             if (q >= 2) drain(q - 2, d2);
             if (!ok) return;
             d2 = d1;
-            d1 = nu - 16 * (q - off_at) >= 8 ? kCutOff : 1.0f;  // a run of few units' offsets adds up seldom
+            d1 = 1.0f;
+            const float loss = offsets_loss(nu - 16 * (q - off_at));
+            // two units' headers at a time: all four take registers that the sums then spill for (777 tokens x [4096 -> 4096] 128 us, so 123)
             const int u = u_begin + ((q - off_at) * 4 + g) * 4;
-            uint4 hd[4];
-#pragma unroll
-            for (int e = 0; e < 4; e++) hd[e] = live && u + e < u_begin + nu ? __ldg(reinterpret_cast<const uint4*>(wrow + (size_t)(u + e) * kPitch)) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
             for (int jj = 0; jj < 2; jj++) {
+                uint4 hd[2];
+#pragma unroll
+                for (int e = 0; e < 2; e++) hd[e] = live && u + 2 * jj + e < u_begin + nu ? __ldg(reinterpret_cast<const uint4*>(wrow + (size_t)(u + 2 * jj + e) * kPitch)) : make_uint4(0u, 0u, 0u, 0u);
                 uint32_t col[16];
-                unpack_mins<TYPE>(hd[2 * jj], up, col);
-                unpack_mins<TYPE>(hd[2 * jj + 1], up, col + 8);
+                unpack_mins<TYPE>(hd[0], up, loss, col);
+                unpack_mins<TYPE>(hd[1], up, loss, col + 8);
                 tmem_st16(a_own + (q & 1) * kColPlace + jj * 16, col);
             }
             operand_ready(q);

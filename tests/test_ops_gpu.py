@@ -253,6 +253,20 @@ def test_many_token_product_in_pairs_of_ctas(gpu, typ, m, k, n):
     assert (np.abs(got[rest] - want) <= 2e-5 * np.sqrt((a[rest].astype(np.float64) ** 2) @ (dense.T ** 2))).all()
 
 
+@pytest.mark.parametrize("typ", [12, 13])
+@pytest.mark.parametrize("m,k,n,bound", [(70, 512, 512, 1.4e-7), (70, 14336, 512, 8e-8), (300, 11008, 512, 5.5e-8), (300, 4096, 4096, 3.4e-7), (300, 8192, 4096, 1.45e-7)])
+def test_many_token_product_of_positive_activations(gpu, typ, m, k, n, bound):
+    """Q4_K and Q5_K, offsets of one sign times positive activations: what the matrix unit cuts off all points one way.  Shares of two, seven, five, sixteen and eleven units.  The bounds lie above
+    what the product of three halves gave where it was nearer (5.5e-8 - 5.8e-8, 5.9e-8 - 6.9e-8, 3.5e-7 - 3.9e-7, 1.3e-7 - 1.4e-7) and below what one correction for all runs of
+    offsets did (1.2e-7, 7.0e-8 - 7.6e-8, 3.7e-7 - 3.9e-7, 1.5e-7 - 1.7e-7); the first holds too much put back in short ones."""
+    r = rng([typ, k, m, n])
+    w, dense = scaled_blocks(gpu, typ, n, k, np.exp2(r.uniform(-1, 0, (n, k // 256))), r)
+    a = np.abs(r.standard_normal((m, k))).astype(np.float32)
+    got = gpu.qmatmul(typ, a.ravel(), w, m, k, n).reshape(m, n)
+    want = a.astype(np.float64) @ dense.T
+    assert np.linalg.norm(got - want) <= bound * np.linalg.norm(want), np.linalg.norm(got - want) / np.linalg.norm(want)
+
+
 @pytest.mark.parametrize("m", [16, 70])
 @pytest.mark.parametrize("typ", [2, 8, 12, 13, 14])
 def test_many_token_product_beside_a_large_activation(gpu, typ, m):
