@@ -1197,6 +1197,12 @@ static int32_t fetch_logits(lc_model* lead, int n_rows, float* host_out) {
         // the next pieces come: 64 rows of 32,000 493 us, in one piece 610; 16 rows 140 / 160.
         const size_t bytes = (size_t)n_rows * Vfull * 4, piece = std::max((size_t)1 << 20, (bytes / kLogitsPieces + 255) & ~(size_t)255);
         char *const to = reinterpret_cast<char*>(host_out), *const pin = reinterpret_cast<char*>(lead->pin_logits);
+        if (bytes <= piece) {
+            LC_CUDA(cudaMemcpyAsync(pin, lead->d_logits, bytes, cudaMemcpyDeviceToHost, lead->stream));
+            LC_CUDA(cudaStreamSynchronize(lead->stream));
+            memcpy(to, pin, bytes);
+            return LC_OK;
+        }
         for (size_t at = 0, i = 0; at < bytes; at += piece, i++) {
             LC_CUDA(cudaMemcpyAsync(pin + at, reinterpret_cast<const char*>(lead->d_logits) + at, std::min(piece, bytes - at), cudaMemcpyDeviceToHost, lead->stream));
             LC_CUDA(cudaEventRecord(lead->ev_logits[i], lead->stream));

@@ -9,6 +9,7 @@ from __future__ import annotations
 import ctypes as C
 import json
 from collections import deque
+from sys import getrefcount
 from typing import Callable, Iterable, Optional, Sequence
 
 import numpy as np
@@ -19,16 +20,6 @@ from ._capi import Counters, ModelConfig, check, load
 
 def _p(a: np.ndarray):
     return a.ctypes.data_as(C.c_void_p)
-
-
-class _Memory:
-    """Ordinary memory of a result; when the last array over it is gone, its engine has it for a later result of the same shape."""
-
-    def __init__(self, spare: deque, memory: np.ndarray):
-        self._spare, self._memory, self.__array_interface__ = spare, memory, memory.__array_interface__
-
-    def __del__(self):
-        self._spare.append(self._memory)
 
 
 class Engine:
@@ -46,7 +37,7 @@ class Engine:
         cfg.rope_mode = {"call_relative": 0, "absolute": 1}[rope_mode]
         cfg.max_seqs, cfg.kv_page_tokens, cfg.kv_pool_tokens, cfg.device = max_seqs, kv_page_tokens, kv_pool_tokens, device
         self.cfg = cfg
-        self._spare = deque(maxlen=2)  # memory of results that are gone
+        self._memory = deque(maxlen=2)  # of the last results (_logits_array)
         self._h = C.c_void_p()
         check(load().lc_model_create(C.byref(cfg), C.byref(self._h)))
         self.vocab_size = vocab_size
@@ -63,7 +54,7 @@ class Engine:
         over.rope_mode = {"call_relative": 0, "absolute": 1}[rope_mode]
         over.max_seqs, over.kv_page_tokens, over.kv_pool_tokens, over.device = max_seqs, kv_page_tokens, kv_pool_tokens, device
         self = cls.__new__(cls)
-        self._spare = deque(maxlen=2)
+        self._memory = deque(maxlen=2)
         self._h = C.c_void_p()
         check(load().lc_model_load_gguf(str(path).encode(), C.byref(over), C.byref(self._h)))
         cfg = ModelConfig()
@@ -76,7 +67,7 @@ class Engine:
     @classmethod
     def _adopt(cls, handle, max_seqs: int) -> "Engine":
         self = cls.__new__(cls)
-        self._spare = deque(maxlen=2)
+        self._memory = deque(maxlen=2)
         self._h = handle
         cfg = ModelConfig()
         check(load().lc_model_get_config(handle, C.byref(cfg)))
@@ -163,15 +154,21 @@ class Engine:
         return out
 
     def _logits_array(self, rows: int) -> np.ndarray:
-        """Where a call's logits go: memory of an earlier result, where there is some (the first write to 8 MB of new pages takes 2 ms, and malloc gives 32 MB and more back)."""
+        """Where a call's logits go: ordinary memory, that of an earlier result where nobody holds one any more (the first write to 8 MB of new pages takes 2 ms, and malloc gives 32 MB
+        and more back).  Whatever is made from a result (views of views too) refers to the array in `_memory` itself, so that its references tell."""
         shape = (rows, self.vocab_size)
-        try:
-            memory = self._spare.pop()
-        except IndexError:
-            memory = None
-        if memory is None or memory.shape != shape:
-            memory = np.empty(shape, np.float32)
-        return np.asarray(_Memory(self._spare, memory))
+        for _ in range(2):
+            try:
+                memory = self._memory.popleft()
+            except IndexError:
+                break
+            free = memory.shape == shape and getrefcount(memory) == 2  # the name here and the argument
+            self._memory.append(memory)
+            if free:
+                return memory.view()
+        memory = np.empty(shape, np.float32)
+        self._memory.append(memory)
+        return memory.view()
 
     def forward_batch(self, seq_ids: Sequence[int], token_lists: Sequence[Sequence[int]], want_logits: bool = True):
         n = len(seq_ids)
@@ -256,7 +253,7 @@ class Engine:
         if self._h:
             load().lc_model_destroy(self._h)
             self._h = C.c_void_p()
-            self._spare = deque(maxlen=0)
+            self._memory.clear()
 
     def __del__(self):
         try:
