@@ -574,7 +574,8 @@ constexpr double kFixedCycles = 8000;
 template <uint32_t TYPE>
 int32_t launch_type(const GemvArgs& a, const GemmWorkspace& ws, GemmParams& p, const GemmGroup* group, int* summed_slices, cudaStream_t s) {
     const int nmat = a.epi == EPI_SILU_MUL ? 2 : 1, tiles = (p.n * nmat + kGemmRows - 1) / kGemmRows;
-    const GemmCut cut = group ? GemmCut{gemm_tokens(group->typical), 1} : gemm_cut(a, ws, p.T, tiles, p.k / kUnitElems, nmat, unit_cycles(gemm_tokens(p.T)), kFixedCycles);
+    const int N = gemm_tokens(group ? group->typical : p.T, 16);
+    const GemmCut cut = group ? GemmCut{N, 1} : gemm_cut(a, ws, p.T, N, tiles, p.k / kUnitElems, nmat, unit_cycles(N), kFixedCycles);
     // five activation chunks (with few tokens eight) and the raw units that fit
     const size_t raw = (size_t)RawUnit<TYPE>::pitch * kGemmRows, fixed = 1024 + 512, b = (size_t)2 * cut.N * 128;
     p.N = cut.N;

@@ -550,7 +550,8 @@ template <uint32_t TYPE>
 int32_t launch_type(const GemvArgs& a, const GemmWorkspace& ws, GemmParams& p, const GemmGroup* group, int* summed_slices, cudaStream_t s) {
     const int nmat = a.epi == EPI_SILU_MUL ? 2 : 1, units = p.k / kUnitElems;
     const int tiles = ((p.n * nmat + kGemmRows - 1) / kGemmRows + 1) / 2 * 2;  // whole pairs
-    const GemmCut cut = group ? GemmCut{gemm_tokens(group->typical), 1} : gemm_cut(a, ws, p.T, tiles, units, nmat, kUnitCycles, kFixedCycles);
+    const int N = gemm_tokens(group ? group->typical : p.T, 32);
+    const GemmCut cut = group ? GemmCut{N, 1} : gemm_cut(a, ws, p.T, N, tiles, units, nmat, kUnitCycles, kFixedCycles);
     const bool wide = cut.N > 64;
     const int box = wide ? cut.N / 2 : cut.N;
     // three raw units, as many activation stages as fit, more raw units
