@@ -22,6 +22,17 @@ def _p(a: np.ndarray):
     return a.ctypes.data_as(C.c_void_p)
 
 
+def _oldest(pool: deque):
+    """The pool's first array, which goes to its end, and its references."""
+    memory = pool.popleft()
+    references = getrefcount(memory)
+    pool.append(memory)
+    return memory, references
+
+
+_FREE = _oldest(deque([np.empty(1)]))[1]  # of an array that only its pool has
+
+
 class Engine:
     def __init__(self, hidden_size: int, num_layers: int, num_heads: int, num_kv_heads: int, intermediate_size: int,
                  vocab_size: int, max_seq_len: int = 4096, rope_theta: float = 10000.0, rms_eps: float = 1e-5,
@@ -157,14 +168,12 @@ class Engine:
         """Where a call's logits go: ordinary memory, that of an earlier result where nobody holds one any more (the first write to 8 MB of new pages takes 2 ms, and malloc gives 32 MB
         and more back).  Whatever is made from a result (views of views too) refers to the array in `_memory` itself, so that its references tell."""
         shape = (rows, self.vocab_size)
-        for _ in range(2):
+        for _ in range(len(self._memory)):
             try:
-                memory = self._memory.popleft()
-            except IndexError:
+                memory, references = _oldest(self._memory)
+            except IndexError:  # another thread has it
                 break
-            free = memory.shape == shape and getrefcount(memory) == 2  # the name here and the argument
-            self._memory.append(memory)
-            if free:
+            if references == _FREE and memory.shape == shape:
                 return memory.view()
         memory = np.empty(shape, np.float32)
         self._memory.append(memory)
