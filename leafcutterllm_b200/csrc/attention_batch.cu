@@ -17,7 +17,8 @@
 //
 // Bound: HBM.  The kernel that had a CTA per (token, head, 1,024 keys), f32 FMAs and the rotation's powers, sines and cosines in each CTA took 594 us for
 // 2.19 GB (64 sequences of 128 - 4,096 tokens, 32 heads) and 88 us for 67 MB (16 of 1,024, 8 kv heads for 32 heads).
-// Now 388 us (5.6 TB/s of measured 6.4) and 29 us; where a step rotates by nothing and there are no kv groups both take 330 - 337 us for 1.98 GB.  Runs of whole pieces per CTA would leave the longest sequence's CTA alone at the end.
+// Now 393 - 404 us (5.4 - 5.6 TB/s of measured 6.4) and 32 us.  Where a step rotates by nothing and there are no kv groups it would gain nothing (attention_batch_applies).
+// Runs of whole pieces per CTA would leave the longest sequence's CTA alone at the end.
 // The rotation's sines and cosines come from a table that the step's first kernel leaves (`rot`).
 #include <algorithm>
 #include <cstdlib>
@@ -559,7 +560,7 @@ int32_t launch_attention_batch(const AttnParams& a, int n_tok, cudaStream_t s) {
     BatchParams P;
     P.a = a; P.n_tok = n_tok;
     const char* const limit = getenv("LC_ATTN_WAITS");  // read per launch so that a test can make the waits run out: 0, before they look
-    P.wait_limit = limit ? (uint32_t)atoi(limit) : 1u << 22;
+    P.wait_limit = limit ? (uint32_t)std::clamp(atoi(limit), 0, 1 << 22) : 1u << 22;
     switch (a.n_heads / a.kv.n_kv) {
         case 1: return launch_batch<1>(P, s);
         case 2: return launch_batch<2>(P, s);

@@ -194,7 +194,7 @@ size_t attention_scratch_bytes(int n_tok, int n_heads, int hd, int max_ctx);
 size_t attention_batch_scratch_bytes(int n_heads, int n_kv, int hd);  // ... and of a handle whose steps pass `rot`
 // counters: n_tok*n_heads ints, zero before the first launch (the kernel leaves them zero).
 // fuse (decode steps only, every token the single new token of its sequence): q is rotated on load and the new
-// key/value are taken from k_new/v_new (rows q_stride floats apart), rotated, and stored into the cache by this kernel,
+// key/value are taken from k_new/v_new (rows kv_stride floats apart), rotated, and stored into the cache by this kernel,
 // so no separate rope/append launch is needed.
 // positions_settled: tok_pos was final before the kernel ahead of this one started (true from the second layer of a
 // step on; false for the first layer, whose positions the end of the previous step may still be writing), so the

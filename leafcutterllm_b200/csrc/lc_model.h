@@ -58,8 +58,9 @@ constexpr int kLogitsPieces = 16;      // most pieces in which logits come to th
 constexpr int kTokTile = 8;
 constexpr int kMoeGroupedTokens = 64;  // most tokens of a call whose experts run as one grouped matrix-vector launch
 // Rows per expert beyond which the experts run as a grouped many-token product instead: the matrix-vector kernel reads the experts again for
-// every four rows.  Mixtral shape, us per step of two layers, matrix-vector / product: 16 sequences (4 rows per expert) 1049 / 1385, 24 (6)
-// 1314 / 1400, 28 (7) 1433 / 1405, 32 (8) 1576 / 1407, 48 (12) 2110 / 1473.  One shape measured.
+// every four rows.  us per step of two layers, matrix-vector / product, at 6, 7 and 8 rows an expert: Mixtral shape 1261 / 1365, 1386 / 1370, 1522 / 1370;
+// 4 experts, top 1, 2048 x 4096 263 / 269, 275 / 271, 294 / 274; 16, top 4, 2048 x 2048 417 / 399, 451 / 403, 481 / 401; 64, top 8, 2048 x 1024 939 / 920, 1017 / 943,
+// 1095 / 962.  Over nine shapes (4 - 64 experts) they meet between five and seven rows; at seven the product is 1 - 16 % faster.
 constexpr float kMoeProductRows = 6.5f;
 
 }  // namespace lc
