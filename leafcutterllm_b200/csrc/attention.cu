@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_staged_kernel(AttnP
         // the token of this step replaces the (stale) staged slot: rotate, round through f16, keep in the cache
         const int row = pos - t_begin;
         float kr[1], vr;
-        load_rotated<1, HD>(p.k_new + (size_t)tok * p.kv_stride + kvh * HD, tid, rp, p.theta, rot, kr);
+        load_rotated<1, HD>(p.k_new + (size_t)tok * p.kv_stride + kvh * HD, tid, rp, rot, kr);
         vr = __ldcg(p.v_new + (size_t)tok * p.kv_stride + kvh * HD + tid);
         const __half hk = __float2half_rn(kr[0]), hv = __float2half_rn(vr);  // cache/mod.rs:35-36
         K_s[row * HD + tid] = hk;
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attention_staged_kernel(AttnP
         float* pout = p.partial + ((size_t)item * p.n_splits + split) * (HD + 2);
         {
             float qv[1];
-            load_rotated<1, HD>(p.q + (size_t)tok * p.q_stride + h * HD, tid, rp, p.theta, rot, qv);
+            load_rotated<1, HD>(p.q + (size_t)tok * p.q_stride + h * HD, tid, rp, rot, qv);
             __syncthreads();  // the previous head is done with q_s / p_s / acc_s
             q_s[tid] = qv[0];
         }
@@ -350,13 +350,14 @@ int32_t launch_attention(const float* q, int q_stride, float* out, int n_tok, in
     p.page_table = page_table; p.pages_per_seq = pages_per_seq; p.chunk = 0; p.n_splits = 1; p.partial = (float*)scratch;
     p.counters = counters;
     p.k_new = fuse ? fuse->k_new : nullptr; p.v_new = fuse ? fuse->v_new : nullptr;
-    p.tok_rope = fuse ? fuse->tok_rope : nullptr; p.theta = fuse ? fuse->theta : 0.f;
+    p.tok_rope = fuse ? fuse->tok_rope : nullptr;
+    LC_CHECK(!fuse || fuse->rot, LC_ERR_INVALID, "attention: a step without its table of rotations");
     p.rot = fuse ? (const float2*)fuse->rot : nullptr;
     p.kv_stride = fuse ? fuse->kv_stride : 0;
     p.positions_settled = (fuse && fuse->positions_settled) ? 1 : 0;
     p.error_flag = gemv_error_flag_dev();
     if (fuse && fuse->stream_slots && attention_stream_applies(p, n_tok)) return launch_attention_stream(p, fuse->stream_slots, s);
-    if (p.rot && attention_batch_applies(p, n_tok, fuse->turns)) return launch_attention_batch(p, n_tok, s);
+    if (fuse && attention_batch_applies(p, n_tok, fuse->turns)) return launch_attention_batch(p, n_tok, s);
     switch (kv.hd) {
         case 32: return launch_attention_hd<32>(p, n_tok, max_ctx, s);
         case 64: return launch_attention_hd<64>(p, n_tok, max_ctx, s);
