@@ -149,7 +149,7 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap ktm, const __grid_co
     const bool fused = p.k_new != nullptr;
     const int rp_of_step = fused ? p.tok_rope[0] : 0;
     // four dims of a head vector of the projection row, rotated (attention.rs:13-34)
-    auto head_vec = [&](const float* plain, size_t off, float (&out4)[4]) { load_rotated<4, kHD>(plain + off, 4 * lane, rp_of_step, p.rot, out4); };
+    auto head_vec = [&](const float* plain, size_t off, float (&out4)[4]) { load_rotated<4, kHD>(plain + off, 4 * lane, rp_of_step, p.theta, p.rot, out4); };
     // attention.rs:93-102: softmax(dot / sqrt(head_dim)).  Scores are kept multiplied by log2(e) so that every exponential is a
     // single ex2; the running maximum is in the same units and goes back to natural units when a warp's state is written out.
     const float sc_log2e = 1.4426950408889634f / sqrtf((float)kHD);

@@ -240,7 +240,7 @@ int32_t attention_block(lc_model* m, int l, const float* x, const float* norm_w,
     float* v = k + (w.fused_qkv ? (size_t)1 : (size_t)T) * m->nkv * m->hd;
     if (decode_step) {
         // one new token per sequence: rotation and the cache append ride inside the attention kernel
-        AttnFusion fz{k, v, kv_stride, m->d_tok_rope};
+        AttnFusion fz{k, v, kv_stride, m->d_tok_rope, m->cfg.rope_theta};
         fz.positions_settled = l > 0;  // the first layer of a step may run while the previous step still advances the positions
         fz.stream_slots = m->d_stream_slots;
         fz.rot = m->d_rot;

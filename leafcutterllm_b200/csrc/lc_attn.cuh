@@ -28,6 +28,7 @@ struct AttnParams {
     const float* k_new;    // null = keys and values are already in the cache and q is already rotated
     const float* v_new;
     const int32_t* tok_rope;
+    float theta;
     const float2* rot;     // [n_tok][hd / 2] cosine and sine of each pair's rotation; with k_new
     int positions_settled; // decode-step fusion: tok_pos may be read before the grid dependency wait
     int* error_flag;       // set when a bounded wait runs out (may be null)
@@ -89,11 +90,11 @@ __device__ __forceinline__ void widen(const RawSlice<DPL, F32>& r, float (&out)[
     }
 }
 
-// Dims d0 .. d0+DPL-1 of a head vector at `base`, rotated by position `rp` (attention.rs:13-34: pairs (d, d + hd/2)).  rp == 0 is the identity.  rot: this token's row of the table that
-// the step's first kernel left.  (Powers, sines and cosines in every CTA cost as much as half of a batch's attention; as a second way in these kernels, which nothing took any
-// more, they cost a single token's attention 2.5 us of 17.7, by their code alone.)
-template <int DPL, int HD>
-__device__ __forceinline__ void load_rotated(const float* base, int d0, int rp, const float2* rot, float (&out)[DPL]) {
+// Dims d0 .. d0+DPL-1 of a head vector at `base`, rotated by position `rp` (attention.rs:13-34: pairs (d, d + hd/2), freq = 1 / theta^(2d/hd)).  rp == 0 is the identity.  rot: this
+// token's row of the table that the step's first kernel left (powers, sines and cosines in every CTA cost as much as half of a batch's attention).  TABLE: from the table only; as a
+// second way in a step's kernels the powers cost a single token's attention 2.5 us of 17.7 by their code alone.
+template <int DPL, int HD, bool TABLE = true>
+__device__ __forceinline__ void load_rotated(const float* base, int d0, int rp, float theta, const float2* rot, float (&out)[DPL]) {
 #pragma unroll
     for (int i = 0; i < DPL; i++) out[i] = __ldcg(base + d0 + i);  // written by another CTA of a persistent kernel: read through L2
     if (rp == 0) return;
@@ -101,7 +102,14 @@ __device__ __forceinline__ void load_rotated(const float* base, int d0, int rp, 
 #pragma unroll
     for (int i = 0; i < DPL; i++) {
         const int d = d0 + i, dd = d < HALF ? d : d - HALF;
-        const float2 cs = __ldcg(rot + dd);
+        float2 cs;
+        if (TABLE || rot) {
+            cs = __ldcg(rot + dd);
+        } else {
+            const float freq = __fdiv_rn(1.0f, powf(theta, __fdiv_rn(__fmul_rn(2.0f, (float)dd), (float)HD)));
+            const float angle = __fmul_rn((float)rp, freq);
+            cs = make_float2(cosf(angle), sinf(angle));
+        }
         const float ca = cs.x, sa = cs.y;
         if (d < HALF) out[i] = __fsub_rn(__fmul_rn(__ldcg(base + d), ca), __fmul_rn(__ldcg(base + d + HALF), sa));
         else out[i] = __fadd_rn(__fmul_rn(__ldcg(base + d - HALF), sa), __fmul_rn(__ldcg(base + d), ca));
@@ -133,7 +141,7 @@ __device__ __forceinline__ void group_sync(int bar_id) {
     else asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "r"(kAttnWarps * 32) : "memory");
 }
 
-template <int HD, bool F32, int BAR>
+template <int HD, bool F32, int BAR, bool STEP>
 __device__ __forceinline__ void attention_item(const AttnParams& p, int item, int split, int tid, float* sh, int bar_id = 0) {
     constexpr int DPL = 16 < HD / 2 ? 16 : HD / 2;
     constexpr int LPK = HD / DPL;
@@ -170,7 +178,7 @@ __device__ __forceinline__ void attention_item(const AttnParams& p, int item, in
         const int rp = p.k_new ? p.tok_rope[tok] : 0;
         const float2* const rot = p.rot ? p.rot + (size_t)tok * (HD / 2) : nullptr;
         float qr[DPL];
-        load_rotated<DPL, HD>(p.q + (size_t)tok * p.q_stride + h * HD, sub * DPL, rp, rot, qr);
+        load_rotated<DPL, HD, STEP>(p.q + (size_t)tok * p.q_stride + h * HD, sub * DPL, rp, p.theta, rot, qr);
 
         auto key_addr = [&](int t) -> size_t {
             int page = pt[t / kv.page_tokens];
@@ -240,7 +248,7 @@ __device__ __forceinline__ void attention_item(const AttnParams& p, int item, in
         if (has_new) {
             // the token of this step: rotate, round through the cache type, and (one head per kv group) store
             float kr[DPL], vr[DPL];
-            load_rotated<DPL, HD>(p.k_new + (size_t)tok * p.kv_stride + kvh * HD, sub * DPL, rp, rot, kr);
+            load_rotated<DPL, HD, STEP>(p.k_new + (size_t)tok * p.kv_stride + kvh * HD, sub * DPL, rp, p.theta, rot, kr);
             const float* vp = p.v_new + (size_t)tok * p.kv_stride + kvh * HD + sub * DPL;
 #pragma unroll
             for (int i = 0; i < DPL; i++) vr[i] = __ldcg(vp + i);

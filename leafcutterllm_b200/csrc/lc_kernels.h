@@ -200,7 +200,7 @@ size_t attention_batch_scratch_bytes(int n_heads, int n_kv, int hd);  // ... and
 // step on; false for the first layer, whose positions the end of the previous step may still be writing), so the
 // kernel may read it, and start fetching cached pages, before it waits for the kernel ahead of it.
 struct AttnFusion {
-    const float* k_new; const float* v_new; int kv_stride; const int32_t* tok_rope; bool positions_settled = false;
+    const float* k_new; const float* v_new; int kv_stride; const int32_t* tok_rope; float theta; bool positions_settled = false;
     // Cross-CTA merge slots of the single-token streaming kernel (attention_stream_slot_bytes of them, all zero before the
     // first launch; the kernel leaves them zero).  They belong to the caller -- one set per model -- because a captured
     // decode step keeps the pointer.
